@@ -141,13 +141,20 @@ __device__ __forceinline__ void store_chunk(const float* v, void* out, int64_t l
   }
 }
 
+__device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, const void* src, int x, int y, int z) {
+  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"
+               ::"l"(map), "r"(smem_u32(src)), "r"(x), "r"(y), "r"(z) : "memory");
+}
+
 // One CTA per SM walks the tiles t = blockIdx.x, blockIdx.x + gridDim.x, ... (n fastest, then m, then the
 // K split): the ring of stages runs on from one tile into the next, and with two accumulators in tensor
 // memory the epilogue warps empty one while the MMAs fill the other.
 // Grouped (`tile_expert` given): W holds several matrices of `expert_rows` outputs each, one after another, and
 // tile_expert[m tile] says which of them the 128 rows of that tile multiply (negative: the tile is skipped).  The list
 // comes from the kernel before, so every role waits for it before its first tile.
-template <int BN, int EPI>
+// HEADS: `n_splits` products side by side instead of shares of K: the maps are three-dimensional ([rows][head][entry]), head z
+// multiplies its own columns of A by its own matrix of W into its own columns of the output, each clipped by its map.
+template <int BN, int EPI, bool HEADS = false>
 __global__ void __launch_bounds__(NUM_THREADS_WIDE, 1)
 linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                       const __grid_constant__ CUtensorMap map_out, int tma_out,
@@ -186,7 +193,7 @@ linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     *m0 = mt * BM;
     const int expert = tile_expert != nullptr ? tile_expert[mt] : 0;
     *w0 = expert < 0 ? -1 : expert * expert_rows + *n0;
-    *kb_begin = *z * kb_per_split;
+    *kb_begin = HEADS ? 0 : *z * kb_per_split;
     const int kb_end = *kb_begin + kb_per_split < kb_total ? *kb_begin + kb_per_split : kb_total;
     *num_kb = kb_end - *kb_begin;
   };
@@ -224,12 +231,15 @@ linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
           const int pre = num_kb < STAGES ? num_kb : STAGES;
           for (int j = 0; j < pre; ++j) {
             mbar_expect_tx(&full_bar[j], T::A_BYTES + T::B_BYTES);
-            tma_load_2d(b_tiles + j * T::B_BYTES, &map_w, &full_bar[j], (kb_begin + j) * BK, w0);
+            if (HEADS) tma_load_3d(b_tiles + j * T::B_BYTES, &map_w, &full_bar[j], j * BK, w0, z);
+            else tma_load_2d(b_tiles + j * T::B_BYTES, &map_w, &full_bar[j], (kb_begin + j) * BK, w0);
           }
           pdl_wait();
           waited = true;
-          for (int j = 0; j < pre; ++j)
-            tma_load_2d(a_tiles + j * T::A_BYTES, &map_a, &full_bar[j], (kb_begin + j) * BK, m0);
+          for (int j = 0; j < pre; ++j) {
+            if (HEADS) tma_load_3d(a_tiles + j * T::A_BYTES, &map_a, &full_bar[j], j * BK, z, m0);
+            else tma_load_2d(a_tiles + j * T::A_BYTES, &map_a, &full_bar[j], (kb_begin + j) * BK, m0);
+          }
           i = pre;
           it = pre;
         }
@@ -237,8 +247,13 @@ linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
           const int s = it % STAGES;
           if (it >= (uint32_t)STAGES && !mbar_wait(&empty_bar[s], ((it / STAGES) & 1) ^ 1)) { ok = false; break; }
           mbar_expect_tx(&full_bar[s], T::A_BYTES + T::B_BYTES);
-          tma_load_2d(a_tiles + s * T::A_BYTES, &map_a, &full_bar[s], (kb_begin + i) * BK, m0);
-          tma_load_2d(b_tiles + s * T::B_BYTES, &map_w, &full_bar[s], (kb_begin + i) * BK, w0);
+          if (HEADS) {
+            tma_load_3d(a_tiles + s * T::A_BYTES, &map_a, &full_bar[s], i * BK, z, m0);
+            tma_load_3d(b_tiles + s * T::B_BYTES, &map_w, &full_bar[s], i * BK, w0, z);
+          } else {
+            tma_load_2d(a_tiles + s * T::A_BYTES, &map_a, &full_bar[s], (kb_begin + i) * BK, m0);
+            tma_load_2d(b_tiles + s * T::B_BYTES, &map_w, &full_bar[s], (kb_begin + i) * BK, w0);
+          }
         }
       }
     }
@@ -367,6 +382,7 @@ linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
           __syncwarp();
           if (lane == 0 && n0 + c0 < N && m0 + quarter * 32 < M) {
             if (EPI == EPI_RESIDUAL) tma_reduce_add_2d(&map_out, slab, n0 + c0, m0 + quarter * 32);
+            else if (HEADS) tma_store_3d(&map_out, slab, n0 + c0, z, m0 + quarter * 32);
             else tma_store_2d(&map_out, slab, n0 + c0, m0 + quarter * 32);
             bulk_commit();
           }
@@ -892,6 +908,45 @@ int launch(const CUtensorMap& ma, const CUtensorMap& mw, const void* bias, int b
   return KVAD_OK;
 }
 
+// [planes][rows][cols] or any other order of three dimensions: sizes and the strides of the outer two in entries, 64 x box_y x box_z a load or store.
+int tensor_map_cube(const void* ptr, const int (&size)[3], const int64_t (&stride)[2], int box_y, int box_z, CUtensorMap* out) {
+  EncodeTiledFn fn = encode_fn();
+  if (fn == nullptr) KVAD_FAIL(KVAD_ERR_CUDA, "linear_tcgen05: the driver does not offer cuTensorMapEncodeTiled");
+  cuuint64_t dims[3] = {(cuuint64_t)size[0], (cuuint64_t)size[1], (cuuint64_t)size[2]};
+  cuuint64_t strides[2] = {(cuuint64_t)stride[0] * 2, (cuuint64_t)stride[1] * 2};
+  cuuint32_t box[3] = {(cuuint32_t)BK, (cuuint32_t)box_y, (cuuint32_t)box_z};
+  cuuint32_t elem[3] = {1, 1, 1};
+  CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS)
+    KVAD_FAIL(KVAD_ERR_CUDA, "linear_tcgen05: cuTensorMapEncodeTiled failed (%d) for [%d, %d, %d] entries", (int)r, size[2], size[1], size[0]);
+  return KVAD_OK;
+}
+
+template <int BN>
+int launch_heads(const void* A, int64_t lda, int64_t a_head, const void* W, void* out, int64_t ldo, int64_t out_head, int M, int heads, int N, int K,
+                 cudaStream_t stream) {
+  using T = Tile<BN>;
+  CUtensorMap ma, mw, mo;
+  int rc = tensor_map_cube(A, {K, heads, M}, {a_head, lda}, 1, BM, &ma);
+  if (rc == KVAD_OK) rc = tensor_map_cube(W, {K, N, heads}, {K, (int64_t)N * K}, BN, 1, &mw);
+  if (rc == KVAD_OK) rc = tensor_map_cube(out, {N, heads, M}, {out_head, ldo}, 1, 32, &mo);
+  if (rc != KVAD_OK) return rc;
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(linear_tcgen05_kernel<BN, EPI_STORE, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::SMEM);
+    if (e != cudaSuccess) KVAD_FAIL(KVAD_ERR_CUDA, "linear_tcgen05: cannot reserve %zu bytes of shared memory: %s", T::SMEM, cudaGetErrorString(e));
+    configured = true;
+  }
+  const int64_t n_tiles = (int64_t)((N + BN - 1) / BN) * ((M + BM - 1) / BM) * heads;
+  KVAD_REQUIRE(n_tiles < (1ll << 30), "linear_tcgen05: %lld tiles are more than one launch takes", (long long)n_tiles);
+  const int ctas = n_tiles < sm_count() ? (int)n_tiles : sm_count();
+  kvad_launch(linear_tcgen05_kernel<BN, EPI_STORE, true>, dim3(ctas), dim3(NUM_THREADS_WIDE), T::SMEM, stream, ma, mw, mo, 1, (const void*)nullptr, 0, out,
+              ldo, M, N, K, (K + BK - 1) / BK, heads, (const int*)nullptr, 0);
+  KVAD_CHECK_LAUNCH("linear_tcgen05 (heads)");
+  return KVAD_OK;
+}
+
 template <int BN>
 int launch_epi(int epilogue, const CUtensorMap& ma, const CUtensorMap& mw, const void* bias, int bias_f32, void* out,
                int64_t ldo, int M, int N, int K, int splits, cudaStream_t stream) {
@@ -1143,8 +1198,6 @@ KVAD_EXPORT int kvad_linear_tcgen05(const void* A, int64_t lda, const void* W, c
   }
 }
 
-// Tests: 1 keeps the swapped form on two-dimensional loads (one per K block) for every K; 2 takes the
-// grouped three-dimensional loads whenever K allows; 0 is the kernel's own choice (them, up to 16 rows).
 // out[p] = W[tile_expert[p / 128]] . A[p] for the rows p of every 128-row tile whose entry is not negative: W is
 // [experts x N, K] (the experts' matrices one after another), A [M, K] with M a multiple of 128, out [M, N] bfloat16 or,
 // with `out_f32`, float32.  No bias, K whole.
@@ -1164,6 +1217,26 @@ KVAD_EXPORT int kvad_linear_tcgen05_grouped(const void* A, int64_t lda, const vo
   return launch<128, EPI_STORE>(ma, mw, nullptr, 0, out, ldo, M, N, K, 1, stream, tile_expert, N);
 }
 
+// out[r, z * out_head + j] = W[z, j, :] . A[r, z * a_head : + K] for every head z in ONE launch (one product a head from the host
+// took 16 launches of 3.9 us, and 18 us of host time each, for 2048 rows of 16 heads 64 x 256).  All strides and K multiples of 8,
+// all three on 16-byte boundaries.  A head is one tile of outputs wide where that is 64, 128 or 256, so that its rows are read once.
+KVAD_EXPORT int kvad_linear_tcgen05_heads(const void* A, int64_t lda, int64_t a_head, const void* W, void* out, int64_t ldo, int64_t out_head,
+                                          int M, int heads, int N, int K, cudaStream_t stream) {
+  KVAD_REQUIRE(M >= 0 && N > 0 && K > 0 && heads > 0, "linear_tcgen05_heads: bad sizes M=%d heads=%d N=%d K=%d", M, heads, N, K);
+  if (K % 8 != 0 || lda % 8 != 0 || a_head % 8 != 0 || ldo % 8 != 0 || out_head % 8 != 0 || (reinterpret_cast<uintptr_t>(A) & 15) ||
+      (reinterpret_cast<uintptr_t>(W) & 15) || (reinterpret_cast<uintptr_t>(out) & 15))
+    KVAD_FAIL(KVAD_ERR_UNSUPPORTED, "linear_tcgen05_heads: K and the strides must be multiples of 8, the tensors on 16-byte boundaries");
+  KVAD_REQUIRE(a_head >= K && out_head >= N && lda >= (heads - 1) * a_head + K && ldo >= (heads - 1) * out_head + N && (M + BM - 1) / BM <= 65535,
+               "linear_tcgen05_heads: the heads do not fit the rows");
+  if (M == 0) return KVAD_OK;
+  if (N <= 64) return launch_heads<64>(A, lda, a_head, W, out, ldo, out_head, M, heads, N, K, stream);
+  if (N <= 128) return launch_heads<128>(A, lda, a_head, W, out, ldo, out_head, M, heads, N, K, stream);
+  if (N <= 192) return launch_heads<192>(A, lda, a_head, W, out, ldo, out_head, M, heads, N, K, stream);
+  return launch_heads<256>(A, lda, a_head, W, out, ldo, out_head, M, heads, N, K, stream);
+}
+
+// Tests: 1 keeps the swapped form on two-dimensional loads (one per K block) for every K; 2 takes the
+// grouped three-dimensional loads whenever K allows; 0 is the kernel's own choice (them, up to 16 rows).
 KVAD_EXPORT void kvad_linear_tcgen05_no_3d(int on) { g_no_3d = on == 1; g_force_3d = on == 2; }
 
 // Tests of the bounded waits: `wait_limit` > 0 sets how many polls a wait makes before it gives up (0: the

@@ -50,9 +50,15 @@ _SIGNATURES = {
         "kvad_linear_simt": [c_int, c_void_p, c_int64, c_void_p, c_void_p, c_int, c_void_p, c_int64, c_int, c_int, c_int,
                              c_int, c_void_p],
     },
+    "linear_split": {
+        "kvad_linear_split": [c_void_p, c_int64, c_void_p, c_void_p, c_int, c_void_p, c_int64, c_int, c_int, c_int, c_int, c_int, c_void_p],
+        "kvad_linear_split_heads": [c_void_p, c_int64, c_int64, c_void_p, c_void_p, c_int64, c_int64, c_int, c_int, c_int, c_int, c_void_p],
+        "kvad_linear_split_status": [],
+    },
     "linear_tcgen05": {
         "kvad_linear_tcgen05": [c_void_p, c_int64, c_void_p, c_void_p, c_int, c_void_p, c_int64, c_int, c_int, c_int,
                                 c_int, c_int, c_void_p],
+        "kvad_linear_tcgen05_heads": [c_void_p, c_int64, c_int64, c_void_p, c_void_p, c_int64, c_int64, c_int, c_int, c_int, c_int, c_void_p],
         "kvad_linear_tcgen05_status": [],
         "kvad_linear_tcgen05_grouped": [c_void_p, c_int64, c_void_p, c_int, c_void_p, c_int64, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
     },
@@ -229,7 +235,7 @@ def lib(name: str) -> ctypes.CDLL:
 
 #: kernel libraries by what needs them: every model ("base"), and the families a part names in `Part.kernel_families`
 _FAMILY_LIBRARIES = {
-    "base": {"any": ("rows", "linear_simt", "sampling"), torch.bfloat16: ("linear_rows", "linear_tcgen05"), torch.float32: ("linear_rows_f32",)},
+    "base": {"any": ("rows", "linear_simt", "sampling"), torch.bfloat16: ("linear_rows", "linear_tcgen05"), torch.float32: ("linear_rows_f32", "linear_split")},
     "causal_attention": {"any": ("attention_simt", "attention_decode"), torch.bfloat16: ("attention_prefill",), torch.float32: ()},
     "norm_rotary": {"any": ("norm_rotary",)},
     "scored_attention": {"any": ("attention_scored",)},
@@ -329,6 +335,8 @@ class Ops:
         # for every row count it takes (the tiled CUDA-core kernel would run one row in a tile of 64).
         self._rows_lib = "linear_rows" if dtype == torch.bfloat16 else "linear_rows_f32"     # one library per element type
         self.rows_linear_max = (2 if dtype == torch.bfloat16 else 16) if self._rows_lib in build.sources() else 0
+        # 32-bit products of many rows on the tensor cores, their operands cut into bfloat16 pieces (linear_split.cu)
+        self.split_linear = dtype == torch.float32 and "linear_split" in build.sources()
         self.tiled_prompt = True    # prompts that the tensor-core kernel does not take: the tiled CUDA-core kernel, not the row-by-row one
         self._counters = None       # zeroed ints the decode kernel counts finished splits in (left zeroed by it)
         # Two 32-bit buffers [16, width] that q/k/v products of 3..16 rows add their shares of K into (see
@@ -345,7 +353,7 @@ class Ops:
         """Everything on the host that decides which kernels a step of a given shape launches; part of
         the key under which a step's CUDA graph is kept."""
         return (_switch_epoch, self.tensor_core_linear, self.tensor_core_prefill, self.fast_decode,
-                self.rows_linear_max, self.qkv_sums, self.SUMS_MIN_K, self.tiled_prompt)
+                self.rows_linear_max, self.qkv_sums, self.SUMS_MIN_K, self.tiled_prompt, self.split_linear)
 
     def begin_step(self) -> None:
         """Called once before a step's first kernel (inside the capture, if the step is being captured)."""
@@ -401,6 +409,10 @@ class Ops:
 
     # -- linear --------------------------------------------------------------------
     ROWS_LINEAR_MAX_OUT = 8192
+    # 32-bit products from this many rows on take the tensor cores (linear_split.cu).  Below, a CTA of 128 rows walks all of K
+    # for few rows: at 33 rows a layer of GPT-2 small's sizes takes 147 us this way and about 100 us as weights streamed in blocks of
+    # 16 rows (a generation from a 33-token prompt: 8.99 ms against 8.25 ms); at 65 rows of 768 x 3072 it is 78 us against the CUDA cores' 165.
+    SPLIT_MIN_ROWS = 65
     ROWS_BLOCKS_MAX = 64           # 32-bit: up to so many rows go through the weight-streaming form in blocks of 16
 
     def linear(self, a, weight, bias, out, epilogue: str = "store", *, tile: int = 0, splits: int = 0,
@@ -447,6 +459,11 @@ class Ops:
             return
         if form == "rows":
             raise KernelError("linear: the weight-streaming form takes at most 16 rows and K a multiple of a 16-byte piece, at most 1024 pieces")
+        if (form == "auto" and self.split_linear and m >= self.SPLIT_MIN_ROWS and k % 4 == 0 and lda % 4 == 0 and a.data_ptr() % 16 == 0
+                and weight.data_ptr() % 16 == 0):
+            h = lib("linear_split")
+            _check(h.kvad_linear_split(_ptr(a), lda, _ptr(weight), _ptr(bias), bias_f32, _ptr(out), ldo, m, n, k, epi, int(tile), _stream()), h)
+            return
         if (form == "auto" and self.dtype == torch.float32 and self.rows_linear_max >= 16 and 16 < m <= self.ROWS_BLOCKS_MAX and k <= 4096
                 and k % ve == 0 and lda % ve == 0 and a.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0 and self._rows_lib in build.sources()):
             # 32-bit, 17..64 rows: the tiled kernel would run a grid of N / 64 CTAs, each walking all of K (17 rows of
@@ -1035,9 +1052,18 @@ class Ops:
             _check(h.kvad_linear_heads(self.code, _ptr(a), ld_a, int(head_stride_a), _ptr(weight), _ptr(out), ld_o, int(head_stride_out),
                                        n, H, n_in, n_out, _ptr(gate), ld_g, _stream()), h)
             return
-        for hd in range(H):
-            self.linear(a[:, hd * head_stride_a: hd * head_stride_a + n_in], weight[hd], None,
-                        out[:, hd * head_stride_out: hd * head_stride_out + n_out])
+        # many rows: one launch for all heads where its loads and stores are whole 16-byte pieces, else one product a head
+        E = 16 // a.element_size()
+        whole = (n_in % E == 0 and head_stride_a % E == 0 and head_stride_out % E == 0 and ld_a % E == 0 and ld_o % E == 0 and head_stride_a >= n_in
+                 and head_stride_out >= n_out and (a.data_ptr() | weight.data_ptr() | out.data_ptr()) % 16 == 0)
+        if whole and (self.tensor_core_linear if self.dtype == torch.bfloat16 else self.split_linear and n >= self.SPLIT_MIN_ROWS):
+            h = lib("linear_tcgen05" if self.dtype == torch.bfloat16 else "linear_split")
+            call = h.kvad_linear_tcgen05_heads if self.dtype == torch.bfloat16 else h.kvad_linear_split_heads
+            _check(call(_ptr(a), ld_a, int(head_stride_a), _ptr(weight), _ptr(out), ld_o, int(head_stride_out), n, H, n_out, n_in, _stream()), h)
+        else:
+            for hd in range(H):
+                self.linear(a[:, hd * head_stride_a: hd * head_stride_a + n_in], weight[hd], None,
+                            out[:, hd * head_stride_out: hd * head_stride_out + n_out])
         if gate is not None:
             self.gate_mul(gate, out, out, "sigmoid")
 

@@ -1,0 +1,91 @@
+"""The 32-bit product on the tensor cores (operands cut into bfloat16 pieces) and the head-wise maps of many rows in one launch."""
+import pytest
+import torch
+
+from kvad_b200.ops import Ops, lib
+
+pytestmark = pytest.mark.gpu
+DT = {"float32": torch.float32, "bfloat16": torch.bfloat16}
+
+
+def rel(got, ref):
+    return float((got.double() - ref).norm() / ref.norm())
+
+
+def randn(g, *shape):
+    return torch.randn(*shape, generator=g, device="cuda")
+
+
+# edges of tiles (128 rows, 64 or 128 outputs), of a block of K (32) and of the four slots, the shortest K, one row past a tile,
+# more tiles than SMs (a CTA goes round its slots over several tiles)
+@pytest.mark.parametrize("m,n,k", [(33, 64, 4), (64, 65, 32), (127, 128, 36), (128, 200, 128), (129, 63, 160), (300, 1031, 96), (1500, 2309, 200), (70, 5, 772)])
+@pytest.mark.parametrize("tile", [64, 128])
+def test_split_product_is_no_further_off_than_the_fmaf_chain(m, n, k, tile):
+    g = torch.Generator(device="cuda")
+    g.manual_seed(m * n + k)
+    ops, chain = Ops(torch.float32), Ops(torch.float32)
+    chain.split_linear, chain.rows_linear_max, ops.SPLIT_MIN_ROWS = False, 0, 1
+    wide = randn(g, m, k + 8)
+    a, w, b, old = wide[:, 4:4 + k], randn(g, n, k) * 0.3, randn(g, n), randn(g, m, n + 3)[:, :n]
+    exact = a.double() @ w.double().t()
+    for epi in ("store", "gelu_tanh", "gelu_erf", "residual", "store_f32"):
+        want = exact + b.double()
+        if epi.startswith("gelu"):
+            want = torch.nn.functional.gelu(want, approximate="tanh" if epi == "gelu_tanh" else "none")
+        if epi == "residual":
+            want = want + old.double()
+        outs = []
+        for o, t in ((ops, tile), (chain, 0)):
+            out = torch.full((m, n + 3), float("nan"), device="cuda")
+            out[:, :n] = old
+            o.linear(a, w, b, out[:, :n], epi, tile=t)
+            assert torch.isnan(out[:, n:]).all()
+            outs.append(rel(out[:, :n], want))
+        # six products leave out less than 2^-23 of |a||w|; single roundings of the result are 2^-25 on average
+        assert outs[0] < max(1.1 * outs[1], 1.5e-7), (epi, outs)
+    assert lib("linear_split").kvad_linear_split_status() == 0
+
+
+def test_split_product_of_values_that_bfloat16_cannot_hold():
+    """Pieces down to the last bit; infinities, NaN and overflow as the fmaf chain gives them; a row's bits whatever its company."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(5)
+    ops, chain = Ops(torch.float32), Ops(torch.float32)
+    chain.split_linear = False
+    a, w = torch.ones(200, 64, device="cuda"), torch.zeros(96, 64, device="cuda")
+    a[:, 0] = 1.0 + 2.0 ** -23 * torch.arange(1, 201, device="cuda")
+    w[:, 0] = 1.0
+    out = torch.empty(200, 96, device="cuda")
+    ops.linear(a, w, None, out)
+    assert torch.equal(out, a[:, :1].expand(200, 96))                     # a product with 1.0 is exact
+    a, w = randn(g, 200, 64), randn(g, 96, 64)
+    a[3, 5], a[7, 1], a[11, 0], a[20, 0], w[30, 0], w[9, 5], w[9, 0] = float("inf"), float("nan"), -float("inf"), 3e38, 3e38, 0.0, 1.0
+    got, want = torch.empty(200, 96, device="cuda"), torch.empty(200, 96, device="cuda")
+    ops.linear(a, w, None, got)
+    chain.linear(a, w, None, want)
+    assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(torch.isinf(got), torch.isinf(want))
+    fine = torch.isfinite(want)
+    assert bool((got[~fine & ~torch.isnan(want)] == want[~fine & ~torch.isnan(want)]).all()) and rel(got[fine][None], want[fine][None].double()) < 1e-6
+    few = torch.empty(70, 96, device="cuda")
+    ops.linear(a[100:170], w, None, few)
+    assert torch.equal(few, got[100:170])
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("n,H,n_in,n_out,pad", [(65, 3, 64, 256, 0), (129, 16, 32, 64, 16), (300, 2, 72, 40, 8), (1030, 5, 136, 200, 24), (70, 1, 8, 300, 0), (130, 3, 12, 20, 4)])
+def test_head_maps_of_many_rows_in_one_launch(dtype, n, H, n_in, n_out, pad):
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n + n_in)
+    ops, t = Ops(DT[dtype]), DT[dtype]
+    a, w = randn(g, n, H * (n_in + pad)).to(t), (randn(g, H, n_out, n_in) * n_in ** -0.5).to(t)
+    a.view(n, H, -1)[:, :, n_in:] = float("nan")                          # what lies between the heads is nobody's
+    out = torch.full((n, H * (n_out + pad) + 8), float("nan"), device="cuda", dtype=t)
+    ops.linear_heads(a, w, out, head_stride_a=n_in + pad, head_stride_out=n_out + pad)
+    got = out[:, :H * (n_out + pad)].view(n, H, -1)
+    want = torch.einsum("rhi,hji->rhj", a.view(n, H, -1)[:, :, :n_in].double(), w.double())
+    assert rel(got[:, :, :n_out], want) < (2e-7 if dtype == "float32" else 3e-3)      # bfloat16: one rounding, 2^-9 at most
+    assert torch.isnan(got[:, :, n_out:]).all() and torch.isnan(out[:, H * (n_out + pad):]).all()
+    gate = randn(g, n, H * n_out).to(t)
+    gated = torch.empty(n, H * n_out, device="cuda", dtype=t)
+    ops.linear_heads(a, w, gated, head_stride_a=n_in + pad, head_stride_out=n_out, gate=gate)
+    assert rel(gated.view(n, H, n_out), want * torch.sigmoid(gate.double()).view(n, H, n_out)) < (3e-7 if dtype == "float32" else 5e-3)
