@@ -1,0 +1,401 @@
+// Softmax attention of prompt rows over the paged cache with shaped scores (`attention_scored.cu` says what a score can be
+// given), on the tensor cores: bfloat16 queries, keys and values, 32-bit scores, softmax weights and sums.
+//
+//   s = q . k        mma.sync m16n8k16, 32-bit accumulation (products of bfloat16 numbers are exact)
+//   p = exp(s - m)   32-bit, in the accumulators' own registers
+//   o += p v         p is cut into bfloat16 pieces, p = h + l (what is left out is below 2^-16 of p), or p = h + m + l
+//                    exactly where the output is 32-bit: a weight is not rounded to 16 bits, the pieces are multiplied one
+//                    after another.  There the tensor core's truncating accumulation is kept to 64 keys, whose sum then
+//                    joins the 32-bit running sum by a rounded addition.
+//
+// A block of eight warps works 128 (token, head) pairs that share a key head - 128 / hp consecutive tokens of one sequence times
+// hp heads of the group, a warp 16 of them - against the cache's pages of 64 keys: a page comes into shared memory by
+// cp.async while the one before is worked on (values that are the keys' first entries come once).  Queries stay in shared memory,
+// all of the running output in registers.  Rows are padded to an odd number of 16-byte pieces, so ldmatrix meets no bank twice.
+// Pages that no pair of the block sees are skipped.  Tiles are launched longest first.
+//
+// Why: on the CUDA cores (`attention_scored.cu`) 2 x 1024 rows of 16 heads over a latent of 256 took 1102 us (15.6 TFLOP/s),
+// 16 heads of 64 on 4 key heads with capped scores and a window of 512 took 342 us.
+#include "common.cuh"
+
+using namespace kvad;
+
+namespace {
+
+constexpr int PAGE = 64, WARPS = 8, THREADS = 32 * WARPS, ROWS = 16 * WARPS;
+constexpr float LOG2E = 1.4426950408889634f, LN2 = 0.6931471805599453f;
+
+struct PromptArgs {
+  const __nv_bfloat16* q; int64_t ld_q;
+  void* out; int64_t ld_out;
+  const __nv_bfloat16* gate; int64_t ld_gate; int gate_heads;    // gate_heads: one number per row and head
+  const float* sinks;
+  const int* seq_starts; const int* kv_lens; const int* page_table; int table_width;
+  const __nv_bfloat16* k_pages; const __nv_bfloat16* v_pages;
+  int64_t k_page_stride, v_page_stride;                           // in entries; a head's page is PAGE x dk (PAGE x dv)
+  int n_heads, n_kv_heads, dk, dv, hp, alias, key_maps;
+  float scale, softcap, slope_span;
+  int window, keep_first, chunk;
+  int k_steps, k_stride, v_stride;                                // 16-entry steps of a key; row strides in shared memory, in entries
+};
+
+__device__ __forceinline__ uint32_t smem_at(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void ldsm4(uint32_t at, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(at) : "memory");
+}
+__device__ __forceinline__ void ldsm4_t(uint32_t at, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(at) : "memory");
+}
+__device__ __forceinline__ void mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// 16 bytes to shared memory, zeros where `live` is false (places of the cache that no row sees yet may hold anything)
+__device__ __forceinline__ void copy16(uint32_t dst, const void* src, bool live) {
+  const int bytes = live ? 16 : 0;
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+// The upper halves of two floats as a pair of bfloat16 (truncated), and what is left of each.
+__device__ __forceinline__ uint32_t cut(float& a, float& b) {
+  const uint32_t x = __float_as_uint(a), y = __float_as_uint(b);
+  a -= __uint_as_float(x & 0xffff0000u);
+  b -= __uint_as_float(y & 0xffff0000u);
+  return __byte_perm(x, y, 0x7632);
+}
+__device__ __forceinline__ uint32_t pack(float a, float b) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+
+// NV: 16-entry groups of a value.
+template <int NV, bool F32OUT>
+__global__ void __launch_bounds__(THREADS, NV <= 4 ? 2 : 1) scored_prompt_kernel(const PromptArgs a) {
+  extern __shared__ uint8_t smem_raw[];
+  __nv_bfloat16* smem = reinterpret_cast<__nv_bfloat16*>(smem_raw);
+  const int hp = a.hp, tok = ROWS / hp, group = a.n_heads / a.n_kv_heads, chunks = group / hp;
+  const int per_seq = a.n_kv_heads * chunks;
+  const int s = blockIdx.x / per_seq, part = blockIdx.x - s * per_seq, kvh = part / chunks, h0 = kvh * group + (part - kvh * chunks) * hp;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int kst = a.k_stride, vst = a.v_stride;
+  __nv_bfloat16* Qs = smem;                                     // [ROWS][kst]
+  __nv_bfloat16* stages = Qs + ROWS * kst;                      // two of: keys [PAGE][kst], values [PAGE][vst] (or none: the keys)
+  const int stage_size = PAGE * kst + (a.alias ? 0 : PAGE * vst);
+  pdl_launch_dependents();
+  // what no copy writes (the rows' padding) must not be NaN: it is multiplied by zeros
+  {
+    const int total = (ROWS * kst + 2 * stage_size + 16) / 8;
+    for (int i = tid; i < total; i += THREADS) reinterpret_cast<uint4*>(smem)[i] = make_uint4(0u, 0u, 0u, 0u);
+  }
+  pdl_wait();
+  const int start = a.seq_starts[s], n_new = a.seq_starts[s + 1] - start, tok0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * tok;
+  if (tok0 >= n_new) return;
+  const int n_tok = min(tok, n_new - tok0), pos0 = a.kv_lens[s] - n_new + tok0, last_pos = pos0 + n_tok - 1;
+  const int* pages = a.page_table + (int64_t)s * a.table_width;
+  __syncthreads();                                              // the zeros lie
+
+  const int q_pieces = a.dk / 8, v_pieces = a.dv / 8;
+  for (int i = tid; i < ROWS * q_pieces; i += THREADS) {
+    const int r = i / q_pieces, c = i - r * q_pieces, ti = r / hp, hi = r - ti * hp;
+    const bool live = ti < n_tok;
+    copy16(smem_at(Qs + r * kst + c * 8), a.q + (int64_t)(start + tok0 + (live ? ti : 0)) * a.ld_q + (int64_t)(h0 + hi) * a.dk + c * 8, live);
+  }
+  const int first_key = a.chunk > 0 ? pos0 - pos0 % a.chunk : ((a.window > 0 && pos0 - a.window + 1 > 0) ? pos0 - a.window + 1 : 0);   // of the block's first token
+  auto next_page = [&](int t) {                                 // the next page that a pair of the block sees (the same for every thread)
+    while (t * PAGE <= last_pos && t * PAGE + PAGE <= first_key && t * PAGE >= a.keep_first) ++t;
+    return t;
+  };
+  auto bring = [&](int t, int stage) {
+    const int page = pages[t], n_live = last_pos - t * PAGE + 1;
+    __nv_bfloat16* ks = stages + stage * stage_size;
+    const __nv_bfloat16* src = a.k_pages + (int64_t)page * a.k_page_stride + (int64_t)kvh * PAGE * a.dk;
+    for (int i = tid; i < PAGE * q_pieces; i += THREADS) {
+      const int r = i / q_pieces, c = i - r * q_pieces;
+      copy16(smem_at(ks + r * kst + c * 8), src + (int64_t)i * 8, r < n_live);
+    }
+    if (!a.alias) {
+      __nv_bfloat16* vs = ks + PAGE * kst;
+      const __nv_bfloat16* vsrc = a.v_pages + (int64_t)page * a.v_page_stride + (int64_t)(kvh / a.key_maps) * PAGE * a.dv;
+      for (int i = tid; i < PAGE * v_pieces; i += THREADS) {
+        const int r = i / v_pieces, c = i - r * v_pieces;
+        copy16(smem_at(vs + r * vst + c * 8), vsrc + (int64_t)i * 8, r < n_live);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+
+  // this thread's two rows of the warp's 16: lane / 4 and that plus 8
+  int pos[2], first[2], head[2];
+  bool live[2];
+  float slope[2], run_max[2] = {-INFINITY, -INFINITY}, run_sum[2] = {0.f, 0.f};      // (maxima in units of log2)
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const int row = warp * 16 + (lane >> 2) + u * 8, ti = row / hp;
+    head[u] = h0 + row - ti * hp;
+    live[u] = ti < n_tok;
+    pos[u] = pos0 + ti;
+    first[u] = a.window > 0 ? pos[u] - a.window + 1 : (a.chunk > 0 ? pos[u] - pos[u] % a.chunk : 0);
+    slope[u] = a.slope_span > 0.f ? exp2f(-a.slope_span * (float)(head[u] + 1) / (float)a.n_heads) * LOG2E : 0.f;
+  }
+  // keys from `clear_from` up to `clear_to` (and the kept first ones) are seen by every live row of the warp
+  const int warp_ti0 = warp * 16 / hp, warp_ti1 = min((warp * 16 + 15) / hp, n_tok - 1);
+  const bool warp_live = warp_ti0 < n_tok;
+  const int clear_to = pos0 + warp_ti0;
+  const int far = pos0 + warp_ti1;
+  const int clear_from = a.window > 0 ? far - a.window + 1 : (a.chunk > 0 ? far - far % a.chunk : 0);
+  float o[2 * NV][4];
+#pragma unroll
+  for (int j = 0; j < 2 * NV; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) o[j][e] = 0.f;
+  const float scale2 = a.scale * LOG2E, inv_cap2 = a.softcap > 0.f ? 2.f * LOG2E * a.scale / a.softcap : 0.f, cap2 = a.softcap * LOG2E;
+  const uint32_t q_at = smem_at(Qs + (warp * 16 + (lane & 15)) * kst + (lane >> 4) * 8);
+
+  int t = next_page(0), stage = 0;
+  bring(t, 0);
+  while (t * PAGE <= last_pos) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();                                            // this page is there, and the one before has been used up
+    const int t_next = next_page(t + 1);
+    if (t_next * PAGE <= last_pos) bring(t_next, stage ^ 1);
+    const int key0 = t * PAGE;
+    const __nv_bfloat16* ks = stages + stage * stage_size;
+    const __nv_bfloat16* vs = a.alias ? ks : ks + PAGE * kst;
+    t = t_next;
+    stage ^= 1;
+    if (!warp_live) continue;
+    float sc[8][4];
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) sc[j][e] = 0.f;
+    const uint32_t k_at = smem_at(ks + ((lane & 7) + (lane >> 4) * 8) * kst + ((lane >> 3) & 1) * 8);
+#pragma unroll 2
+    for (int kk = 0; kk < a.k_steps; ++kk) {
+      uint32_t qa[4];
+      ldsm4(q_at + kk * 32, qa);
+#pragma unroll
+      for (int ng = 0; ng < 4; ++ng) {
+        uint32_t kb[4];
+        ldsm4(k_at + kk * 32 + ng * 16 * kst * 2, kb);
+        mma(sc[2 * ng], qa, kb[0], kb[1]);
+        mma(sc[2 * ng + 1], qa, kb[2], kb[3]);
+      }
+    }
+    // scores in units of log2, shaped and masked
+    const bool all_seen = key0 + PAGE - 1 <= clear_to && (key0 >= clear_from || key0 + PAGE <= a.keep_first);
+    float top[2] = {-INFINITY, -INFINITY};
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int u = e >> 1, key = key0 + j * 8 + (lane & 3) * 2 + (e & 1);
+        float x = sc[j][e];
+        if (a.softcap > 0.f) {                                  // cap tanh(s / cap), tanh(y) = 1 - 2 / (exp(2 y) + 1)
+          x = F32OUT ? cap2 * tanhf(x * a.scale / a.softcap) : fmaf(-2.f * cap2, __fdividef(1.f, exp2f(x * inv_cap2) + 1.f), cap2);
+        } else {
+          x *= scale2;
+        }
+        x -= slope[u] * (float)(pos[u] - key);
+        if (!all_seen && !(key <= pos[u] && (key >= first[u] || key < a.keep_first))) x = -INFINITY;
+        sc[j][e] = x;
+        top[u] = fmaxf(top[u], x);
+      }
+    float base[2], keep[2], sum[2] = {0.f, 0.f};
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      top[u] = fmaxf(top[u], __shfl_xor_sync(0xffffffffu, top[u], 1));
+      top[u] = fmaxf(top[u], __shfl_xor_sync(0xffffffffu, top[u], 2));
+      const float new_max = fmaxf(run_max[u], top[u]);
+      base[u] = new_max == -INFINITY ? 0.f : new_max;
+      keep[u] = run_max[u] == -INFINITY ? 0.f : exp2f(run_max[u] - base[u]);
+      run_max[u] = new_max;
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int u = e >> 1;
+        sc[j][e] = exp2f(sc[j][e] - base[u]);
+        sum[u] += sc[j][e];
+      }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      sum[u] += __shfl_xor_sync(0xffffffffu, sum[u], 1);
+      sum[u] += __shfl_xor_sync(0xffffffffu, sum[u], 2);
+      run_sum[u] = run_sum[u] * keep[u] + sum[u];
+    }
+    const uint32_t v_at = smem_at(vs + ((lane & 7) + ((lane >> 3) & 1) * 8) * vst + (lane >> 4) * 8);
+    if (!F32OUT) {
+#pragma unroll
+      for (int j = 0; j < 2 * NV; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[j][e] *= keep[e >> 1];
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk) {
+        uint32_t ph[4], pl[4];
+#pragma unroll
+        for (int f = 0; f < 4; ++f) {
+          float x = sc[2 * kk + (f >> 1)][(f & 1) * 2], y = sc[2 * kk + (f >> 1)][(f & 1) * 2 + 1];
+          ph[f] = cut(x, y);
+          pl[f] = pack(x, y);
+        }
+#pragma unroll
+        for (int ng = 0; ng < NV; ++ng) {
+          uint32_t vb[4];
+          ldsm4_t(v_at + kk * 16 * vst * 2 + ng * 32, vb);
+          mma(o[2 * ng], pl, vb[0], vb[1]);
+          mma(o[2 * ng + 1], pl, vb[2], vb[3]);
+          mma(o[2 * ng], ph, vb[0], vb[1]);
+          mma(o[2 * ng + 1], ph, vb[2], vb[3]);
+        }
+      }
+    } else {
+      uint32_t ph[4][4], pm[4][4], pl[4][4];
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+        for (int f = 0; f < 4; ++f) {
+          float x = sc[2 * kk + (f >> 1)][(f & 1) * 2], y = sc[2 * kk + (f >> 1)][(f & 1) * 2 + 1];
+          ph[kk][f] = cut(x, y);
+          pm[kk][f] = cut(x, y);
+          pl[kk][f] = pack(x, y);
+        }
+#pragma unroll
+      for (int ng = 0; ng < NV; ++ng) {
+        float low[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}}, page[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) {
+          uint32_t vb[4];
+          ldsm4_t(v_at + kk * 16 * vst * 2 + ng * 32, vb);
+#pragma unroll
+          for (int w = 0; w < 2; ++w) {
+            mma(low[w], pl[kk], vb[2 * w], vb[2 * w + 1]);
+            mma(low[w], pm[kk], vb[2 * w], vb[2 * w + 1]);
+            mma(page[w], ph[kk], vb[2 * w], vb[2 * w + 1]);
+          }
+        }
+#pragma unroll
+        for (int w = 0; w < 2; ++w)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) o[2 * ng + w][e] = fmaf(o[2 * ng + w][e], keep[e >> 1], page[w][e] + low[w][e]);
+      }
+    }
+  }
+
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    if (!live[u]) continue;
+    const int row = warp * 16 + (lane >> 2) + u * 8, h = head[u];
+    const int64_t grow = start + tok0 + row / hp;
+    float inv;
+    if (a.sinks == nullptr) {
+      inv = 1.0f / run_sum[u];
+    } else {                                                    // a sink is one more term of the denominator
+      const float mine = run_max[u] * LN2, sink = a.sinks[h], m = fmaxf(mine, sink), f = expf(mine - m);
+      inv = f / fmaf(run_sum[u], f, expf(sink - m));
+    }
+    float head_factor = 1.f;
+    if (a.gate != nullptr && a.gate_heads) head_factor = 1.0f / (1.0f + expf(-__bfloat162float(a.gate[grow * a.ld_gate + h])));
+#pragma unroll
+    for (int j = 0; j < 2 * NV; ++j) {
+      const int d = j * 8 + (lane & 3) * 2;                     // (dv is a multiple of 8)
+      if (d >= a.dv) continue;
+      float x = o[j][2 * u] * inv, y = o[j][2 * u + 1] * inv;
+      if (F32OUT) {
+        *reinterpret_cast<float2*>(reinterpret_cast<float*>(a.out) + grow * a.ld_out + (int64_t)h * a.dv + d) = make_float2(x, y);
+      } else {
+        if (a.gate != nullptr && !a.gate_heads) {
+          const __nv_bfloat162 z = *reinterpret_cast<const __nv_bfloat162*>(a.gate + grow * a.ld_gate + (int64_t)h * a.dv + d);
+          x *= 1.0f / (1.0f + expf(-__bfloat162float(z.x)));
+          y *= 1.0f / (1.0f + expf(-__bfloat162float(z.y)));
+        } else {
+          x *= head_factor;
+          y *= head_factor;
+        }
+        *reinterpret_cast<uint32_t*>(reinterpret_cast<__nv_bfloat16*>(a.out) + grow * a.ld_out + (int64_t)h * a.dv + d) = pack(x, y);
+      }
+    }
+  }
+}
+
+template <int NV, bool F32OUT>
+int launch(const PromptArgs& a, int n_seqs, int max_new, size_t smem, cudaStream_t stream) {
+  static size_t configured = 0;
+  if (smem > configured) {
+    cudaError_t e = cudaFuncSetAttribute(scored_prompt_kernel<NV, F32OUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) KVAD_FAIL(KVAD_ERR_CUDA, "attention (scored, prompts): cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
+    configured = smem;
+  }
+  const int tok = ROWS / a.hp;
+  const int64_t columns = (int64_t)n_seqs * (a.n_heads / a.hp);
+  KVAD_REQUIRE(columns < (1ll << 31) && (max_new + tok - 1) / tok <= 65535, "attention (scored, prompts): more tiles than one launch takes");
+  kvad_launch(scored_prompt_kernel<NV, F32OUT>, dim3((unsigned)columns, (max_new + tok - 1) / tok), dim3(THREADS), smem, stream, a);
+  KVAD_CHECK_LAUNCH("attention_scored_prompt");
+  return KVAD_OK;
+}
+
+struct Layout { int k_stride, v_stride; size_t smem; };
+// Row strides of an odd number of 16-byte pieces over whole 16-entry steps; all of shared memory with the slack of one step that the last
+// row's unused value columns may read.
+Layout layout_of(int dk, int dv, bool alias) {
+  Layout z;
+  z.k_stride = (dk + 15) / 16 * 16 + 8;
+  z.v_stride = alias ? z.k_stride : (dv + 15) / 16 * 16 + 8;
+  z.smem = ((size_t)ROWS * z.k_stride + 2 * ((size_t)PAGE * z.k_stride + (alias ? 0 : (size_t)PAGE * z.v_stride)) + 256 + 16) * 2;
+  return z;
+}
+
+}  // namespace
+
+// 1 if prompts of these sizes run here: whole 16-byte pieces, values up to 256 entries (128 where the output is 32-bit), everything in shared memory.
+KVAD_EXPORT int kvad_attention_scored_prompt_takes(int dk, int dv, int alias, int out_f32) {
+  return dk > 0 && dv > 0 && dk % 8 == 0 && dv % 8 == 0 && dv <= (out_f32 ? 128 : 256) && layout_of(dk, dv, alias != 0).smem <= 220 * 1024 ? 1 : 0;
+}
+
+KVAD_EXPORT int kvad_attention_scored_prompt(const void* q, int64_t ld_q, void* out, int64_t ld_out, const void* gate, int64_t ld_gate, int gate_heads,
+                                             const float* sinks, const int* seq_starts, const int* kv_lens, const int* page_table, int table_width,
+                                             const void* k_pages, const void* v_pages, int n_seqs, int n_heads, int n_kv_heads, int dk, int dv,
+                                             int page_size, int max_new, float scale, float softcap, float slope_span, int window, int keep_first,
+                                             int chunk, int key_maps, int out_f32, cudaStream_t stream) {
+  KVAD_REQUIRE(n_seqs >= 0 && n_heads > 0 && n_kv_heads > 0 && dk > 0 && dv > 0 && table_width > 0 && max_new >= 0 && keep_first >= 0,
+               "attention (scored, prompts): bad sizes seqs=%d heads=%d kv_heads=%d dk=%d dv=%d", n_seqs, n_heads, n_kv_heads, dk, dv);
+  KVAD_REQUIRE(n_heads % n_kv_heads == 0, "attention (scored, prompts): %d heads do not divide into %d key/value heads", n_heads, n_kv_heads);
+  KVAD_REQUIRE(chunk <= 0 || window <= 0, "attention (scored, prompts): a chunk goes without a window");
+  const bool alias = v_pages == k_pages;
+  KVAD_REQUIRE(key_maps >= 1 && n_kv_heads % key_maps == 0 && (key_maps == 1 || !alias), "attention (scored, prompts): %d key heads do not share values %d by %d", n_kv_heads, key_maps, key_maps);
+  KVAD_REQUIRE(!out_f32 || gate == nullptr, "attention (scored, prompts): a 32-bit output takes no gate");
+  KVAD_REQUIRE(!alias || dv <= dk, "attention (scored, prompts): values read from the keys cannot be longer than a key");
+  if (page_size != PAGE || !kvad_attention_scored_prompt_takes(dk, dv, alias, out_f32))
+    KVAD_FAIL(KVAD_ERR_UNSUPPORTED, "attention (scored, prompts): pages of %d, keys of %d, values of %d are not taken", page_size, dk, dv);
+  const uintptr_t all = reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k_pages) | reinterpret_cast<uintptr_t>(v_pages);
+  if ((all & 15) || ld_q % 8 != 0 || (reinterpret_cast<uintptr_t>(out) & 7) || ld_out % 2 != 0 ||
+      (gate != nullptr && ((reinterpret_cast<uintptr_t>(gate) & 3) || ld_gate % 2 != 0)))
+    KVAD_FAIL(KVAD_ERR_UNSUPPORTED, "attention (scored, prompts): rows must lie on 16-byte boundaries");
+  if (n_seqs == 0 || max_new == 0) return KVAD_OK;
+  PromptArgs a;
+  a.q = (const __nv_bfloat16*)q; a.ld_q = ld_q; a.out = out; a.ld_out = ld_out; a.gate = (const __nv_bfloat16*)gate; a.ld_gate = ld_gate;
+  a.gate_heads = gate_heads; a.sinks = sinks; a.seq_starts = seq_starts; a.kv_lens = kv_lens; a.page_table = page_table; a.table_width = table_width;
+  a.k_pages = (const __nv_bfloat16*)k_pages; a.v_pages = (const __nv_bfloat16*)v_pages;
+  a.k_page_stride = (int64_t)n_kv_heads * PAGE * dk; a.v_page_stride = (int64_t)(n_kv_heads / key_maps) * PAGE * dv;
+  a.n_heads = n_heads; a.n_kv_heads = n_kv_heads; a.dk = dk; a.dv = dv; a.alias = alias ? 1 : 0; a.key_maps = key_maps;
+  a.scale = scale; a.softcap = softcap; a.slope_span = slope_span; a.window = window > 0 ? window : 0; a.keep_first = window > 0 ? keep_first : 0;
+  a.chunk = chunk > 0 ? chunk : 0;
+  // heads a tile: as many of the group as divide it, up to a warp's 16 rows (a tile then spans few tokens: little of its last page is masked)
+  a.hp = 1;
+  while (a.hp < 16 && (n_heads / n_kv_heads) % (a.hp * 2) == 0) a.hp *= 2;
+  const Layout z = layout_of(dk, dv, alias);
+  a.k_steps = (dk + 15) / 16; a.k_stride = z.k_stride; a.v_stride = z.v_stride;
+#define KVAD_SP(N)                                                                          \
+  do {                                                                                      \
+    if (out_f32) return launch<(N > 8 ? 8 : N), true>(a, n_seqs, max_new, z.smem, stream);  \
+    return launch<N, false>(a, n_seqs, max_new, z.smem, stream);                            \
+  } while (0)
+  if (dv <= 32) KVAD_SP(2);
+  if (dv <= 64) KVAD_SP(4);
+  if (dv <= 128) KVAD_SP(8);
+  if (dv <= 192) KVAD_SP(12);
+  KVAD_SP(16);
+#undef KVAD_SP
+}
+
+KVAD_DEFINE_LAST_ERROR()

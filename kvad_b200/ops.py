@@ -125,6 +125,12 @@ _SIGNATURES = {
         "kvad_latent_store": [c_int, c_void_p, c_int64, c_void_p, c_int, c_float, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
                               c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int64, c_void_p, c_int, c_void_p, c_int64, c_int, c_void_p],
     },
+    "attention_scored_prompt": {
+        "kvad_attention_scored_prompt": [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
+                                         c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_float, c_int, c_int,
+                                         c_int, c_int, c_int, c_void_p],
+        "kvad_attention_scored_prompt_takes": [c_int, c_int, c_int, c_int],
+    },
     "retention": {
         "kvad_retention": [c_int, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64,
                            c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
@@ -238,7 +244,7 @@ _FAMILY_LIBRARIES = {
     "base": {"any": ("rows", "linear_simt", "sampling"), torch.bfloat16: ("linear_rows", "linear_tcgen05"), torch.float32: ("linear_rows_f32", "linear_split")},
     "causal_attention": {"any": ("attention_simt", "attention_decode"), torch.bfloat16: ("attention_prefill",), torch.float32: ()},
     "norm_rotary": {"any": ("norm_rotary",)},
-    "scored_attention": {"any": ("attention_scored",)},
+    "scored_attention": {"any": ("attention_scored",), torch.bfloat16: ("attention_scored_prompt",)},
     "prompt_attention": {torch.bfloat16: ("attention_prefill",)},
     "retention": {"any": ("retention",)},
     "gated_recurrence": {"any": ("gated_recurrence",)},
@@ -337,6 +343,7 @@ class Ops:
         self.rows_linear_max = (2 if dtype == torch.bfloat16 else 16) if self._rows_lib in build.sources() else 0
         # 32-bit products of many rows on the tensor cores, their operands cut into bfloat16 pieces (linear_split.cu)
         self.split_linear = dtype == torch.float32 and "linear_split" in build.sources()
+        self.scored_prompt = dtype == torch.bfloat16 and "attention_scored_prompt" in build.sources()     # shaped scores of prompt rows on the tensor cores
         self.tiled_prompt = True    # prompts that the tensor-core kernel does not take: the tiled CUDA-core kernel, not the row-by-row one
         self._counters = None       # zeroed ints the decode kernel counts finished splits in (left zeroed by it)
         # Two 32-bit buffers [16, width] that q/k/v products of 3..16 rows add their shares of K into (see
@@ -353,7 +360,7 @@ class Ops:
         """Everything on the host that decides which kernels a step of a given shape launches; part of
         the key under which a step's CUDA graph is kept."""
         return (_switch_epoch, self.tensor_core_linear, self.tensor_core_prefill, self.fast_decode,
-                self.rows_linear_max, self.qkv_sums, self.SUMS_MIN_K, self.tiled_prompt, self.split_linear)
+                self.rows_linear_max, self.qkv_sums, self.SUMS_MIN_K, self.tiled_prompt, self.split_linear, self.scored_prompt)
 
     def begin_step(self) -> None:
         """Called once before a step's first kernel (inside the capture, if the step is being captured)."""
@@ -1067,6 +1074,8 @@ class Ops:
         if gate is not None:
             self.gate_mul(gate, out, out, "sigmoid")
 
+    SCORED_PROMPT_MIN_NEW = 2
+
     def attention_scored(self, q, out, seq_starts, kv_lens, n_seqs: int, max_new: int, page_table, k_pages, v_pages, n_heads: int,
                          scale: float, *, value_dim: Optional[int] = None, softcap: float = 0.0, slope_span: float = 0.0,
                          window: int = 0, keep_first: int = 0, gate=None, heads_per_block: int = 1, n_splits: int = 1,
@@ -1109,6 +1118,17 @@ class Ops:
         if n_splits > 1 and (max_new != 1 or scratch is None or scratch.dtype != torch.float32
                              or scratch.numel() < q.shape[0] * n_heads * n_splits * (dv + 2)):
             raise KernelError("attention_scored: splitting keys goes with single-token rows and float32 scratch of rows x heads x splits x (value size + 2)")
+        if (self.scored_prompt and max_new >= self.SCORED_PROMPT_MIN_NEW and n_splits == 1 and page == 64 and ld_q % 8 == 0 and ld_o % 2 == 0 and ld_g % 2 == 0
+                and (q.data_ptr() | k_pages.data_ptr() | v_ptr.data_ptr()) % 16 == 0 and out.data_ptr() % 8 == 0
+                and (gate is None or gate.data_ptr() % 4 == 0) and (v_pages is not None or dv <= dk)
+                and lib("attention_scored_prompt").kvad_attention_scored_prompt_takes(dk, dv, int(v_pages is None), int(out_f32)) == 1):
+            h = lib("attention_scored_prompt")
+            _check(h.kvad_attention_scored_prompt(_ptr(q), ld_q, _ptr(out), ld_o, _ptr(gate), ld_g, int(gate_heads), _ptr(sinks), _ptr(seq_starts),
+                                                  _ptr(kv_lens), _ptr(page_table), page_table.shape[1], _ptr(k_pages), _ptr(v_ptr), int(n_seqs),
+                                                  int(n_heads), n_kv, dk, dv, page, int(max_new), float(scale), float(softcap or 0.0),
+                                                  float(slope_span or 0.0), int(window or 0), int(keep_first or 0), int(chunk or 0), int(key_maps),
+                                                  int(out_f32), _stream()), h)
+            return
         h = lib("attention_scored")
         _check(h.kvad_attention_scored(self.code, _ptr(q), ld_q, _ptr(out), ld_o, _ptr(gate), ld_g, _ptr(seq_starts), _ptr(kv_lens),
                                        _ptr(page_table), page_table.shape[1], _ptr(k_pages), _ptr(v_ptr), int(n_seqs), int(n_heads), n_kv,
