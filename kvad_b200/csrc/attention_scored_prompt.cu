@@ -55,6 +55,17 @@ __device__ __forceinline__ void copy16(uint32_t dst, const void* src, bool live)
   const int bytes = live ? 16 : 0;
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
+// 2^x and 1/x by the special-function unit (2 units in the last place; results below 2^-126 are zero).
+__device__ __forceinline__ float exp2_fast(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float rcp_fast(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
 // The upper halves of two floats as a pair of bfloat16 (truncated), and what is left of each.
 __device__ __forceinline__ uint32_t cut(float& a, float& b) {
   const uint32_t x = __float_as_uint(a), y = __float_as_uint(b);
@@ -148,6 +159,8 @@ __global__ void __launch_bounds__(THREADS, NV <= 4 ? 2 : 1) scored_prompt_kernel
 #pragma unroll
     for (int e = 0; e < 4; ++e) o[j][e] = 0.f;
   const float scale2 = a.scale * LOG2E, inv_cap2 = a.softcap > 0.f ? 2.f * LOG2E * a.scale / a.softcap : 0.f, cap2 = a.softcap * LOG2E;
+  const bool plain = !(a.softcap > 0.f) && !(a.slope_span > 0.f) && a.scale > 0.f;
+  const float unit = plain ? scale2 : 1.f;
   const uint32_t q_at = smem_at(Qs + (warp * 16 + (lane & 15)) * kst + (lane >> 4) * 8);
 
   int t = next_page(0), stage = 0;
@@ -181,33 +194,50 @@ __global__ void __launch_bounds__(THREADS, NV <= 4 ? 2 : 1) scored_prompt_kernel
         mma(sc[2 * ng + 1], qa, kb[2], kb[3]);
       }
     }
-    // scores in units of log2, shaped and masked
-    const bool all_seen = key0 + PAGE - 1 <= clear_to && (key0 >= clear_from || key0 + PAGE <= a.keep_first);
+    // Scores in units of log2, or, where nothing but a positive factor is on them, as they are with the factor `unit` still owed.
+    // (Whole passes over the 32 scores under tests that are the same for every thread: this part is bound by instructions.)
+    if (!plain) {
+      if (a.softcap > 0.f) {                                    // cap tanh(s / cap), tanh(y) = 1 - 2 / (exp(2 y) + 1)
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            sc[j][e] = F32OUT ? cap2 * tanhf(sc[j][e] * a.scale / a.softcap) : fmaf(-2.f * cap2, rcp_fast(exp2_fast(sc[j][e] * inv_cap2) + 1.f), cap2);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) sc[j][e] *= scale2;
+      }
+      if (a.slope_span > 0.f) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) sc[j][e] -= slope[e >> 1] * (float)(pos[e >> 1] - (key0 + j * 8 + (lane & 3) * 2 + (e & 1)));
+      }
+    }
+    if (!(key0 + PAGE - 1 <= clear_to && (key0 >= clear_from || key0 + PAGE <= a.keep_first))) {      // some pair does not see all of the page
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int u = e >> 1, key = key0 + j * 8 + (lane & 3) * 2 + (e & 1);
+          if (!(key <= pos[u] && (key >= first[u] || key < a.keep_first))) sc[j][e] = -INFINITY;
+        }
+    }
     float top[2] = {-INFINITY, -INFINITY};
 #pragma unroll
     for (int j = 0; j < 8; ++j)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int u = e >> 1, key = key0 + j * 8 + (lane & 3) * 2 + (e & 1);
-        float x = sc[j][e];
-        if (a.softcap > 0.f) {                                  // cap tanh(s / cap), tanh(y) = 1 - 2 / (exp(2 y) + 1)
-          x = F32OUT ? cap2 * tanhf(x * a.scale / a.softcap) : fmaf(-2.f * cap2, __fdividef(1.f, exp2f(x * inv_cap2) + 1.f), cap2);
-        } else {
-          x *= scale2;
-        }
-        x -= slope[u] * (float)(pos[u] - key);
-        if (!all_seen && !(key <= pos[u] && (key >= first[u] || key < a.keep_first))) x = -INFINITY;
-        sc[j][e] = x;
-        top[u] = fmaxf(top[u], x);
-      }
+      for (int e = 0; e < 4; ++e) top[e >> 1] = fmaxf(top[e >> 1], sc[j][e]);
     float base[2], keep[2], sum[2] = {0.f, 0.f};
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       top[u] = fmaxf(top[u], __shfl_xor_sync(0xffffffffu, top[u], 1));
       top[u] = fmaxf(top[u], __shfl_xor_sync(0xffffffffu, top[u], 2));
-      const float new_max = fmaxf(run_max[u], top[u]);
+      const float new_max = fmaxf(run_max[u], top[u] * unit);
       base[u] = new_max == -INFINITY ? 0.f : new_max;
-      keep[u] = run_max[u] == -INFINITY ? 0.f : exp2f(run_max[u] - base[u]);
+      keep[u] = run_max[u] == -INFINITY ? 0.f : exp2_fast(run_max[u] - base[u]);
       run_max[u] = new_max;
     }
 #pragma unroll
@@ -215,7 +245,7 @@ __global__ void __launch_bounds__(THREADS, NV <= 4 ? 2 : 1) scored_prompt_kernel
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const int u = e >> 1;
-        sc[j][e] = exp2f(sc[j][e] - base[u]);
+        sc[j][e] = exp2_fast(fmaf(sc[j][e], unit, -base[u]));
         sum[u] += sc[j][e];
       }
 #pragma unroll
@@ -226,10 +256,12 @@ __global__ void __launch_bounds__(THREADS, NV <= 4 ? 2 : 1) scored_prompt_kernel
     }
     const uint32_t v_at = smem_at(vs + ((lane & 7) + ((lane >> 3) & 1) * 8) * vst + (lane >> 4) * 8);
     if (!F32OUT) {
+      if (__any_sync(0xffffffffu, keep[0] != 1.f || keep[1] != 1.f)) {      // (after a few pages the maxima seldom move)
 #pragma unroll
-      for (int j = 0; j < 2 * NV; ++j)
+        for (int j = 0; j < 2 * NV; ++j)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) o[j][e] *= keep[e >> 1];
+          for (int e = 0; e < 4; ++e) o[j][e] *= keep[e >> 1];
+      }
 #pragma unroll
       for (int kk = 0; kk < 4; ++kk) {
         uint32_t ph[4], pl[4];
