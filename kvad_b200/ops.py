@@ -138,6 +138,20 @@ _SIGNATURES = {
         "kvad_retention_needs_raw": [c_int, c_int],
         "kvad_row_norm_gate": [c_int, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int, c_void_p, c_int64, c_int, c_int, c_float, c_void_p],
     },
+    "chunked_recurrence": {
+        "kvad_chunk_places": [c_int, c_int],
+        "kvad_retention_chunked": [c_int, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64,
+                                   c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
+                                   c_int, c_float, c_float, c_int, c_int, c_int, c_void_p, c_void_p],
+        "kvad_matrix_memory_chunked": [c_int, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_int,
+                                       c_void_p, c_int64, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_void_p, c_void_p,
+                                       c_void_p],
+    },
+    "chunked_channels": {
+        "kvad_channels_work": [c_int, c_int],
+        "kvad_channels_chunked": [c_int, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64,
+                                  c_int, c_void_p, c_int64, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p, c_void_p],
+    },
     "gated_recurrence": {
         "kvad_gated_recurrence": [c_int, c_int, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64,
                                   c_void_p, c_void_p, c_int, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_void_p, c_int, c_int, c_int,
@@ -246,8 +260,8 @@ _FAMILY_LIBRARIES = {
     "norm_rotary": {"any": ("norm_rotary",)},
     "scored_attention": {"any": ("attention_scored",), torch.bfloat16: ("attention_scored_prompt",)},
     "prompt_attention": {torch.bfloat16: ("attention_prefill",)},
-    "retention": {"any": ("retention",)},
-    "gated_recurrence": {"any": ("gated_recurrence",)},
+    "retention": {"any": ("retention", "chunked_recurrence")},
+    "gated_recurrence": {"any": ("gated_recurrence", "chunked_recurrence", "chunked_channels")},
     "moe": {"any": ("moe",)},
     "channel_recurrence": {"any": ("channel_recurrence",)},
     "streams": {"any": ("streams",)},
@@ -344,6 +358,7 @@ class Ops:
         # 32-bit products of many rows on the tensor cores, their operands cut into bfloat16 pieces (linear_split.cu)
         self.split_linear = dtype == torch.float32 and "linear_split" in build.sources()
         self.scored_prompt = dtype == torch.bfloat16 and "attention_scored_prompt" in build.sources()     # shaped scores of prompt rows on the tensor cores
+        self.chunked_recurrences = "chunked_recurrence" in build.sources()     # recurrences of prompts: products of 64 rows, not a walk
         self.tiled_prompt = True    # prompts that the tensor-core kernel does not take: the tiled CUDA-core kernel, not the row-by-row one
         self._counters = None       # zeroed ints the decode kernel counts finished splits in (left zeroed by it)
         # Two 32-bit buffers [16, width] that q/k/v products of 3..16 rows add their shares of K into (see
@@ -360,7 +375,7 @@ class Ops:
         """Everything on the host that decides which kernels a step of a given shape launches; part of
         the key under which a step's CUDA graph is kept."""
         return (_switch_epoch, self.tensor_core_linear, self.tensor_core_prefill, self.fast_decode,
-                self.rows_linear_max, self.qkv_sums, self.SUMS_MIN_K, self.tiled_prompt, self.split_linear, self.scored_prompt)
+                self.rows_linear_max, self.qkv_sums, self.SUMS_MIN_K, self.tiled_prompt, self.split_linear, self.scored_prompt, self.chunked_recurrences)
 
     def begin_step(self) -> None:
         """Called once before a step's first kernel (inside the capture, if the step is being captured)."""
@@ -1149,6 +1164,11 @@ class Ops:
         want = (int(per_sm) * (n_sms or sm_count())) // blocks
         return max(1, min(want, -(-reach // 64) + 1, 16))
 
+    # Recurrences of steps with so many rows a sequence, on average, are taken in chunks of 64 rows.  (By the step's shape only.  The walk takes
+    # 0.35 us a row of the longest sequence, the chunks' three kernels 35 .. 75 us for few chunks: 8 heads of 128 x 128, one sequence of 128
+    # rows: 59 us walked, 74 in chunks; four of 245 + 23 + 153 + 76: 102 and 60.)
+    CHUNK_MIN_ROWS = 160
+
     # -- retention ------------------------------------------------------------------------
     def retention(self, q, k, v, out, state, seq_starts, kv_lens, seq_slots, n_seqs: int, decay, n_heads: int, *, inv_freq=None,
                   rot_dims: int = 0, interleaved: bool = False, k_scale: float = 1.0, gate=None, unit_norm_eps: Optional[float] = None,
@@ -1184,6 +1204,20 @@ class Ops:
                 raise KernelError("retention: the gate must have the output's shape and dtype")
         if raw is not None and (raw.dtype != torch.float32 or not raw.is_contiguous() or raw.numel() < n * n_heads * dv):
             raise KernelError("retention: the scratch must be contiguous float32 [rows, heads x dv]")
+        E = 2 if self.dtype == torch.bfloat16 else 4          # bytes of an entry
+        if (self.chunked_recurrences and n >= self.CHUNK_MIN_ROWS * n_seqs and dk <= 128 and dv <= 128 and dk % 4 == 0 and dv % 4 == 0
+                and (ld_q | ld_k | ld_v | ld_g) % 4 == 0 and (q.data_ptr() | k.data_ptr() | v.data_ptr() | (gate.data_ptr() if gate is not None else 0)) % (4 * E) == 0
+                and state.data_ptr() % 16 == 0 and (not raw_only or raw.data_ptr() % 16 == 0)):
+            global _launches
+            h = lib("chunked_recurrence")
+            work = torch.empty(h.kvad_chunk_places(n, int(n_seqs)) * n_heads * dk * dv, dtype=torch.float32, device=q.device)
+            _check(h.kvad_retention_chunked(self.code, _ptr(q), ld_q, _ptr(k), ld_k, _ptr(v), ld_v, _ptr(gate), ld_g, _ptr(out), ld_o, _ptr(raw), n, _ptr(state),
+                                            _ptr(seq_starts), _ptr(kv_lens), _ptr(seq_slots), _ptr(decay), _ptr(inv_freq), int(rot_dims),
+                                            int(bool(interleaved)), int(n_seqs), int(n_heads), dk, dv, float(k_scale),
+                                            float(unit_norm_eps or 0.0), 0 if unit_norm_eps is None else 1, int(bool(silu_inputs)), 0 if raw_only else 1,
+                                            _ptr(work), _stream()), h)
+            _launches += 2          # three kernels: the chunks' sums, the state from chunk to chunk, the read-outs
+            return
         h = lib("retention")
         _check(h.kvad_retention(self.code, _ptr(q), ld_q, _ptr(k), ld_k, _ptr(v), ld_v, _ptr(gate), ld_g, _ptr(out), ld_o, _ptr(raw), n, _ptr(state),
                                 _ptr(seq_starts), _ptr(kv_lens), _ptr(seq_slots), _ptr(decay), _ptr(inv_freq), int(rot_dims),
@@ -1256,6 +1290,29 @@ class Ops:
             p_f32 = 1 if a_log.dtype == torch.float32 else 0
         if not tau > 0:
             raise KernelError("gated_recurrence: tau must be positive")
+        global _launches
+        E = 2 if q.dtype == torch.bfloat16 else 4          # bytes of an entry
+        if (mode == 0 and self.chunked_recurrences and n >= self.CHUNK_MIN_ROWS * n_seqs and dk <= 128 and dv <= 128 and dk % 4 == 0 and dv % 4 == 0
+                and (ld_q | ld_k | ld_v | ld_o | state.stride(0)) % 4 == 0 and (q.data_ptr() | k.data_ptr() | v.data_ptr()) % (4 * E) == 0
+                and (state.data_ptr() | out.data_ptr()) % 16 == 0):
+            h = lib("chunked_recurrence")
+            places = h.kvad_chunk_places(n, int(n_seqs))
+            work = torch.empty(places * n_heads * dk * dv, dtype=torch.float32, device=q.device)
+            work_n = torch.empty(places * n_heads * (dk + 3), dtype=torch.float32, device=q.device)
+            _check(h.kvad_matrix_memory_chunked(_code(q.dtype), _ptr(q), ld_q, _ptr(k), ld_k, _ptr(v), ld_v, _ptr(gates), ld_g, _ptr(out), ld_o, n, _ptr(state),
+                                                state.stride(0), _ptr(seq_starts), _ptr(seq_slots), int(n_seqs), int(n_heads), int(n_kv_heads), int(dk), int(dv),
+                                                float(q_scale), float(cap), _ptr(work), _ptr(work_n), _stream()), h)
+            _launches += 3          # four kernels: the chunks' sums, the state from chunk to chunk, the running maxima, the read-outs
+            return
+        if (mode != 0 and gates_ready and self.chunked_recurrences and n >= self.CHUNK_MIN_ROWS * n_seqs and dk <= 128 and dk % 4 == 0
+                and (ld_q | ld_k | ld_g) % 4 == 0 and (q.data_ptr() | k.data_ptr()) % (4 * E) == 0 and gates.data_ptr() % 16 == 0):
+            h = lib("chunked_channels")
+            work = torch.empty((n // 64 + int(n_seqs)) * int(n_heads) * h.kvad_channels_work(int(dk), int(dv)), dtype=torch.float32, device=q.device)
+            _check(h.kvad_channels_chunked(_code(q.dtype), _ptr(q), ld_q, _ptr(k), ld_k, _ptr(v), ld_v, _ptr(gates), ld_g, _ptr(beta if mode == 1 else None), ld_b,
+                                           _ptr(out), ld_o, n, _ptr(state), state.stride(0), _ptr(seq_starts), _ptr(seq_slots), int(n_seqs), int(n_heads),
+                                           int(n_kv_heads), int(dk), int(dv), float(q_scale), _ptr(work), _stream()), h)
+            _launches += 1          # two kernels: the chunks by themselves, the walk from chunk to chunk
+            return
         h = lib("gated_recurrence")
         _check(h.kvad_gated_recurrence(mode, _code(q.dtype), _ptr(q), ld_q, _ptr(k), ld_k, _ptr(v), ld_v, _ptr(gates), ld_g, _ptr(beta), ld_b,
                                        _ptr(a_log), _ptr(dt_bias), p_f32, _ptr(out), ld_o, _ptr(state), state.stride(0), _ptr(seq_starts),

@@ -1,0 +1,219 @@
+"""Recurrences of prompts taken in chunks of 64 rows, against the row by row formulas in 64 bits: ragged lengths around the edges of chunks
+and blocks, states carried on, sizes that fill no tile, decays of 0 and 1."""
+import numpy as np
+import pytest
+import torch
+
+from kvad_b200.ops import Ops
+
+pytestmark = pytest.mark.gpu
+DT = {"float32": torch.float32, "bfloat16": torch.bfloat16}
+LENS = [65, 1, 129, 64, 300, 16, 63]
+SLOTS = [6, 0, 3, 8, 1, 5, 2]                 # slots 4 and 7 belong to nobody
+
+
+def rel(got, ref):
+    return float((got.double() - ref).norm() / ref.norm().clamp(min=1e-30))
+
+
+def i32(x):
+    return torch.tensor(x, dtype=torch.int32, device="cuda")
+
+
+def starts(lens):
+    return i32([0] + list(np.cumsum(lens)))
+
+
+def portions():
+    """All rows at once; and in two steps, the second of which carries the first one's state on."""
+    yield [LENS]
+    yield [[min(n, 70) for n in LENS], [n - min(n, 70) for n in LENS]]
+
+
+def rows(x, lens, done, part):
+    at = np.cumsum([0] + lens[:-1])
+    return torch.cat([x[a + d:a + d + p] for a, d, p in zip(at, done, part)])
+
+
+def walk(lens, H, dk, dv, q, k, v, g, beta=None, w=None):
+    """S = g S + w k u^T row by row; `g` [n, H, dk] or [n, H, 1].  Read-outs and the states at the ends."""
+    outs, ends, at = [], [], 0
+    for n in lens:
+        S = torch.zeros(H, dk, dv, dtype=torch.float64, device="cuda")
+        for t in range(at, at + n):
+            S = S * g[t][:, :, None]
+            u = v[t] if beta is None else beta[t][:, None] * (v[t] - (S * k[t][:, :, None]).sum(1))
+            S = S + (k[t] if w is None else k[t] * w[t][:, None])[:, :, None] * u[:, None, :]
+            outs.append((S * q[t][:, :, None]).sum(1))
+        ends.append(S)
+        at += n
+    return torch.stack(outs), ends
+
+
+def through(call, lens, out_width):
+    """The rows in the given portions through `call(select, starts, slots, lens after, n, out)`; read-outs of all rows in their order."""
+    got = []
+    for cuts in portions():
+        out = torch.full((sum(lens), out_width), float("nan"), device="cuda")
+        state, done, at = None, [0] * len(lens), np.cumsum([0] + lens[:-1])
+        for part in cuts:
+            live = [i for i in range(len(lens)) if part[i]]
+            o = torch.full((sum(part), out_width), float("nan"), device="cuda")
+            after = [done[i] + part[i] for i in live]
+            state = call(lambda x: rows(x, lens, done, part), starts([part[i] for i in live]), i32([SLOTS[i] for i in live]), i32(after), len(live), o, state)
+            pos = 0
+            for i in live:
+                out[at[i] + done[i]:at[i] + done[i] + part[i]] = o[pos:pos + part[i]]
+                pos += part[i]
+            done = [d + p for d, p in zip(done, part)]
+        got.append((out, state))
+    return got
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("H,dk,dv,rot,inter,act", [(2, 128, 128, 128, False, False), (3, 64, 20, 0, False, True), (1, 4, 64, 4, True, False), (2, 100, 68, 32, False, False)])
+def test_retention_in_chunks(dtype, H, dk, dv, rot, inter, act):
+    g, ops = torch.Generator(device="cuda"), Ops(DT[dtype])
+    g.manual_seed(dk + dv)
+    ops.CHUNK_MIN_ROWS = 1
+    N, t = sum(LENS), DT[dtype]
+    q, k, v, gate = (torch.randn(N, H * d, generator=g, device="cuda").to(t) for d in (dk, dk, dv, dv))
+    decay = torch.linspace(0.9, 1.0, H, device="cuda") if H > 1 else torch.tensor([0.97], device="cuda")
+    freq = (100.0 ** (-torch.arange(0, max(rot, 2), 2, device="cuda") / max(rot, 2))).float() if rot else None
+    ks, eps = dk ** -0.5, 1e-5
+    s = torch.nn.functional.silu if act else (lambda x: x)
+    qd, kd, vd = (s(x.double()).view(N, H, -1).clone() for x in (q, k, v))
+    pos = torch.cat([torch.arange(n, device="cuda") for n in LENS]).double()
+    if rot:
+        ang = (pos[:, None].float() * freq).double()[:, None, :]          # angles as the kernel has them, in 32 bits
+        c, sn = torch.cos(ang), torch.sin(ang)
+        for x in (qd, kd):
+            a, b = (x[..., 0:rot:2], x[..., 1:rot:2]) if inter else (x[..., :rot // 2], x[..., rot // 2:rot])
+            a1, b1 = a * c - b * sn, b * c + a * sn
+            if inter:
+                x[..., 0:rot:2], x[..., 1:rot:2] = a1, b1
+            else:
+                x[..., :rot // 2], x[..., rot // 2:rot] = a1, b1
+    raw, ends = walk(LENS, H, dk, dv, qd, kd * ks, vd, decay.double()[None, :, None].expand(N, H, 1))
+    kw = dict(inv_freq=freq, rot_dims=rot, interleaved=inter, k_scale=ks, silu_inputs=act)
+
+    def run(finish):
+        def call(pick, st, sl, after, n, out, state):
+            state = torch.zeros(9, H, dk, dv, device="cuda") if state is None else state
+            if finish:
+                o = torch.full(out.shape, float("nan"), device="cuda", dtype=t)
+                scratch = torch.empty(out.shape, device="cuda")
+                ops.retention(pick(q), pick(k), pick(v), o, state, st, after, sl, n, decay, H, gate=pick(gate), unit_norm_eps=eps, raw=scratch, **kw)
+                out.copy_(o)
+            else:
+                ops.retention(pick(q), pick(k), pick(v), None, state, st, after, sl, n, decay, H, raw=out, raw_only=True, **kw)
+            return state
+        return through(call, LENS, H * dv)
+
+    gd = gate.double().view(N, H, dv)
+    done = raw / torch.sqrt(raw.square().mean(-1, keepdim=True) + eps) * gd * torch.sigmoid(gd)
+    for finish, want in ((False, raw), (True, done)):
+        for out, state in run(finish):
+            # 32-bit sums of up to 192 terms a chunk; 32-bit sines; the finished rows of bfloat16 are rounded once
+            assert rel(out.view(N, H, dv), want) < (5e-3 if finish and dtype == "bfloat16" else 3e-6)
+            assert all(rel(state[SLOTS[i]], e) < 3e-6 for i, e in enumerate(ends)) and float(state[[4, 7]].abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("H,G,dk,dv", [(2, 2, 128, 128), (4, 2, 64, 20), (1, 1, 4, 64), (3, 1, 100, 72)])
+def test_matrix_memory_in_chunks(dtype, H, G, dk, dv):
+    g, ops, cap = torch.Generator(device="cuda"), Ops(DT[dtype]), 15.0
+    g.manual_seed(dk + dv)
+    ops.CHUNK_MIN_ROWS = 1
+    N, t, tiles = sum(LENS), DT[dtype], -(-dv // 16)
+    q, k, v = (torch.randn(N, n * d, generator=g, device="cuda").to(t) for n, d in ((G, dk), (G, dk), (H, dv)))
+    gates = torch.randn(N, 2 * H, generator=g, device="cuda") * 3.0
+    gates[:, H:] += 4.0
+    gates[200:230, H:] -= 200.0                # a stretch that forgets at the cap: sums of logarithms in the hundreds
+    scale = dk ** -0.5
+    qd, kd, vd = (x.double().view(N, -1, d).repeat_interleave(r, 1) for x, d, r in ((q, dk, H // G), (k, dk, H // G), (v, dv, 1)))
+    gi, gf = cap * torch.tanh(gates[:, :H].double() / cap), torch.nn.functional.logsigmoid(cap * torch.tanh(gates[:, H:].double() / cap))
+    m, f, w = (torch.empty(N, H, dtype=torch.float64, device="cuda") for _ in range(3))
+    at = 0
+    for n in LENS:
+        last = torch.zeros(H, dtype=torch.float64, device="cuda")
+        for r in range(at, at + n):
+            m[r] = torch.maximum(gf[r] + last, gi[r])
+            f[r], w[r] = torch.exp(gf[r] + last - m[r]), torch.exp(gi[r] - m[r])
+            last = m[r]
+        at += n
+    one = torch.ones(N, H, 1, dtype=torch.float64, device="cuda")
+    num, ends = walk(LENS, H, dk, dv, qd * scale, kd, vd, f[:, :, None], w=w)
+    den, n_ends = walk(LENS, H, dk, 1, qd * scale, kd, one, f[:, :, None], w=w)
+    want = num / (torch.maximum(den.abs(), torch.exp(-m)[:, :, None]) + 1e-6)
+
+    def call(pick, st, sl, after, n, out, state):
+        state = torch.zeros(9, ops.recurrence_state_size("matrix_memory", H, dk, dv), device="cuda") if state is None else state
+        state = torch.nn.functional.pad(state, (0, -state.shape[1] % 4)) if state.shape[1] % 4 else state
+        ops.gated_recurrence("matrix_memory", pick(q), pick(k), pick(v), pick(gates), out, state, st, sl, n, H, G, dk, dv, q_scale=scale, cap=cap)
+        return state
+
+    # The gates' logarithms are 32-bit numbers whose errors add up over a reach of rows, in either kernel: a logarithm of up to 15 is off by
+    # 2^-21, and a memory reaches back at most 129 rows that such errors do not cancel over: sqrt(129) 2^-21 times three.
+    tol = 3.0 * 129 ** 0.5 * 2.0 ** -21
+    for out, state in through(call, LENS, H * dv):
+        # a quotient whose sums can nearly cancel
+        assert rel(out.view(N, H, dv), want) < 5e-5
+        last = np.cumsum(LENS) - 1
+        for i, (e, ne) in enumerate(zip(ends, n_ends)):
+            st = state[SLOTS[i]]
+            assert rel(st[:H * dv * dk].view(H, dv, dk).transpose(1, 2), e) < tol
+            norms = st[H * dv * dk:H * dv * dk + H * tiles * dk].view(H, tiles, dk)
+            assert all(rel(norms[:, j], ne[..., 0]) < tol for j in range(tiles))
+            maxima = st[H * dv * dk + H * tiles * dk:H * dv * dk + H * tiles * (dk + 1)].view(H, tiles).double()
+            assert torch.allclose(maxima, m[last[i]][:, None].expand(-1, tiles), rtol=tol, atol=tol)
+        assert float(state[[4, 7]].abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("kind", ["delta_rule", "gated_linear"])
+@pytest.mark.parametrize("H,G,dk,dv", [(2, 2, 128, 128), (4, 2, 64, 20), (1, 1, 4, 64), (3, 1, 100, 72), (2, 1, 36, 7)])
+def test_channel_recurrences_in_chunks(dtype, kind, H, G, dk, dv):
+    g, ops = torch.Generator(device="cuda"), Ops(DT[dtype])
+    g.manual_seed(dk + dv)
+    ops.CHUNK_MIN_ROWS = 1
+    N, t, delta = sum(LENS), DT[dtype], kind == "delta_rule"
+    q, k, v = (torch.randn(N, n, d, generator=g, device="cuda") for n, d in ((G, dk), (G, dk), (H, dv)))
+    if delta:
+        k = torch.nn.functional.normalize(k, dim=-1)
+        k[40:60] = k[40]                          # one key again and again: what was written is taken back every time
+    q, k, v = q.reshape(N, -1).to(t), k.reshape(N, -1).to(t), v.reshape(N, -1).to(t)
+    decay = torch.sigmoid(torch.randn(N, H, dk, generator=g, device="cuda") + 2.0)
+    decay[:, :, 0], decay[:, :, 1] = 1.0, 0.0     # a channel that keeps everything, one that keeps nothing
+    decay[100:103, :, 2] = 1e-30                  # products of these underflow
+    beta = torch.sigmoid(torch.randn(N, H, generator=g, device="cuda"))
+    scale = 0.5
+    qd, kd = (x.double().view(N, G, dk).repeat_interleave(H // G, 1) for x in (q, k))
+    want, ends = walk(LENS, H, dk, dv, qd * scale, kd, v.double().view(N, H, dv), decay.double(), beta=beta.double() if delta else None)
+    more = dict(beta=beta, a_log=torch.zeros(H, device="cuda"), dt_bias=torch.zeros(H * dk, device="cuda")) if delta else {}
+
+    def call(pick, st, sl, after, n, out, state):
+        state = torch.zeros(9, ops.recurrence_state_size(kind, H, dk, dv) + 3, device="cuda") if state is None else state
+        kw = dict(more, beta=pick(beta)) if delta else {}
+        ops.gated_recurrence(kind, pick(q), pick(k), pick(v), pick(decay.view(N, -1)), out, state, st, sl, n, H, G, dk, dv, q_scale=scale, gates_ready=True, **kw)
+        return state
+
+    for out, state in through(call, LENS, H * dv):
+        assert rel(out.view(N, H, dv), want) < 3e-6
+        for i, e in enumerate(ends):
+            assert rel(state[SLOTS[i]][:H * dv * dk].view(H, dv, dk).transpose(1, 2), e) < 3e-6
+        assert float(state[[4, 7]].abs().max()) == 0.0
+
+
+def test_the_walk_still_takes_what_the_chunks_do_not():
+    """Short steps, decays that are not worked out yet, keys of more than 128 entries and odd sizes: the same answers by the other kernel."""
+    g, ops = torch.Generator(device="cuda"), Ops(torch.float32)
+    g.manual_seed(1)
+    for n, dk, ready in ((80, 64, True), (400, 64, False), (400, 132, True), (400, 62, True)):
+        q, k, v = (torch.randn(n, d, generator=g, device="cuda") for d in (dk, dk, 16))
+        z = torch.randn(n, dk, generator=g, device="cuda")
+        decay = torch.sigmoid(z.double())
+        want, _ = walk([n], 1, dk, 16, q.double()[:, None], k.double()[:, None], v.double()[:, None], decay[:, None])
+        out, state = torch.full((n, 16), float("nan"), device="cuda"), torch.zeros(1, ops.recurrence_state_size("gated_linear", 1, dk, 16), device="cuda")
+        ops.gated_recurrence("gated_linear", q, k, v, decay.float() if ready else z, out, state, starts([n]), i32([0]), 1, 1, 1, dk, 16, gates_ready=ready)
+        assert rel(out, want[:, 0]) < 3e-6
