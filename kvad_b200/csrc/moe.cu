@@ -461,22 +461,81 @@ grouped_linear_kernel(const T* __restrict__ a, int64_t ld_a, const int* __restri
   }
 }
 
-// The same product for steps of a few rows (decoding): a stream of the chosen experts' weights.  A warp owns two outputs
-// of one tile; its lanes take every 32nd 16-byte piece of the two weight rows (several on their way at once) and
-// multiply them with the same pieces of up to eight of the tile's rows (which stay in the L1); a shuffle tree per
-// (row, output) at the end.  A tile with more than eight rows streams its weights again per eight, from the L2.
-template <typename T, typename TO>
-__global__ void __launch_bounds__(256)
+// The same product for steps of a few rows (decoding): a stream of the chosen experts' weights.  A block owns 8 CU outputs of a
+// tile, whose weight rows lie side by side in memory: ONE bulk copy brings all of them (45 KB at K = 1408), asked for as soon as the
+// tile's expert is known and before its rows are looked up, so that with three blocks an SM some 130 KB a SM are on their way.  A warp
+// then has CU outputs; its lanes take every 32nd 16-byte piece of the weight rows, from shared memory, and multiply them with the same pieces
+// of 1, 2, 4 or 8 of the tile's rows (which stay in the L1); a shuffle tree per (row, output) at the end.  A tile with more than
+// eight rows goes over its weights again per eight.  (With the weights fetched into registers piece by piece, 8 x 4 loads a warp, 64
+// pairs of 16 experts of 1408 x 1024 took 44 us: a block held its registers through three trips to memory one after another.)
+__device__ int g_rows_timeouts = 0;
+constexpr uint32_t ROWS_WAIT_LIMIT = 1u << 24;
+
+template <typename T, typename TO, int R, int CU>
+__device__ __forceinline__ void rows_times(const T* __restrict__ a, int64_t ld_a, const int* rows_in, const int* rows_out, int n, const T* w,
+                                           TO* __restrict__ out, int64_t ld_out, int col0, int n_out, int k_dim, int lane) {
+  constexpr int PIECE = 16 / (int)sizeof(T);
+  const T* ar[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) ar[r] = a + (int64_t)rows_in[r < n ? r : 0] * ld_a;
+  float acc[R][CU] = {};
+#pragma unroll 2
+  for (int k = lane * PIECE; k < k_dim; k += 32 * PIECE) {
+    float wv[CU][PIECE], av[PIECE];
+#pragma unroll
+    for (int c = 0; c < CU; ++c) load_piece<T, PIECE>(w + c * k_dim + k, PIECE, true, wv[c]);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      load_piece<T, PIECE>(ar[r] + k, PIECE, true, av);
+#pragma unroll
+      for (int j = 0; j < PIECE; ++j) {
+#pragma unroll
+        for (int c = 0; c < CU; ++c) acc[r][c] = fmaf(av[j], wv[c][j], acc[r][c]);
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    if (r < n) {
+      float sums[CU];
+#pragma unroll
+      for (int c = 0; c < CU; ++c) sums[c] = warp_sum(acc[r][c]);
+      if (lane == 0) {
+        TO* o = out + (int64_t)rows_out[r] * ld_out + col0;
+#pragma unroll
+        for (int c = 0; c < CU; ++c)
+          if (col0 + c < n_out) o[c] = from_f32<TO>(sums[c]);
+      }
+    }
+  }
+}
+
+template <typename T, typename TO, int CU>
+__global__ void __launch_bounds__(256, 3)
 grouped_rows_kernel(const T* __restrict__ a, int64_t ld_a, const int* __restrict__ in_rows, const T* __restrict__ w,
                     int64_t expert_stride, TO* __restrict__ out, int64_t ld_out, const int* __restrict__ out_rows,
                     const int* __restrict__ valid, const int* __restrict__ tile_expert, int n_out, int k_dim) {
-  constexpr int R = 8, CU = 2, PIECE = 16 / (int)sizeof(T);       // (four outputs a warp: 4 % slower on the step, fewer blocks and more registers)
+  extern __shared__ __align__(128) uint8_t rows_smem[];
+  T* ws = reinterpret_cast<T*>(rows_smem);      // [8 CU][k_dim]
   __shared__ int rows_in[TM], rows_out[TM], n_valid;
+  __shared__ uint64_t here;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, tile = blockIdx.y, first = blockIdx.x * 8 * CU;
+  const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&here);
+  if (tid == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
   pdl_launch_dependents();
   pdl_wait();
-  const int tile = blockIdx.y, expert = tile_expert[tile];
+  const int expert = tile_expert[tile];
   if (expert < 0) return;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid == 0) {
+    const uint32_t bytes = (uint32_t)min(8 * CU, n_out - first) * (uint32_t)k_dim * (uint32_t)sizeof(T);
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"((uint32_t)__cvta_generic_to_shared(ws)), "l"(w + (int64_t)expert * expert_stride + (int64_t)first * k_dim), "r"(bytes), "r"(bar) : "memory");
+  }
   if (tid < TM) {                               // the tile's used positions, side by side
     const int p = tile * TM + tid;
     const bool used = valid[p] >= 0;
@@ -489,48 +548,28 @@ grouped_rows_kernel(const T* __restrict__ a, int64_t ld_a, const int* __restrict
     if (tid == 0) n_valid = __popc(mask);
   }
   __syncthreads();
-  const int col0 = (blockIdx.x * 8 + warp) * CU;
+  bool there = false;
+  for (uint32_t i = 0; i < ROWS_WAIT_LIMIT && !there; ++i) {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar) : "memory");
+    there = ok != 0;
+  }
+  if (!there) {                                 // (the copy never came: say so, write nothing)
+    if (lane == 0) atomicAdd(&g_rows_timeouts, 1);
+    return;
+  }
+  const int col0 = first + warp * CU;
   if (col0 >= n_out) return;
-  const T* we = w + (int64_t)expert * expert_stride;
-  const T* wr[CU];
-#pragma unroll
-  for (int c = 0; c < CU; ++c) wr[c] = we + (int64_t)(col0 + c < n_out ? col0 + c : col0) * k_dim;
-  for (int r0 = 0; r0 < n_valid; r0 += R) {
-    const int nr = min(R, n_valid - r0);
-    float acc[R][CU] = {};
-#pragma unroll 4
-    for (int k = lane * PIECE; k < k_dim; k += 32 * PIECE) {
-      float wv[CU][PIECE], av[PIECE];
-#pragma unroll
-      for (int c = 0; c < CU; ++c) load_piece<T, PIECE>(wr[c] + k, PIECE, true, wv[c]);
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        if (r < nr) {
-          load_piece<T, PIECE>(a + (int64_t)rows_in[r0 + r] * ld_a + k, PIECE, true, av);
-#pragma unroll
-          for (int j = 0; j < PIECE; ++j) {
-#pragma unroll
-            for (int c = 0; c < CU; ++c) acc[r][c] = fmaf(av[j], wv[c][j], acc[r][c]);
-          }
-        }
-      }
-    }
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      if (r < nr) {
-        float sums[CU];
-#pragma unroll
-        for (int c = 0; c < CU; ++c) sums[c] = warp_sum(acc[r][c]);
-        if (lane == 0) {
-          TO* o = out + (int64_t)rows_out[r0 + r] * ld_out + col0;
-#pragma unroll
-          for (int c = 0; c < CU; ++c)
-            if (col0 + c < n_out) o[c] = from_f32<TO>(sums[c]);
-        }
-      }
-    }
+  const T* wr = ws + (int64_t)warp * CU * k_dim;      // (rows past the last output are not there: what they give is not written)
+  for (int r0 = 0; r0 < n_valid; r0 += 8) {
+    const int n = min(8, n_valid - r0);
+    if (n == 1) rows_times<T, TO, 1, CU>(a, ld_a, rows_in + r0, rows_out + r0, n, wr, out, ld_out, col0, n_out, k_dim, lane);
+    else if (n == 2) rows_times<T, TO, 2, CU>(a, ld_a, rows_in + r0, rows_out + r0, n, wr, out, ld_out, col0, n_out, k_dim, lane);
+    else if (n <= 4) rows_times<T, TO, 4, CU>(a, ld_a, rows_in + r0, rows_out + r0, n, wr, out, ld_out, col0, n_out, k_dim, lane);
+    else rows_times<T, TO, 8, CU>(a, ld_a, rows_in + r0, rows_out + r0, n, wr, out, ld_out, col0, n_out, k_dim, lane);
   }
 }
+
 
 __device__ __forceinline__ float clamped_glu_f(float gate, float up, float limit, float alpha) {
   const float g = fminf(gate, limit);
@@ -723,6 +762,19 @@ inline int flat_blocks(int64_t total, int threads) {
   return (int)(b < 148 * 16 ? (b < 1 ? 1 : b) : 148 * 16);
 }
 
+template <typename T, typename TO, int CU>
+int launch_rows(dim3 grid, size_t smem, cudaStream_t stream, const T* a, int64_t ld_a, const int* in_rows, const T* w, int64_t expert_stride, TO* out, int64_t ld_out,
+                const int* out_rows, const int* valid, const int* tile_expert, int n_out, int k_dim) {
+  static size_t configured = 48 * 1024;
+  if (smem > configured) {
+    cudaError_t e = cudaFuncSetAttribute(grouped_rows_kernel<T, TO, CU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) KVAD_FAIL(KVAD_ERR_CUDA, "grouped_linear: cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
+    configured = smem;
+  }
+  kvad_launch(grouped_rows_kernel<T, TO, CU>, grid, dim3(256), smem, stream, a, ld_a, in_rows, w, expert_stride, out, ld_out, out_rows, valid, tile_expert, n_out, k_dim);
+  return KVAD_OK;
+}
+
 }  // namespace
 
 KVAD_EXPORT int kvad_moe_tile_rows() { return TM; }
@@ -781,6 +833,14 @@ KVAD_EXPORT int kvad_moe_sort(int* chosen, int n_slots, int top, int n_experts, 
   return KVAD_OK;
 }
 
+// How many waits for a block's weights have run out since the library was loaded (0 in a healthy run).  Synchronises the device.
+KVAD_EXPORT int kvad_moe_status() {
+  int n = 0;
+  cudaError_t e = cudaMemcpyFromSymbol(&n, g_rows_timeouts, sizeof(int));
+  if (e != cudaSuccess) KVAD_FAIL(KVAD_ERR_CUDA, "moe_status: %s", cudaGetErrorString(e));
+  return n;
+}
+
 // Position p reads row in_rows[p] of `a` (null: row p) and writes row out_rows[p] of `out` (null: row p); valid[p] < 0: padding.
 // few_rows: the step has so few rows that most of a tile is padding; where the sizes allow 16-byte pieces the weight-streaming
 // form runs.
@@ -794,11 +854,18 @@ KVAD_EXPORT int kvad_grouped_linear(int dtype, int out_f32, const void* a, int64
   const int piece = dtype == KVAD_DTYPE_F32 ? 4 : 8;
   const int vec = (k_dim % piece == 0 && ld_a % piece == 0 && expert_stride % piece == 0 &&
                    ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w)) & 15) == 0) ? 1 : 0;
-  if (few_rows && vec) {
-    dim3 rgrid((n_out + 15) / 16, max_tiles);
-#define KVAD_GR(T, TO)                                                                                                     \
-  kvad_launch(grouped_rows_kernel<T, TO>, rgrid, block, 0, stream, (const T*)a, ld_a, in_rows, (const T*)w, expert_stride, (TO*)out, \
-              ld_out, out_rows, valid, tile_expert, n_out, k_dim)
+  // the weight rows of a block in shared memory, two outputs a warp where 16 rows are at most 64 KB, else one (up to 200 KB: beyond, the tiled form)
+  const size_t row_bytes = (size_t)k_dim * (dtype == KVAD_DTYPE_F32 ? 4 : 2);
+  if (few_rows && vec && 8 * row_bytes <= 200 * 1024) {
+    const int cu = 16 * row_bytes <= 64 * 1024 ? 2 : 1;
+    const size_t smem = 8 * cu * row_bytes;
+    dim3 rgrid((n_out + 8 * cu - 1) / (8 * cu), max_tiles);
+#define KVAD_GR(T, TO)                                                                                                         \
+  do {                                                                                                                         \
+    int rc = cu == 2 ? launch_rows<T, TO, 2>(rgrid, smem, stream, (const T*)a, ld_a, in_rows, (const T*)w, expert_stride, (TO*)out, ld_out, out_rows, valid, tile_expert, n_out, k_dim)  \
+                     : launch_rows<T, TO, 1>(rgrid, smem, stream, (const T*)a, ld_a, in_rows, (const T*)w, expert_stride, (TO*)out, ld_out, out_rows, valid, tile_expert, n_out, k_dim); \
+    if (rc != KVAD_OK) return rc;                                                                                              \
+  } while (0)
     if (dtype == KVAD_DTYPE_F32) KVAD_GR(float, float);
     else if (dtype == KVAD_DTYPE_BF16 && out_f32) KVAD_GR(__nv_bfloat16, float);
     else if (dtype == KVAD_DTYPE_BF16) KVAD_GR(__nv_bfloat16, __nv_bfloat16);

@@ -166,6 +166,7 @@ _SIGNATURES = {
     },
     "moe": {
         "kvad_moe_tile_rows": [],
+        "kvad_moe_status": [],
         "kvad_moe_route_apart_rows": [],
         "kvad_moe_route": [c_void_p, c_int64, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p],
         "kvad_moe_sort": [c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_void_p,
