@@ -315,6 +315,255 @@ __global__ void __launch_bounds__(32 * NW) scored_attention_kernel(const ScoredA
   }
 }
 
+// ---- single-token rows on the tensor cores (bfloat16) ---------------------------------------------------------------------
+// A block has one row's heads that share a key head - 16 of them at most, the 16 rows of an mma.sync m16n8k16 - and its share of the pages.
+// Per page of 64 keys a warp of four takes the scores of 16 keys (products of bfloat16 numbers, summed in 32 bits), the warps meet twice in
+// shared memory for the row's maximum and sum, and each takes a quarter of the values' columns.  A softmax weight enters that product as
+// three bfloat16 pieces (p = h + m + l, by truncation: all 24 bits of it), and a page's sum joins the running one by a rounded addition.
+// The next page is on its way while one is worked.  Such a row is a chain of latencies, not of bytes: on the CUDA cores, a page a block and
+// four heads a warp, 8 rows of 16 heads at 520 keys of a latent of 288 took 20.4 us.
+__device__ __forceinline__ uint32_t smem_at(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void ldsm4(uint32_t at, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(at) : "memory");
+}
+__device__ __forceinline__ void ldsm4_t(uint32_t at, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(at) : "memory");
+}
+__device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void copy16(void* dst, const void* src, bool live) {      // zeros where `live` is false
+  const int bytes = live ? 16 : 0;
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_at(dst)), "l"(src), "r"(bytes) : "memory");
+}
+
+constexpr int STEP_HEADS = 16, STEP_LDP = PAGE + 8;
+struct StepLayout { int k_stride, v_stride; size_t smem; };
+inline StepLayout step_layout(int dk, int dv, bool alias) {
+  StepLayout z;
+  z.k_stride = (dk + 15) / 16 * 16 + 8;                 // an odd number of 16-byte pieces: ldmatrix meets no bank twice
+  z.v_stride = alias ? z.k_stride : (dv + 15) / 16 * 16 + 8;
+  z.smem = ((size_t)STEP_HEADS * z.k_stride + 2 * ((size_t)PAGE * z.k_stride + (alias ? 0 : (size_t)PAGE * z.v_stride)) + 256 + 3 * STEP_HEADS * STEP_LDP) * 2;
+  return z;
+}
+
+// NT: pairs of 8-entry groups of a value that a warp owns.
+template <int NT>
+__global__ void __launch_bounds__(128) scored_step_kernel(const ScoredArgs a, int kst, int vst) {
+  using T = __nv_bfloat16;
+  extern __shared__ float smem[];
+  __shared__ float red_max[4][STEP_HEADS], red_sum[4][STEP_HEADS];
+  T* Qs = reinterpret_cast<T*>(smem);                   // [16][kst]
+  T* Ps = Qs + STEP_HEADS * kst;                        // [3][16][STEP_LDP]: the weights' pieces
+  T* stages = Ps + 3 * STEP_HEADS * STEP_LDP;
+  const int stage_size = PAGE * kst + (a.v_alias ? 0 : PAGE * vst);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  pdl_launch_dependents();
+  // what no copy writes (the rows' padding) must not be NaN: it is multiplied by zeros
+  for (int i = tid; i < (STEP_HEADS * kst + 3 * STEP_HEADS * STEP_LDP + 2 * stage_size) / 8; i += 128) reinterpret_cast<uint4*>(smem)[i] = make_uint4(0u, 0u, 0u, 0u);
+  pdl_wait();
+  const int group = a.n_heads / a.n_kv_heads, chunks = (group + STEP_HEADS - 1) / STEP_HEADS;
+  const int s = blockIdx.y, kvh = blockIdx.z / chunks, chunk = blockIdx.z - kvh * chunks, n_splits = a.n_splits, split = blockIdx.x;
+  const int start = a.seq_starts[s];
+  if (a.seq_starts[s + 1] <= start) return;
+  const int pos = a.kv_lens[s] - 1, h0 = kvh * group + chunk * STEP_HEADS, n_h = min(STEP_HEADS, group - chunk * STEP_HEADS);
+  const int* pages = a.page_table + (int64_t)s * a.table_width;
+  __syncthreads();                                      // the zeros lie
+  const int q_pieces = a.dk / 8, v_pieces = a.dv / 8;
+  for (int i = tid; i < n_h * q_pieces; i += 128) {
+    const int r = i / q_pieces, c = i - r * q_pieces;
+    copy16(Qs + r * kst + c * 8, (const T*)a.q + (int64_t)start * a.ld_q + (int64_t)(h0 + r) * a.dk + c * 8, true);
+  }
+  const int first_key = a.window > 0 ? max(0, pos - a.window + 1) : (a.chunk > 0 ? pos - pos % a.chunk : 0);
+  int dealt = 0;
+  auto next_page = [&](int t) {                         // this block's next page from t on (the same for every thread)
+    for (; t * PAGE <= pos; ++t) {
+      if (t * PAGE + PAGE <= first_key && t * PAGE >= a.keep_first) continue;
+      if (dealt++ % n_splits == split) break;
+    }
+    return t;
+  };
+  auto bring = [&](int t, int stage) {
+    const int64_t page = pages[t];
+    const int n_live = pos - t * PAGE + 1;
+    T* ks = stages + stage * stage_size;
+    const T* src = (const T*)a.k_pages + page * a.k_page_stride + (int64_t)kvh * a.k_head_stride;
+    for (int i = tid; i < PAGE * q_pieces; i += 128) {
+      const int r = i / q_pieces, c = i - r * q_pieces;
+      copy16(ks + r * kst + c * 8, src + (int64_t)r * a.ld_k + c * 8, r < n_live);
+    }
+    if (!a.v_alias) {
+      const T* vsrc = (const T*)a.v_pages + page * a.v_page_stride + (int64_t)(kvh / a.key_maps) * a.v_head_stride;
+      for (int i = tid; i < PAGE * v_pieces; i += 128) {
+        const int r = i / v_pieces, c = i - r * v_pieces;
+        copy16(ks + PAGE * kst + r * vst + c * 8, vsrc + (int64_t)r * a.ld_v + c * 8, r < n_live);
+      }
+    }
+  };
+  const int g = lane >> 2, c2 = (lane & 3) * 2;         // this thread's rows g and g + 8, its columns of a tile
+  float slope[2], run_max[2] = {-INFINITY, -INFINITY}, run_sum[2] = {0.f, 0.f}, o[2 * NT][4];
+#pragma unroll
+  for (int u = 0; u < 2; ++u) slope[u] = a.slope_span > 0.f ? exp2f(-a.slope_span * (float)(h0 + g + 8 * u + 1) / (float)a.n_heads) : 0.f;
+#pragma unroll
+  for (int j = 0; j < 2 * NT; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) o[j][e] = 0.f;
+  int t = next_page(0), stage = 0;
+  if (t * PAGE <= pos) bring(t, 0);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  const int steps = (a.dk + 15) / 16;
+  while (t * PAGE <= pos) {
+    const int t_next = next_page(t + 1);
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();                                    // this page is there, and the one before has been used up
+    if (t_next * PAGE <= pos) bring(t_next, stage ^ 1);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    const int key0 = t * PAGE;
+    const T* ks = stages + stage * stage_size;
+    const T* vs = a.v_alias ? ks : ks + PAGE * kst;
+    t = t_next;
+    stage ^= 1;
+    float sc[2][4] = {};
+    const uint32_t q_at = smem_at(Qs + (lane & 15) * kst + (lane >> 4) * 8);
+    const uint32_t k_at = smem_at(ks + (warp * 16 + (lane & 7) + (lane >> 4) * 8) * kst + ((lane >> 3) & 1) * 8);
+#pragma unroll 4
+    for (int kk = 0; kk < steps; ++kk) {
+      uint32_t qa[4], kb[4];
+      ldsm4(q_at + kk * 32, qa);
+      ldsm4(k_at + kk * 32, kb);
+      mma_bf16(sc[0], qa, kb[0], kb[1]);
+      mma_bf16(sc[1], qa, kb[2], kb[3]);
+    }
+    float top[2] = {-INFINITY, -INFINITY};
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int u = e >> 1, key = key0 + warp * 16 + j * 8 + c2 + (e & 1);
+        float x = sc[j][e] * a.scale;
+        if (a.softcap > 0.f) x = a.softcap * tanhf(x / a.softcap);
+        x -= slope[u] * (float)(pos - key);
+        if (!(key <= pos && (key >= first_key || key < a.keep_first))) x = -INFINITY;
+        sc[j][e] = x;
+        top[u] = fmaxf(top[u], x);
+      }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      top[u] = fmaxf(top[u], __shfl_xor_sync(0xffffffffu, top[u], 1));
+      top[u] = fmaxf(top[u], __shfl_xor_sync(0xffffffffu, top[u], 2));
+      if ((lane & 3) == 0) red_max[warp][g + 8 * u] = top[u];
+    }
+    __syncthreads();
+    float base[2], keep[2], sum[2] = {0.f, 0.f};
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int r = g + 8 * u;
+      const float new_max = fmaxf(fmaxf(run_max[u], fmaxf(red_max[0][r], red_max[1][r])), fmaxf(red_max[2][r], red_max[3][r]));
+      base[u] = new_max == -INFINITY ? 0.f : new_max;
+      keep[u] = run_max[u] == -INFINITY ? 0.f : expf(run_max[u] - base[u]);
+      run_max[u] = new_max;
+    }
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        float p0 = sc[j][2 * u] == -INFINITY ? 0.f : expf(sc[j][2 * u] - base[u]), p1 = sc[j][2 * u + 1] == -INFINITY ? 0.f : expf(sc[j][2 * u + 1] - base[u]);
+        sum[u] += p0 + p1;
+        T* at = Ps + (g + 8 * u) * STEP_LDP + warp * 16 + j * 8 + c2;
+#pragma unroll
+        for (int piece = 0; piece < 3; ++piece) {
+          const uint32_t x = __float_as_uint(p0), y = __float_as_uint(p1);
+          p0 -= __uint_as_float(x & 0xffff0000u);
+          p1 -= __uint_as_float(y & 0xffff0000u);
+          *reinterpret_cast<uint32_t*>(at + piece * STEP_HEADS * STEP_LDP) = __byte_perm(x, y, 0x7632);
+        }
+      }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      sum[u] += __shfl_xor_sync(0xffffffffu, sum[u], 1);
+      sum[u] += __shfl_xor_sync(0xffffffffu, sum[u], 2);
+      if ((lane & 3) == 0) red_sum[warp][g + 8 * u] = sum[u];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int r = g + 8 * u;
+      run_sum[u] = run_sum[u] * keep[u] + ((red_sum[0][r] + red_sum[1][r]) + (red_sum[2][r] + red_sum[3][r]));
+    }
+    float low[2 * NT][4] = {}, high[2 * NT][4] = {};
+    const uint32_t p_at = smem_at(Ps + (lane & 15) * STEP_LDP + (lane >> 4) * 8);
+    const uint32_t v_at = smem_at(vs + ((lane & 7) + ((lane >> 3) & 1) * 8) * vst + warp * 16 * NT + (lane >> 4) * 8);
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk) {
+      uint32_t p[3][4];
+#pragma unroll
+      for (int piece = 0; piece < 3; ++piece) ldsm4(p_at + (piece * STEP_HEADS * STEP_LDP + kk * 16) * 2, p[piece]);
+#pragma unroll
+      for (int n = 0; n < NT; ++n) {
+        uint32_t vb[4];
+        ldsm4_t(v_at + kk * 16 * vst * 2 + n * 32, vb);
+#pragma unroll
+        for (int w = 0; w < 2; ++w) {
+          mma_bf16(low[2 * n + w], p[2], vb[2 * w], vb[2 * w + 1]);
+          mma_bf16(low[2 * n + w], p[1], vb[2 * w], vb[2 * w + 1]);
+          mma_bf16(high[2 * n + w], p[0], vb[2 * w], vb[2 * w + 1]);
+        }
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 2 * NT; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) o[j][e] = fmaf(o[j][e], keep[e >> 1], high[j][e] + low[j][e]);
+  }
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const int r = g + 8 * u, h = h0 + r;
+    if (r >= n_h) continue;
+    float* dst = nullptr;
+    float inv = 1.f;
+    if (n_splits > 1) {
+      dst = a.partial + (((int64_t)start * a.n_heads + h) * n_splits + split) * (a.dv + 2);
+      if (warp == 0 && c2 == 0) {
+        dst[0] = run_max[u];
+        dst[1] = run_sum[u];
+      }
+    } else {
+      inv = softmax_factor(run_max[u], run_sum[u], a.sinks, h);
+    }
+#pragma unroll
+    for (int j = 0; j < 2 * NT; ++j) {
+      const int d = warp * 16 * NT + j * 8 + c2;        // (dv is a multiple of 8)
+      if (d >= a.dv) continue;
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        float y = o[j][2 * u + e] * inv;
+        if (n_splits > 1) {
+          dst[2 + d + e] = y;
+        } else {
+          if (a.gate != nullptr) y *= gate_factor((const T*)a.gate, a.ld_gate, a.gate_heads, start, h, a.dv, d + e);
+          if (a.out_f32) reinterpret_cast<float*>(a.out)[(int64_t)start * a.ld_out + (int64_t)h * a.dv + d + e] = y;
+          else reinterpret_cast<T*>(a.out)[(int64_t)start * a.ld_out + (int64_t)h * a.dv + d + e] = from_f32<T>(y);
+        }
+      }
+    }
+  }
+}
+
+template <int NT>
+int launch_step(const ScoredArgs& a, int n_seqs, const StepLayout& z, cudaStream_t stream) {
+  static size_t configured = 48 * 1024;
+  if (z.smem > configured) {
+    cudaError_t e = cudaFuncSetAttribute(scored_step_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)z.smem);
+    if (e != cudaSuccess) KVAD_FAIL(KVAD_ERR_CUDA, "attention (scored): cannot reserve %zu bytes of shared memory: %s", z.smem, cudaGetErrorString(e));
+    configured = z.smem;
+  }
+  const int group = a.n_heads / a.n_kv_heads, chunks = (group + STEP_HEADS - 1) / STEP_HEADS;
+  kvad_launch(scored_step_kernel<NT>, dim3(a.n_splits, n_seqs, a.n_kv_heads * chunks), dim3(128), z.smem, stream, a, z.k_stride, z.v_stride);
+  KVAD_CHECK_LAUNCH("attention_scored (single-token rows)");
+  return KVAD_OK;
+}
+
 // The parts that `n_splits` (32 at most) blocks left of one (row, head) become its output: a block per (row, head), a thread per
 // output entry.  Every warp takes the parts' maxima and sums by itself, a lane a part, and hands the parts' factors round by
 // shuffles; a thread adds the parts in split order, so the result does not depend on which block finished first.
@@ -398,6 +647,16 @@ scored_merge_diff_kernel(const float* __restrict__ partial, int n_splits, int n_
   }
 }
 
+template <typename T>
+int launch_merge(const ScoredArgs& a, int n_seqs, cudaStream_t stream) {
+  if (a.n_splits > 1 && a.merge) {       // (rows are single tokens here: row = sequence)
+    kvad_launch(scored_merge_kernel<T>, dim3(n_seqs, a.n_heads), dim3(a.dv <= 64 ? 64 : 128), 0, stream, (const float*)a.partial, a.n_splits,
+                a.n_heads, a.dv, (T*)a.out, a.ld_out, (const T*)a.gate, a.ld_gate, a.gate_heads, a.out_f32, a.sinks);
+    KVAD_CHECK_LAUNCH("attention_scored (merge)");
+  }
+  return KVAD_OK;
+}
+
 template <typename T, int KPL, int DPL, int NW, int RPW = 8>
 int launch_scored(const ScoredArgs& a, int n_seqs, int max_new, size_t smem, cudaStream_t stream) {
   constexpr int TR = RPW * NW, THREADS = 32 * NW;
@@ -411,16 +670,22 @@ int launch_scored(const ScoredArgs& a, int n_seqs, int max_new, size_t smem, cud
   dim3 grid(((max_new + tok - 1) / tok) * a.n_splits, n_seqs, a.n_kv_heads * chunks);
   kvad_launch(scored_attention_kernel<T, KPL, DPL, NW, RPW>, grid, dim3(THREADS), smem, stream, a);
   KVAD_CHECK_LAUNCH("attention_scored");
-  if (a.n_splits > 1 && a.merge) {       // (rows are single tokens here: row = sequence)
-    kvad_launch(scored_merge_kernel<T>, dim3(n_seqs, a.n_heads), dim3(a.dv <= 64 ? 64 : 128), 0, stream, (const float*)a.partial, a.n_splits,
-                a.n_heads, a.dv, (T*)a.out, a.ld_out, (const T*)a.gate, a.ld_gate, a.gate_heads, a.out_f32, a.sinks);
-    KVAD_CHECK_LAUNCH("attention_scored (merge)");
-  }
-  return KVAD_OK;
+  return launch_merge<T>(a, n_seqs, stream);
 }
 
 template <typename T>
 int dispatch_scored(const ScoredArgs& a, int n_seqs, int max_new, cudaStream_t stream) {
+  // bfloat16 rows of one token, whole 16-byte pieces: the tensor cores
+  if (sizeof(T) == 2 && max_new == 1 && a.vec_q && a.vec_k && (a.v_alias || a.vec_v) && a.dv % 8 == 0 && a.dv <= 256) {
+    const StepLayout z = step_layout(a.dk, a.dv, a.v_alias != 0);
+    if (z.smem <= 200 * 1024) {
+      int rc;
+      if (a.dv <= 64) rc = launch_step<1>(a, n_seqs, z, stream);
+      else if (a.dv <= 128) rc = launch_step<2>(a, n_seqs, z, stream);
+      else rc = launch_step<4>(a, n_seqs, z, stream);
+      return rc != KVAD_OK ? rc : launch_merge<T>(a, n_seqs, stream);
+    }
+  }
   const size_t limit = 224 * 1024;
   const size_t dkp = (size_t)((a.dk + 3) & ~3);
   auto need = [&](int tk, int tr) {
