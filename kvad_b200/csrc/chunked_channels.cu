@@ -25,7 +25,7 @@ using namespace kvad;
 
 namespace {
 
-constexpr int C = 64, B = 16, THREADS = 256, LDT = C + 4, COLS = 16;
+constexpr int C = 64, B = 16, THREADS = 256, LDT = C + 4, COLS = 16, LDC = COLS + 4;
 
 struct ChannelArgs {
   const void* q; const void* k; const void* v;
@@ -313,21 +313,39 @@ __global__ void __launch_bounds__(THREADS, 2) channel_prepare_kernel(const Chann
 __device__ __forceinline__ void copy16(void* dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
 }
-// acc[4][4] += sum over n of X[n][0 .. 3] Y[n][0 .. 3]
-__device__ __forceinline__ void product(float (&acc)[4][4], const float* X, int ldx, const float* Y, int ldy, int n) {
-#pragma unroll 8
-  for (int t = 0; t < n; ++t) {
-    const float4 x = *reinterpret_cast<const float4*>(X + t * ldx), y = *reinterpret_cast<const float4*>(Y + t * ldy);
-    const float xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w};
+// The walk's tiles of 16 columns ([rows][COLS]) keep row r at place (r % 4) * (rows / 4) + r / 4, places LDC apart: 4 x 4 tiles of eight
+// neighbouring lanes then go to and come from different banks (with the rows in order they all meet in the same four).
+template <int ROWS>
+__device__ __forceinline__ int place_of(int r) { return ((r & 3) * (ROWS / 4) + (r >> 2)) * LDC; }
+// acc[4][4] += sum over n of X[n][0 .. 3] Y[row n][0 .. 3]; Y points at the place of a row that is a multiple of 4, n too.
+template <int ROWS>
+__device__ __forceinline__ void product(float (&acc)[4][4], const float* X, int ldx, const float* Y, int n) {
+#pragma unroll 2
+  for (int t4 = 0; t4 < n / 4; ++t4) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int e = 0; e < 4; ++e) {
+      const float4 x = *reinterpret_cast<const float4*>(X + (t4 * 4 + e) * ldx), y = *reinterpret_cast<const float4*>(Y + (e * (ROWS / 4) + t4) * LDC);
+      const float xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w};
 #pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(xs[i], ys[j], acc[i][j]);
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(xs[i], ys[j], acc[i][j]);
+    }
   }
 }
-__device__ __forceinline__ void put_tile(float* dst, const float (&v)[4][4]) {
+// Rows 4 q .. + 3 of a tile.
+template <int ROWS>
+__device__ __forceinline__ void put_tile(float* dst, int q, const float (&v)[4][4]) {
 #pragma unroll
-  for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(dst + i * COLS) = make_float4(v[i][0], v[i][1], v[i][2], v[i][3]);
+  for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(dst + (i * (ROWS / 4) + q) * LDC) = make_float4(v[i][0], v[i][1], v[i][2], v[i][3]);
+}
+template <int ROWS>
+__device__ __forceinline__ void add_tile(const float* src, int q, float (&v)[4][4]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float4 o = *reinterpret_cast<const float4*>(src + (i * (ROWS / 4) + q) * LDC);
+    v[i][0] += o.x; v[i][1] += o.y; v[i][2] += o.z; v[i][3] += o.w;
+  }
 }
 
 template <typename TI, int DK, bool DELTA>
@@ -338,9 +356,9 @@ __global__ void __launch_bounds__(THREADS, 1) channel_walk_kernel(const ChannelA
   float* kt = wq + DK * WROWS;                        // [64][DK]
   float* at = kt + C * DK;                            // [64][64]
   float* S = at + C * C;                              // [DK][COLS]
-  float* D = S + DK * COLS;                           // [64][COLS]: u
-  float* part = D + C * COLS;                         // partial sums: up to 3 x 64 x COLS, or 128 x COLS
-  float* part2 = part + 3 * C * COLS;                 // [DK][COLS]
+  float* D = S + DK * LDC;                            // [64][COLS]: u
+  float* part = D + C * LDC;                          // partial sums: 3 x [64][COLS], or [128][COLS]
+  float* part2 = part + 3 * C * LDC;                  // [DK][COLS]
   pdl_launch_dependents();
   pdl_wait();
   const int s = blockIdx.x / a.heads, h = blockIdx.x - s * a.heads, c0 = blockIdx.y * COLS, tid = threadIdx.x;
@@ -350,7 +368,7 @@ __global__ void __launch_bounds__(THREADS, 1) channel_walk_kernel(const ChannelA
   float* st = a.state + (int64_t)a.seq_slots[s] * a.state_stride + (int64_t)h * a.dv * a.dk;
   for (int i = tid; i < DK * COLS; i += THREADS) {
     const int c = i / DK, d = i - c * DK;
-    S[d * COLS + c] = d < a.dk && c0 + c < a.dv ? st[(int64_t)(c0 + c) * a.dk + d] : 0.f;
+    S[place_of<DK>(d) + c] = d < a.dk && c0 + c < a.dv ? st[(int64_t)(c0 + c) * a.dk + d] : 0.f;
   }
   auto bring_wq = [&](int c) {
     const float* src = a.wq + ((int64_t)(first + c) * a.heads + h) * DK * 128 + (128 - WROWS);
@@ -393,38 +411,34 @@ __global__ void __launch_bounds__(THREADS, 1) channel_walk_kernel(const ChannelA
     // [W | q B]^T S: rows r4 of both, a half of the channels a group (without W: 64 rows, a quarter of the channels)
     float acc[4][4] = {};
     if (DELTA) {
-      product(acc, wq + group * (DK / 2) * WROWS + r4 * 4, WROWS, S + group * (DK / 2) * COLS + c4, COLS, DK / 2);
-      if (group == 1) put_tile(part + r4 * 4 * COLS + c4, acc);
+      product<DK>(acc, wq + group * (DK / 2) * WROWS + r4 * 4, WROWS, S + place_of<DK>(group * (DK / 2)) + c4, DK / 2);
+      if (group == 1) put_tile<128>(part + c4, r4, acc);
       __syncthreads();
       if (group == 0) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float4 o = *reinterpret_cast<const float4*>(part + (r4 * 4 + i) * COLS + c4);
-          acc[i][0] += o.x; acc[i][1] += o.y; acc[i][2] += o.z; acc[i][3] += o.w;
-        }
-        if (r4 < 16) put_tile(D + r4 * 4 * COLS + c4, acc);
+        add_tile<128>(part + c4, r4, acc);
+        if (r4 < 16) put_tile<C>(D + c4, r4, acc);
       }
       __syncthreads();
-      const float4 w = *reinterpret_cast<const float4*>(D + ur * COLS + uc);      // u = X - W S
-      *reinterpret_cast<float4*>(D + ur * COLS + uc) = make_float4(given[0] - w.x, given[1] - w.y, given[2] - w.z, given[3] - w.w);
+      const float4 w = *reinterpret_cast<const float4*>(D + place_of<C>(ur) + uc);      // u = X - W S
+      *reinterpret_cast<float4*>(D + place_of<C>(ur) + uc) = make_float4(given[0] - w.x, given[1] - w.y, given[2] - w.z, given[3] - w.w);
     } else {
-      *reinterpret_cast<float4*>(D + ur * COLS + uc) = make_float4(given[0], given[1], given[2], given[3]);
-      product(acc, wq + quarter * (DK / 4) * WROWS + q4 * 4, WROWS, S + quarter * (DK / 4) * COLS + c4, COLS, DK / 4);
+      *reinterpret_cast<float4*>(D + place_of<C>(ur) + uc) = make_float4(given[0], given[1], given[2], given[3]);
+      product<DK>(acc, wq + quarter * (DK / 4) * WROWS + q4 * 4, WROWS, S + place_of<DK>(quarter * (DK / 4)) + c4, DK / 4);
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();                                  // u lies, keys and A are there, W and q B have been used up
     if (c + 1 < n_chunks) bring_wq(c + 1);
     // the state: S' = B S + K^T u, a half of the rows a group
     float add[4][4] = {};
-    if (r4 * 4 < DK) product(add, kt + group * 32 * DK + r4 * 4, DK, D + group * 32 * COLS + c4, COLS, 32);
-    if (group == 1 && r4 * 4 < DK) put_tile(part2 + r4 * 4 * COLS + c4, add);
+    if (r4 * 4 < DK) product<C>(add, kt + group * 32 * DK + r4 * 4, DK, D + place_of<C>(group * 32) + c4, 32);
+    if (group == 1 && r4 * 4 < DK) put_tile<DK>(part2 + c4, r4, add);
     // the read-outs: A u, a quarter of the rows j a thread, plus (q B)^T S
     float read[4][4];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int j = 0; j < 4; ++j) read[i][j] = DELTA ? 0.f : acc[i][j];
-    product(read, at + quarter * B * C + q4 * 4, C, D + quarter * B * COLS + c4, COLS, B);
+    product<C>(read, at + quarter * B * C + q4 * 4, C, D + place_of<C>(quarter * B) + c4, B);
     // (delta rule: the threads of group 0 with rows from 64 on hold (q B)^T S: they are the second quarter, for the same rows and columns)
     if (DELTA && quarter == 1) {
 #pragma unroll
@@ -432,17 +446,14 @@ __global__ void __launch_bounds__(THREADS, 1) channel_walk_kernel(const ChannelA
 #pragma unroll
         for (int j = 0; j < 4; ++j) read[i][j] += acc[i][j];
     }
-    if (quarter > 0) put_tile(part + ((quarter - 1) * C + q4 * 4) * COLS + c4, read);
+    if (quarter > 0) put_tile<C>(part + (quarter - 1) * C * LDC + c4, q4, read);
     __syncthreads();
     if (quarter == 0) {
 #pragma unroll
+      for (int m = 0; m < 3; ++m) add_tile<C>(part + m * C * LDC + c4, q4, read);
+#pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int r = q4 * 4 + i;
-#pragma unroll
-        for (int m = 0; m < 3; ++m) {
-          const float4 o = *reinterpret_cast<const float4*>(part + (m * C + r) * COLS + c4);
-          read[i][0] += o.x; read[i][1] += o.y; read[i][2] += o.z; read[i][3] += o.w;
-        }
         if (r < n) {
           float* o = a.out + (int64_t)(row0 + r) * a.ld_out + h * a.dv + c0 + c4;
 #pragma unroll
@@ -452,26 +463,26 @@ __global__ void __launch_bounds__(THREADS, 1) channel_walk_kernel(const ChannelA
       }
     }
     if (group == 0 && r4 * 4 < DK) {
+      add_tile<DK>(part2 + c4, r4, add);
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        float4* at_s = reinterpret_cast<float4*>(S + (r4 * 4 + i) * COLS + c4);
-        const float4 o = *reinterpret_cast<const float4*>(part2 + (r4 * 4 + i) * COLS + c4), was = *at_s;
-        *at_s = make_float4(fmaf(keep[i], was.x, add[i][0] + o.x), fmaf(keep[i], was.y, add[i][1] + o.y), fmaf(keep[i], was.z, add[i][2] + o.z),
-                            fmaf(keep[i], was.w, add[i][3] + o.w));
+        float4* at_s = reinterpret_cast<float4*>(S + (i * (DK / 4) + r4) * LDC + c4);
+        const float4 was = *at_s;
+        *at_s = make_float4(fmaf(keep[i], was.x, add[i][0]), fmaf(keep[i], was.y, add[i][1]), fmaf(keep[i], was.z, add[i][2]), fmaf(keep[i], was.w, add[i][3]));
       }
     }
     __syncthreads();                                  // the new state lies; keys, A and the partial sums have been used up
   }
   for (int i = tid; i < DK * COLS; i += THREADS) {
     const int c = i / DK, d = i - c * DK;
-    if (d < a.dk && c0 + c < a.dv) st[(int64_t)(c0 + c) * a.dk + d] = S[d * COLS + c];
+    if (d < a.dk && c0 + c < a.dv) st[(int64_t)(c0 + c) * a.dk + d] = S[place_of<DK>(d) + c];
   }
 }
 
 template <typename TI, int DK, bool DELTA>
 int launch(const ChannelArgs& a, cudaStream_t stream) {
   constexpr size_t prepare_smem = ((size_t)4 * HD * LDT + 2 * C * LDT + 4 * HD) * 4;
-  constexpr size_t walk_smem = ((size_t)DK * (DELTA ? 128 : 64) + C * DK + C * C + DK * COLS + C * COLS + 3 * C * COLS + DK * COLS) * 4;
+  constexpr size_t walk_smem = ((size_t)DK * (DELTA ? 128 : 64) + C * DK + C * C + 2 * DK * LDC + 4 * C * LDC) * 4;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(channel_prepare_kernel<TI, DK, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prepare_smem);
