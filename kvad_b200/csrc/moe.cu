@@ -762,6 +762,120 @@ inline int flat_blocks(int64_t total, int threads) {
   return (int)(b < 148 * 16 ? (b < 1 ? 1 : b) : 148 * 16);
 }
 
+// The bfloat16 form on mma.sync: a block's 16 weight rows are the M side, up to eight of the tile's rows the N side, its eight warps take
+// every eighth 32 of K.  A lane reads 16 bytes of its two weight rows and of its row at the same place of K - the sum's order is free, so
+// neighbouring k go to one lane - which is two m16n8k16.  The tensor core truncates where it accumulates, so a sum stays in it for those 32
+// of K only and then joins a register by a rounded addition; the warps' sums meet in shared memory.  (Error against 64 bits at K = 1408: 7e-8,
+// as the chain of fused multiply-adds it replaces; that chain cost more instructions than the copy cost time.)
+template <typename TO>
+__global__ void __launch_bounds__(256, 4)
+grouped_rows_mma_kernel(const __nv_bfloat16* __restrict__ a, int64_t ld_a, const int* __restrict__ in_rows, const __nv_bfloat16* __restrict__ w,
+                        int64_t expert_stride, TO* __restrict__ out, int64_t ld_out, const int* __restrict__ out_rows,
+                        const int* __restrict__ valid, const int* __restrict__ tile_expert, int n_out, int k_dim) {
+  constexpr int OUTS = 16;
+  extern __shared__ __align__(128) uint8_t rows_smem[];
+  const __nv_bfloat16* ws = reinterpret_cast<const __nv_bfloat16*>(rows_smem);      // [16][k_dim]
+  __shared__ int rows_in[TM], rows_out[TM], n_valid;
+  __shared__ float sums[8][8][OUTS + 1];                                             // [warp][row][output]
+  __shared__ uint64_t here;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, tile = blockIdx.y, first = blockIdx.x * OUTS;
+  const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&here);
+  if (tid == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  pdl_launch_dependents();
+  pdl_wait();
+  const int expert = tile_expert[tile];
+  if (expert < 0) return;
+  const int n_rows_w = min(OUTS, n_out - first);
+  if (tid == 0) {
+    const uint32_t bytes = (uint32_t)n_rows_w * (uint32_t)k_dim * 2u;
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"((uint32_t)__cvta_generic_to_shared(ws)), "l"(w + (int64_t)expert * expert_stride + (int64_t)first * k_dim), "r"(bytes), "r"(bar) : "memory");
+  }
+  if (tid < TM) {                               // the tile's used positions, side by side
+    const int p = tile * TM + tid;
+    const bool used = valid[p] >= 0;
+    const unsigned mask = __ballot_sync(0xffffffffu, used);
+    if (used) {
+      const int at = __popc(mask & ((1u << tid) - 1u));
+      rows_in[at] = in_rows ? in_rows[p] : p;
+      rows_out[at] = out_rows ? out_rows[p] : p;
+    }
+    if (tid == 0) n_valid = __popc(mask);
+  }
+  __syncthreads();
+  const int g = lane >> 2, k_of = (lane & 3) * 8;
+  bool waited = false;
+  for (int r0 = 0; r0 < n_valid; r0 += 8) {
+    const int n = min(8, n_valid - r0);
+    const __nv_bfloat16* ar = a + (int64_t)rows_in[r0 + (g < n ? g : 0)] * ld_a + k_of;
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    uint4 next = make_uint4(0u, 0u, 0u, 0u);
+    if (g < n && warp * 32 + k_of < k_dim) next = *reinterpret_cast<const uint4*>(ar + warp * 32);
+    if (!waited) {                              // (the first rows are on their way meanwhile)
+      bool there = false;
+      for (uint32_t i = 0; i < ROWS_WAIT_LIMIT && !there; ++i) {
+        uint32_t ok;
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar) : "memory");
+        there = ok != 0;
+      }
+      waited = true;
+      if (!there) {                             // (the copy never came: say so, write nothing that means anything)
+        if (lane == 0) atomicAdd(&g_rows_timeouts, 1);
+      }
+    }
+#pragma unroll 2
+    for (int k0 = warp * 32; k0 < k_dim; k0 += 256) {
+      const uint4 b = next;
+      const int k1 = k0 + 256;
+      next = make_uint4(0u, 0u, 0u, 0u);
+      if (g < n && k1 + k_of < k_dim) next = *reinterpret_cast<const uint4*>(ar + k1);
+      uint4 lo = make_uint4(0u, 0u, 0u, 0u), hi = lo;      // outputs g and g + 8
+      if (k0 + k_of < k_dim) {
+        if (g < n_rows_w) lo = *reinterpret_cast<const uint4*>(ws + (int64_t)g * k_dim + k0 + k_of);
+        if (g + 8 < n_rows_w) hi = *reinterpret_cast<const uint4*>(ws + (int64_t)(g + 8) * k_dim + k0 + k_of);
+      }
+      float c[4] = {0.f, 0.f, 0.f, 0.f};
+      asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                   : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(lo.x), "r"(hi.x), "r"(lo.y), "r"(hi.y), "r"(b.x), "r"(b.y));
+      asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                   : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(lo.z), "r"(hi.z), "r"(lo.w), "r"(hi.w), "r"(b.z), "r"(b.w));
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[e] += c[e];
+    }
+    if (r0 > 0) __syncthreads();                // the sums before have been read
+#pragma unroll
+    for (int e = 0; e < 4; ++e) sums[warp][(lane & 3) * 2 + (e & 1)][g + (e >> 1) * 8] = acc[e];
+    __syncthreads();
+    if (tid < 8 * OUTS) {
+      const int r = tid / OUTS, o = tid % OUTS;
+      if (r < n && first + o < n_out) {
+        const float y = ((sums[0][r][o] + sums[1][r][o]) + (sums[2][r][o] + sums[3][r][o])) + ((sums[4][r][o] + sums[5][r][o]) + (sums[6][r][o] + sums[7][r][o]));
+        out[(int64_t)rows_out[r0 + r] * ld_out + first + o] = from_f32<TO>(y);
+      }
+    }
+  }
+}
+
+template <typename TO>
+int launch_rows_mma(int n_out, int max_tiles, size_t smem, cudaStream_t stream, const __nv_bfloat16* a, int64_t ld_a, const int* in_rows, const __nv_bfloat16* w,
+                    int64_t expert_stride, TO* out, int64_t ld_out, const int* out_rows, const int* valid, const int* tile_expert, int k_dim) {
+  static size_t configured = 48 * 1024;
+  if (smem > configured) {
+    cudaError_t e = cudaFuncSetAttribute(grouped_rows_mma_kernel<TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) KVAD_FAIL(KVAD_ERR_CUDA, "grouped_linear: cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
+    configured = smem;
+  }
+  kvad_launch(grouped_rows_mma_kernel<TO>, dim3((n_out + 15) / 16, max_tiles), dim3(256), smem, stream, a, ld_a, in_rows, w, expert_stride, out, ld_out, out_rows,
+              valid, tile_expert, n_out, k_dim);
+  KVAD_CHECK_LAUNCH("grouped_linear");
+  return KVAD_OK;
+}
+
 template <typename T, typename TO, int CU>
 int launch_rows(dim3 grid, size_t smem, cudaStream_t stream, const T* a, int64_t ld_a, const int* in_rows, const T* w, int64_t expert_stride, TO* out, int64_t ld_out,
                 const int* out_rows, const int* valid, const int* tile_expert, int n_out, int k_dim) {
@@ -857,6 +971,13 @@ KVAD_EXPORT int kvad_grouped_linear(int dtype, int out_f32, const void* a, int64
   // the weight rows of a block in shared memory, two outputs a warp where 16 rows are at most 64 KB, else one (up to 200 KB: beyond, the tiled form)
   const size_t row_bytes = (size_t)k_dim * (dtype == KVAD_DTYPE_F32 ? 4 : 2);
   if (few_rows && vec && 8 * row_bytes <= 200 * 1024) {
+    if (dtype == KVAD_DTYPE_BF16 && 16 * row_bytes <= 200 * 1024) {
+      if (out_f32)
+        return launch_rows_mma<float>(n_out, max_tiles, 16 * row_bytes, stream, (const __nv_bfloat16*)a, ld_a, in_rows, (const __nv_bfloat16*)w, expert_stride,
+                                      (float*)out, ld_out, out_rows, valid, tile_expert, k_dim);
+      return launch_rows_mma<__nv_bfloat16>(n_out, max_tiles, 16 * row_bytes, stream, (const __nv_bfloat16*)a, ld_a, in_rows, (const __nv_bfloat16*)w, expert_stride,
+                                            (__nv_bfloat16*)out, ld_out, out_rows, valid, tile_expert, k_dim);
+    }
     const int cu = 16 * row_bytes <= 64 * 1024 ? 2 : 1;
     const size_t smem = 8 * cu * row_bytes;
     dim3 rgrid((n_out + 8 * cu - 1) / (8 * cu), max_tiles);
