@@ -552,7 +552,7 @@ __global__ void __launch_bounds__(128) scored_step_kernel(const ScoredArgs a, in
 
 template <int NT>
 int launch_step(const ScoredArgs& a, int n_seqs, const StepLayout& z, cudaStream_t stream) {
-  static size_t configured = 48 * 1024;
+  static size_t configured = 40 * 1024;      // (static shared memory counts towards the 48 KB that need no asking)
   if (z.smem > configured) {
     cudaError_t e = cudaFuncSetAttribute(scored_step_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)z.smem);
     if (e != cudaSuccess) KVAD_FAIL(KVAD_ERR_CUDA, "attention (scored): cannot reserve %zu bytes of shared memory: %s", z.smem, cudaGetErrorString(e));

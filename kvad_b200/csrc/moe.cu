@@ -864,7 +864,7 @@ grouped_rows_mma_kernel(const __nv_bfloat16* __restrict__ a, int64_t ld_a, const
 template <typename TO>
 int launch_rows_mma(int n_out, int max_tiles, size_t smem, cudaStream_t stream, const __nv_bfloat16* a, int64_t ld_a, const int* in_rows, const __nv_bfloat16* w,
                     int64_t expert_stride, TO* out, int64_t ld_out, const int* out_rows, const int* valid, const int* tile_expert, int k_dim) {
-  static size_t configured = 48 * 1024;
+  static size_t configured = 40 * 1024;      // (static shared memory counts towards the 48 KB that need no asking)
   if (smem > configured) {
     cudaError_t e = cudaFuncSetAttribute(grouped_rows_mma_kernel<TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) KVAD_FAIL(KVAD_ERR_CUDA, "grouped_linear: cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
@@ -879,7 +879,7 @@ int launch_rows_mma(int n_out, int max_tiles, size_t smem, cudaStream_t stream, 
 template <typename T, typename TO, int CU>
 int launch_rows(dim3 grid, size_t smem, cudaStream_t stream, const T* a, int64_t ld_a, const int* in_rows, const T* w, int64_t expert_stride, TO* out, int64_t ld_out,
                 const int* out_rows, const int* valid, const int* tile_expert, int n_out, int k_dim) {
-  static size_t configured = 48 * 1024;
+  static size_t configured = 40 * 1024;      // (static shared memory counts towards the 48 KB that need no asking)
   if (smem > configured) {
     cudaError_t e = cudaFuncSetAttribute(grouped_rows_kernel<T, TO, CU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) KVAD_FAIL(KVAD_ERR_CUDA, "grouped_linear: cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
