@@ -341,11 +341,12 @@ class Ops:
     def __init__(self, dtype: torch.dtype):
         self.dtype = dtype
         self.code = _code(dtype)
+        have = set(build.sources())          # (one look at the folder, not one a switch)
         self.use_tensor_cores = dtype == torch.bfloat16
         # set to False to keep the bfloat16 engine on the CUDA-core kernels (tests compare both)
-        self.tensor_core_linear = dtype == torch.bfloat16 and "linear_tcgen05" in build.sources()
-        self.tensor_core_prefill = dtype == torch.bfloat16 and "attention_prefill" in build.sources()
-        self.fast_decode = "attention_decode" in build.sources()        # both dtypes: the decode kernel is templated on the storage type
+        self.tensor_core_linear = dtype == torch.bfloat16 and "linear_tcgen05" in have
+        self.tensor_core_prefill = dtype == torch.bfloat16 and "attention_prefill" in have
+        self.fast_decode = "attention_decode" in have        # both dtypes: the decode kernel is templated on the storage type
         # Up to 16 rows the product can also run as a stream of weights through registers on the CUDA cores
         # (linear_rows.cu).  Measured on a B200 it beats the tensor-core kernel at one or two rows (qkv at 1 row:
         # 2.4 us against 3.9 us; a GPT-2 small decode step at batch 1: 0.286 ms against 0.326 ms, at batch 2: 0.314
@@ -355,11 +356,11 @@ class Ops:
         # In 32-bit there are no tensor cores to lose to: the weight stream is the decode road of the float32 engine
         # for every row count it takes (the tiled CUDA-core kernel would run one row in a tile of 64).
         self._rows_lib = "linear_rows" if dtype == torch.bfloat16 else "linear_rows_f32"     # one library per element type
-        self.rows_linear_max = (2 if dtype == torch.bfloat16 else 16) if self._rows_lib in build.sources() else 0
+        self.rows_linear_max = (2 if dtype == torch.bfloat16 else 16) if self._rows_lib in have else 0
         # 32-bit products of many rows on the tensor cores, their operands cut into bfloat16 pieces (linear_split.cu)
-        self.split_linear = dtype == torch.float32 and "linear_split" in build.sources()
-        self.scored_prompt = dtype == torch.bfloat16 and "attention_scored_prompt" in build.sources()     # shaped scores of prompt rows on the tensor cores
-        self.chunked_recurrences = "chunked_recurrence" in build.sources()     # recurrences of prompts: products of 64 rows, not a walk
+        self.split_linear = dtype == torch.float32 and "linear_split" in have
+        self.scored_prompt = dtype == torch.bfloat16 and "attention_scored_prompt" in have     # shaped scores of prompt rows on the tensor cores
+        self.chunked_recurrences = "chunked_recurrence" in have     # recurrences of prompts: products of 64 rows, not a walk
         self.tiled_prompt = True    # prompts that the tensor-core kernel does not take: the tiled CUDA-core kernel, not the row-by-row one
         self._counters = None       # zeroed ints the decode kernel counts finished splits in (left zeroed by it)
         # Two 32-bit buffers [16, width] that q/k/v products of 3..16 rows add their shares of K into (see
