@@ -461,10 +461,10 @@ grouped_linear_kernel(const T* __restrict__ a, int64_t ld_a, const int* __restri
   }
 }
 
-// The same product for steps of a few rows (decoding): a stream of the chosen experts' weights.  A block owns 8 CU outputs of a
+// The same product for steps of a few rows (decoding): a stream of the chosen experts' weights.  A block owns CU outputs a warp of a
 // tile, whose weight rows lie side by side in memory: ONE bulk copy brings all of them (45 KB at K = 1408), asked for as soon as the
-// tile's expert is known and before its rows are looked up, so that with three blocks an SM some 130 KB a SM are on their way.  A warp
-// then has CU outputs; its lanes take every 32nd 16-byte piece of the weight rows, from shared memory, and multiply them with the same pieces
+// tile's expert is known and before its rows are looked up, so that with three blocks an SM some 130 KB a SM are on their way.  A warp's
+// lanes take every 32nd 16-byte piece of the weight rows, from shared memory, and multiply them with the same pieces
 // of 1, 2, 4 or 8 of the tile's rows (which stay in the L1); a shuffle tree per (row, output) at the end.  A tile with more than
 // eight rows goes over its weights again per eight.  (With the weights fetched into registers piece by piece, 8 x 4 loads a warp, 64
 // pairs of 16 experts of 1408 x 1024 took 44 us: a block held its registers through three trips to memory one after another.)
@@ -516,10 +516,11 @@ grouped_rows_kernel(const T* __restrict__ a, int64_t ld_a, const int* __restrict
                     int64_t expert_stride, TO* __restrict__ out, int64_t ld_out, const int* __restrict__ out_rows,
                     const int* __restrict__ valid, const int* __restrict__ tile_expert, int n_out, int k_dim) {
   extern __shared__ __align__(128) uint8_t rows_smem[];
-  T* ws = reinterpret_cast<T*>(rows_smem);      // [8 CU][k_dim]
+  T* ws = reinterpret_cast<T*>(rows_smem);      // [warps * CU][k_dim]
   __shared__ int rows_in[TM], rows_out[TM], n_valid;
   __shared__ uint64_t here;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, tile = blockIdx.y, first = blockIdx.x * 8 * CU;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, tile = blockIdx.y;
+  const int per_block = (blockDim.x >> 5) * CU, first = blockIdx.x * per_block;
   const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&here);
   if (tid == 0) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
@@ -531,7 +532,7 @@ grouped_rows_kernel(const T* __restrict__ a, int64_t ld_a, const int* __restrict
   const int expert = tile_expert[tile];
   if (expert < 0) return;
   if (tid == 0) {
-    const uint32_t bytes = (uint32_t)min(8 * CU, n_out - first) * (uint32_t)k_dim * (uint32_t)sizeof(T);
+    const uint32_t bytes = (uint32_t)min(per_block, n_out - first) * (uint32_t)k_dim * (uint32_t)sizeof(T);
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"((uint32_t)__cvta_generic_to_shared(ws)), "l"(w + (int64_t)expert * expert_stride + (int64_t)first * k_dim), "r"(bytes), "r"(bar) : "memory");
@@ -765,8 +766,18 @@ inline int flat_blocks(int64_t total, int threads) {
 // The bfloat16 form on mma.sync: a block's 16 weight rows are the M side, up to eight of the tile's rows the N side, its eight warps take
 // every eighth 32 of K.  A lane reads 16 bytes of its two weight rows and of its row at the same place of K - the sum's order is free, so
 // neighbouring k go to one lane - which is two m16n8k16.  The tensor core truncates where it accumulates, so a sum stays in it for those 32
-// of K only and then joins a register by a rounded addition; the warps' sums meet in shared memory.  (Error against 64 bits at K = 1408: 7e-8,
-// as the chain of fused multiply-adds it replaces; that chain cost more instructions than the copy cost time.)
+// of K only and then joins a register by a rounded addition; what those additions round away is carried beside the sum (`add_exactly`) and
+// joins it at the end, which pays for the truncation: the error against 64 bits
+// is 5.3e-8 at K = 704 .. 4096 (7.7e-8 without, 7.3e-8 the chain of fused multiply-adds).  64 pairs of 16 experts of 1408 x 1024: 38 us with the
+// weights fetched into registers, 27 with the bulk copy and that chain (more instructions than the copy costs time), 13.7 this way.
+__device__ __forceinline__ float add_exactly(float a, float b, float& lost) {      // a + b rounded; what the rounding lost is added to `lost` (Knuth's two-sum)
+  const float s = __fadd_rn(a, b), of_b = __fsub_rn(s, a);
+  lost = __fadd_rn(lost, __fadd_rn(__fsub_rn(a, __fsub_rn(s, of_b)), __fsub_rn(b, of_b)));
+  return s;
+}
+// The sum with what it lost; a sum that is infinite or no number stays as it is (what it lost is no number then).
+__device__ __forceinline__ float with_lost(float s, float lost) { return fabsf(s) <= 3.402823466e38f ? s + lost : s; }
+
 template <typename TO>
 __global__ void __launch_bounds__(256, 4)
 grouped_rows_mma_kernel(const __nv_bfloat16* __restrict__ a, int64_t ld_a, const int* __restrict__ in_rows, const __nv_bfloat16* __restrict__ w,
@@ -810,10 +821,10 @@ grouped_rows_mma_kernel(const __nv_bfloat16* __restrict__ a, int64_t ld_a, const
   __syncthreads();
   const int g = lane >> 2, k_of = (lane & 3) * 8;
   bool waited = false;
-  for (int r0 = 0; r0 < n_valid; r0 += 8) {
+  for (int r0 = 0; r0 < max(n_valid, 1); r0 += 8) {      // (a tile without rows waits for its copy too)
     const int n = min(8, n_valid - r0);
-    const __nv_bfloat16* ar = a + (int64_t)rows_in[r0 + (g < n ? g : 0)] * ld_a + k_of;
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    const __nv_bfloat16* ar = a + (g < n ? (int64_t)rows_in[r0 + g] * ld_a : 0) + k_of;
+    float acc[4] = {0.f, 0.f, 0.f, 0.f}, lost[4] = {0.f, 0.f, 0.f, 0.f};
     uint4 next = make_uint4(0u, 0u, 0u, 0u);
     if (g < n && warp * 32 + k_of < k_dim) next = *reinterpret_cast<const uint4*>(ar + warp * 32);
     if (!waited) {                              // (the first rows are on their way meanwhile)
@@ -845,17 +856,19 @@ grouped_rows_mma_kernel(const __nv_bfloat16* __restrict__ a, int64_t ld_a, const
       asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                    : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(lo.z), "r"(hi.z), "r"(lo.w), "r"(hi.w), "r"(b.z), "r"(b.w));
 #pragma unroll
-      for (int e = 0; e < 4; ++e) acc[e] += c[e];
+      for (int e = 0; e < 4; ++e) acc[e] = add_exactly(acc[e], c[e], lost[e]);
     }
     if (r0 > 0) __syncthreads();                // the sums before have been read
 #pragma unroll
-    for (int e = 0; e < 4; ++e) sums[warp][(lane & 3) * 2 + (e & 1)][g + (e >> 1) * 8] = acc[e];
+    for (int e = 0; e < 4; ++e) sums[warp][(lane & 3) * 2 + (e & 1)][g + (e >> 1) * 8] = with_lost(acc[e], lost[e]);
     __syncthreads();
     if (tid < 8 * OUTS) {
       const int r = tid / OUTS, o = tid % OUTS;
       if (r < n && first + o < n_out) {
-        const float y = ((sums[0][r][o] + sums[1][r][o]) + (sums[2][r][o] + sums[3][r][o])) + ((sums[4][r][o] + sums[5][r][o]) + (sums[6][r][o] + sums[7][r][o]));
-        out[(int64_t)rows_out[r0 + r] * ld_out + first + o] = from_f32<TO>(y);
+        float y = sums[0][r][o], left = 0.f;
+#pragma unroll
+        for (int i = 1; i < 8; ++i) y = add_exactly(y, sums[i][r][o], left);
+        out[(int64_t)rows_out[r0 + r] * ld_out + first + o] = from_f32<TO>(with_lost(y, left));
       }
     }
   }
@@ -877,7 +890,7 @@ int launch_rows_mma(int n_out, int max_tiles, size_t smem, cudaStream_t stream, 
 }
 
 template <typename T, typename TO, int CU>
-int launch_rows(dim3 grid, size_t smem, cudaStream_t stream, const T* a, int64_t ld_a, const int* in_rows, const T* w, int64_t expert_stride, TO* out, int64_t ld_out,
+int launch_rows(dim3 grid, int warps, size_t smem, cudaStream_t stream, const T* a, int64_t ld_a, const int* in_rows, const T* w, int64_t expert_stride, TO* out, int64_t ld_out,
                 const int* out_rows, const int* valid, const int* tile_expert, int n_out, int k_dim) {
   static size_t configured = 40 * 1024;      // (static shared memory counts towards the 48 KB that need no asking)
   if (smem > configured) {
@@ -885,7 +898,7 @@ int launch_rows(dim3 grid, size_t smem, cudaStream_t stream, const T* a, int64_t
     if (e != cudaSuccess) KVAD_FAIL(KVAD_ERR_CUDA, "grouped_linear: cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
     configured = smem;
   }
-  kvad_launch(grouped_rows_kernel<T, TO, CU>, grid, dim3(256), smem, stream, a, ld_a, in_rows, w, expert_stride, out, ld_out, out_rows, valid, tile_expert, n_out, k_dim);
+  kvad_launch(grouped_rows_kernel<T, TO, CU>, grid, dim3(32 * warps), smem, stream, a, ld_a, in_rows, w, expert_stride, out, ld_out, out_rows, valid, tile_expert, n_out, k_dim);
   return KVAD_OK;
 }
 
@@ -968,9 +981,10 @@ KVAD_EXPORT int kvad_grouped_linear(int dtype, int out_f32, const void* a, int64
   const int piece = dtype == KVAD_DTYPE_F32 ? 4 : 8;
   const int vec = (k_dim % piece == 0 && ld_a % piece == 0 && expert_stride % piece == 0 &&
                    ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w)) & 15) == 0) ? 1 : 0;
-  // the weight rows of a block in shared memory, two outputs a warp where 16 rows are at most 64 KB, else one (up to 200 KB: beyond, the tiled form)
+  // the weight rows of a block in shared memory: two outputs a warp where 16 rows are at most 64 KB, else one, and fewer warps where eight rows
+  // are more than the 200 KB a block may take (beyond one row, the tiled form)
   const size_t row_bytes = (size_t)k_dim * (dtype == KVAD_DTYPE_F32 ? 4 : 2);
-  if (few_rows && vec && 8 * row_bytes <= 200 * 1024) {
+  if (few_rows && vec && row_bytes <= 200 * 1024) {
     if (dtype == KVAD_DTYPE_BF16 && 16 * row_bytes <= 200 * 1024) {
       if (out_f32)
         return launch_rows_mma<float>(n_out, max_tiles, 16 * row_bytes, stream, (const __nv_bfloat16*)a, ld_a, in_rows, (const __nv_bfloat16*)w, expert_stride,
@@ -978,19 +992,20 @@ KVAD_EXPORT int kvad_grouped_linear(int dtype, int out_f32, const void* a, int64
       return launch_rows_mma<__nv_bfloat16>(n_out, max_tiles, 16 * row_bytes, stream, (const __nv_bfloat16*)a, ld_a, in_rows, (const __nv_bfloat16*)w, expert_stride,
                                             (__nv_bfloat16*)out, ld_out, out_rows, valid, tile_expert, k_dim);
     }
-    const int cu = 16 * row_bytes <= 64 * 1024 ? 2 : 1;
-    const size_t smem = 8 * cu * row_bytes;
-    dim3 rgrid((n_out + 8 * cu - 1) / (8 * cu), max_tiles);
-#define KVAD_GR(T, TO)                                                                                                         \
-  do {                                                                                                                         \
-    int rc = cu == 2 ? launch_rows<T, TO, 2>(rgrid, smem, stream, (const T*)a, ld_a, in_rows, (const T*)w, expert_stride, (TO*)out, ld_out, out_rows, valid, tile_expert, n_out, k_dim)  \
-                     : launch_rows<T, TO, 1>(rgrid, smem, stream, (const T*)a, ld_a, in_rows, (const T*)w, expert_stride, (TO*)out, ld_out, out_rows, valid, tile_expert, n_out, k_dim); \
-    if (rc != KVAD_OK) return rc;                                                                                              \
-  } while (0)
-    if (dtype == KVAD_DTYPE_F32) KVAD_GR(float, float);
-    else if (dtype == KVAD_DTYPE_BF16 && out_f32) KVAD_GR(__nv_bfloat16, float);
-    else if (dtype == KVAD_DTYPE_BF16) KVAD_GR(__nv_bfloat16, __nv_bfloat16);
+    const int cu = dtype == KVAD_DTYPE_F32 && 16 * row_bytes <= 64 * 1024 ? 2 : 1;
+    int warps = 8;
+    while (warps * cu * row_bytes > 200 * 1024) warps /= 2;
+    const size_t smem = warps * cu * row_bytes;
+    dim3 rgrid((n_out + warps * cu - 1) / (warps * cu), max_tiles);
+    int rc;
+#define KVAD_GR(T, TO, CU)                                                                                                     \
+  rc = launch_rows<T, TO, CU>(rgrid, warps, smem, stream, (const T*)a, ld_a, in_rows, (const T*)w, expert_stride, (TO*)out, ld_out, out_rows, valid, tile_expert, n_out, k_dim)
+    if (dtype == KVAD_DTYPE_F32 && cu == 2) KVAD_GR(float, float, 2);
+    else if (dtype == KVAD_DTYPE_F32) KVAD_GR(float, float, 1);
+    else if (dtype == KVAD_DTYPE_BF16 && out_f32) KVAD_GR(__nv_bfloat16, float, 1);
+    else if (dtype == KVAD_DTYPE_BF16) KVAD_GR(__nv_bfloat16, __nv_bfloat16, 1);
     else KVAD_FAIL(KVAD_ERR_UNSUPPORTED, "grouped_linear: unknown dtype %d", dtype);
+    if (rc != KVAD_OK) return rc;
 #undef KVAD_GR
     KVAD_CHECK_LAUNCH("grouped_linear");
     return KVAD_OK;

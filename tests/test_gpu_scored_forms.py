@@ -1,0 +1,152 @@
+"""Attention with shaped scores in bfloat16 on the tensor cores, prompt rows and single-token rows, against the formula in 64 bits and against
+the CUDA-core kernel: sequences that end one row before and after a tile and a page, pages in any order with no number in the places that no
+row has reached, every shaping of a score, one to many heads of a group, values of 8 to 256 entries."""
+import pytest
+import torch
+
+from kvad_b200.ops import Ops, lib
+
+pytestmark = pytest.mark.gpu
+PAGE = 64
+
+
+def i32(x):
+    return torch.tensor(x, dtype=torch.int32, device="cuda")
+
+
+class Case:
+    """A paged cache, queries for the last `new` of each sequence's positions, and the exact answer with a bound on the error."""
+
+    def __init__(self, seqs, H, G, dk, dv, *, alias=False, key_maps=1, cap=0.0, span=0.0, window=0, keep=0, chunk=0, gate=None, sinks=False, seed=0):
+        g = torch.Generator(device="cuda")
+        g.manual_seed(seed + dk * 7 + dv)
+        rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").to(torch.bfloat16)
+        self.seqs, self.H, self.dv, self.alias, self.scale = seqs, H, dv, alias, 1.5 / dk ** 0.5
+        width = -(-max(c + n for c, n in seqs) // PAGE)
+        n_pages = width * len(seqs) + 2
+        order = torch.randperm(n_pages, generator=torch.Generator().manual_seed(seed + 3))
+        self.table = order[:width * len(seqs)].reshape(len(seqs), width).to(torch.int32).cuda().contiguous()
+        self.kp = torch.full((n_pages, G, PAGE, dk), float("nan"), dtype=torch.bfloat16, device="cuda")
+        self.vp = None if alias else torch.full((n_pages, G // key_maps, PAGE, dv), float("nan"), dtype=torch.bfloat16, device="cuda")
+        n_rows = sum(n for _, n in seqs)
+        self.q = rnd(n_rows, H * dk + 8)[:, :H * dk]
+        self.gate = {None: None, "entry": rnd(n_rows, H * dv), "head": rnd(n_rows, H)}[gate]
+        self.sinks = torch.randn(H, generator=g, device="cuda") if sinks else None
+        self.kw = dict(softcap=cap, slope_span=span, window=window, keep_first=keep, chunk=chunk, key_maps=key_maps, sinks=self.sinks, gate=self.gate,
+                       value_dim=dv if alias else None)
+        want, slack, at = [], [], 0
+        for s, (cached, new) in enumerate(seqs):
+            L = cached + new
+            k = rnd(G, L, dk)
+            v = k[:, :, :dv] if alias else rnd(G // key_maps, L, dv)
+            for p in range(-(-L // PAGE)):
+                n = min(PAGE, L - p * PAGE)
+                self.kp[self.table[s, p].long(), :, :n] = k[:, p * PAGE:p * PAGE + n]
+                if not alias:
+                    self.vp[self.table[s, p].long(), :, :n] = v[:, p * PAGE:p * PAGE + n]
+            kd = k.double().repeat_interleave(H // G, 0)
+            vd = v.double().repeat_interleave(key_maps, 0).repeat_interleave(H // G, 0)
+            qd = self.q[at:at + new].double().reshape(new, H, dk).transpose(0, 1)
+            x = qd @ kd.transpose(1, 2) * self.scale
+            # a score's error: the tensor core truncates after every 16 products (2^-22 of the sum of magnitudes a step is generous); the cap goes
+            # through exponentials and a reciprocal good to 2 units in the last place of 1
+            ds = (qd.abs() @ kd.abs().transpose(1, 2)).max().item() * self.scale * (dk / 16 + 2) * 2.0 ** -22 + cap * 2.0 ** -20
+            if cap:
+                x = cap * torch.tanh(x / cap)
+            pos, key = torch.arange(cached, L, device="cuda"), torch.arange(L, device="cuda")
+            if span:
+                slopes = 2.0 ** (-span * torch.arange(1, H + 1, device="cuda", dtype=torch.float64) / H)
+                x = x - slopes[:, None, None] * (pos[:, None] - key[None, :])
+                ds += span and L * 2.0 ** -22
+            seen = key[None, :] <= pos[:, None]
+            if window:
+                seen &= (key[None, :] > pos[:, None] - window) | (key[None, :] < keep)
+            if chunk:
+                seen &= key[None, :] >= (pos - pos % chunk)[:, None]
+            x = x.masked_fill(~seen, float("-inf"))
+            if sinks:
+                x = torch.cat([x, self.sinks.double()[:, None, None].expand(H, new, 1)], 2)
+            p = torch.softmax(x, 2)[:, :, :L]
+            f = 1.0 if gate is None else torch.sigmoid(self.gate[at:at + new].double().reshape(new, H, -1)).transpose(0, 1)
+            want.append(((p @ vd) * f).transpose(0, 1).reshape(new, H * dv))
+            # a weight's relative error: twice the scores', 2^-16 for its pieces, and 2^-17 for sums of up to L terms and exponentials of up to 2^7
+            slack.append(((p @ vd.abs()) * f * (2 * ds + 2.0 ** -15)).transpose(0, 1).reshape(new, H * dv))
+            at += new
+        self.want, self.slack = torch.cat(want), torch.cat(slack)
+        starts = [0]
+        for _, n in seqs:
+            starts.append(starts[-1] + n)
+        self.starts, self.lens, self.max_new = i32(starts), i32([c + n for c, n in seqs]), max(n for _, n in seqs)
+
+    def run(self, ops, out_dtype=torch.bfloat16, **extra):
+        out = torch.full((self.q.shape[0], self.want.shape[1] + 8), float("nan"), dtype=out_dtype, device="cuda")
+        ops.attention_scored(self.q, out[:, :-8], self.starts, self.lens, len(self.seqs), self.max_new, self.table, self.kp, self.vp, self.H, self.scale,
+                             **self.kw, **extra)
+        torch.cuda.synchronize()
+        assert out[:, -8:].isnan().all()                  # nothing is written beside the heads
+        return out[:, :-8].double()
+
+    def check(self, got, out_dtype=torch.bfloat16):
+        bound = self.slack + (2.0 ** -8 if out_dtype == torch.bfloat16 else 2.0 ** -23) * self.want.abs() + 1e-30
+        worst = ((got - self.want).abs() / bound).max().item()
+        assert worst <= 1.0, worst
+
+
+EDGES = [(0, 129), (63, 2), (200, 65), (5, 1), (0, 64), (1, 127)]
+SHAPES = [
+    (4, 4, 64, 64, {}),                                                       # one head a group: a tile of 128 tokens
+    (16, 1, 96, 96, dict(alias=True)),
+    (16, 1, 256, 256, dict(alias=True, gate="entry")),                        # a latent of 256
+    (6, 2, 72, 40, dict(cap=30.0)),                                           # three heads a group, sizes that fill no 16
+    (8, 2, 128, 128, dict(window=50, keep=4, gate="entry")),
+    (20, 1, 64, 8, dict(window=1)),                                           # every row sees itself alone
+    (12, 4, 32, 192, dict(chunk=96, sinks=True)),
+    (4, 2, 128, 64, dict(span=8.0, gate="head")),
+    (8, 8, 64, 64, dict(key_maps=2)),
+    (2, 1, 8, 8, dict(sinks=True, window=130, keep=70, cap=5.0, span=4.0)),
+]
+
+
+@pytest.mark.parametrize("H,G,dk,dv,form", SHAPES)
+def test_prompt_rows_on_the_tensor_cores(H, G, dk, dv, form):
+    ops, cores = Ops(torch.bfloat16), Ops(torch.bfloat16)
+    cores.scored_prompt = False
+    c = Case(EDGES, H, G, dk, dv, **form)
+    outs = [torch.bfloat16] if c.gate is not None or dv > 128 else [torch.bfloat16, torch.float32]
+    for out in outs:
+        assert lib("attention_scored_prompt").kvad_attention_scored_prompt_takes(dk, dv, int(c.alias), int(out == torch.float32)) == 1
+        for o in (ops, cores):
+            c.check(c.run(o, out), out)
+
+
+@pytest.mark.parametrize("dk,dv,page,shift", [(64, 264, 64, 0), (20, 16, 64, 0), (64, 64, 32, 0), (64, 64, 64, 4)])
+def test_prompt_rows_it_does_not_take_go_to_the_cuda_cores(dk, dv, page, shift):
+    """Values, keys, pages and addresses out of its range: the same answer as with the tensor cores off, to the last bit."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(1)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").to(torch.bfloat16)
+    q, kp, vp = rnd(70, 2 * dk + 8)[:, shift:shift + 2 * dk], rnd(3, 1, page, dk), rnd(3, 1, page, dv)
+    outs = []
+    for on in (True, False):
+        ops = Ops(torch.bfloat16)
+        ops.scored_prompt = on
+        out = torch.full((70, 2 * dv), float("nan"), dtype=torch.bfloat16, device="cuda")
+        ops.attention_scored(q, out, i32([0, 70]), i32([80]), 1, 70, i32([[2, 0, 1]]), kp, vp, 2, 0.1)
+        outs.append(out)
+    assert torch.equal(*outs) and outs[0].isfinite().all()
+
+
+STEPS = [(0, 1), (63, 1), (64, 1), (129, 1), (700, 1), (191, 1)]
+
+
+@pytest.mark.parametrize("splits", [1, 3, 16])
+@pytest.mark.parametrize("H,G,dk,dv,form", SHAPES + [(16, 4, 64, 64, dict(cap=30.0, window=512, keep=4)), (17, 1, 40, 136, {}), (40, 1, 64, 64, dict(span=8.0))])
+def test_single_token_rows_on_the_tensor_cores(H, G, dk, dv, form, splits):
+    ops = Ops(torch.bfloat16)
+    c = Case(STEPS, H, G, dk, dv, **form)
+    scratch = torch.full((len(STEPS) * H * splits * (dv + 2),), float("nan"), device="cuda")
+    for out in (torch.bfloat16, torch.float32):
+        if out == torch.float32 and c.gate is not None:
+            continue
+        for per_block in (1, H // G):
+            c.check(c.run(ops, out, n_splits=splits, scratch=scratch, heads_per_block=per_block), out)
