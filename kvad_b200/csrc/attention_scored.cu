@@ -1,5 +1,6 @@
 // Softmax attention over the paged cache with everything a score can be given on its way to the softmax,
-// on the CUDA cores in 32-bit arithmetic, for prompts and for single-token rows alike:
+// in 32-bit arithmetic: on the CUDA cores for prompts and for single-token rows alike, and bfloat16 single-token rows in
+// whole 16-byte pieces on the tensor cores (`scored_step_kernel`; bfloat16 prompts: attention_scored_prompt.cu):
 //
 //   s = (q . k) * scale;  s = cap * tanh(s / cap)  (cap > 0);  s -= slope_h * (i - j)  (slope_span > 0,
 //   slope_h = 2^(-slope_span * (h + 1) / n_heads));  query i sees key j if j <= i and

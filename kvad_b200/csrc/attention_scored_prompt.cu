@@ -22,7 +22,7 @@ using namespace kvad;
 
 namespace {
 
-constexpr int PAGE = 64, WARPS = 8, THREADS = 32 * WARPS, ROWS = 16 * WARPS;
+constexpr int PAGE = 64, WARPS = 4, THREADS = 32 * WARPS, ROWS = 16 * WARPS;
 constexpr float LOG2E = 1.4426950408889634f, LN2 = 0.6931471805599453f;
 
 struct PromptArgs {
@@ -80,7 +80,7 @@ __device__ __forceinline__ uint32_t pack(float a, float b) {
 
 // NV: 16-entry groups of a value.
 template <int NV, bool F32OUT>
-__global__ void __launch_bounds__(THREADS, NV <= 4 ? 2 : 1) scored_prompt_kernel(const PromptArgs a) {
+__global__ void __launch_bounds__(THREADS, NV <= 4 ? 4 : 2) scored_prompt_kernel(const PromptArgs a) {
   extern __shared__ uint8_t smem_raw[];
   __nv_bfloat16* smem = reinterpret_cast<__nv_bfloat16*>(smem_raw);
   const int hp = a.hp, tok = ROWS / hp, group = a.n_heads / a.n_kv_heads, chunks = group / hp;
@@ -115,21 +115,29 @@ __global__ void __launch_bounds__(THREADS, NV <= 4 ? 2 : 1) scored_prompt_kernel
     while (t * PAGE <= last_pos && t * PAGE + PAGE <= first_key && t * PAGE >= a.keep_first) ++t;
     return t;
   };
+  // this thread's first piece of a page of keys and of values; from one of its pieces to the next by addition (a division a piece cost as much as
+  // the scores)
+  const int kr = tid / q_pieces, kc = tid - kr * q_pieces, vr = tid / v_pieces, vc = tid - vr * v_pieces;
+  const int k_rows = THREADS / q_pieces, k_rest = THREADS - k_rows * q_pieces, v_rows = THREADS / v_pieces, v_rest = THREADS - v_rows * v_pieces;
+  auto bring_rows = [&](__nv_bfloat16* dst, int stride, const __nv_bfloat16* src, int pieces, int r, int c, int n_live) {
+    const int rows = pieces == q_pieces ? k_rows : v_rows, rest = pieces == q_pieces ? k_rest : v_rest;
+#pragma unroll 4
+    for (int i = tid; i < PAGE * pieces; i += THREADS) {
+      copy16(smem_at(dst + r * stride + c * 8), src + (int64_t)i * 8, r < n_live);
+      r += rows;
+      c += rest;
+      if (c >= pieces) { c -= pieces; ++r; }
+    }
+  };
   auto bring = [&](int t, int stage) {
     const int page = pages[t], n_live = last_pos - t * PAGE + 1;
     __nv_bfloat16* ks = stages + stage * stage_size;
     const __nv_bfloat16* src = a.k_pages + (int64_t)page * a.k_page_stride + (int64_t)kvh * PAGE * a.dk;
-    for (int i = tid; i < PAGE * q_pieces; i += THREADS) {
-      const int r = i / q_pieces, c = i - r * q_pieces;
-      copy16(smem_at(ks + r * kst + c * 8), src + (int64_t)i * 8, r < n_live);
-    }
+    bring_rows(ks, kst, src, q_pieces, kr, kc, n_live);
     if (!a.alias) {
       __nv_bfloat16* vs = ks + PAGE * kst;
       const __nv_bfloat16* vsrc = a.v_pages + (int64_t)page * a.v_page_stride + (int64_t)(kvh / a.key_maps) * PAGE * a.dv;
-      for (int i = tid; i < PAGE * v_pieces; i += THREADS) {
-        const int r = i / v_pieces, c = i - r * v_pieces;
-        copy16(smem_at(vs + r * vst + c * 8), vsrc + (int64_t)i * 8, r < n_live);
-      }
+      bring_rows(vs, vst, vsrc, v_pieces, vr, vc, n_live);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
@@ -249,11 +257,7 @@ __global__ void __launch_bounds__(THREADS, NV <= 4 ? 2 : 1) scored_prompt_kernel
         sum[u] += sc[j][e];
       }
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      sum[u] += __shfl_xor_sync(0xffffffffu, sum[u], 1);
-      sum[u] += __shfl_xor_sync(0xffffffffu, sum[u], 2);
-      run_sum[u] = run_sum[u] * keep[u] + sum[u];
-    }
+    for (int u = 0; u < 2; ++u) run_sum[u] = run_sum[u] * keep[u] + sum[u];      // (of this thread's keys; the row's four threads meet at the end)
     const uint32_t v_at = smem_at(vs + ((lane & 7) + ((lane >> 3) & 1) * 8) * vst + (lane >> 4) * 8);
     if (!F32OUT) {
       if (__any_sync(0xffffffffu, keep[0] != 1.f || keep[1] != 1.f)) {      // (after a few pages the maxima seldom move)
@@ -271,14 +275,16 @@ __global__ void __launch_bounds__(THREADS, NV <= 4 ? 2 : 1) scored_prompt_kernel
           ph[f] = cut(x, y);
           pl[f] = pack(x, y);
         }
+        constexpr int GV = NV == 8 || NV == 4 ? 4 : 2;          // (the two products of an accumulator 2 GV products apart)
 #pragma unroll
-        for (int ng = 0; ng < NV; ++ng) {
-          uint32_t vb[4];
-          ldsm4_t(v_at + kk * 16 * vst * 2 + ng * 32, vb);
-          mma(o[2 * ng], pl, vb[0], vb[1]);
-          mma(o[2 * ng + 1], pl, vb[2], vb[3]);
-          mma(o[2 * ng], ph, vb[0], vb[1]);
-          mma(o[2 * ng + 1], ph, vb[2], vb[3]);
+        for (int n0 = 0; n0 < NV; n0 += GV) {
+          uint32_t vb[GV][4];
+#pragma unroll
+          for (int g = 0; g < GV; ++g) ldsm4_t(v_at + kk * 16 * vst * 2 + (n0 + g) * 32, vb[g]);
+#pragma unroll
+          for (int g = 0; g < 2 * GV; ++g) mma(o[2 * n0 + g], pl, vb[g >> 1][2 * (g & 1)], vb[g >> 1][2 * (g & 1) + 1]);
+#pragma unroll
+          for (int g = 0; g < 2 * GV; ++g) mma(o[2 * n0 + g], ph, vb[g >> 1][2 * (g & 1)], vb[g >> 1][2 * (g & 1) + 1]);
         }
       }
     } else {
@@ -300,11 +306,11 @@ __global__ void __launch_bounds__(THREADS, NV <= 4 ? 2 : 1) scored_prompt_kernel
           uint32_t vb[4];
           ldsm4_t(v_at + kk * 16 * vst * 2 + ng * 32, vb);
 #pragma unroll
-          for (int w = 0; w < 2; ++w) {
-            mma(low[w], pl[kk], vb[2 * w], vb[2 * w + 1]);
-            mma(low[w], pm[kk], vb[2 * w], vb[2 * w + 1]);
-            mma(page[w], ph[kk], vb[2 * w], vb[2 * w + 1]);
-          }
+          for (int w = 0; w < 2; ++w) mma(low[w], pl[kk], vb[2 * w], vb[2 * w + 1]);
+#pragma unroll
+          for (int w = 0; w < 2; ++w) mma(page[w], ph[kk], vb[2 * w], vb[2 * w + 1]);
+#pragma unroll
+          for (int w = 0; w < 2; ++w) mma(low[w], pm[kk], vb[2 * w], vb[2 * w + 1]);
         }
 #pragma unroll
         for (int w = 0; w < 2; ++w)
@@ -316,6 +322,8 @@ __global__ void __launch_bounds__(THREADS, NV <= 4 ? 2 : 1) scored_prompt_kernel
 
 #pragma unroll
   for (int u = 0; u < 2; ++u) {
+    run_sum[u] += __shfl_xor_sync(0xffffffffu, run_sum[u], 1);
+    run_sum[u] += __shfl_xor_sync(0xffffffffu, run_sum[u], 2);
     if (!live[u]) continue;
     const int row = warp * 16 + (lane >> 2) + u * 8, h = head[u];
     const int64_t grow = start + tok0 + row / hp;

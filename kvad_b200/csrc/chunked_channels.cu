@@ -19,6 +19,8 @@
 // Two kernels.  `prepare`, a block per (chunk, head): A, the decayed keys and queries, and for the delta rule X and W by forward
 // substitution, a column a thread, all of it in registers.  `walk`, a block per (sequence, head, 16 value columns): from chunk to chunk,
 // four products a chunk.  All 32-bit on the CUDA cores.
+//
+// Measured, delta rule, 2 x 1024 rows of 8 heads of 128 x 128: 434 -> 155 us (prepare 64 of them, the walk 92: 16 chunks one after another).
 #include "common.cuh"
 
 using namespace kvad;

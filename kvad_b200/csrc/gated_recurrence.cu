@@ -21,7 +21,8 @@
 // share a column, each with an eighth of its key entries in registers (four neighbours at a time), and meet by three shuffles for the two dot
 // products a row needs.  The rows' q, k and gates are staged 16 (or 8) rows at a time in shared memory, where the
 // scalar recurrences (the running maximum) and the transcendental functions are done once per block.  One row is
-// the same walk, so decoding, whole prompts and prompts in portions give the same bits.  The state of a slot is
+// the same walk, so decoding and portions of few rows give the same bits (prompts of many rows a sequence run in chunks,
+// chunked_recurrence.cu and chunked_channels.cu: the same sums in another order).  The state of a slot is
 // [heads, dv, dk] (a column's key entries side by side), then for the matrix memory n [heads, tiles, dk] and
 // m [heads, tiles] (a copy per block of 16 columns, so that no block reads what another writes).
 #include "common.cuh"

@@ -17,8 +17,8 @@
 // registers, the `split` threads of a column pair are neighbouring lanes and meet by shuffles.  Where one block
 // has all columns of a head, it also divides the outputs by their root mean square and applies the gate; where
 // a head's columns are spread over blocks, the raw 32-bit outputs go to `raw` and a second kernel finishes them.
-// A single-token row is the same walk with one row, so decoding and prompts (whole or in portions) give the
-// same bits.  The state is read from the sequence's slot at the start and written back at the end.
+// A single-token row is the same walk with one row, so decoding and portions of few rows give the same bits (prompts of
+// many rows a sequence run in chunks, chunked_recurrence.cu: the same sums in another order).  The state is read from the sequence's slot at the start and written back at the end.
 #include "common.cuh"
 
 using namespace kvad;

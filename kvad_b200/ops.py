@@ -1057,7 +1057,8 @@ class Ops:
     def linear_heads(self, a, weight, out, *, head_stride_a: int, head_stride_out: int, gate=None) -> None:
         """out[r, h * head_stride_out + j] = sum_i weight[h, j, i] * a[r, h * head_stride_a + i] for every head h: one small
         linear map per head (no bias).  Up to `HEADS_LINEAR_MAX_ROWS` rows and 768 inputs a head in ONE launch on the
-        CUDA cores (32-bit sums); more rows: one product per head through `linear` (the tensor cores where they take it).
+        CUDA cores (32-bit sums); more rows: one launch on the tensor cores where rows, outputs and strides are whole 16-byte
+        pieces, else one product per head through `linear`.
         `gate` [rows, heads x outputs]: the outputs times sigmoid(gate) (few rows: where they are written; more: by a pass of its own)."""
         _need_cuda(a, weight, out, gate)
         ld_a, ld_o = _rows_view(a, "head-wise input"), _rows_view(out, "head-wise output")
@@ -1107,7 +1108,7 @@ class Ops:
         heads x n_splits x (value size + 2)).  `key_maps` > 1: that many consecutive key heads read one value head (the values'
         pages have kv heads / key_maps heads).  `out` may be float32 whatever the compute dtype (no gate then).  `merge` False (with
         `n_splits` > 1): the parts stay in `scratch` for a merge of the caller's (`scored_merge_diff`), `out` is not written.  32-bit
-        arithmetic on the CUDA cores."""
+        scores, weights and sums; bfloat16 in whole 16-byte pieces on the tensor cores (the weights in bfloat16 pieces), else on the CUDA cores."""
         _need_cuda(q, out, seq_starts, kv_lens, page_table, k_pages, v_pages, gate, sinks)
         if sinks is not None and (sinks.dtype != torch.float32 or sinks.numel() != n_heads or not sinks.is_contiguous()):
             raise KernelError("attention_scored: sinks are float32, one per query head")

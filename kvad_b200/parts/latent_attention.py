@@ -7,8 +7,7 @@ key/value latent and one rotated key part are cached.
 
 The cache holds [c | k_r] per position: one "head" of kv_rank + rot_dim entries and no values.  The
 keys and values of the heads are never rebuilt: q_n . (W_uk c) = (W_uk^T q_n) . c, so each head's query is
-carried into the latent's space (a head-wise map: one launch for a few rows, one product a head for many),
-attention runs with ONE shared key [c | k_r] and the latent c itself as the value, and W_uv is applied to
+carried into the latent's space (a head-wise map, one launch), attention runs with ONE shared key [c | k_r] and the latent c itself as the value, and W_uv is applied to
 the attended latent (head-wise again) before the output projection.  Prompts and single-token rows take the same road.
 
 Without a `position` there is no rotated part: queries are W_q h (or W_uq c_q) as they are, the cache holds c alone.  `sink_name`: a

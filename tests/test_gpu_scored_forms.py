@@ -119,13 +119,13 @@ def test_prompt_rows_on_the_tensor_cores(H, G, dk, dv, form):
             c.check(c.run(o, out), out)
 
 
-@pytest.mark.parametrize("dk,dv,page,shift", [(64, 264, 64, 0), (20, 16, 64, 0), (64, 64, 32, 0), (64, 64, 64, 4)])
-def test_prompt_rows_it_does_not_take_go_to_the_cuda_cores(dk, dv, page, shift):
-    """Values, keys, pages and addresses out of its range: the same answer as with the tensor cores off, to the last bit."""
+@pytest.mark.parametrize("dk,dv,shift", [(64, 264, 0), (20, 16, 0), (64, 64, 4)])
+def test_prompt_rows_it_does_not_take_go_to_the_cuda_cores(dk, dv, shift):
+    """Values, keys and addresses out of its range: the same answer as with the tensor cores off, to the last bit."""
     g = torch.Generator(device="cuda")
     g.manual_seed(1)
     rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").to(torch.bfloat16)
-    q, kp, vp = rnd(70, 2 * dk + 8)[:, shift:shift + 2 * dk], rnd(3, 1, page, dk), rnd(3, 1, page, dv)
+    q, kp, vp = rnd(70, 2 * dk + 8)[:, shift:shift + 2 * dk], rnd(3, 1, PAGE, dk), rnd(3, 1, PAGE, dv)
     outs = []
     for on in (True, False):
         ops = Ops(torch.bfloat16)
@@ -148,5 +148,5 @@ def test_single_token_rows_on_the_tensor_cores(H, G, dk, dv, form, splits):
     for out in (torch.bfloat16, torch.float32):
         if out == torch.float32 and c.gate is not None:
             continue
-        for per_block in (1, H // G):
+        for per_block in (1, min(H // G, 32)):
             c.check(c.run(ops, out, n_splits=splits, scratch=scratch, heads_per_block=per_block), out)
