@@ -20,7 +20,7 @@
 // substitution, a column a thread, all of it in registers.  `walk`, a block per (sequence, head, 16 value columns): from chunk to chunk,
 // four products a chunk.  All 32-bit on the CUDA cores.
 //
-// Measured, delta rule, 2 x 1024 rows of 8 heads of 128 x 128: 434 -> 155 us (prepare 64 of them, the walk 92: 16 chunks one after another).
+// Measured, delta rule, 2 x 1024 rows of 8 heads of 128 x 128: 434 -> 150 us (prepare 60 of them, the walk 92: 16 chunks one after another).
 #include "common.cuh"
 
 using namespace kvad;
@@ -68,11 +68,13 @@ __device__ __forceinline__ float4 load4(const __nv_bfloat16* p) {
   const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
   return make_float4(a.x, a.y, b.x, b.y);
 }
-// A chunk's rows of one head, transposed [entry][row] (lanes over rows: no two meet in a bank); what does not exist is `fill`.
+// A chunk's rows of one head, transposed [entry][row]; what does not exist is `fill`.  `width_to` is a multiple of 16: a warp takes 8 rows by 4
+// neighbouring quads, whole sectors of memory, and its stores meet a bank twice.
 template <typename TI>
 __device__ __forceinline__ void bring(float* dst, const TI* src, int64_t ld, const Place& p, int width, int width_to, float scale, float fill) {
+#pragma unroll 4
   for (int i = threadIdx.x; i < C * width_to / 4; i += THREADS) {
-    const int r = i % C, d = i / C * 4;
+    const int r = (i & 7) + (i >> 5) % (C / 8) * 8, d = (((i >> 3) & 3) + (i >> 5) / (C / 8) * 4) * 4;
     float4 x = make_float4(fill, fill, fill, fill);
     if (r < p.n && d < width) {
       x = load4(src + (int64_t)(p.row0 + r) * ld + d);

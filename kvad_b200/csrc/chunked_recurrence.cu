@@ -16,8 +16,8 @@
 // keeps its last places.  The matrix memory's running maximum goes along: a chunk's own maximum at its end, the maximum carried over
 // the chunks in step 2, and per row m_i = F_i + max(m_c, max_(j <= i) (i_j - F_j)); every weight is at most 1.
 //
-// Measured: 2 x 1024 rows of 8 heads of 128 x 128 (rotated, normed, gated, bfloat16) 387 -> 90 us; the matrix memory over 1000 + 517 + 37 rows of 8
-// heads of 64 x 128 334 -> 59 us.
+// Measured: 2 x 1024 rows of 8 heads of 128 x 128 (rotated, normed, gated, bfloat16) 387 -> 85 us; the matrix memory over 1000 + 517 + 37 rows of 8
+// heads of 64 x 128 334 -> 50 us.  (92 and 53 before the state came a piece ahead by way of registers and rows by whole sectors.)
 //
 // Chunks of all sequences lie in one list: chunk c of sequence s is place seq_starts[s] / 64 + s + c, which never collides.
 #include "common.cuh"
@@ -129,8 +129,10 @@ __device__ __forceinline__ void chunk_gates(const ChunkArgs& a, const Place& p, 
 template <typename TI, bool TRANSPOSED>
 __device__ __forceinline__ void bring(float* dst, int ld, const TI* src, int64_t ld_src, const Place& p, int width, int width_to, bool act, float scale_from, int scaled_from) {
   const int quads = width_to / 4;
+#pragma unroll 4
   for (int i = threadIdx.x; i < C * quads; i += THREADS) {
-    const int r = TRANSPOSED ? i % C : i / quads, c = (TRANSPOSED ? i / C : i % quads) * 4;
+    // transposed: a warp takes 8 rows by 4 neighbouring quads (whole 32-byte sectors of bfloat16, and stores that meet a bank twice)
+    const int r = TRANSPOSED ? (i & 7) + (i >> 5) % (C / 8) * 8 : i / quads, c = (TRANSPOSED ? ((i >> 3) & 3) + (i >> 5) / (C / 8) * 4 : i % quads) * 4;
     float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
     if (r < p.n && c < width) x = load4(src + (int64_t)(p.row0 + r) * ld_src + c);
     float v[4] = {x.x, x.y, x.z, x.w};
@@ -375,6 +377,23 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_read_kernel(const ChunkArgs 
   }
   __syncthreads();
 
+  // The state before the chunk comes a piece at a time by way of registers, each piece asked for before the arithmetic that runs ahead of it.
+  // (The matrix memory's is [dv][dk]: a thread takes four neighbours along dk of one column.)
+  constexpr int FETCH = DV / 32;
+  const float* S = a.work + ((int64_t)blockIdx.x * a.heads + h) * a.dk * a.dv;
+  float4 piece[FETCH];
+  auto fetch = [&](int d0) {
+    const int nd = min(PIECE, a.dk - d0);
+#pragma unroll
+    for (int f = 0; f < FETCH; ++f) {
+      const int i = threadIdx.x + f * THREADS;
+      const int c = KIND == MEMORY ? i % DV : i % (DV / 4) * 4, d = KIND == MEMORY ? i / DV * 4 : i / (DV / 4);
+      piece[f] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (c < a.dv && d < nd) piece[f] = *reinterpret_cast<const float4*>(KIND == MEMORY ? S + (int64_t)c * a.dk + d0 + d : S + (int64_t)(d0 + d) * a.dv + c);
+    }
+  };
+  fetch(0);
+
   float sc[4][4] = {};
 #pragma unroll 1
   for (int d0 = 0; d0 < DK; d0 += PIECE) {              // (sums of 32 terms, added up: less rounding than one chain of 128)
@@ -420,28 +439,23 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_read_kernel(const ChunkArgs 
 
   constexpr int TC = DV / 16;
   float acc[4][TC] = {};
-  const float* S = a.work + ((int64_t)blockIdx.x * a.heads + h) * a.dk * a.dv;
   for (int d0 = 0; d0 < a.dk; d0 += PIECE) {
     const int nd = min(PIECE, a.dk - d0);
     if (d0 > 0) __syncthreads();
-    if (KIND == MEMORY) {                   // [dv][dk]: a thread takes four neighbours along dk of one column
-      for (int i = threadIdx.x; i < DV * (PIECE / 4); i += THREADS) {
+#pragma unroll
+    for (int f = 0; f < FETCH; ++f) {
+      const int i = threadIdx.x + f * THREADS;
+      if (KIND == MEMORY) {
         const int c = i % DV, d = i / DV * 4;
-        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (c < a.dv && d < nd) x = *reinterpret_cast<const float4*>(S + (int64_t)c * a.dk + d0 + d);
-        ss[d * LDS + c] = x.x;
-        ss[(d + 1) * LDS + c] = x.y;
-        ss[(d + 2) * LDS + c] = x.z;
-        ss[(d + 3) * LDS + c] = x.w;
-      }
-    } else {
-      for (int i = threadIdx.x; i < PIECE * (DV / 4); i += THREADS) {
-        const int d = i / (DV / 4), c = i % (DV / 4) * 4;
-        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (c < a.dv && d < nd) x = *reinterpret_cast<const float4*>(S + (int64_t)(d0 + d) * a.dv + c);
-        *reinterpret_cast<float4*>(ss + d * LDS + c) = x;
+        ss[d * LDS + c] = piece[f].x;
+        ss[(d + 1) * LDS + c] = piece[f].y;
+        ss[(d + 2) * LDS + c] = piece[f].z;
+        ss[(d + 3) * LDS + c] = piece[f].w;
+      } else {
+        *reinterpret_cast<float4*>(ss + i / (DV / 4) * LDS + i % (DV / 4) * 4) = piece[f];
       }
     }
+    if (d0 + PIECE < a.dk) fetch(d0 + PIECE);
     __syncthreads();
     float part[4][TC] = {};
     outer<4, TC>(part, qt + d0 * LDT, LDT, ss, LDS, nd, ty, tx);
