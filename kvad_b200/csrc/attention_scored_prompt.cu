@@ -8,21 +8,27 @@
 //                    after another.  There the tensor core's truncating accumulation is kept to 64 keys, whose sum then
 //                    joins the 32-bit running sum by a rounded addition.
 //
-// A block of eight warps works 128 (token, head) pairs that share a key head - 128 / hp consecutive tokens of one sequence times
-// hp heads of the group, a warp 16 of them - against the cache's pages of 64 keys: a page comes into shared memory by
-// cp.async while the one before is worked on (values that are the keys' first entries come once).  Queries stay in shared memory,
-// all of the running output in registers.  Rows are padded to an odd number of 16-byte pieces, so ldmatrix meets no bank twice.
+// A block works 64 (token, head) pairs that share a key head - 64 / hp consecutive tokens of one sequence times hp heads of the
+// group, a warp 16 of them - against the cache's pages of 64 keys, by two halves of four warps that take the pages the block sees in
+// turn and put their sums together at the end (`layout_of`: or by one half alone).  What bounds it is the chain through one
+// warp, ~1000 instructions and 5000 cycles a page with the products' latency; more warps at once and half as many pages a warp is what helps, and
+// four warps a barrier, so that halves and blocks are out of step and one's softmax runs under another's products.  A page comes into
+// shared memory by cp.async while the one before is worked on (values that are the keys' first entries come once).  Queries stay in shared
+// memory, all of the running output in registers.  Rows are padded to an odd number of 16-byte pieces, so ldmatrix meets no bank twice.
 // Pages that no pair of the block sees are skipped.  Tiles are launched longest first.
 //
-// Why: on the CUDA cores (`attention_scored.cu`) 2 x 1024 rows of 16 heads over a latent of 256 took 1102 us (15.6 TFLOP/s),
-// 16 heads of 64 on 4 key heads with capped scores and a window of 512 took 342 us.
+// Why: on the CUDA cores (`attention_scored.cu`) 2 x 1024 rows of 16 heads over a latent of 256 took 1102 us (15.6 TFLOP/s) and take LAT here,
+// 16 heads of 64 on 4 key heads with capped scores, gates and a window of 512 took 342 us and take WIN.
+#include <algorithm>
+
 #include "common.cuh"
 
 using namespace kvad;
 
 namespace {
 
-constexpr int PAGE = 64, WARPS = 4, THREADS = 32 * WARPS, ROWS = 16 * WARPS;
+constexpr int PAGE = 64, WARPS = 4, HALF = 32 * WARPS, THREADS = 2 * HALF, ROWS = 16 * WARPS;
+constexpr size_t SMEM_MOST = 220 * 1024, SMEM_HALF = 112 * 1024;      // (a block's; so that two fit an SM)
 constexpr float LOG2E = 1.4426950408889634f, LN2 = 0.6931471805599453f;
 
 struct PromptArgs {
@@ -33,7 +39,7 @@ struct PromptArgs {
   const int* seq_starts; const int* kv_lens; const int* page_table; int table_width;
   const __nv_bfloat16* k_pages; const __nv_bfloat16* v_pages;
   int64_t k_page_stride, v_page_stride;                           // in entries; a head's page is PAGE x dk (PAGE x dv)
-  int n_heads, n_kv_heads, dk, dv, hp, alias, key_maps;
+  int n_heads, n_kv_heads, dk, dv, hp, alias, key_maps, halves;
   float scale, softcap, slope_span;
   int window, keep_first, chunk;
   int k_steps, k_stride, v_stride;                                // 16-entry steps of a key; row strides in shared memory, in entries
@@ -80,32 +86,32 @@ __device__ __forceinline__ uint32_t pack(float a, float b) {
 
 // NV: 16-entry groups of a value.
 template <int NV, bool F32OUT>
-__global__ void __launch_bounds__(THREADS, NV <= 4 ? 4 : 2) scored_prompt_kernel(const PromptArgs a) {
+__global__ void __launch_bounds__(NV <= 4 ? THREADS : HALF, 2) scored_prompt_kernel(const PromptArgs a) {
   extern __shared__ uint8_t smem_raw[];
   __nv_bfloat16* smem = reinterpret_cast<__nv_bfloat16*>(smem_raw);
   const int hp = a.hp, tok = ROWS / hp, group = a.n_heads / a.n_kv_heads, chunks = group / hp;
   const int per_seq = a.n_kv_heads * chunks;
   const int s = blockIdx.x / per_seq, part = blockIdx.x - s * per_seq, kvh = part / chunks, h0 = kvh * group + (part - kvh * chunks) * hp;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int half = threadIdx.x / HALF, tid = threadIdx.x - half * HALF, lane = tid & 31, warp = tid >> 5;      // (tid, warp: within the half)
   const int kst = a.k_stride, vst = a.v_stride;
   __nv_bfloat16* Qs = smem;                                     // [ROWS][kst]
-  __nv_bfloat16* stages = Qs + ROWS * kst;                      // two of: keys [PAGE][kst], values [PAGE][vst] (or none: the keys)
   const int stage_size = PAGE * kst + (a.alias ? 0 : PAGE * vst);
+  __nv_bfloat16* stages = Qs + ROWS * kst + half * 2 * stage_size;      // each half: two of: keys [PAGE][kst], values [PAGE][vst] (or none: the keys)
   pdl_launch_dependents();
-  // what no copy writes (the rows' padding) must not be NaN: it is multiplied by zeros
-  {
-    const int total = (ROWS * kst + 2 * stage_size + 16) / 8;
-    for (int i = tid; i < total; i += THREADS) reinterpret_cast<uint4*>(smem)[i] = make_uint4(0u, 0u, 0u, 0u);
+  // The last step's entries past the key that no copy writes must not be NaN: zeros.  (Values past the last reach only outputs that are not written.)
+  if (a.dk % 16 != 0) {
+    for (int i = tid; i < ROWS + 2 * PAGE; i += HALF) {
+      __nv_bfloat16* at = i < ROWS ? Qs + i * kst : stages + ((i - ROWS) / PAGE) * stage_size + ((i - ROWS) % PAGE) * kst;
+      *reinterpret_cast<uint4*>(at + a.dk) = make_uint4(0u, 0u, 0u, 0u);
+    }
   }
   pdl_wait();
   const int start = a.seq_starts[s], n_new = a.seq_starts[s + 1] - start, tok0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * tok;
   if (tok0 >= n_new) return;
   const int n_tok = min(tok, n_new - tok0), pos0 = a.kv_lens[s] - n_new + tok0, last_pos = pos0 + n_tok - 1;
   const int* pages = a.page_table + (int64_t)s * a.table_width;
-  __syncthreads();                                              // the zeros lie
-
   const int q_pieces = a.dk / 8, v_pieces = a.dv / 8;
-  for (int i = tid; i < ROWS * q_pieces; i += THREADS) {
+  for (int i = threadIdx.x; i < ROWS * q_pieces; i += blockDim.x) {
     const int r = i / q_pieces, c = i - r * q_pieces, ti = r / hp, hi = r - ti * hp;
     const bool live = ti < n_tok;
     copy16(smem_at(Qs + r * kst + c * 8), a.q + (int64_t)(start + tok0 + (live ? ti : 0)) * a.ld_q + (int64_t)(h0 + hi) * a.dk + c * 8, live);
@@ -115,17 +121,22 @@ __global__ void __launch_bounds__(THREADS, NV <= 4 ? 4 : 2) scored_prompt_kernel
     while (t * PAGE <= last_pos && t * PAGE + PAGE <= first_key && t * PAGE >= a.keep_first) ++t;
     return t;
   };
-  // this thread's first piece of a page of keys and of values; from one of its pieces to the next by addition (a division a piece cost as much as
-  // the scores)
-  const int kr = tid / q_pieces, kc = tid - kr * q_pieces, vr = tid / v_pieces, vc = tid - vr * v_pieces;
-  const int k_rows = THREADS / q_pieces, k_rest = THREADS - k_rows * q_pieces, v_rows = THREADS / v_pieces, v_rest = THREADS - v_rows * v_pieces;
-  auto bring_rows = [&](__nv_bfloat16* dst, int stride, const __nv_bfloat16* src, int pieces, int r, int c, int n_live) {
-    const int rows = pieces == q_pieces ? k_rows : v_rows, rest = pieces == q_pieces ? k_rest : v_rest;
+  // A thread steps from one of its pieces to the next by additions (a division a piece cost as much as the scores); where registers are to spare the
+  // first step is worked out once, not once a page.
+  struct Steps { int r, c, rows, rest; };
+  auto steps_of = [&](int pieces) {
+    const int rows = HALF / pieces, r = tid / pieces;
+    return Steps{r, tid - r * pieces, rows, HALF - rows * pieces};
+  };
+  constexpr bool ONCE = NV == 8;
+  const Steps k_once = ONCE ? steps_of(q_pieces) : Steps{}, v_once = ONCE ? steps_of(v_pieces) : Steps{};
+  auto bring_rows = [&](__nv_bfloat16* dst, int stride, const __nv_bfloat16* src, int pieces, const Steps& z, int n_live) {
+    int r = z.r, c = z.c;
 #pragma unroll 4
-    for (int i = tid; i < PAGE * pieces; i += THREADS) {
+    for (int i = tid; i < PAGE * pieces; i += HALF) {
       copy16(smem_at(dst + r * stride + c * 8), src + (int64_t)i * 8, r < n_live);
-      r += rows;
-      c += rest;
+      r += z.rows;
+      c += z.rest;
       if (c >= pieces) { c -= pieces; ++r; }
     }
   };
@@ -133,11 +144,11 @@ __global__ void __launch_bounds__(THREADS, NV <= 4 ? 4 : 2) scored_prompt_kernel
     const int page = pages[t], n_live = last_pos - t * PAGE + 1;
     __nv_bfloat16* ks = stages + stage * stage_size;
     const __nv_bfloat16* src = a.k_pages + (int64_t)page * a.k_page_stride + (int64_t)kvh * PAGE * a.dk;
-    bring_rows(ks, kst, src, q_pieces, kr, kc, n_live);
+    bring_rows(ks, kst, src, q_pieces, ONCE ? k_once : steps_of(q_pieces), n_live);
     if (!a.alias) {
       __nv_bfloat16* vs = ks + PAGE * kst;
       const __nv_bfloat16* vsrc = a.v_pages + (int64_t)page * a.v_page_stride + (int64_t)(kvh / a.key_maps) * PAGE * a.dv;
-      bring_rows(vs, vst, vsrc, v_pieces, vr, vc, n_live);
+      bring_rows(vs, vst, vsrc, v_pieces, ONCE ? v_once : steps_of(v_pieces), n_live);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
@@ -171,12 +182,22 @@ __global__ void __launch_bounds__(THREADS, NV <= 4 ? 4 : 2) scored_prompt_kernel
   const float unit = plain ? scale2 : 1.f;
   const uint32_t q_at = smem_at(Qs + (warp * 16 + (lane & 15)) * kst + (lane >> 4) * 8);
 
+  // the pages that the block sees, dealt out to the halves in turn
   int t = next_page(0), stage = 0;
-  bring(t, 0);
+  if (half == 1) t = next_page(t + 1);
+  if (t * PAGE <= last_pos) bring(t, 0);
+  asm volatile("cp.async.wait_all;" ::: "memory");              // (a half without pages has queries on their way)
+  __syncthreads();                                              // the queries, brought by both halves, and each half's first page
+  bool first_page = true;
   while (t * PAGE <= last_pos) {
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();                                            // this page is there, and the one before has been used up
-    const int t_next = next_page(t + 1);
+    if (!first_page) {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      if (half == 0) asm volatile("bar.sync 1, %0;" ::"n"(HALF) : "memory");      // this page is there, and the one before has been used up
+      else asm volatile("bar.sync 2, %0;" ::"n"(HALF) : "memory");
+    }
+    first_page = false;
+    int t_next = next_page(t + 1);
+    if (a.halves == 2) t_next = next_page(t_next + 1);
     if (t_next * PAGE <= last_pos) bring(t_next, stage ^ 1);
     const int key0 = t * PAGE;
     const __nv_bfloat16* ks = stages + stage * stage_size;
@@ -320,10 +341,45 @@ __global__ void __launch_bounds__(THREADS, NV <= 4 ? 4 : 2) scored_prompt_kernel
     }
   }
 
+  // The second half's sums join the first's: its threads hold the same rows and entries.
 #pragma unroll
   for (int u = 0; u < 2; ++u) {
     run_sum[u] += __shfl_xor_sync(0xffffffffu, run_sum[u], 1);
     run_sum[u] += __shfl_xor_sync(0xffffffffu, run_sum[u], 2);
+  }
+  if (a.halves == 2) {
+    float* meet = reinterpret_cast<float*>(smem_raw) + tid;
+    __syncthreads();                                              // nobody reads queries or pages any more
+    if (half == 1) {
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        meet[u * HALF] = run_max[u];
+        meet[(2 + u) * HALF] = run_sum[u];
+      }
+#pragma unroll
+      for (int j = 0; j < 2 * NV; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) meet[(4 + j * 4 + e) * HALF] = o[j][e];
+    }
+    __syncthreads();
+    if (half == 1) return;
+    float mine[2], theirs[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const float their_max = meet[u * HALF], m = fmaxf(run_max[u], their_max), base = m == -INFINITY ? 0.f : m;
+      mine[u] = exp2_fast(run_max[u] - base);
+      theirs[u] = exp2_fast(their_max - base);
+      run_sum[u] = run_sum[u] * mine[u] + meet[(2 + u) * HALF] * theirs[u];
+      run_max[u] = m;
+    }
+#pragma unroll
+    for (int j = 0; j < 2 * NV; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) o[j][e] = o[j][e] * mine[e >> 1] + meet[(4 + j * 4 + e) * HALF] * theirs[e >> 1];
+  }
+
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
     if (!live[u]) continue;
     const int row = warp * 16 + (lane >> 2) + u * 8, h = head[u];
     const int64_t grow = start + tok0 + row / hp;
@@ -369,19 +425,30 @@ int launch(const PromptArgs& a, int n_seqs, int max_new, size_t smem, cudaStream
   const int tok = ROWS / a.hp;
   const int64_t columns = (int64_t)n_seqs * (a.n_heads / a.hp);
   KVAD_REQUIRE(columns < (1ll << 31) && (max_new + tok - 1) / tok <= 65535, "attention (scored, prompts): more tiles than one launch takes");
-  kvad_launch(scored_prompt_kernel<NV, F32OUT>, dim3((unsigned)columns, (max_new + tok - 1) / tok), dim3(THREADS), smem, stream, a);
+  kvad_launch(scored_prompt_kernel<NV, F32OUT>, dim3((unsigned)columns, (max_new + tok - 1) / tok), dim3(a.halves * HALF), smem, stream, a);
   KVAD_CHECK_LAUNCH("attention_scored_prompt");
   return KVAD_OK;
 }
 
-struct Layout { int k_stride, v_stride; size_t smem; };
-// Row strides of an odd number of 16-byte pieces over whole 16-entry steps; all of shared memory with the slack of one step that the last
-// row's unused value columns may read.
+// 16-entry groups of a value that the kernel is built for.
+int groups_of(int dv) { return dv <= 32 ? 2 : (dv <= 64 ? 4 : (dv <= 128 ? 8 : (dv <= 192 ? 12 : 16))); }
+
+struct Layout { int k_stride, v_stride, halves; size_t smem; };
+// Row strides of an odd number of 16-byte pieces over whole 16-entry steps; all of shared memory with the slack that the last row's unused
+// value columns may read (values are read in the kernel's groups of 16 entries), and room for the second half's sums at the end.
 Layout layout_of(int dk, int dv, bool alias) {
   Layout z;
   z.k_stride = (dk + 15) / 16 * 16 + 8;
   z.v_stride = alias ? z.k_stride : (dv + 15) / 16 * 16 + 8;
-  z.smem = ((size_t)ROWS * z.k_stride + 2 * ((size_t)PAGE * z.k_stride + (alias ? 0 : (size_t)PAGE * z.v_stride)) + 256 + 16) * 2;
+  // Two halves where two such blocks fit an SM (values of up to 64 entries: 128 registers a thread), else one: two halves that are the SM's
+  // only block leave it idle where they begin and end.  (Measured, 2 x 1024 rows, two halves against one: 12 heads of 64: 36 us and 50; 32 heads of
+  // 128 on 8: 148 and 112; 16 heads over a latent of 256: 152 and 108.)
+  auto need = [&](int halves) {
+    return ((size_t)ROWS * z.k_stride + 2 * halves * ((size_t)PAGE * z.k_stride + (alias ? 0 : (size_t)PAGE * z.v_stride)) + 256 + 16) * 2;
+  };
+  z.halves = groups_of(dv) <= 4 && need(2) <= SMEM_HALF ? 2 : 1;
+  z.smem = need(z.halves);
+  if (z.halves == 2) z.smem = std::max(z.smem, (size_t)(8 * groups_of(dv) + 4) * HALF * sizeof(float));
   return z;
 }
 
@@ -389,7 +456,7 @@ Layout layout_of(int dk, int dv, bool alias) {
 
 // 1 if prompts of these sizes run here: whole 16-byte pieces, values up to 256 entries (128 where the output is 32-bit), everything in shared memory.
 KVAD_EXPORT int kvad_attention_scored_prompt_takes(int dk, int dv, int alias, int out_f32) {
-  return dk > 0 && dv > 0 && dk % 8 == 0 && dv % 8 == 0 && dv <= (out_f32 ? 128 : 256) && layout_of(dk, dv, alias != 0).smem <= 220 * 1024 ? 1 : 0;
+  return dk > 0 && dv > 0 && dk % 8 == 0 && dv % 8 == 0 && dv <= (out_f32 ? 128 : 256) && layout_of(dk, dv, alias != 0).smem <= SMEM_MOST ? 1 : 0;
 }
 
 KVAD_EXPORT int kvad_attention_scored_prompt(const void* q, int64_t ld_q, void* out, int64_t ld_out, const void* gate, int64_t ld_gate, int gate_heads,
@@ -424,17 +491,19 @@ KVAD_EXPORT int kvad_attention_scored_prompt(const void* q, int64_t ld_q, void* 
   a.hp = 1;
   while (a.hp < 16 && (n_heads / n_kv_heads) % (a.hp * 2) == 0) a.hp *= 2;
   const Layout z = layout_of(dk, dv, alias);
-  a.k_steps = (dk + 15) / 16; a.k_stride = z.k_stride; a.v_stride = z.v_stride;
+  a.halves = z.halves; a.k_steps = (dk + 15) / 16; a.k_stride = z.k_stride; a.v_stride = z.v_stride;
 #define KVAD_SP(N)                                                                          \
   do {                                                                                      \
     if (out_f32) return launch<(N > 8 ? 8 : N), true>(a, n_seqs, max_new, z.smem, stream);  \
     return launch<N, false>(a, n_seqs, max_new, z.smem, stream);                            \
   } while (0)
-  if (dv <= 32) KVAD_SP(2);
-  if (dv <= 64) KVAD_SP(4);
-  if (dv <= 128) KVAD_SP(8);
-  if (dv <= 192) KVAD_SP(12);
-  KVAD_SP(16);
+  switch (groups_of(dv)) {
+    case 2: KVAD_SP(2);
+    case 4: KVAD_SP(4);
+    case 8: KVAD_SP(8);
+    case 12: KVAD_SP(12);
+    default: KVAD_SP(16);
+  }
 #undef KVAD_SP
 }
 

@@ -20,7 +20,7 @@
 // substitution, a column a thread, all of it in registers.  `walk`, a block per (sequence, head, 16 value columns): from chunk to chunk,
 // four products a chunk.  All 32-bit on the CUDA cores.
 //
-// Measured, delta rule, 2 x 1024 rows of 8 heads of 128 x 128: 434 -> 150 us (prepare 60 of them, the walk 92: 16 chunks one after another).
+// Measured, delta rule, 2 x 1024 rows of 8 heads of 128 x 128: 434 -> 150 us (the walk 92 of them: 16 chunks one after another).
 #include "common.cuh"
 
 using namespace kvad;

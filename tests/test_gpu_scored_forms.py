@@ -97,6 +97,8 @@ SHAPES = [
     (4, 4, 64, 64, {}),                                                       # one head a group: a tile of 128 tokens
     (16, 1, 96, 96, dict(alias=True)),
     (16, 1, 256, 256, dict(alias=True, gate="entry")),                        # a latent of 256
+    (4, 2, 256, 256, {}),                                                     # no room for two halves
+    (2, 1, 400, 64, dict(alias=True)),
     (6, 2, 72, 40, dict(cap=30.0)),                                           # three heads a group, sizes that fill no 16
     (8, 2, 128, 128, dict(window=50, keep=4, gate="entry")),
     (20, 1, 64, 8, dict(window=1)),                                           # every row sees itself alone
