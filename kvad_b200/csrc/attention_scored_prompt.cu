@@ -3,10 +3,9 @@
 //
 //   s = q . k        mma.sync m16n8k16, 32-bit accumulation (products of bfloat16 numbers are exact)
 //   p = exp(s - m)   32-bit, in the accumulators' own registers
-//   o += p v         p is cut into bfloat16 pieces, p = h + l (what is left out is below 2^-16 of p), or p = h + m + l
-//                    exactly where the output is 32-bit: a weight is not rounded to 16 bits, the pieces are multiplied one
-//                    after another.  There the tensor core's truncating accumulation is kept to 64 keys, whose sum then
-//                    joins the 32-bit running sum by a rounded addition.
+//   o += p v         p is cut into three bfloat16 pieces, p = h + m + l exactly: a weight keeps its 24 bits, the pieces are
+//                    multiplied one after another.  Where the output is 32-bit, the tensor core's truncating accumulation is
+//                    kept to 64 keys, whose sum then joins the 32-bit running sum by a rounded addition.
 //
 // A block works 64 (token, head) pairs that share a key head - 64 / hp consecutive tokens of one sequence times hp heads of the
 // group, a warp 16 of them - against the cache's pages of 64 keys, by two halves of four warps that take the pages the block sees in
@@ -17,8 +16,8 @@
 // memory, all of the running output in registers.  Rows are padded to an odd number of 16-byte pieces, so ldmatrix meets no bank twice.
 // Pages that no pair of the block sees are skipped.  Tiles are launched longest first.
 //
-// Why: on the CUDA cores (`attention_scored.cu`) 2 x 1024 rows of 16 heads over a latent of 256 took 1102 us (15.6 TFLOP/s) and take 110 here,
-// 16 heads of 64 on 4 key heads with capped scores, gates and a window of 512 took 358 us and take 51.
+// Why: on the CUDA cores (`attention_scored.cu`) 2 x 1024 rows of 16 heads over a latent of 256 took 1102 us (15.6 TFLOP/s) and take 130 here,
+// 16 heads of 64 on 4 key heads with capped scores, gates and a window of 512 took 358 us and take 57.
 #include <algorithm>
 
 #include "common.cuh"
@@ -289,14 +288,15 @@ __global__ void __launch_bounds__(NV <= 4 ? THREADS : HALF, 2) scored_prompt_ker
       }
 #pragma unroll
       for (int kk = 0; kk < 4; ++kk) {
-        uint32_t ph[4], pl[4];
+        uint32_t ph[4], pm[4], pl[4];
 #pragma unroll
         for (int f = 0; f < 4; ++f) {
           float x = sc[2 * kk + (f >> 1)][(f & 1) * 2], y = sc[2 * kk + (f >> 1)][(f & 1) * 2 + 1];
           ph[f] = cut(x, y);
+          pm[f] = cut(x, y);
           pl[f] = pack(x, y);
         }
-        constexpr int GV = NV == 8 || NV == 4 ? 4 : 2;          // (the two products of an accumulator 2 GV products apart)
+        constexpr int GV = NV == 8 || NV == 4 ? 4 : 2;          // (the three products of an accumulator 2 GV products apart)
 #pragma unroll
         for (int n0 = 0; n0 < NV; n0 += GV) {
           uint32_t vb[GV][4];
@@ -304,6 +304,8 @@ __global__ void __launch_bounds__(NV <= 4 ? THREADS : HALF, 2) scored_prompt_ker
           for (int g = 0; g < GV; ++g) ldsm4_t(v_at + kk * 16 * vst * 2 + (n0 + g) * 32, vb[g]);
 #pragma unroll
           for (int g = 0; g < 2 * GV; ++g) mma(o[2 * n0 + g], pl, vb[g >> 1][2 * (g & 1)], vb[g >> 1][2 * (g & 1) + 1]);
+#pragma unroll
+          for (int g = 0; g < 2 * GV; ++g) mma(o[2 * n0 + g], pm, vb[g >> 1][2 * (g & 1)], vb[g >> 1][2 * (g & 1) + 1]);
 #pragma unroll
           for (int g = 0; g < 2 * GV; ++g) mma(o[2 * n0 + g], ph, vb[g >> 1][2 * (g & 1)], vb[g >> 1][2 * (g & 1) + 1]);
         }

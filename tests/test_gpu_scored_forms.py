@@ -152,3 +152,50 @@ def test_single_token_rows_on_the_tensor_cores(H, G, dk, dv, form, splits):
             continue
         for per_block in (1, min(H // G, 32)):
             c.check(c.run(ops, out, n_splits=splits, scratch=scratch, heads_per_block=per_block), out)
+
+
+def paged(k, v, order_seed=1):
+    """One sequence's keys [G, L, dk] and values (None: the keys' first entries) as pages in any order, with its page table."""
+    G, L, _ = k.shape
+    n = -(-L // PAGE)
+    order = torch.randperm(n, generator=torch.Generator().manual_seed(order_seed))
+    table = order.to(torch.int32).cuda()[None].contiguous()
+
+    def pages(x):
+        out = torch.full((n, G, PAGE, x.shape[2]), float("nan"), dtype=torch.bfloat16, device="cuda")
+        for p in range(n):
+            m = min(PAGE, L - p * PAGE)
+            out[order[p], :, :m] = x[:, p * PAGE:p * PAGE + m]
+        return out
+    return pages(k), None if v is None else pages(v), table
+
+
+@pytest.mark.parametrize("H,dk,dv,alias", [(1, 64, 64, False), (16, 32, 32, False), (4, 128, 128, False), (2, 224, 192, True), (16, 288, 256, True)])
+def test_prompt_weights_keep_their_32_bits(H, dk, dv, alias):
+    """Two keys a row whose values are each other's opposites and whose scores differ by about 2^-13: what is left of the output is the difference
+    of two weights near 1, which a weight of 16 bits (2^-17 off) gives to one or two digits only."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(dk)
+    L = 200
+    k = torch.zeros(1, L, dk, dtype=torch.bfloat16, device="cuda")
+    tail = dv if alias else 0                                                # (the entries that the queries look at)
+    k[0, :, tail] = 0.25
+    k[0, :, tail + 1] = (torch.rand(L, generator=g, device="cuda") * 2.0 ** -12).bfloat16()
+    v = ((torch.rand(dv, generator=g, device="cuda") + 0.5) * (1.0 - 2.0 * (torch.arange(L, device="cuda") % 2))[:, None]).bfloat16()
+    if alias:
+        k[0, :, :dv] = v
+    q = torch.zeros(L, H, dk, dtype=torch.bfloat16, device="cuda")
+    q[:, :, tail] = torch.rand(L, H, generator=g, device="cuda").bfloat16()
+    q[:, :, tail + 1] = 1.0
+    kp, vp, table = paged(k, None if alias else v[None])
+    out = torch.full((L, H * dv), float("nan"), dtype=torch.bfloat16, device="cuda")
+    ops = Ops(torch.bfloat16)
+    assert lib("attention_scored_prompt").kvad_attention_scored_prompt_takes(dk, dv, int(alias), 0) == 1
+    ops.attention_scored(q.view(L, -1), out, i32([0, L]), i32([L]), 1, L, table, kp, vp, H, 1.0, value_dim=dv if alias else None, window=2)
+    x = torch.einsum("thd,sd->hts", q.double(), k[0].double())
+    pos = torch.arange(L, device="cuda")
+    x = x.masked_fill((pos[None] > pos[:, None]) | (pos[None] <= pos[:, None] - 2), float("-inf"))
+    want = torch.einsum("hts,sd->thd", torch.softmax(x, 2), v.double()).reshape(L, -1)
+    # scores of at most 1/4 + 2^-12, rounded a few times: 2^-24 of a weight; an exponential good to 2 units in the last place: 2^-23; the output's own rounding
+    bound = 2.0 ** -8 * want.abs() + 2.0 ** -21 * v.double().abs().max(0).values.repeat(H)
+    assert ((out.double() - want).abs() <= bound).all(), ((out.double() - want).abs() / bound).max().item()
