@@ -4,8 +4,9 @@
 //   s = q . k        mma.sync m16n8k16, 32-bit accumulation (products of bfloat16 numbers are exact)
 //   p = exp(s - m)   32-bit, in the accumulators' own registers
 //   o += p v         p is cut into three bfloat16 pieces, p = h + m + l exactly: a weight keeps its 24 bits, the pieces are
-//                    multiplied one after another.  Where the output is 32-bit, the tensor core's truncating accumulation is
-//                    kept to 64 keys, whose sum then joins the 32-bit running sum by a rounded addition.
+//                    multiplied one after another.  The tensor core's truncating accumulation is kept to 64 keys, whose sum
+//                    then joins the 32-bit running sum by a rounded addition: over all pages it left the sums of 8 k even weights
+//                    8e-5 short.
 //
 // A block works 64 (token, head) pairs that share a key head - 64 / hp consecutive tokens of one sequence times hp heads of the
 // group, a warp 16 of them - against the cache's pages of 64 keys, by two halves of four warps that take the pages the block sees in
@@ -16,8 +17,8 @@
 // memory, all of the running output in registers.  Rows are padded to an odd number of 16-byte pieces, so ldmatrix meets no bank twice.
 // Pages that no pair of the block sees are skipped.  Tiles are launched longest first.
 //
-// Why: on the CUDA cores (`attention_scored.cu`) 2 x 1024 rows of 16 heads over a latent of 256 took 1102 us (15.6 TFLOP/s) and take 130 here,
-// 16 heads of 64 on 4 key heads with capped scores, gates and a window of 512 took 358 us and take 57.
+// Why: on the CUDA cores (`attention_scored.cu`) 2 x 1024 rows of 16 heads over a latent of 256 took 1102 us (15.6 TFLOP/s) and take 127 here,
+// 16 heads of 64 on 4 key heads with capped scores, gates and a window of 512 took 358 us and take 58.
 #include <algorithm>
 
 #include "common.cuh"
@@ -279,67 +280,34 @@ __global__ void __launch_bounds__(NV <= 4 ? THREADS : HALF, 2) scored_prompt_ker
 #pragma unroll
     for (int u = 0; u < 2; ++u) run_sum[u] = run_sum[u] * keep[u] + sum[u];      // (of this thread's keys; the row's four threads meet at the end)
     const uint32_t v_at = smem_at(vs + ((lane & 7) + ((lane >> 3) & 1) * 8) * vst + (lane >> 4) * 8);
-    if (!F32OUT) {
-      if (__any_sync(0xffffffffu, keep[0] != 1.f || keep[1] != 1.f)) {      // (after a few pages the maxima seldom move)
+    uint32_t ph[4][4], pm[4][4], pl[4][4];
 #pragma unroll
-        for (int j = 0; j < 2 * NV; ++j)
+    for (int kk = 0; kk < 4; ++kk)
 #pragma unroll
-          for (int e = 0; e < 4; ++e) o[j][e] *= keep[e >> 1];
+      for (int f = 0; f < 4; ++f) {
+        float x = sc[2 * kk + (f >> 1)][(f & 1) * 2], y = sc[2 * kk + (f >> 1)][(f & 1) * 2 + 1];
+        ph[kk][f] = cut(x, y);
+        pm[kk][f] = cut(x, y);
+        pl[kk][f] = pack(x, y);
       }
+#pragma unroll
+    for (int ng = 0; ng < NV; ++ng) {
+      float low[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}}, page[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll
       for (int kk = 0; kk < 4; ++kk) {
-        uint32_t ph[4], pm[4], pl[4];
+        uint32_t vb[4];
+        ldsm4_t(v_at + kk * 16 * vst * 2 + ng * 32, vb);
 #pragma unroll
-        for (int f = 0; f < 4; ++f) {
-          float x = sc[2 * kk + (f >> 1)][(f & 1) * 2], y = sc[2 * kk + (f >> 1)][(f & 1) * 2 + 1];
-          ph[f] = cut(x, y);
-          pm[f] = cut(x, y);
-          pl[f] = pack(x, y);
-        }
-        constexpr int GV = NV == 8 || NV == 4 ? 4 : 2;          // (the three products of an accumulator 2 GV products apart)
+        for (int w = 0; w < 2; ++w) mma(low[w], pl[kk], vb[2 * w], vb[2 * w + 1]);
 #pragma unroll
-        for (int n0 = 0; n0 < NV; n0 += GV) {
-          uint32_t vb[GV][4];
+        for (int w = 0; w < 2; ++w) mma(page[w], ph[kk], vb[2 * w], vb[2 * w + 1]);
 #pragma unroll
-          for (int g = 0; g < GV; ++g) ldsm4_t(v_at + kk * 16 * vst * 2 + (n0 + g) * 32, vb[g]);
-#pragma unroll
-          for (int g = 0; g < 2 * GV; ++g) mma(o[2 * n0 + g], pl, vb[g >> 1][2 * (g & 1)], vb[g >> 1][2 * (g & 1) + 1]);
-#pragma unroll
-          for (int g = 0; g < 2 * GV; ++g) mma(o[2 * n0 + g], pm, vb[g >> 1][2 * (g & 1)], vb[g >> 1][2 * (g & 1) + 1]);
-#pragma unroll
-          for (int g = 0; g < 2 * GV; ++g) mma(o[2 * n0 + g], ph, vb[g >> 1][2 * (g & 1)], vb[g >> 1][2 * (g & 1) + 1]);
-        }
+        for (int w = 0; w < 2; ++w) mma(low[w], pm[kk], vb[2 * w], vb[2 * w + 1]);
       }
-    } else {
-      uint32_t ph[4][4], pm[4][4], pl[4][4];
 #pragma unroll
-      for (int kk = 0; kk < 4; ++kk)
+      for (int w = 0; w < 2; ++w)
 #pragma unroll
-        for (int f = 0; f < 4; ++f) {
-          float x = sc[2 * kk + (f >> 1)][(f & 1) * 2], y = sc[2 * kk + (f >> 1)][(f & 1) * 2 + 1];
-          ph[kk][f] = cut(x, y);
-          pm[kk][f] = cut(x, y);
-          pl[kk][f] = pack(x, y);
-        }
-#pragma unroll
-      for (int ng = 0; ng < NV; ++ng) {
-        float low[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}}, page[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-#pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {
-          uint32_t vb[4];
-          ldsm4_t(v_at + kk * 16 * vst * 2 + ng * 32, vb);
-#pragma unroll
-          for (int w = 0; w < 2; ++w) mma(low[w], pl[kk], vb[2 * w], vb[2 * w + 1]);
-#pragma unroll
-          for (int w = 0; w < 2; ++w) mma(page[w], ph[kk], vb[2 * w], vb[2 * w + 1]);
-#pragma unroll
-          for (int w = 0; w < 2; ++w) mma(low[w], pm[kk], vb[2 * w], vb[2 * w + 1]);
-        }
-#pragma unroll
-        for (int w = 0; w < 2; ++w)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) o[2 * ng + w][e] = fmaf(o[2 * ng + w][e], keep[e >> 1], page[w][e] + low[w][e]);
-      }
+        for (int e = 0; e < 4; ++e) o[2 * ng + w][e] = fmaf(o[2 * ng + w][e], keep[e >> 1], page[w][e] + low[w][e]);
     }
   }
 

@@ -199,3 +199,30 @@ def test_prompt_weights_keep_their_32_bits(H, dk, dv, alias):
     # scores of at most 1/4 + 2^-12, rounded a few times: 2^-24 of a weight; an exponential good to 2 units in the last place: 2^-23; the output's own rounding
     bound = 2.0 ** -8 * want.abs() + 2.0 ** -21 * v.double().abs().max(0).values.repeat(H)
     assert ((out.double() - want).abs() <= bound).all(), ((out.double() - want).abs() / bound).max().item()
+
+
+@pytest.mark.parametrize("H,dk,dv,alias,cached", [(16, 64, 64, False, 16384), (16, 128, 128, True, 8192), (16, 256, 256, True, 8192)])
+def test_a_long_cache_adds_no_bias(H, dk, dv, alias, cached):
+    """Positive values under nearly even weights: a sum that truncates at every step falls behind the longer it gets.  The outputs' own roundings, spread by a
+    gate, average out over the rows."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(dv)
+    new = 256
+    L = cached + new
+    k = (torch.rand(1, L, dk, generator=g, device="cuda") + 0.5).bfloat16()
+    v = None if alias else (torch.rand(1, L, dv, generator=g, device="cuda") + 0.5).bfloat16()
+    q, gate = (torch.randn(new, H * d, generator=g, device="cuda").bfloat16() for d in (dk, dv))
+    kp, vp, table = paged(k, v)
+    out = torch.full((new, H * dv), float("nan"), dtype=torch.bfloat16, device="cuda")
+    scale = 0.1 / dk ** 0.5
+    Ops(torch.bfloat16).attention_scored(q, out, i32([0, new]), i32([L]), 1, new, table, kp, vp, H, scale, value_dim=dv if alias else None, gate=gate)
+    seen = torch.arange(L, device="cuda")[None] <= torch.arange(cached, L, device="cuda")[:, None]
+    vd = (k if alias else v)[0, :, :dv].double()
+    error = 0.0
+    for h in range(H):
+        x = (q[:, h * dk:(h + 1) * dk].double() @ k[0].double().t() * scale).masked_fill(~seen, float("-inf"))
+        want = torch.softmax(x, 1) @ vd * torch.sigmoid(gate[:, h * dv:(h + 1) * dv].double())
+        error += ((out[:, h * dv:(h + 1) * dv].double() - want) / want).mean().item() / H
+    # single roundings to bfloat16 are 2^-9 at most and of either sign: 256 rows of 1024 outputs or more leave 2^-9 / 2^9 / sqrt(3) of them, four times that
+    # is 2^-16.8; 32-bit sums by rounding are far below
+    assert abs(error) < 2.0 ** -17, error
