@@ -18,7 +18,7 @@
 // Pages that no pair of the block sees are skipped.  Tiles are launched longest first.
 //
 // Why: on the CUDA cores (`attention_scored.cu`) 2 x 1024 rows of 16 heads over a latent of 256 took 1102 us (15.6 TFLOP/s) and take 127 here,
-// 16 heads of 64 on 4 key heads with capped scores, gates and a window of 512 took 358 us and take 58.
+// 16 heads of 64 on 4 key heads with capped scores, gates and a window of 512 took 358 us and take 64.
 #include <algorithm>
 
 #include "common.cuh"
@@ -41,6 +41,7 @@ struct PromptArgs {
   int64_t k_page_stride, v_page_stride;                           // in entries; a head's page is PAGE x dk (PAGE x dv)
   int n_heads, n_kv_heads, dk, dv, hp, alias, key_maps, halves;
   float scale, softcap, slope_span;
+  float cap_in, cap_out;                                          // a capped score: cap_out * tanh(cap_in * (q . k)), in units of log2
   int window, keep_first, chunk;
   int k_steps, k_stride, v_stride;                                // 16-entry steps of a key; row strides in shared memory, in entries
 };
@@ -61,15 +62,11 @@ __device__ __forceinline__ void copy16(uint32_t dst, const void* src, bool live)
   const int bytes = live ? 16 : 0;
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
-// 2^x and 1/x by the special-function unit (2 units in the last place; results below 2^-126 are zero).
+// 2^x by the special-function unit (2 units in the last place; a weight below 2^-126 of its row's largest is zero).  With it a 32-bit output is off
+// by 1.4e-7 (16 heads of 64) to 1.8e-7 (a latent of 128) over 1024 rows, the CUDA-core kernel's by 2.6e-7 to 3.2e-7.
 __device__ __forceinline__ float exp2_fast(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-__device__ __forceinline__ float rcp_fast(float x) {
-  float y;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
 // The upper halves of two floats as a pair of bfloat16 (truncated), and what is left of each.
@@ -177,7 +174,7 @@ __global__ void __launch_bounds__(NV <= 4 ? THREADS : HALF, 2) scored_prompt_ker
   for (int j = 0; j < 2 * NV; ++j)
 #pragma unroll
     for (int e = 0; e < 4; ++e) o[j][e] = 0.f;
-  const float scale2 = a.scale * LOG2E, inv_cap2 = a.softcap > 0.f ? 2.f * LOG2E * a.scale / a.softcap : 0.f, cap2 = a.softcap * LOG2E;
+  const float scale2 = a.scale * LOG2E;
   const bool plain = !(a.softcap > 0.f) && !(a.slope_span > 0.f) && a.scale > 0.f;
   const float unit = plain ? scale2 : 1.f;
   const uint32_t q_at = smem_at(Qs + (warp * 16 + (lane & 15)) * kst + (lane >> 4) * 8);
@@ -226,12 +223,12 @@ __global__ void __launch_bounds__(NV <= 4 ? THREADS : HALF, 2) scored_prompt_ker
     // Scores in units of log2, or, where nothing but a positive factor is on them, as they are with the factor `unit` still owed.
     // (Whole passes over the 32 scores under tests that are the same for every thread: this part is bound by instructions.)
     if (!plain) {
-      if (a.softcap > 0.f) {                                    // cap tanh(s / cap), tanh(y) = 1 - 2 / (exp(2 y) + 1)
+      if (a.softcap > 0.f) {                                    // cap tanh(s / cap): by `tanhf`, whose error follows its result (1 - 2 / (exp(2 y) + 1): off by 2^-22 of the CAP)
 #pragma unroll
         for (int j = 0; j < 8; ++j)
 #pragma unroll
           for (int e = 0; e < 4; ++e)
-            sc[j][e] = F32OUT ? cap2 * tanhf(sc[j][e] * a.scale / a.softcap) : fmaf(-2.f * cap2, rcp_fast(exp2_fast(sc[j][e] * inv_cap2) + 1.f), cap2);
+            sc[j][e] = a.cap_out * tanhf(sc[j][e] * a.cap_in);
       } else {
 #pragma unroll
         for (int j = 0; j < 8; ++j)
@@ -457,6 +454,9 @@ KVAD_EXPORT int kvad_attention_scored_prompt(const void* q, int64_t ld_q, void* 
   a.n_heads = n_heads; a.n_kv_heads = n_kv_heads; a.dk = dk; a.dv = dv; a.alias = alias ? 1 : 0; a.key_maps = key_maps;
   a.scale = scale; a.softcap = softcap; a.slope_span = slope_span; a.window = window > 0 ? window : 0; a.keep_first = window > 0 ? keep_first : 0;
   a.chunk = chunk > 0 ? chunk : 0;
+  // (scale / cap stays an ordinary number: a cap above 2^100 moves no score below 2^87, one of nothing makes every score but 0 the cap)
+  const float cap = std::min(softcap, 1.2676506e30f), ratio = scale / cap;
+  a.cap_in = softcap > 0.f ? std::max(-3.402823466e38f, std::min(3.402823466e38f, ratio)) : 0.f; a.cap_out = cap * LOG2E;
   // heads a tile: as many of the group as divide it, up to a warp's 16 rows (a tile then spans few tokens: little of its last page is masked)
   a.hp = 1;
   while (a.hp < 16 && (n_heads / n_kv_heads) % (a.hp * 2) == 0) a.hp *= 2;

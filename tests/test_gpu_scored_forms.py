@@ -48,10 +48,11 @@ class Case:
             vd = v.double().repeat_interleave(key_maps, 0).repeat_interleave(H // G, 0)
             qd = self.q[at:at + new].double().reshape(new, H, dk).transpose(0, 1)
             x = qd @ kd.transpose(1, 2) * self.scale
-            # a score's error: the tensor core truncates after every 16 products (2^-22 of the sum of magnitudes a step is generous); the cap goes
-            # through exponentials and a reciprocal good to 2 units in the last place of 1
-            ds = (qd.abs() @ kd.abs().transpose(1, 2)).max().item() * self.scale * (dk / 16 + 2) * 2.0 ** -22 + cap * 2.0 ** -20
+            # a score's error: the tensor core truncates after every 16 products (2^-22 of the sum of magnitudes a step is generous); the cap rounds what it
+            # gives, which is no larger than the score and the cap, a few times
+            ds = (qd.abs() @ kd.abs().transpose(1, 2)).max().item() * self.scale * (dk / 16 + 2) * 2.0 ** -22
             if cap:
+                ds += min(cap, x.abs().max().item()) * 2.0 ** -21
                 x = cap * torch.tanh(x / cap)
             pos, key = torch.arange(cached, L, device="cuda"), torch.arange(L, device="cuda")
             if span:
@@ -226,3 +227,14 @@ def test_a_long_cache_adds_no_bias(H, dk, dv, alias, cached):
     # single roundings to bfloat16 are 2^-9 at most and of either sign: 256 rows of 1024 outputs or more leave 2^-9 / 2^9 / sqrt(3) of them, four times that
     # is 2^-16.8; 32-bit sums by rounding are far below
     assert abs(error) < 2.0 ** -17, error
+
+
+@pytest.mark.parametrize("cap", [0.5, 5.0, 30.0, 1000.0, 1e6, 3e38])
+@pytest.mark.parametrize("H,G,dk,dv,form", [(4, 2, 64, 64, {}), (16, 1, 128, 128, dict(alias=True, sinks=True)), (4, 4, 256, 256, dict(window=90))])
+def test_score_caps_of_any_size(H, G, dk, dv, form, cap):
+    """The error of a capped score follows the score, not the cap: prompts and single-token rows, 16-bit and 32-bit outputs."""
+    ops = Ops(torch.bfloat16)
+    for seqs in (EDGES, STEPS):
+        c = Case(seqs, H, G, dk, dv, cap=cap, **form)
+        for out in (torch.bfloat16, torch.float32):
+            c.check(c.run(ops, out), out)
