@@ -40,6 +40,7 @@ struct PromptArgs {
   const __nv_bfloat16* k_pages; const __nv_bfloat16* v_pages;
   int64_t k_page_stride, v_page_stride;                           // in entries; a head's page is PAGE x dk (PAGE x dv)
   int n_heads, n_kv_heads, dk, dv, hp, alias, key_maps, halves;
+  int columns;                                                    // tiles of one place in their sequence: sequences x heads / hp (the grid is these, the last place first)
   float scale, softcap, slope_span;
   float cap_in, cap_out;                                          // a capped score: cap_out * tanh(cap_in * (q . k)), in units of log2
   int window, keep_first, chunk;
@@ -87,8 +88,8 @@ __global__ void __launch_bounds__(NV <= 4 ? THREADS : HALF, 2) scored_prompt_ker
   extern __shared__ uint8_t smem_raw[];
   __nv_bfloat16* smem = reinterpret_cast<__nv_bfloat16*>(smem_raw);
   const int hp = a.hp, tok = ROWS / hp, group = a.n_heads / a.n_kv_heads, chunks = group / hp;
-  const int per_seq = a.n_kv_heads * chunks;
-  const int s = blockIdx.x / per_seq, part = blockIdx.x - s * per_seq, kvh = part / chunks, h0 = kvh * group + (part - kvh * chunks) * hp;
+  const int per_seq = a.n_kv_heads * chunks, from_end = blockIdx.x / a.columns, column = blockIdx.x - from_end * a.columns;
+  const int s = column / per_seq, part = column - s * per_seq, kvh = part / chunks, h0 = kvh * group + (part - kvh * chunks) * hp;
   const int half = threadIdx.x / HALF, tid = threadIdx.x - half * HALF, lane = tid & 31, warp = tid >> 5;      // (tid, warp: within the half)
   const int kst = a.k_stride, vst = a.v_stride;
   __nv_bfloat16* Qs = smem;                                     // [ROWS][kst]
@@ -103,7 +104,7 @@ __global__ void __launch_bounds__(NV <= 4 ? THREADS : HALF, 2) scored_prompt_ker
     }
   }
   pdl_wait();
-  const int start = a.seq_starts[s], n_new = a.seq_starts[s + 1] - start, tok0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * tok;
+  const int start = a.seq_starts[s], n_new = a.seq_starts[s + 1] - start, tok0 = ((int)gridDim.x / a.columns - 1 - from_end) * tok;
   if (tok0 >= n_new) return;
   const int n_tok = min(tok, n_new - tok0), pos0 = a.kv_lens[s] - n_new + tok0, last_pos = pos0 + n_tok - 1;
   const int* pages = a.page_table + (int64_t)s * a.table_width;
@@ -382,7 +383,7 @@ __global__ void __launch_bounds__(NV <= 4 ? THREADS : HALF, 2) scored_prompt_ker
 }
 
 template <int NV, bool F32OUT>
-int launch(const PromptArgs& a, int n_seqs, int max_new, size_t smem, cudaStream_t stream) {
+int launch(const PromptArgs& a, int max_new, size_t smem, cudaStream_t stream) {
   static size_t configured = 0;
   if (smem > configured) {
     cudaError_t e = cudaFuncSetAttribute(scored_prompt_kernel<NV, F32OUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -390,9 +391,9 @@ int launch(const PromptArgs& a, int n_seqs, int max_new, size_t smem, cudaStream
     configured = smem;
   }
   const int tok = ROWS / a.hp;
-  const int64_t columns = (int64_t)n_seqs * (a.n_heads / a.hp);
-  KVAD_REQUIRE(columns < (1ll << 31) && (max_new + tok - 1) / tok <= 65535, "attention (scored, prompts): more tiles than one launch takes");
-  kvad_launch(scored_prompt_kernel<NV, F32OUT>, dim3((unsigned)columns, (max_new + tok - 1) / tok), dim3(a.halves * HALF), smem, stream, a);
+  const int64_t tiles = (int64_t)a.columns * ((max_new + tok - 1) / tok);
+  KVAD_REQUIRE(tiles < (1ll << 31), "attention (scored, prompts): %lld tiles are more than one launch takes", (long long)tiles);
+  kvad_launch(scored_prompt_kernel<NV, F32OUT>, dim3((unsigned)tiles), dim3(a.halves * HALF), smem, stream, a);
   KVAD_CHECK_LAUNCH("attention_scored_prompt");
   return KVAD_OK;
 }
@@ -460,12 +461,14 @@ KVAD_EXPORT int kvad_attention_scored_prompt(const void* q, int64_t ld_q, void* 
   // heads a tile: as many of the group as divide it, up to a warp's 16 rows (a tile then spans few tokens: little of its last page is masked)
   a.hp = 1;
   while (a.hp < 16 && (n_heads / n_kv_heads) % (a.hp * 2) == 0) a.hp *= 2;
+  KVAD_REQUIRE((int64_t)n_seqs * (n_heads / a.hp) < (1ll << 31), "attention (scored, prompts): %d sequences x %d heads are more than one launch takes", n_seqs, n_heads);
+  a.columns = n_seqs * (n_heads / a.hp);
   const Layout z = layout_of(dk, dv, alias);
   a.halves = z.halves; a.k_steps = (dk + 15) / 16; a.k_stride = z.k_stride; a.v_stride = z.v_stride;
 #define KVAD_SP(N)                                                                          \
   do {                                                                                      \
-    if (out_f32) return launch<(N > 8 ? 8 : N), true>(a, n_seqs, max_new, z.smem, stream);  \
-    return launch<N, false>(a, n_seqs, max_new, z.smem, stream);                            \
+    if (out_f32) return launch<(N > 8 ? 8 : N), true>(a, max_new, z.smem, stream);  \
+    return launch<N, false>(a, max_new, z.smem, stream);                            \
   } while (0)
   switch (groups_of(dv)) {
     case 2: KVAD_SP(2);

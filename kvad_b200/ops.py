@@ -1138,7 +1138,7 @@ class Ops:
             raise KernelError("attention_scored: splitting keys goes with single-token rows and float32 scratch of rows x heads x splits x (value size + 2)")
         if (self.scored_prompt and max_new >= self.SCORED_PROMPT_MIN_NEW and n_splits == 1 and page == 64 and ld_q % 8 == 0 and ld_o % 2 == 0 and ld_g % 2 == 0
                 and (q.data_ptr() | k_pages.data_ptr() | v_ptr.data_ptr()) % 16 == 0 and out.data_ptr() % 8 == 0
-                and (gate is None or gate.data_ptr() % 4 == 0) and (v_pages is not None or dv <= dk)
+                and (gate is None or gate.data_ptr() % 4 == 0) and (v_pages is not None or dv <= dk) and n_seqs * n_heads * (max_new // 64 + 1) < 1 << 31
                 and lib("attention_scored_prompt").kvad_attention_scored_prompt_takes(dk, dv, int(v_pages is None), int(out_f32)) == 1):
             h = lib("attention_scored_prompt")
             _check(h.kvad_attention_scored_prompt(_ptr(q), ld_q, _ptr(out), ld_o, _ptr(gate), ld_g, int(gate_heads), _ptr(sinks), _ptr(seq_starts),

@@ -238,3 +238,25 @@ def test_score_caps_of_any_size(H, G, dk, dv, form, cap):
         c = Case(seqs, H, G, dk, dv, cap=cap, **form)
         for out in (torch.bfloat16, torch.float32):
             c.check(c.run(ops, out), out)
+
+
+def test_a_prompt_of_more_tiles_than_a_grid_dimension_holds():
+    """16 heads on one key make tiles of 4 tokens: from 262 141 rows on there are more than 65 535 of them."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(3)
+    new, H, dk = 65535 * 4 + 70, 16, 8
+    L = new + 5
+    k = torch.randn(1, L, dk, generator=g, device="cuda").bfloat16()
+    q = torch.randn(new, H * dk, generator=g, device="cuda").bfloat16()
+    kp, _, table = paged(k, None)
+    out = torch.full((new, H * dk), float("nan"), dtype=torch.bfloat16, device="cuda")
+    ops = Ops(torch.bfloat16)
+    kw = dict(value_dim=dk, window=40)
+    ops.attention_scored(q, out, i32([0, new]), i32([L]), 1, new, table, kp, None, H, 0.3, **kw)
+    cut = new - 3000
+    part = torch.full((3000, H * dk), float("nan"), dtype=torch.bfloat16, device="cuda")
+    ops.attention_scored(q[cut:], part, i32([0, 3000]), i32([L]), 1, 3000, table, kp, None, H, 0.3, **kw)
+    assert torch.equal(out[cut:], part)
+    first = torch.full((3000, H * dk), float("nan"), dtype=torch.bfloat16, device="cuda")
+    ops.attention_scored(q[:3000], first, i32([0, 3000]), i32([3005]), 1, 3000, table, kp, None, H, 0.3, **kw)
+    assert torch.equal(out[:3000], first) and out.isfinite().all()
