@@ -445,7 +445,7 @@ class Ops:
 
         `form`: "auto"; "rows" (at most 16 rows: weights streamed through registers on the CUDA cores);
         "wide" / "swapped" (the tensor-core kernel's two operand roles).  `tile` and `splits` fix the
-        tensor-core kernel's tile width and K split (0: its own choice)."""
+        tensor-core kernel's tile width and K split (0: its own choice; 32-bit products take notice of widths of 64 and 128 alone)."""
         _need_cuda(a, weight, bias, out)
         epi = EPILOGUES[epilogue]
         lda, ldo = _rows_view(a, "linear input"), _rows_view(out, "linear output")
@@ -486,7 +486,8 @@ class Ops:
         if (form == "auto" and self.split_linear and m >= self.SPLIT_MIN_ROWS and k % 4 == 0 and lda % 4 == 0 and a.data_ptr() % 16 == 0
                 and weight.data_ptr() % 16 == 0):
             h = lib("linear_split")
-            _check(h.kvad_linear_split(_ptr(a), lda, _ptr(weight), _ptr(bias), bias_f32, _ptr(out), ldo, m, n, k, epi, int(tile), _stream()), h)
+            width = int(tile) if tile in (64, 128) else 0          # (its own widths; the bfloat16 kernel's others say nothing to it)
+            _check(h.kvad_linear_split(_ptr(a), lda, _ptr(weight), _ptr(bias), bias_f32, _ptr(out), ldo, m, n, k, epi, width, _stream()), h)
             return
         if (form == "auto" and self.dtype == torch.float32 and self.rows_linear_max >= 16 and 16 < m <= self.ROWS_BLOCKS_MAX and k <= 4096
                 and k % ve == 0 and lda % ve == 0 and a.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0 and self._rows_lib in build.sources()):

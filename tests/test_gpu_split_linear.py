@@ -89,3 +89,15 @@ def test_head_maps_of_many_rows_in_one_launch(dtype, n, H, n_in, n_out, pad):
     gated = torch.empty(n, H * n_out, device="cuda", dtype=t)
     ops.linear_heads(a, w, gated, head_stride_a=n_in + pad, head_stride_out=n_out, gate=gate)
     assert rel(gated.view(n, H, n_out), want * torch.sigmoid(gate.double()).view(n, H, n_out)) < (3e-7 if dtype == "float32" else 5e-3)
+
+
+@pytest.mark.parametrize("tile", [16, 32, 96, 192, 256])
+def test_a_tile_width_of_the_other_kernels_is_the_split_products_own_choice(tile):
+    """`tile` fixes the width of the bfloat16 kernel's tiles; the 32-bit product has 64 and 128 only and takes no notice of others."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(tile)
+    ops, a, w = Ops(torch.float32), randn(g, 200, 64), randn(g, 300, 64)
+    want, got = torch.empty(200, 300, device="cuda"), torch.empty(200, 300, device="cuda")
+    ops.linear(a, w, None, want)
+    ops.linear(a, w, None, got, tile=tile)
+    assert torch.equal(got, want)
