@@ -424,13 +424,15 @@ __global__ void __launch_bounds__(THREADS, 1) channel_walk_kernel(const ChannelA
       }
       __syncthreads();
       const float4 w = *reinterpret_cast<const float4*>(D + place_of<C>(ur) + uc);      // u = X - W S
-      *reinterpret_cast<float4*>(D + place_of<C>(ur) + uc) = make_float4(given[0] - w.x, given[1] - w.y, given[2] - w.z, given[3] - w.w);
+      given[0] -= w.x; given[1] -= w.y; given[2] -= w.z; given[3] -= w.w;
+      *reinterpret_cast<float4*>(D + place_of<C>(ur) + uc) = make_float4(given[0], given[1], given[2], given[3]);
     } else {
       *reinterpret_cast<float4*>(D + place_of<C>(ur) + uc) = make_float4(given[0], given[1], given[2], given[3]);
       product<DK>(acc, wq + quarter * (DK / 4) * WROWS + q4 * 4, WROWS, S + place_of<DK>(quarter * (DK / 4)) + c4, DK / 4);
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();                                  // u lies, keys and A are there, W and q B have been used up
+    // u lies, keys and A are there, W and q B have been used up
+    const bool odd = __syncthreads_or(given[0] * 0.f + given[1] * 0.f + given[2] * 0.f + given[3] * 0.f != 0.f);
     if (c + 1 < n_chunks) bring_wq(c + 1);
     // the state: S' = B S + K^T u, a half of the rows a group
     float add[4][4] = {};
@@ -442,7 +444,21 @@ __global__ void __launch_bounds__(THREADS, 1) channel_walk_kernel(const ChannelA
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int j = 0; j < 4; ++j) read[i][j] = DELTA ? 0.f : acc[i][j];
-    product<C>(read, at + quarter * B * C + q4 * 4, C, D + place_of<C>(quarter * B) + c4, B);
+    if (!odd) {
+      product<C>(read, at + quarter * B * C + q4 * 4, C, D + place_of<C>(quarter * B) + c4, B);
+    } else {                                          // a row u is not finite: A's zeros would make NaN of it, so only the rows that a row sees
+#pragma unroll 1
+      for (int j = quarter * B; j < min(quarter * B + B, q4 * 4 + 4); ++j) {
+        const float4 x = *reinterpret_cast<const float4*>(at + j * C + q4 * 4), y = *reinterpret_cast<const float4*>(D + place_of<C>(j) + c4);
+        const float xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (j <= q4 * 4 + i) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) read[i][e] = fmaf(xs[i], ys[e], read[i][e]);
+          }
+      }
+    }
     // (delta rule: the threads of group 0 with rows from 64 on hold (q B)^T S: they are the second quarter, for the same rows and columns)
     if (DELTA && quarter == 1) {
 #pragma unroll

@@ -412,9 +412,9 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_read_kernel(const ChunkArgs 
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int c = tx * 4 + j;
-      float w = 0.f;
-      if (c <= r && r < p.n) w = KIND == MEMORY ? expf((float)((double)in[c] - F[c] - (double)mx[r])) : power[r - c];
-      sc[i][j] *= w;
+      // (a row that is not seen counts for nothing, also where its score is no number)
+      if (c <= r && r < p.n) sc[i][j] *= KIND == MEMORY ? expf((float)((double)in[c] - F[c] - (double)mx[r])) : power[r - c];
+      else sc[i][j] = 0.f;
       sum += sc[i][j];
     }
     if (KIND == MEMORY) {
@@ -470,7 +470,22 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_read_kernel(const ChunkArgs 
 #pragma unroll
     for (int j = 0; j < TC; ++j) acc[i][j] *= w;
   }
-  outer<4, TC>(acc, pt, LDT, vs, DV, p.n, ty, tx);
+  // values of the rows that a row sees, and no others: a zero weight would make NaN of a value that is not finite
+  outer<4, TC>(acc, pt, LDT, vs, DV, min(p.n, ty * 4), ty, tx);
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const int t = ty * 4 + e;
+    if (t >= p.n) break;
+    float y[TC];
+#pragma unroll
+    for (int g = 0; g < TC; g += 4) *reinterpret_cast<float4*>(y + g) = *reinterpret_cast<const float4*>(vs + t * DV + tx * 4 + g * 16);
+#pragma unroll
+    for (int i = e; i < 4; ++i) {
+      const float x = pt[t * LDT + ty * 4 + i];
+#pragma unroll
+      for (int j = 0; j < TC; ++j) acc[i][j] = fmaf(x, y[j], acc[i][j]);
+    }
+  }
 
 #pragma unroll
   for (int i = 0; i < 4; ++i) {

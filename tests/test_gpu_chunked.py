@@ -217,3 +217,48 @@ def test_the_walk_still_takes_what_the_chunks_do_not():
         out, state = torch.full((n, 16), float("nan"), device="cuda"), torch.zeros(1, ops.recurrence_state_size("gated_linear", 1, dk, 16), device="cuda")
         ops.gated_recurrence("gated_linear", q, k, v, decay.float() if ready else z, out, state, starts([n]), i32([0]), 1, 1, 1, dk, 16, gates_ready=ready)
         assert rel(out, want[:, 0]) < 3e-6
+
+
+@pytest.mark.parametrize("kind", ["retention", "retention finished", "matrix_memory", "delta_rule", "gated_linear"])
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+@pytest.mark.parametrize("row,what", [(40, "v"), (43, "k"), (42, "kv"), (63, "v"), (1, "kv"), (97, "kv")])
+def test_a_row_that_is_not_finite_reaches_no_row_before_it(kind, bad, row, what):
+    """As in the row by row walk: the rows before it have the bits that they have beside finite rows, other heads and sequences too; the ones after it do not
+    pass it off as finite."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(row)
+    H, dk, dv, lens = 2, 64, 128, [130, 70]
+    N = sum(lens)
+    q, k, v, gate = (torch.randn(N, H * d, generator=g, device="cuda") for d in (dk, dk, dv, dv))
+    memory = kind == "matrix_memory"
+    gates = torch.randn(N, 2 * H, generator=g, device="cuda") + 3.0 if memory else torch.sigmoid(torch.randn(N, H * dk, generator=g, device="cuda") + 3.0)
+    beta, decay = torch.sigmoid(torch.randn(N, H, generator=g, device="cuda")), torch.tensor([0.9, 0.97], device="cuda")
+    if kind == "delta_rule":
+        k = torch.nn.functional.normalize(k.view(N, H, dk), dim=-1).view(N, -1)
+    ops = Ops(torch.float32)
+    ops.CHUNK_MIN_ROWS = 1
+
+    def run(k, v):
+        out = torch.full((N, H * dv), float("nan"), device="cuda")
+        if kind.startswith("retention"):
+            state, done = torch.zeros(2, H, dk, dv, device="cuda"), kind.endswith("finished")
+            ops.retention(q, k, v, out if done else None, state, starts(lens), i32(lens), i32([0, 1]), 2, decay, H, raw=torch.empty_like(out) if done else out,
+                          raw_only=not done, **(dict(gate=gate, unit_norm_eps=1e-5) if done else {}))
+        else:
+            state = torch.zeros(2, ops.recurrence_state_size(kind, H, dk, dv), device="cuda")
+            more = {"delta_rule": dict(beta=beta, a_log=torch.zeros(H, device="cuda"), dt_bias=torch.zeros(H * dk, device="cuda"), gates_ready=True),
+                    "gated_linear": dict(gates_ready=True), "matrix_memory": dict(cap=15.0)}[kind]
+            ops.gated_recurrence(kind, q, k, v, gates, out, state, starts(lens), i32([0, 1]), 2, H, H, dk, dv, **more)
+        return out, state
+
+    want, end = run(k, v)
+    assert want.isfinite().all()
+    k2, v2 = k.clone(), v.clone()
+    if "k" in what:
+        k2[row, 3] = bad
+    if "v" in what:
+        v2[row, 5] = bad
+    got, end2 = run(k2, v2)
+    assert torch.equal(got[:row], want[:row])                                           # the rows before, of both heads
+    assert torch.equal(got[:, dv:], want[:, dv:]) and torch.equal(got[130:], want[130:]) and torch.equal(end2[1], end[1])       # the other head and sequence
+    assert not got[row:130, 5].isfinite().any() and not end2[0].isfinite().all()
