@@ -18,9 +18,11 @@
 //
 // Two kernels.  `prepare`, a block per (chunk, head): A, the decayed keys and queries, and for the delta rule X and W by forward
 // substitution, a column a thread, all of it in registers.  `walk`, a block per (sequence, head, 16 value columns): from chunk to chunk,
-// four products a chunk.  All 32-bit on the CUDA cores.
+// four products a chunk.  All 32-bit on the CUDA cores; sums of 16 terms added up and decays whose products carry what they lose keep the
+// error beside the walk's: over 1024 rows of 128 x 128 the delta rule's outputs are off by 1.21e-7 (row by row 1.17e-7, with longer chains and
+// plain products 1.43e-7) and its states by 8.9e-8 (8.9e-8, 9.9e-8), the gated linear kind's by 1.30e-7 (1.27e-7, 1.71e-7) and 9.0e-8 (1.00e-7, 1.26e-7).
 //
-// Measured, delta rule, 2 x 1024 rows of 8 heads of 128 x 128: 434 -> 150 us (the walk 92 of them: 16 chunks one after another).
+// Measured, delta rule, 2 x 1024 rows of 8 heads of 128 x 128: 434 -> 155 us (the walk 92 of them: 16 chunks one after another).
 #include "common.cuh"
 
 using namespace kvad;
@@ -100,6 +102,17 @@ __device__ __forceinline__ void put16(float* dst, const float (&v)[B]) {
 // The channels come 64 at a time, so that two blocks fit an SM.
 constexpr int HD = 64;
 
+// A product of decays that carries what its roundings lose (up to 64 of them in a row otherwise, which every state and output would inherit).
+struct Decay {
+  float w = 1.f, lost = 0.f;
+  __device__ __forceinline__ void by(float g) {
+    const float p = w * g;
+    lost = fmaf(lost, g, fmaf(w, g, -p));
+    w = p;
+  }
+  __device__ __forceinline__ float value() const { return w + lost; }
+};
+
 template <typename TI, int DK, bool DELTA>
 __global__ void __launch_bounds__(THREADS, 2) channel_prepare_kernel(const ChannelArgs a) {
   extern __shared__ float smem[];
@@ -140,12 +153,15 @@ __global__ void __launch_bounds__(THREADS, 2) channel_prepare_kernel(const Chann
         get16(gv, gt + d * LDT + i0);
         if (DELTA) get16(kv, kt + d * LDT + i0);
         const float own = kt[d * LDT + i0 + j];
-        float w = 0.f;
+        float w = 0.f, lost = 0.f;                 // (the key's entry as it decays, and what the roundings of that lose)
 #pragma unroll
         for (int i = 0; i < B; ++i) {
-          w = i == j ? own : w * gv[i];            // (before row j: zero)
-          sq[i] = fmaf(qv[i], w, sq[i]);
-          if (DELTA) sk[i] = fmaf(kv[i], w, sk[i]);
+          const float next = w * gv[i];
+          lost = i == j ? 0.f : fmaf(lost, gv[i], fmaf(w, gv[i], -next));
+          w = i == j ? own : next;                 // (before row j: zero)
+          const float key = w + lost;
+          sq[i] = fmaf(qv[i], key, sq[i]);
+          if (DELTA) sk[i] = fmaf(kv[i], key, sk[i]);
         }
       }
       // the quarters meet: neighbouring half-warps by shuffles, the two warps in shared memory
@@ -170,23 +186,23 @@ __global__ void __launch_bounds__(THREADS, 2) channel_prepare_kernel(const Chann
     // decays along a block, a (channel, block) a thread
     {
       const int d = tid % HD, blk = tid / HD, at_d = d * LDT + blk * B;
-      float g[B], k[B], x[B], w = 1.f;
+      float g[B], k[B], x[B];
+      Decay after, before;
       get16(g, gt + at_d);
       get16(k, kt + at_d);
 #pragma unroll
       for (int r = B - 1; r >= 0; --r) {
-        x[r] = k[r] * w;
-        w *= g[r];
+        x[r] = k[r] * after.value();
+        after.by(g[r]);
       }
       put16(kh + at_d, x);
-      block_g[blk * HD + d] = w;
+      block_g[blk * HD + d] = after.value();
       get16(x, qt + at_d);
-      w = 1.f;
 #pragma unroll
       for (int r = 0; r < B; ++r) {
-        w *= g[r];
-        x[r] *= w;
-        k[r] *= w;
+        before.by(g[r]);
+        x[r] *= before.value();
+        k[r] *= before.value();
       }
       put16(qt + at_d, x);
       if (DELTA) put16(kt + at_d, k);
@@ -199,19 +215,27 @@ __global__ void __launch_bounds__(THREADS, 2) channel_prepare_kernel(const Chann
       const int i0 = late * B + (lane & 3) * 4, j0 = early * B + ((lane >> 2) & 3) * 4;
       if (DELTA || lane < 16) {
         float s[4][4] = {};
+#pragma unroll 1
+        for (int d0 = 0; d0 < HD; d0 += 16) {      // (sums of 16 terms, added up)
+          float part[4][4] = {};
 #pragma unroll 4
-        for (int d = 0; d < HD; ++d) {
-          float x[4], y[4], w = 1.f;
-          *reinterpret_cast<float4*>(x) = *reinterpret_cast<const float4*>(rows + d * LDT + i0);
-          *reinterpret_cast<float4*>(y) = *reinterpret_cast<const float4*>(kh + d * LDT + j0);
-          if (late - early > 1) w = block_g[(early + 1) * HD + d];
-          if (late - early > 2) w *= block_g[(early + 2) * HD + d];
+          for (int d = d0; d < d0 + 16; ++d) {
+            float x[4], y[4], w = 1.f;
+            *reinterpret_cast<float4*>(x) = *reinterpret_cast<const float4*>(rows + d * LDT + i0);
+            *reinterpret_cast<float4*>(y) = *reinterpret_cast<const float4*>(kh + d * LDT + j0);
+            if (late - early > 1) w = block_g[(early + 1) * HD + d];
+            if (late - early > 2) w *= block_g[(early + 2) * HD + d];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const float xi = x[i] * w;
+            for (int i = 0; i < 4; ++i) {
+              const float xi = x[i] * w;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) s[i][j] = fmaf(xi, y[j], s[i][j]);
+              for (int j = 0; j < 4; ++j) part[i][j] = fmaf(xi, y[j], part[i][j]);
+            }
           }
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) s[i][j] += part[i][j];
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i)
@@ -268,7 +292,7 @@ __global__ void __launch_bounds__(THREADS, 2) channel_prepare_kernel(const Chann
       }
       if (is_w) {
         const float* decay = g + (int64_t)p.row0 * a.ld_gates + own;
-        float w = 1.f;
+        Decay before;
 #pragma unroll
         for (int i0 = 0; i0 < C; i0 += B) {
           float y[B];
@@ -279,8 +303,8 @@ __global__ void __launch_bounds__(THREADS, 2) channel_prepare_kernel(const Chann
           }
 #pragma unroll
           for (int i = 0; i < B; ++i) {
-            w *= y[i];
-            x[i0 + i] *= w;
+            before.by(y[i]);
+            x[i0 + i] *= before.value();
           }
         }
       }
@@ -321,20 +345,29 @@ __device__ __forceinline__ void copy16(void* dst, const void* src) {
 // neighbouring lanes then go to and come from different banks (with the rows in order they all meet in the same four).
 template <int ROWS>
 __device__ __forceinline__ int place_of(int r) { return ((r & 3) * (ROWS / 4) + (r >> 2)) * LDC; }
-// acc[4][4] += sum over n of X[n][0 .. 3] Y[row n][0 .. 3]; Y points at the place of a row that is a multiple of 4, n too.
+// acc[4][4] += sum over n of X[n][0 .. 3] Y[row n][0 .. 3]; Y points at the place of a row that is a multiple of 4, n is a multiple of 16.
+// Sums of 16 terms, added up: less rounding than one chain (of 8: less again by 2 %, for 6 us of 148).
 template <int ROWS>
 __device__ __forceinline__ void product(float (&acc)[4][4], const float* X, int ldx, const float* Y, int n) {
-#pragma unroll 2
-  for (int t4 = 0; t4 < n / 4; ++t4) {
+#pragma unroll 1
+  for (int t0 = 0; t0 < n / 4; t0 += 4) {
+    float part[4][4] = {};
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float4 x = *reinterpret_cast<const float4*>(X + (t4 * 4 + e) * ldx), y = *reinterpret_cast<const float4*>(Y + (e * (ROWS / 4) + t4) * LDC);
-      const float xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w};
+    for (int t4 = t0; t4 < t0 + 4; ++t4) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int e = 0; e < 4; ++e) {
+        const float4 x = *reinterpret_cast<const float4*>(X + (t4 * 4 + e) * ldx), y = *reinterpret_cast<const float4*>(Y + (e * (ROWS / 4) + t4) * LDC);
+        const float xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w};
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(xs[i], ys[j], acc[i][j]);
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) part[i][j] = fmaf(xs[i], ys[j], part[i][j]);
+      }
     }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][j] += part[i][j];
   }
 }
 // Rows 4 q .. + 3 of a tile.
@@ -447,6 +480,7 @@ __global__ void __launch_bounds__(THREADS, 1) channel_walk_kernel(const ChannelA
     if (!odd) {
       product<C>(read, at + quarter * B * C + q4 * 4, C, D + place_of<C>(quarter * B) + c4, B);
     } else {                                          // a row u is not finite: A's zeros would make NaN of it, so only the rows that a row sees
+      float sum[4][4] = {};                           // (in the same order, for the same bits)
 #pragma unroll 1
       for (int j = quarter * B; j < min(quarter * B + B, q4 * 4 + 4); ++j) {
         const float4 x = *reinterpret_cast<const float4*>(at + j * C + q4 * 4), y = *reinterpret_cast<const float4*>(D + place_of<C>(j) + c4);
@@ -455,9 +489,13 @@ __global__ void __launch_bounds__(THREADS, 1) channel_walk_kernel(const ChannelA
         for (int i = 0; i < 4; ++i)
           if (j <= q4 * 4 + i) {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) read[i][e] = fmaf(xs[i], ys[e], read[i][e]);
+            for (int e = 0; e < 4; ++e) sum[i][e] = fmaf(xs[i], ys[e], sum[i][e]);
           }
       }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) read[i][e] += sum[i][e];
     }
     // (delta rule: the threads of group 0 with rows from 64 on hold (q B)^T S: they are the second quarter, for the same rows and columns)
     if (DELTA && quarter == 1) {
