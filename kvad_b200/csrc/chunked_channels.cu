@@ -37,7 +37,8 @@ struct ChannelArgs {
   const float* gates; int64_t ld_gates;        // [rows, heads * dk]: the decays
   const float* beta; int64_t ld_beta;          // [rows, heads], or null: the gated linear kind
   const int* seq_starts; const int* seq_slots;
-  int n_seqs, heads, group, dk, dv, places;
+  int n_seqs, heads, group, dk, dv;
+  int place0, places;       // the span of the list of chunks that the scratch holds: its first place, how many (see chunked_recurrence.cu)
   float q_scale;
   float* wq;          // [places, heads, DK, 128]: columns 0..63 W (delta rule), 64..127 q B, transposed
   float* kt;          // [places, heads, 64, DK]: keys decayed to the chunk's end
@@ -127,7 +128,7 @@ __global__ void __launch_bounds__(THREADS, 2) channel_prepare_kernel(const Chann
   pdl_launch_dependents();
   pdl_wait();
   const int h = blockIdx.y, qh = h / a.group, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const Place p = find(a, blockIdx.x);
+  const Place p = find(a, a.place0 + blockIdx.x);
   if (p.n == 0) return;
   const int64_t at = (int64_t)blockIdx.x * a.heads + h;
   for (int i = tid; i < 2 * C * LDT; i += THREADS) As[i] = 0.f;
@@ -401,7 +402,9 @@ __global__ void __launch_bounds__(THREADS, 1) channel_walk_kernel(const ChannelA
   const int s = blockIdx.x / a.heads, h = blockIdx.x - s * a.heads, c0 = blockIdx.y * COLS, tid = threadIdx.x;
   const int start = a.seq_starts[s], n_new = a.seq_starts[s + 1] - start;
   if (n_new <= 0) return;
-  const int n_chunks = (n_new + C - 1) / C, first = start / C + s;
+  // the chunks that lie in the span, and where chunk 0 would lie in its scratch
+  const int n_chunks = (n_new + C - 1) / C, first = start / C + s - a.place0, c_begin = max(0, -first), c_end = min(n_chunks, a.places - first);
+  if (c_begin >= c_end) return;
   float* st = a.state + (int64_t)a.seq_slots[s] * a.state_stride + (int64_t)h * a.dv * a.dk;
   for (int i = tid; i < DK * COLS; i += THREADS) {
     const int c = i / DK, d = i - c * DK;
@@ -426,8 +429,8 @@ __global__ void __launch_bounds__(THREADS, 1) channel_walk_kernel(const ChannelA
   const int group = tid >> 7;                         // halves of a sum
   const int r4 = tid & 31, c4 = ((tid >> 5) & 3) * 4;
   const int q4 = tid & 15, quarter = (tid >> 4 & 1) + 2 * group;      // 64 rows: quarters of a sum
-  bring_wq(0);
-  for (int c = 0; c < n_chunks; ++c) {
+  bring_wq(c_begin);
+  for (int c = c_begin; c < c_end; ++c) {
     const int64_t place = (int64_t)(first + c) * a.heads + h;
     const int n = min(C, n_new - c * C), row0 = start + c * C;
     bring_rest(c);                                    // on its way under the first product
@@ -466,7 +469,7 @@ __global__ void __launch_bounds__(THREADS, 1) channel_walk_kernel(const ChannelA
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     // u lies, keys and A are there, W and q B have been used up
     const bool odd = __syncthreads_or(given[0] * 0.f + given[1] * 0.f + given[2] * 0.f + given[3] * 0.f != 0.f);
-    if (c + 1 < n_chunks) bring_wq(c + 1);
+    if (c + 1 < c_end) bring_wq(c + 1);
     // the state: S' = B S + K^T u, a half of the rows a group
     float add[4][4] = {};
     if (r4 * 4 < DK) product<C>(add, kt + group * 32 * DK + r4 * 4, DK, D + place_of<C>(group * 32) + c4, 32);
@@ -538,7 +541,7 @@ __global__ void __launch_bounds__(THREADS, 1) channel_walk_kernel(const ChannelA
 }
 
 template <typename TI, int DK, bool DELTA>
-int launch(const ChannelArgs& a, cudaStream_t stream) {
+int launch(ChannelArgs a, int span, cudaStream_t stream) {
   constexpr size_t prepare_smem = ((size_t)4 * HD * LDT + 2 * C * LDT + 4 * HD) * 4;
   constexpr size_t walk_smem = ((size_t)DK * (DELTA ? 128 : 64) + C * DK + C * C + 2 * DK * LDC + 4 * C * LDC) * 4;
   static bool configured = false;
@@ -548,16 +551,20 @@ int launch(const ChannelArgs& a, cudaStream_t stream) {
     if (e != cudaSuccess) KVAD_FAIL(KVAD_ERR_CUDA, "chunked channels: cannot reserve shared memory: %s", cudaGetErrorString(e));
     configured = true;
   }
-  kvad_launch(channel_prepare_kernel<TI, DK, DELTA>, dim3(a.places, a.heads), dim3(THREADS), prepare_smem, stream, a);
-  kvad_launch(channel_walk_kernel<TI, DK, DELTA>, dim3(a.n_seqs * a.heads, (a.dv + COLS - 1) / COLS), dim3(THREADS), walk_smem, stream, a);
+  const int total = a.places;
+  for (a.place0 = 0; a.place0 < total; a.place0 += span) {
+    a.places = total - a.place0 < span ? total - a.place0 : span;
+    kvad_launch(channel_prepare_kernel<TI, DK, DELTA>, dim3(a.places, a.heads), dim3(THREADS), prepare_smem, stream, a);
+    kvad_launch(channel_walk_kernel<TI, DK, DELTA>, dim3(a.n_seqs * a.heads, (a.dv + COLS - 1) / COLS), dim3(THREADS), walk_smem, stream, a);
+  }
   KVAD_CHECK_LAUNCH("chunked channels");
   return KVAD_OK;
 }
 
 template <typename TI>
-int dispatch(const ChannelArgs& a, bool delta, cudaStream_t stream) {
-  if (a.dk <= 64) return delta ? launch<TI, 64, true>(a, stream) : launch<TI, 64, false>(a, stream);
-  return delta ? launch<TI, 128, true>(a, stream) : launch<TI, 128, false>(a, stream);
+int dispatch(const ChannelArgs& a, bool delta, int span, cudaStream_t stream) {
+  if (a.dk <= 64) return delta ? launch<TI, 64, true>(a, span, stream) : launch<TI, 64, false>(a, span, stream);
+  return delta ? launch<TI, 128, true>(a, span, stream) : launch<TI, 128, false>(a, span, stream);
 }
 
 inline int64_t work_per(int dk, int dv) {
@@ -567,17 +574,17 @@ inline int64_t work_per(int dk, int dv) {
 
 }  // namespace
 
-// Scratch in floats for one chunk of one head; `n` rows of `s` sequences are n / 64 + s chunks at most.
+// Scratch in floats for one chunk of one head; `n` rows of `s` sequences are n / 64 + s places of chunks, and `work` holds `span` of them at a time.
 KVAD_EXPORT int kvad_channels_work(int dk, int dv) { return (int)work_per(dk, dv); }
 
 // The gated delta rule (`beta` given) or the gated linear kind over prompt rows; `gates` are the decays themselves (see kvad_gated_recurrence).
 KVAD_EXPORT int kvad_channels_chunked(int dtype, const void* q, int64_t ld_q, const void* k, int64_t ld_k, const void* v, int64_t ld_v, const float* gates,
                                       int64_t ld_gates, const float* beta, int64_t ld_beta, float* out, int64_t ld_out, int n_rows, float* state,
                                       int64_t state_stride, const int* seq_starts, const int* seq_slots, int n_seqs, int heads, int kv_heads, int dk, int dv,
-                                      float q_scale, float* work, cudaStream_t stream) {
+                                      float q_scale, float* work, int span, cudaStream_t stream) {
   KVAD_REQUIRE(n_rows >= 0 && n_seqs > 0 && heads > 0 && kv_heads > 0 && heads % kv_heads == 0 && dk > 0 && dv > 0, "chunked channels: bad sizes seqs=%d heads=%d dk=%d dv=%d",
                n_seqs, heads, dk, dv);
-  KVAD_REQUIRE(q && k && v && gates && out && state && seq_starts && seq_slots && work, "chunked channels: bad arguments");
+  KVAD_REQUIRE(q && k && v && gates && out && state && seq_starts && seq_slots && work && span > 0, "chunked channels: bad arguments");
   KVAD_REQUIRE(heads <= 65535 && (int64_t)n_seqs * heads < (1ll << 31) && (dv + COLS - 1) / COLS <= 65535, "chunked channels: more than one launch takes");
   const uintptr_t unit = dtype == KVAD_DTYPE_F32 ? 15 : 7;
   if (dk > 128 || dk % 4 || ld_q % 4 || ld_k % 4 || ld_gates % 4 || ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k)) & unit) ||
@@ -587,14 +594,14 @@ KVAD_EXPORT int kvad_channels_chunked(int dtype, const void* q, int64_t ld_q, co
   a.q = q; a.k = k; a.v = v; a.ld_q = ld_q; a.ld_k = ld_k; a.ld_v = ld_v; a.gates = gates; a.ld_gates = ld_gates; a.beta = beta; a.ld_beta = ld_beta;
   a.seq_starts = seq_starts; a.seq_slots = seq_slots; a.n_seqs = n_seqs; a.heads = heads; a.group = heads / kv_heads; a.dk = dk; a.dv = dv;
   a.places = n_rows / C + n_seqs; a.q_scale = q_scale; a.out = out; a.ld_out = ld_out; a.state = state; a.state_stride = state_stride;
-  const int64_t DK = dk <= 64 ? 64 : 128, places = (int64_t)a.places * heads;
+  const int64_t DK = dk <= 64 ? 64 : 128, places = (int64_t)span * heads;
   a.wq = work;
   a.kt = a.wq + places * DK * 128;
   a.at = a.kt + places * C * DK;
   a.whole = a.at + places * C * C;
   a.x = a.whole + places * DK;
-  if (dtype == KVAD_DTYPE_F32) return dispatch<float>(a, beta != nullptr, stream);
-  if (dtype == KVAD_DTYPE_BF16) return dispatch<__nv_bfloat16>(a, beta != nullptr, stream);
+  if (dtype == KVAD_DTYPE_F32) return dispatch<float>(a, beta != nullptr, span, stream);
+  if (dtype == KVAD_DTYPE_BF16) return dispatch<__nv_bfloat16>(a, beta != nullptr, span, stream);
   KVAD_FAIL(KVAD_ERR_UNSUPPORTED, "chunked channels: unknown dtype %d", dtype);
 }
 

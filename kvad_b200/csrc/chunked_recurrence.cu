@@ -19,7 +19,8 @@
 // Measured: 2 x 1024 rows of 8 heads of 128 x 128 (rotated, normed, gated, bfloat16) 387 -> 85 us; the matrix memory over 1000 + 517 + 37 rows of 8
 // heads of 64 x 128 334 -> 50 us.  (92 and 53 before the state came a piece ahead by way of registers and rows by whole sectors.)
 //
-// Chunks of all sequences lie in one list: chunk c of sequence s is place seq_starts[s] / 64 + s + c, which never collides.
+// Chunks of all sequences lie in one list: chunk c of sequence s is place seq_starts[s] / 64 + s + c, which never collides.  The list is taken in
+// spans of as many places as the scratch holds, one after another: the sequences' own states carry over from one to the next.
 #include "common.cuh"
 
 using namespace kvad;
@@ -36,7 +37,8 @@ struct ChunkArgs {
   const void* q; const void* k; const void* v;
   int64_t ld_q, ld_k, ld_v;
   const int* seq_starts; const int* kv_lens; const int* seq_slots;
-  int n_seqs, heads, group, dk, dv, places;
+  int n_seqs, heads, group, dk, dv;
+  int place0, places;       // the span: its first place, how many
   float* work;              // [places, heads, dk * dv]: U of a chunk, then the state before it (in the state's own order of entries)
   float* state; int64_t state_stride;
   // retention
@@ -76,6 +78,18 @@ __device__ __forceinline__ Place find(const ChunkArgs& a, int place) {
   p.n = max(0, min(C, n_new - first));
   p.pos0 = a.kv_lens != nullptr ? a.kv_lens[lo] - n_new + first : 0;
   return p;
+}
+// The chunks of sequence `s` that lie in the span: from `begin` up to `end`, and where chunk 0 would lie in the span's scratch.
+struct Run { int begin, end, n_new, n_chunks, base; };
+__device__ __forceinline__ Run run_of(const ChunkArgs& a, int s) {
+  Run r;
+  const int start = a.seq_starts[s];
+  r.n_new = a.seq_starts[s + 1] - start;
+  r.n_chunks = r.n_new > 0 ? (r.n_new + C - 1) / C : 0;
+  r.base = start / C + s - a.place0;
+  r.begin = max(0, -r.base);
+  r.end = min(r.n_chunks, a.places - r.base);
+  return r;
 }
 
 // The matrix memory's gates of a chunk's rows, by the block's first 64 threads: F (the forget gates' logarithms summed up from the chunk's
@@ -195,7 +209,7 @@ __global__ void __launch_bounds__(THREADS) chunk_sum_kernel(const ChunkArgs a) {
   pdl_launch_dependents();
   pdl_wait();
   const int h = blockIdx.y, qh = h / a.group;
-  const Place p = find(a, blockIdx.x);
+  const Place p = find(a, a.place0 + blockIdx.x);
   if (p.n == 0) return;
   const bool half = KIND == RETENTION && a.rot_dims > 0;
   bring<TI, false>(ks, DK, (const TI*)a.k + qh * a.dk, a.ld_k, p, a.dk, DK, KIND == RETENTION && a.act, a.k_scale, a.rot_dims);
@@ -259,9 +273,9 @@ __global__ void __launch_bounds__(THREADS) chunk_scan_kernel(const ChunkArgs a) 
   pdl_launch_dependents();
   pdl_wait();
   const int s = blockIdx.x / a.heads, h = blockIdx.x - s * a.heads;
-  const int start = a.seq_starts[s], n_new = a.seq_starts[s + 1] - start;
-  if (n_new <= 0) return;
-  const int n_chunks = (n_new + C - 1) / C, entries = a.dk * a.dv, first = start / C + s;
+  const Run run = run_of(a, s);
+  if (run.begin >= run.end) return;
+  const int entries = a.dk * a.dv;
   const int at = (blockIdx.y * THREADS + threadIdx.x) * 4;
   float* slot = a.state + (int64_t)a.seq_slots[s] * a.state_stride;
   float* st = slot + (int64_t)h * entries;
@@ -275,15 +289,15 @@ __global__ void __launch_bounds__(THREADS) chunk_scan_kernel(const ChunkArgs a) 
   const float lambda = KIND == RETENTION ? a.decay[h] : 0.f;
   const float whole = KIND == RETENTION ? powf(lambda, (float)C) : 0.f;
   const int64_t step = (int64_t)a.heads * entries, n_step = (int64_t)a.heads * (a.dk + 2);
-  float* w = a.work + (int64_t)first * step + (int64_t)h * entries + at;
-  float* wn = KIND == MEMORY ? a.work_n + (int64_t)first * n_step + (int64_t)h * (a.dk + 2) : nullptr;
+  float* w = a.work + (int64_t)run.base * step + (int64_t)h * entries + at;
+  float* wn = KIND == MEMORY ? a.work_n + (int64_t)run.base * n_step + (int64_t)h * (a.dk + 2) : nullptr;
   constexpr int AHEAD = 8;
-  for (int c0 = 0; c0 < n_chunks; c0 += AHEAD) {
+  for (int c0 = run.begin; c0 < run.end; c0 += AHEAD) {
     float4 u[AHEAD];
     float f[AHEAD], top[AHEAD], un[AHEAD];
 #pragma unroll
     for (int i = 0; i < AHEAD; ++i) {
-      const bool in = c0 + i < n_chunks;
+      const bool in = c0 + i < run.end;
       u[i] = in && mine ? *reinterpret_cast<const float4*>(w + (c0 + i) * step) : make_float4(0.f, 0.f, 0.f, 0.f);
       if (KIND == MEMORY) {
         f[i] = in ? wn[(c0 + i) * n_step + a.dk] : 0.f;
@@ -294,7 +308,7 @@ __global__ void __launch_bounds__(THREADS) chunk_scan_kernel(const ChunkArgs a) 
 #pragma unroll
     for (int i = 0; i < AHEAD; ++i) {
       const int c = c0 + i;
-      if (c >= n_chunks) break;
+      if (c >= run.end) break;
       float keep = whole, take = 1.f;
       if (mine) *reinterpret_cast<float4*>(w + c * step) = S;
       if (KIND == MEMORY) {
@@ -302,11 +316,11 @@ __global__ void __launch_bounds__(THREADS) chunk_scan_kernel(const ChunkArgs a) 
         keep = expf(f[i] + m - next);
         take = expf(top[i] - next);
         if (norm) wn[c * n_step + threadIdx.x] = N;
-        if (blockIdx.y == 0 && threadIdx.x == 0) a.work_m[(int64_t)(first + c) * a.heads + h] = m;
+        if (blockIdx.y == 0 && threadIdx.x == 0) a.work_m[(int64_t)(run.base + c) * a.heads + h] = m;
         m = next;
         N = fmaf(keep, N, take * un[i]);
-      } else if (c == n_chunks - 1) {
-        keep = powf(lambda, (float)(n_new - c * C));
+      } else if (c == run.n_chunks - 1) {
+        keep = powf(lambda, (float)(run.n_new - c * C));
       }
       S.x = fmaf(keep, S.x, take * u[i].x);
       S.y = fmaf(keep, S.y, take * u[i].y);
@@ -325,9 +339,9 @@ __global__ void chunk_max_kernel(const ChunkArgs a) {
   pdl_launch_dependents();
   pdl_wait();
   const int s = blockIdx.x;
-  const int start = a.seq_starts[s], n_new = a.seq_starts[s + 1] - start;
-  if (n_new <= 0) return;
-  const int last = start / C + s + (n_new + C - 1) / C - 1;
+  const Run run = run_of(a, s);
+  if (run.begin >= run.end) return;
+  const int last = run.base + run.end - 1;
   float* slot = a.state + (int64_t)a.seq_slots[s] * a.state_stride + (int64_t)a.heads * a.dk * a.dv + (int64_t)a.heads * a.tiles * a.dk;
   for (int h = threadIdx.x; h < a.heads; h += blockDim.x) {
     const float* end = a.work_n + ((int64_t)last * a.heads + h) * (a.dk + 2) + a.dk;
@@ -352,7 +366,7 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_read_kernel(const ChunkArgs 
   pdl_launch_dependents();
   pdl_wait();
   const int h = blockIdx.y, qh = h / a.group;
-  const Place p = find(a, blockIdx.x);
+  const Place p = find(a, a.place0 + blockIdx.x);
   if (p.n == 0) return;
   const bool act = KIND == RETENTION && a.act;
   bring<TI, true>(qt, LDT, (const TI*)a.q + qh * a.dk, a.ld_q, p, a.dk, DK, act, a.q_scale, 0);
@@ -534,7 +548,7 @@ int room(K kernel, size_t smem) {
 }
 
 template <int KIND, typename TI, int DK, int DV>
-int launch(const ChunkArgs& a, cudaStream_t stream) {
+int launch(ChunkArgs a, int span, cudaStream_t stream) {
   constexpr size_t sum_smem = (size_t)C * (DK + DV) * 4;
   constexpr int LDS = DV + 4, region = DK * LDT > C * LDT + 32 * LDS ? DK * LDT : C * LDT + 32 * LDS;
   constexpr size_t read_smem = ((size_t)DK * LDT + region + C * DV) * 4;
@@ -546,23 +560,28 @@ int launch(const ChunkArgs& a, cudaStream_t stream) {
     configured = true;
   }
   const int entries = a.dk * a.dv;
-  kvad_launch(chunk_sum_kernel<KIND, TI, DK, DV>, dim3(a.places, a.heads), dim3(THREADS), sum_smem, stream, a);
-  kvad_launch(chunk_scan_kernel<KIND>, dim3(a.n_seqs * a.heads, (entries / 4 + THREADS - 1) / THREADS), dim3(THREADS), 0, stream, a);
-  if (KIND == MEMORY) kvad_launch(chunk_max_kernel, dim3(a.n_seqs), dim3(64), 0, stream, a);
-  kvad_launch(chunk_read_kernel<KIND, TI, DK, DV>, dim3(a.places, a.heads), dim3(THREADS), read_smem, stream, a);
+  const int total = a.places;
+  for (a.place0 = 0; a.place0 < total; a.place0 += span) {
+    a.places = total - a.place0 < span ? total - a.place0 : span;
+    kvad_launch(chunk_sum_kernel<KIND, TI, DK, DV>, dim3(a.places, a.heads), dim3(THREADS), sum_smem, stream, a);
+    kvad_launch(chunk_scan_kernel<KIND>, dim3(a.n_seqs * a.heads, (entries / 4 + THREADS - 1) / THREADS), dim3(THREADS), 0, stream, a);
+    if (KIND == MEMORY) kvad_launch(chunk_max_kernel, dim3(a.n_seqs), dim3(64), 0, stream, a);
+    kvad_launch(chunk_read_kernel<KIND, TI, DK, DV>, dim3(a.places, a.heads), dim3(THREADS), read_smem, stream, a);
+  }
   KVAD_CHECK_LAUNCH("chunked recurrence");
   return KVAD_OK;
 }
 
 template <int KIND, typename TI>
-int dispatch(const ChunkArgs& a, cudaStream_t stream) {
-  if (a.dk <= 64) return a.dv <= 64 ? launch<KIND, TI, 64, 64>(a, stream) : launch<KIND, TI, 64, 128>(a, stream);
-  return a.dv <= 64 ? launch<KIND, TI, 128, 64>(a, stream) : launch<KIND, TI, 128, 128>(a, stream);
+int dispatch(const ChunkArgs& a, int span, cudaStream_t stream) {
+  if (a.dk <= 64) return a.dv <= 64 ? launch<KIND, TI, 64, 64>(a, span, stream) : launch<KIND, TI, 64, 128>(a, span, stream);
+  return a.dv <= 64 ? launch<KIND, TI, 128, 64>(a, span, stream) : launch<KIND, TI, 128, 128>(a, span, stream);
 }
 
-int check(const ChunkArgs& a, int dtype, int n_rows) {
+int check(const ChunkArgs& a, int dtype, int n_rows, int span) {
   const uintptr_t unit = dtype == KVAD_DTYPE_F32 ? 15 : 7;
   KVAD_REQUIRE(a.n_seqs > 0 && a.heads > 0 && a.dk > 0 && a.dv > 0 && n_rows >= 0, "chunked recurrence: bad sizes seqs=%d heads=%d dk=%d dv=%d", a.n_seqs, a.heads, a.dk, a.dv);
+  KVAD_REQUIRE(span > 0, "chunked recurrence: scratch for no chunk at all");
   KVAD_REQUIRE(a.state && a.seq_starts && a.seq_slots && a.work, "chunked recurrence: needs state, sequences and scratch");
   KVAD_REQUIRE(a.heads <= 65535 && (int64_t)a.n_seqs * a.heads < (1ll << 31), "chunked recurrence: %d sequences x %d heads are more than one launch takes", a.n_seqs, a.heads);
   if (a.dk > 128 || a.dv > 128 || a.dk % 4 || a.dv % 4 || a.ld_q % 4 || a.ld_k % 4 || a.ld_v % 4 ||
@@ -577,46 +596,46 @@ int check(const ChunkArgs& a, int dtype, int n_rows) {
 // Places of chunks that `n_rows` rows of `n_seqs` sequences may take.
 KVAD_EXPORT int kvad_chunk_places(int n_rows, int n_seqs) { return n_rows / C + n_seqs; }
 
-// Retention of prompt rows (see kvad_retention for the arguments).  `work`: float32 [places, heads, dk, dv].  With `finish` the rows of `out` are
+// Retention of prompt rows (see kvad_retention for the arguments).  `work`: float32 [span, heads, dk, dv] for `span` places at a time.  With `finish` the rows of `out` are
 // written, else the 32-bit read-outs [rows, heads * dv] to `raw`.
 KVAD_EXPORT int kvad_retention_chunked(int dtype, const void* q, int64_t ld_q, const void* k, int64_t ld_k, const void* v, int64_t ld_v, const void* gate,
                                        int64_t ld_gate, void* out, int64_t ld_out, float* raw, int n_rows, float* state, const int* seq_starts,
                                        const int* kv_lens, const int* seq_slots, const float* decay, const float* inv_freq, int rot_dims,
                                        int interleaved, int n_seqs, int heads, int dk, int dv, float k_scale, float eps, int unit_norm, int act,
-                                       int finish, float* work, cudaStream_t stream) {
+                                       int finish, float* work, int span, cudaStream_t stream) {
   ChunkArgs a = {};
   a.q = q; a.k = k; a.v = v; a.ld_q = ld_q; a.ld_k = ld_k; a.ld_v = ld_v; a.seq_starts = seq_starts; a.kv_lens = kv_lens; a.seq_slots = seq_slots;
   a.n_seqs = n_seqs; a.heads = heads; a.group = 1; a.dk = dk; a.dv = dv; a.places = kvad_chunk_places(n_rows, n_seqs); a.work = work;
   a.state = state; a.state_stride = (int64_t)heads * dk * dv; a.decay = decay; a.inv_freq = inv_freq; a.rot_dims = inv_freq != nullptr ? rot_dims : 0;
   a.interleaved = interleaved; a.act = act; a.k_scale = k_scale; a.q_scale = 1.f; a.raw = finish ? nullptr : raw; a.ld_raw = (int64_t)heads * dv;
   a.out = out; a.ld_out = ld_out; a.gate = gate; a.ld_gate = ld_gate; a.unit_norm = unit_norm; a.finish = finish; a.eps = eps;
-  int rc = check(a, dtype, n_rows);
+  int rc = check(a, dtype, n_rows, span);
   if (rc != KVAD_OK) return rc;
   KVAD_REQUIRE(kv_lens && decay && (finish ? out != nullptr : raw != nullptr), "retention (chunked): bad arguments");
   KVAD_REQUIRE(rot_dims >= 0 && rot_dims % 2 == 0 && rot_dims <= dk, "retention (chunked): %d rotated entries of %d", rot_dims, dk);
   const uintptr_t unit = dtype == KVAD_DTYPE_F32 ? 15 : 7;
   if (gate != nullptr && (ld_gate % 4 || (reinterpret_cast<uintptr_t>(gate) & unit)))
     KVAD_FAIL(KVAD_ERR_UNSUPPORTED, "retention (chunked): the gate comes in whole quads");
-  if (dtype == KVAD_DTYPE_F32) return dispatch<RETENTION, float>(a, stream);
-  if (dtype == KVAD_DTYPE_BF16) return dispatch<RETENTION, __nv_bfloat16>(a, stream);
+  if (dtype == KVAD_DTYPE_F32) return dispatch<RETENTION, float>(a, span, stream);
+  if (dtype == KVAD_DTYPE_BF16) return dispatch<RETENTION, __nv_bfloat16>(a, span, stream);
   KVAD_FAIL(KVAD_ERR_UNSUPPORTED, "retention (chunked): unknown dtype %d", dtype);
 }
 
-// The matrix memory over prompt rows (see kvad_gated_recurrence).  `work`: float32 [places, heads, dk * dv]; `work_n`: float32 places x heads x (dk + 3).
+// The matrix memory over prompt rows (see kvad_gated_recurrence).  `work`: float32 [span, heads, dk * dv]; `work_n`: float32 span x heads x (dk + 3).
 KVAD_EXPORT int kvad_matrix_memory_chunked(int dtype, const void* q, int64_t ld_q, const void* k, int64_t ld_k, const void* v, int64_t ld_v, const float* gates,
                                            int64_t ld_gates, float* out, int64_t ld_out, int n_rows, float* state, int64_t state_stride, const int* seq_starts,
                                            const int* seq_slots, int n_seqs, int heads, int kv_heads, int dk, int dv, float q_scale, float cap, float* work,
-                                           float* work_n, cudaStream_t stream) {
+                                           float* work_n, int span, cudaStream_t stream) {
   KVAD_REQUIRE(kv_heads > 0 && heads % kv_heads == 0 && gates && work_n && out, "matrix memory (chunked): bad arguments");
   ChunkArgs a = {};
   a.q = q; a.k = k; a.v = v; a.ld_q = ld_q; a.ld_k = ld_k; a.ld_v = ld_v; a.seq_starts = seq_starts; a.seq_slots = seq_slots;
   a.n_seqs = n_seqs; a.heads = heads; a.group = heads / kv_heads; a.dk = dk; a.dv = dv; a.places = kvad_chunk_places(n_rows, n_seqs); a.work = work;
   a.state = state; a.state_stride = state_stride; a.k_scale = 1.f; a.q_scale = q_scale; a.gates = gates; a.ld_gates = ld_gates; a.cap = cap;
-  a.work_n = work_n; a.work_m = work_n + (int64_t)a.places * heads * (dk + 2); a.tiles = (dv + 15) / 16; a.raw = out; a.ld_raw = ld_out;
-  int rc = check(a, dtype, n_rows);
+  a.work_n = work_n; a.work_m = work_n + (int64_t)span * heads * (dk + 2); a.tiles = (dv + 15) / 16; a.raw = out; a.ld_raw = ld_out;
+  int rc = check(a, dtype, n_rows, span);
   if (rc != KVAD_OK) return rc;
-  if (dtype == KVAD_DTYPE_F32) return dispatch<MEMORY, float>(a, stream);
-  if (dtype == KVAD_DTYPE_BF16) return dispatch<MEMORY, __nv_bfloat16>(a, stream);
+  if (dtype == KVAD_DTYPE_F32) return dispatch<MEMORY, float>(a, span, stream);
+  if (dtype == KVAD_DTYPE_BF16) return dispatch<MEMORY, __nv_bfloat16>(a, span, stream);
   KVAD_FAIL(KVAD_ERR_UNSUPPORTED, "matrix memory (chunked): unknown dtype %d", dtype);
 }
 

@@ -154,6 +154,7 @@ class Engine:
         self.use_graphs = model.graph_safe and not profile.enabled()
         self.max_graphs = 48            # captured step shapes kept (least recently used go first)
         self._graphs: "collections.OrderedDict" = collections.OrderedDict()
+        self._graph_pool = None         # what captured steps allocate and give back within the step is one piece of memory for all of them (they never run side by side)
         self._decode_plans: dict = {}
         self.h2d_bytes = 0          # bytes copied host -> device by steps and sampling (for measurement)
         self.d2h_bytes = 0
@@ -312,7 +313,9 @@ class Engine:
         torch.cuda.synchronize()
         graph = torch.cuda.CUDAGraph()
         before = ops_mod.launch_count()
-        with torch.cuda.graph(graph):
+        if self._graph_pool is None:
+            self._graph_pool = torch.cuda.graph_pool_handle()
+        with torch.cuda.graph(graph, pool=self._graph_pool):
             result = body()
         n_kernels = ops_mod.launch_count() - before
         self._graphs[key] = (graph, result, n_kernels)

@@ -142,15 +142,15 @@ _SIGNATURES = {
         "kvad_chunk_places": [c_int, c_int],
         "kvad_retention_chunked": [c_int, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64,
                                    c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
-                                   c_int, c_float, c_float, c_int, c_int, c_int, c_void_p, c_void_p],
+                                   c_int, c_float, c_float, c_int, c_int, c_int, c_void_p, c_int, c_void_p],
         "kvad_matrix_memory_chunked": [c_int, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_int,
                                        c_void_p, c_int64, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_void_p, c_void_p,
-                                       c_void_p],
+                                       c_int, c_void_p],
     },
     "chunked_channels": {
         "kvad_channels_work": [c_int, c_int],
         "kvad_channels_chunked": [c_int, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64,
-                                  c_int, c_void_p, c_int64, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p, c_void_p],
+                                  c_int, c_void_p, c_int64, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p, c_int, c_void_p],
     },
     "gated_recurrence": {
         "kvad_gated_recurrence": [c_int, c_int, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64,
@@ -1172,6 +1172,17 @@ class Ops:
     # 0.35 us a row of the longest sequence, the chunks' three kernels 35 .. 75 us for few chunks: 8 heads of 128 x 128, one sequence of 128
     # rows: 59 us walked, 74 in chunks; four of 245 + 23 + 153 + 76: 102 and 60.)
     CHUNK_MIN_ROWS = 160
+    # What the chunks of a step may take beside the model, at most: 64 KB a chunk of 64 rows and head of 128 x 128 (retention, the matrix memory), 148 KB
+    # (decays by channel).  Longer lists of chunks go in spans of equal length, one after another; a span of 128 MB keeps every SM busy (8 heads:
+    # 113 chunks by channel, 1808 blocks of two an SM).
+    CHUNK_WORK_BYTES = 128 << 20
+
+    def _chunk_span(self, n: int, n_seqs: int, per_place: int) -> tuple:
+        """How many places of chunks `n` rows take, how many of them a span holds (`per_place`: scratch of one, in bytes), how many spans there are."""
+        places = n // 64 + int(n_seqs)
+        spans = -(-places // max(1, self.CHUNK_WORK_BYTES // per_place))
+        span = -(-places // spans)
+        return span, -(-places // span)
 
     # -- retention ------------------------------------------------------------------------
     def retention(self, q, k, v, out, state, seq_starts, kv_lens, seq_slots, n_seqs: int, decay, n_heads: int, *, inv_freq=None,
@@ -1214,13 +1225,14 @@ class Ops:
                 and state.data_ptr() % 16 == 0 and (not raw_only or raw.data_ptr() % 16 == 0)):
             global _launches
             h = lib("chunked_recurrence")
-            work = torch.empty(h.kvad_chunk_places(n, int(n_seqs)) * n_heads * dk * dv, dtype=torch.float32, device=q.device)
+            span, spans = self._chunk_span(n, n_seqs, n_heads * dk * dv * 4)
+            work = torch.empty(span * n_heads * dk * dv, dtype=torch.float32, device=q.device)
             _check(h.kvad_retention_chunked(self.code, _ptr(q), ld_q, _ptr(k), ld_k, _ptr(v), ld_v, _ptr(gate), ld_g, _ptr(out), ld_o, _ptr(raw), n, _ptr(state),
                                             _ptr(seq_starts), _ptr(kv_lens), _ptr(seq_slots), _ptr(decay), _ptr(inv_freq), int(rot_dims),
                                             int(bool(interleaved)), int(n_seqs), int(n_heads), dk, dv, float(k_scale),
                                             float(unit_norm_eps or 0.0), 0 if unit_norm_eps is None else 1, int(bool(silu_inputs)), 0 if raw_only else 1,
-                                            _ptr(work), _stream()), h)
-            _launches += 2          # three kernels: the chunks' sums, the state from chunk to chunk, the read-outs
+                                            _ptr(work), span, _stream()), h)
+            _launches += 3 * spans - 1          # three kernels a span: the chunks' sums, the state from chunk to chunk, the read-outs
             return
         h = lib("retention")
         _check(h.kvad_retention(self.code, _ptr(q), ld_q, _ptr(k), ld_k, _ptr(v), ld_v, _ptr(gate), ld_g, _ptr(out), ld_o, _ptr(raw), n, _ptr(state),
@@ -1300,22 +1312,24 @@ class Ops:
                 and (ld_q | ld_k | ld_v | ld_o | state.stride(0)) % 4 == 0 and (q.data_ptr() | k.data_ptr() | v.data_ptr()) % (4 * E) == 0
                 and (state.data_ptr() | out.data_ptr()) % 16 == 0):
             h = lib("chunked_recurrence")
-            places = h.kvad_chunk_places(n, int(n_seqs))
-            work = torch.empty(places * n_heads * dk * dv, dtype=torch.float32, device=q.device)
-            work_n = torch.empty(places * n_heads * (dk + 3), dtype=torch.float32, device=q.device)
+            span, spans = self._chunk_span(n, n_seqs, n_heads * (dk * dv + dk + 3) * 4)
+            work = torch.empty(span * n_heads * dk * dv, dtype=torch.float32, device=q.device)
+            work_n = torch.empty(span * n_heads * (dk + 3), dtype=torch.float32, device=q.device)
             _check(h.kvad_matrix_memory_chunked(_code(q.dtype), _ptr(q), ld_q, _ptr(k), ld_k, _ptr(v), ld_v, _ptr(gates), ld_g, _ptr(out), ld_o, n, _ptr(state),
                                                 state.stride(0), _ptr(seq_starts), _ptr(seq_slots), int(n_seqs), int(n_heads), int(n_kv_heads), int(dk), int(dv),
-                                                float(q_scale), float(cap), _ptr(work), _ptr(work_n), _stream()), h)
-            _launches += 3          # four kernels: the chunks' sums, the state from chunk to chunk, the running maxima, the read-outs
+                                                float(q_scale), float(cap), _ptr(work), _ptr(work_n), span, _stream()), h)
+            _launches += 4 * spans - 1          # four kernels a span: the chunks' sums, the state from chunk to chunk, the running maxima, the read-outs
             return
         if (mode != 0 and gates_ready and self.chunked_recurrences and n >= self.CHUNK_MIN_ROWS * n_seqs and dk <= 128 and dk % 4 == 0
                 and (ld_q | ld_k | ld_g) % 4 == 0 and (q.data_ptr() | k.data_ptr()) % (4 * E) == 0 and gates.data_ptr() % 16 == 0):
             h = lib("chunked_channels")
-            work = torch.empty((n // 64 + int(n_seqs)) * int(n_heads) * h.kvad_channels_work(int(dk), int(dv)), dtype=torch.float32, device=q.device)
+            per_head = h.kvad_channels_work(int(dk), int(dv))
+            span, spans = self._chunk_span(n, n_seqs, int(n_heads) * per_head * 4)
+            work = torch.empty(span * int(n_heads) * per_head, dtype=torch.float32, device=q.device)
             _check(h.kvad_channels_chunked(_code(q.dtype), _ptr(q), ld_q, _ptr(k), ld_k, _ptr(v), ld_v, _ptr(gates), ld_g, _ptr(beta if mode == 1 else None), ld_b,
                                            _ptr(out), ld_o, n, _ptr(state), state.stride(0), _ptr(seq_starts), _ptr(seq_slots), int(n_seqs), int(n_heads),
-                                           int(n_kv_heads), int(dk), int(dv), float(q_scale), _ptr(work), _stream()), h)
-            _launches += 1          # two kernels: the chunks by themselves, the walk from chunk to chunk
+                                           int(n_kv_heads), int(dk), int(dv), float(q_scale), _ptr(work), span, _stream()), h)
+            _launches += 2 * spans - 1          # two kernels a span: the chunks by themselves, the walk from chunk to chunk
             return
         h = lib("gated_recurrence")
         _check(h.kvad_gated_recurrence(mode, _code(q.dtype), _ptr(q), ld_q, _ptr(k), ld_k, _ptr(v), ld_v, _ptr(gates), ld_g, _ptr(beta), ld_b,

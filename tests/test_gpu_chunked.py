@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 import torch
 
-from kvad_b200.ops import Ops
+from kvad_b200.ops import Ops, lib
 
 pytestmark = pytest.mark.gpu
 DT = {"float32": torch.float32, "bfloat16": torch.bfloat16}
@@ -291,3 +291,48 @@ def test_chunks_of_channel_decays_are_no_less_exact_than_the_walk(kind, H, dk, d
             sums[chunks][0] += rel(out.view(n, H, dv), want)
             sums[chunks][1] += rel(state[0][:H * dv * dk].view(H, dv, dk).transpose(1, 2), end)
     assert sums[True][0] < sums[False][0] * 1.15 and sums[True][1] < sums[False][1] * 1.12, sums
+
+
+@pytest.mark.parametrize("kind", ["retention", "matrix_memory", "delta_rule", "gated_linear"])
+def test_long_steps_go_in_spans_of_bounded_scratch(kind):
+    """A list of chunks in spans gives the bits that it gives at once, whatever the spans cut; and scratch stays within its bound however long the step."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(7)
+    H, dk, dv = 2, 64, 64
+    memory = kind == "matrix_memory"
+
+    def run(lens, budget=None):
+        g.manual_seed(sum(lens))
+        N, ops = sum(lens), Ops(torch.float32)
+        ops.CHUNK_MIN_ROWS = 1
+        if budget is not None:
+            ops.CHUNK_WORK_BYTES = budget
+        q, k, v = (torch.randn(N, H * d, generator=g, device="cuda") for d in (dk, dk, dv))
+        gates = torch.randn(N, 2 * H, generator=g, device="cuda") + 3.0 if memory else torch.sigmoid(torch.randn(N, H * dk, generator=g, device="cuda") + 3.0)
+        beta, decay = torch.sigmoid(torch.randn(N, H, generator=g, device="cuda")), torch.tensor([0.9, 0.97], device="cuda")
+        if kind == "delta_rule":
+            k = torch.nn.functional.normalize(k.view(N, H, dk), dim=-1).view(N, -1)
+        out, st, sl, n = torch.full((N, H * dv), float("nan"), device="cuda"), starts(lens), i32(list(range(len(lens)))), len(lens)
+        size = dk * dv * H if kind == "retention" else ops.recurrence_state_size(kind, H, dk, dv)
+        state = torch.randn(n, size, generator=g, device="cuda") if not memory else torch.zeros(n, size, device="cuda")
+        torch.cuda.synchronize()
+        torch.cuda.reset_peak_memory_stats()
+        before = torch.cuda.memory_allocated()
+        if kind == "retention":
+            ops.retention(q, k, v, None, state.view(n, H, dk, dv), st, i32(lens), sl, n, decay, H, raw=out, raw_only=True)
+        else:
+            more = {"delta_rule": dict(beta=beta, a_log=torch.zeros(H, device="cuda"), dt_bias=torch.zeros(H * dk, device="cuda"), gates_ready=True),
+                    "gated_linear": dict(gates_ready=True), "matrix_memory": dict(cap=15.0)}[kind]
+            ops.gated_recurrence(kind, q, k, v, gates, out, state, st, sl, n, H, H, dk, dv, **more)
+        torch.cuda.synchronize()
+        return out, state, torch.cuda.max_memory_allocated() - before
+
+    whole, end, _ = run(LENS)
+    per_place = H * (dk * dv + dk + 3) * 4 if memory else H * dk * dv * 4 if kind == "retention" else H * lib("chunked_channels").kvad_channels_work(dk, dv) * 4
+    for places in (1, 2, 5):
+        out, state, _ = run(LENS, places * per_place)
+        assert torch.equal(out, whole) and torch.equal(state, end)
+    budget = 16 * per_place
+    out, state, peak = run([20000, 1, 300], budget)
+    assert peak <= budget + (1 << 16), (peak, budget)
+    assert out.isfinite().all()
