@@ -38,6 +38,7 @@ struct ChannelArgs {
   const float* beta; int64_t ld_beta;          // [rows, heads], or null: the gated linear kind
   const int* seq_starts; const int* seq_slots;
   int n_seqs, heads, group, dk, dv;
+  int from;                 // only sequences of so many new rows or more (the others: gated_recurrence.cu)
   int place0, places;       // the span of the list of chunks that the scratch holds: its first place, how many (see chunked_recurrence.cu)
   float q_scale;
   float* wq;          // [places, heads, DK, 128]: columns 0..63 W (delta rule), 64..127 q B, transposed
@@ -61,7 +62,7 @@ __device__ __forceinline__ Place find(const ChannelArgs& a, int place) {
   const int start = a.seq_starts[lo], n_new = a.seq_starts[lo + 1] - start, first = (place - (start / C + lo)) * C;
   p.s = lo;
   p.row0 = start + first;
-  p.n = max(0, min(C, n_new - first));
+  p.n = n_new < a.from ? 0 : max(0, min(C, n_new - first));
   return p;
 }
 
@@ -401,7 +402,7 @@ __global__ void __launch_bounds__(THREADS, 1) channel_walk_kernel(const ChannelA
   pdl_wait();
   const int s = blockIdx.x / a.heads, h = blockIdx.x - s * a.heads, c0 = blockIdx.y * COLS, tid = threadIdx.x;
   const int start = a.seq_starts[s], n_new = a.seq_starts[s + 1] - start;
-  if (n_new <= 0) return;
+  if (n_new <= 0 || n_new < a.from) return;
   // the chunks that lie in the span, and where chunk 0 would lie in its scratch
   const int n_chunks = (n_new + C - 1) / C, first = start / C + s - a.place0, c_begin = max(0, -first), c_end = min(n_chunks, a.places - first);
   if (c_begin >= c_end) return;
@@ -581,7 +582,7 @@ KVAD_EXPORT int kvad_channels_work(int dk, int dv) { return (int)work_per(dk, dv
 KVAD_EXPORT int kvad_channels_chunked(int dtype, const void* q, int64_t ld_q, const void* k, int64_t ld_k, const void* v, int64_t ld_v, const float* gates,
                                       int64_t ld_gates, const float* beta, int64_t ld_beta, float* out, int64_t ld_out, int n_rows, float* state,
                                       int64_t state_stride, const int* seq_starts, const int* seq_slots, int n_seqs, int heads, int kv_heads, int dk, int dv,
-                                      float q_scale, float* work, int span, cudaStream_t stream) {
+                                      float q_scale, float* work, int span, int from, cudaStream_t stream) {
   KVAD_REQUIRE(n_rows >= 0 && n_seqs > 0 && heads > 0 && kv_heads > 0 && heads % kv_heads == 0 && dk > 0 && dv > 0, "chunked channels: bad sizes seqs=%d heads=%d dk=%d dv=%d",
                n_seqs, heads, dk, dv);
   KVAD_REQUIRE(q && k && v && gates && out && state && seq_starts && seq_slots && work && span > 0, "chunked channels: bad arguments");
@@ -593,7 +594,7 @@ KVAD_EXPORT int kvad_channels_chunked(int dtype, const void* q, int64_t ld_q, co
   ChannelArgs a = {};
   a.q = q; a.k = k; a.v = v; a.ld_q = ld_q; a.ld_k = ld_k; a.ld_v = ld_v; a.gates = gates; a.ld_gates = ld_gates; a.beta = beta; a.ld_beta = ld_beta;
   a.seq_starts = seq_starts; a.seq_slots = seq_slots; a.n_seqs = n_seqs; a.heads = heads; a.group = heads / kv_heads; a.dk = dk; a.dv = dv;
-  a.places = n_rows / C + n_seqs; a.q_scale = q_scale; a.out = out; a.ld_out = ld_out; a.state = state; a.state_stride = state_stride;
+  a.from = from; a.places = n_rows / C + n_seqs; a.q_scale = q_scale; a.out = out; a.ld_out = ld_out; a.state = state; a.state_stride = state_stride;
   const int64_t DK = dk <= 64 ? 64 : 128, places = (int64_t)span * heads;
   a.wq = work;
   a.kt = a.wq + places * DK * 128;

@@ -38,6 +38,7 @@ struct ChunkArgs {
   int64_t ld_q, ld_k, ld_v;
   const int* seq_starts; const int* kv_lens; const int* seq_slots;
   int n_seqs, heads, group, dk, dv;
+  int from;                 // only sequences of so many new rows or more (the others: retention.cu, gated_recurrence.cu)
   int place0, places;       // the span: its first place, how many
   float* work;              // [places, heads, dk * dv]: U of a chunk, then the state before it (in the state's own order of entries)
   float* state; int64_t state_stride;
@@ -75,7 +76,7 @@ __device__ __forceinline__ Place find(const ChunkArgs& a, int place) {
   const int start = a.seq_starts[lo], n_new = a.seq_starts[lo + 1] - start, first = (place - (start / C + lo)) * C;
   p.s = lo;
   p.row0 = start + first;
-  p.n = max(0, min(C, n_new - first));
+  p.n = n_new < a.from ? 0 : max(0, min(C, n_new - first));
   p.pos0 = a.kv_lens != nullptr ? a.kv_lens[lo] - n_new + first : 0;
   return p;
 }
@@ -85,7 +86,7 @@ __device__ __forceinline__ Run run_of(const ChunkArgs& a, int s) {
   Run r;
   const int start = a.seq_starts[s];
   r.n_new = a.seq_starts[s + 1] - start;
-  r.n_chunks = r.n_new > 0 ? (r.n_new + C - 1) / C : 0;
+  r.n_chunks = r.n_new >= a.from ? (r.n_new + C - 1) / C : 0;
   r.base = start / C + s - a.place0;
   r.begin = max(0, -r.base);
   r.end = min(r.n_chunks, a.places - r.base);
@@ -602,13 +603,14 @@ KVAD_EXPORT int kvad_retention_chunked(int dtype, const void* q, int64_t ld_q, c
                                        int64_t ld_gate, void* out, int64_t ld_out, float* raw, int n_rows, float* state, const int* seq_starts,
                                        const int* kv_lens, const int* seq_slots, const float* decay, const float* inv_freq, int rot_dims,
                                        int interleaved, int n_seqs, int heads, int dk, int dv, float k_scale, float eps, int unit_norm, int act,
-                                       int finish, float* work, int span, cudaStream_t stream) {
+                                       int finish, float* work, int span, int from, cudaStream_t stream) {
   ChunkArgs a = {};
   a.q = q; a.k = k; a.v = v; a.ld_q = ld_q; a.ld_k = ld_k; a.ld_v = ld_v; a.seq_starts = seq_starts; a.kv_lens = kv_lens; a.seq_slots = seq_slots;
   a.n_seqs = n_seqs; a.heads = heads; a.group = 1; a.dk = dk; a.dv = dv; a.places = kvad_chunk_places(n_rows, n_seqs); a.work = work;
   a.state = state; a.state_stride = (int64_t)heads * dk * dv; a.decay = decay; a.inv_freq = inv_freq; a.rot_dims = inv_freq != nullptr ? rot_dims : 0;
   a.interleaved = interleaved; a.act = act; a.k_scale = k_scale; a.q_scale = 1.f; a.raw = finish ? nullptr : raw; a.ld_raw = (int64_t)heads * dv;
   a.out = out; a.ld_out = ld_out; a.gate = gate; a.ld_gate = ld_gate; a.unit_norm = unit_norm; a.finish = finish; a.eps = eps;
+  a.from = from;
   int rc = check(a, dtype, n_rows, span);
   if (rc != KVAD_OK) return rc;
   KVAD_REQUIRE(kv_lens && decay && (finish ? out != nullptr : raw != nullptr), "retention (chunked): bad arguments");
@@ -625,13 +627,14 @@ KVAD_EXPORT int kvad_retention_chunked(int dtype, const void* q, int64_t ld_q, c
 KVAD_EXPORT int kvad_matrix_memory_chunked(int dtype, const void* q, int64_t ld_q, const void* k, int64_t ld_k, const void* v, int64_t ld_v, const float* gates,
                                            int64_t ld_gates, float* out, int64_t ld_out, int n_rows, float* state, int64_t state_stride, const int* seq_starts,
                                            const int* seq_slots, int n_seqs, int heads, int kv_heads, int dk, int dv, float q_scale, float cap, float* work,
-                                           float* work_n, int span, cudaStream_t stream) {
+                                           float* work_n, int span, int from, cudaStream_t stream) {
   KVAD_REQUIRE(kv_heads > 0 && heads % kv_heads == 0 && gates && work_n && out, "matrix memory (chunked): bad arguments");
   ChunkArgs a = {};
   a.q = q; a.k = k; a.v = v; a.ld_q = ld_q; a.ld_k = ld_k; a.ld_v = ld_v; a.seq_starts = seq_starts; a.seq_slots = seq_slots;
   a.n_seqs = n_seqs; a.heads = heads; a.group = heads / kv_heads; a.dk = dk; a.dv = dv; a.places = kvad_chunk_places(n_rows, n_seqs); a.work = work;
   a.state = state; a.state_stride = state_stride; a.k_scale = 1.f; a.q_scale = q_scale; a.gates = gates; a.ld_gates = ld_gates; a.cap = cap;
   a.work_n = work_n; a.work_m = work_n + (int64_t)span * heads * (dk + 2); a.tiles = (dv + 15) / 16; a.raw = out; a.ld_raw = ld_out;
+  a.from = from;
   int rc = check(a, dtype, n_rows, span);
   if (rc != KVAD_OK) return rc;
   if (dtype == KVAD_DTYPE_F32) return dispatch<MEMORY, float>(a, span, stream);

@@ -48,6 +48,7 @@ struct RecArgs {
   const int* seq_starts; const int* seq_slots;
   int heads, group, dk, dv, tiles;
   int gates_ready;                     // delta rule, gated linear: `gates` already holds the decays themselves (see decay_gate)
+  int below;                           // only sequences of fewer new rows than this (the others: chunked_recurrence.cu, chunked_channels.cu)
   float q_scale, cap, gate_rate;       // gate_rate: 1 / tau of the gated linear kind
 };
 
@@ -78,6 +79,7 @@ __global__ void __launch_bounds__(128) recurrence_kernel(const RecArgs p) {
   pdl_launch_dependents();
   pdl_wait();
   const int row0 = p.seq_starts[s], row1 = p.seq_starts[s + 1];
+  if (row1 - row0 >= p.below) return;
   float* st = p.state + (int64_t)p.seq_slots[s] * p.state_stride;
   const bool col_ok = col < dv;
   float* S_g = st + ((int64_t)h * dv + (col_ok ? col : 0)) * dk;
@@ -395,7 +397,7 @@ KVAD_EXPORT int kvad_gated_recurrence(int mode, int in_dtype, const void* q, int
                                       const void* a_log, const void* dt_bias, int params_f32, float* out, int64_t ld_out, float* state,
                                       int64_t state_stride, const int* seq_starts, const int* seq_slots, int n_seqs, int heads,
                                       int kv_heads, int dk, int dv, float q_scale, float cap, int gates_ready, float gate_rate,
-                                      cudaStream_t stream) {
+                                      int below, cudaStream_t stream) {
   KVAD_REQUIRE(heads > 0 && kv_heads > 0 && heads % kv_heads == 0 && dk > 0 && dv > 0 && n_seqs >= 0,
                "gated_recurrence: bad sizes heads=%d kv_heads=%d dk=%d dv=%d", heads, kv_heads, dk, dv);
   KVAD_REQUIRE(dk <= 512, "gated_recurrence: heads of up to 512 key entries, not %d", dk);
@@ -412,7 +414,7 @@ KVAD_EXPORT int kvad_gated_recurrence(int mode, int in_dtype, const void* q, int
   a.out = out; a.ld_out = ld_out; a.state = state; a.state_stride = state_stride;
   a.seq_starts = seq_starts; a.seq_slots = seq_slots;
   a.heads = heads; a.group = heads / kv_heads; a.dk = dk; a.dv = dv; a.tiles = (dv + COLS - 1) / COLS;
-  a.q_scale = q_scale; a.cap = cap; a.gates_ready = gates_ready; a.gate_rate = gate_rate;
+  a.q_scale = q_scale; a.cap = cap; a.gates_ready = gates_ready; a.gate_rate = gate_rate; a.below = below;
   if (in_dtype == KVAD_DTYPE_F32) {
     if (mode == 0) launch_recurrence<float, MEMORY>(a, n_seqs, stream);
     else if (mode == 1) launch_recurrence<float, DELTA>(a, n_seqs, stream);

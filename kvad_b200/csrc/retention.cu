@@ -41,6 +41,7 @@ struct RetentionArgs {
   float k_scale, eps;
   int unit_norm;
   int act;                              // 1: q, k and v pass a silu as they are staged
+  int below;                            // only sequences of fewer new rows than this (the others: chunked_recurrence.cu)
   int finish;                           // 0: only the raw 32-bit read-outs are written (to `raw`)
 };
 
@@ -93,6 +94,7 @@ __global__ void __launch_bounds__(256) retention_kernel(const RetentionArgs a) {
   pdl_wait();
   const int s = blockIdx.x, h = blockIdx.y, v_base = blockIdx.z * vc, tid = threadIdx.x, nthreads = blockDim.x;
   const int start = a.seq_starts[s], n_new = a.seq_starts[s + 1] - start;
+  if (n_new >= a.below) return;
   const int pos0 = a.kv_lens[s] - n_new;
   const int ci = tid / split, si = tid - ci * split;               // column pair, share of the key entries
   const int c0 = ci * VPT;                                          // first of the thread's columns, within the block's range
@@ -383,12 +385,13 @@ int dispatch_retention(RetentionArgs& a, int n_seqs, int n_rows, cudaStream_t st
 // 1 if heads of this shape have their value columns spread over blocks, so that kvad_retention needs `raw`.
 KVAD_EXPORT int kvad_retention_needs_raw(int dk, int dv) { return spread_of(dk, dv).fused ? 0 : 1; }
 
-// `raw`: float32 [rows, heads * dv] (see kvad_retention_needs_raw), `n_rows`: the step's rows.
+// `raw`: float32 [rows, heads * dv] (see kvad_retention_needs_raw), `n_rows`: the step's rows.  Sequences of `below` new rows or more are left alone; where
+// heads are spread over blocks, their rows of `out` are written with what `raw` holds, for the caller to write afterwards.
 KVAD_EXPORT int kvad_retention(int dtype, const void* q, int64_t ld_q, const void* k, int64_t ld_k, const void* v, int64_t ld_v,
                                const void* gate, int64_t ld_gate, void* out, int64_t ld_out, float* raw, int n_rows, float* state, const int* seq_starts,
                                const int* kv_lens, const int* seq_slots, const float* decay, const float* inv_freq, int rot_dims,
                                int interleaved, int n_seqs, int heads, int dk, int dv, float k_scale, float eps, int unit_norm,
-                               int act, int finish, cudaStream_t stream) {
+                               int act, int finish, int below, cudaStream_t stream) {
   KVAD_REQUIRE(n_seqs >= 0 && heads > 0 && dk > 0 && dv > 0, "retention: bad sizes seqs=%d heads=%d dk=%d dv=%d", n_seqs, heads, dk, dv);
   KVAD_REQUIRE(state != nullptr && decay != nullptr && seq_starts && kv_lens && seq_slots, "retention: needs state, decays and the step's sequences");
   KVAD_REQUIRE(rot_dims >= 0 && rot_dims % 2 == 0 && rot_dims <= dk, "retention: %d rotated entries of %d", rot_dims, dk);
@@ -398,7 +401,7 @@ KVAD_EXPORT int kvad_retention(int dtype, const void* q, int64_t ld_q, const voi
   a.q = q; a.k = k; a.v = v; a.gate = gate; a.ld_q = ld_q; a.ld_k = ld_k; a.ld_v = ld_v; a.ld_gate = ld_gate;
   a.out = out; a.ld_out = ld_out; a.raw = raw; a.vc = 0; a.fused = 1; a.vec = 0; a.state = state; a.seq_starts = seq_starts; a.kv_lens = kv_lens; a.seq_slots = seq_slots;
   a.decay = decay; a.inv_freq = rot_dims > 0 ? inv_freq : nullptr; a.rot_dims = rot_dims; a.interleaved = interleaved;
-  a.heads = heads; a.dk = dk; a.dv = dv; a.split = 1; a.k_scale = k_scale; a.eps = eps; a.unit_norm = unit_norm; a.act = act ? 1 : 0; a.finish = finish ? 1 : 0;
+  a.heads = heads; a.dk = dk; a.dv = dv; a.split = 1; a.k_scale = k_scale; a.eps = eps; a.unit_norm = unit_norm; a.act = act ? 1 : 0; a.finish = finish ? 1 : 0; a.below = below;
   KVAD_REQUIRE(finish || raw != nullptr, "retention: raw read-outs need the 32-bit scratch");
   if (dtype == KVAD_DTYPE_F32) return dispatch_retention<float>(a, n_seqs, n_rows, stream);
   if (dtype == KVAD_DTYPE_BF16) return dispatch_retention<__nv_bfloat16>(a, n_seqs, n_rows, stream);

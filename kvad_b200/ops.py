@@ -134,7 +134,7 @@ _SIGNATURES = {
     "retention": {
         "kvad_retention": [c_int, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64,
                            c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
-                           c_int, c_float, c_float, c_int, c_int, c_int, c_void_p],
+                           c_int, c_float, c_float, c_int, c_int, c_int, c_int, c_void_p],
         "kvad_retention_needs_raw": [c_int, c_int],
         "kvad_row_norm_gate": [c_int, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int, c_void_p, c_int64, c_int, c_int, c_float, c_void_p],
     },
@@ -142,20 +142,20 @@ _SIGNATURES = {
         "kvad_chunk_places": [c_int, c_int],
         "kvad_retention_chunked": [c_int, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64,
                                    c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
-                                   c_int, c_float, c_float, c_int, c_int, c_int, c_void_p, c_int, c_void_p],
+                                   c_int, c_float, c_float, c_int, c_int, c_int, c_void_p, c_int, c_int, c_void_p],
         "kvad_matrix_memory_chunked": [c_int, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_int,
                                        c_void_p, c_int64, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_void_p, c_void_p,
-                                       c_int, c_void_p],
+                                       c_int, c_int, c_void_p],
     },
     "chunked_channels": {
         "kvad_channels_work": [c_int, c_int],
         "kvad_channels_chunked": [c_int, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64,
-                                  c_int, c_void_p, c_int64, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p, c_int, c_void_p],
+                                  c_int, c_void_p, c_int64, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p, c_int, c_int, c_void_p],
     },
     "gated_recurrence": {
         "kvad_gated_recurrence": [c_int, c_int, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64,
                                   c_void_p, c_void_p, c_int, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_void_p, c_int, c_int, c_int,
-                                  c_int, c_int, c_float, c_float, c_int, c_float, c_void_p],
+                                  c_int, c_int, c_float, c_float, c_int, c_float, c_int, c_void_p],
         "kvad_gated_recurrence_state": [c_int, c_int, c_int, c_int],
         "kvad_decay_gate": [c_void_p, c_int64, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_void_p],
         "kvad_short_conv": [c_int, c_void_p, c_int64, c_void_p, c_void_p, c_int64, c_void_p, c_int64, c_int64, c_void_p, c_void_p, c_void_p,
@@ -1168,10 +1168,22 @@ class Ops:
         want = (int(per_sm) * (n_sms or sm_count())) // blocks
         return max(1, min(want, -(-reach // 64) + 1, 16))
 
-    # Recurrences of steps with so many rows a sequence, on average, are taken in chunks of 64 rows.  (By the step's shape only.  The walk takes
-    # 0.35 us a row of the longest sequence, the chunks' three kernels 35 .. 75 us for few chunks: 8 heads of 128 x 128, one sequence of 128
-    # rows: 59 us walked, 74 in chunks; four of 245 + 23 + 153 + 76: 102 and 60.)
+    # Recurrences of steps whose longest run of new rows is so long are taken in chunks of 64 rows.  (The walk takes 0.35 us a row of the longest
+    # sequence, the chunks' kernels 45 .. 75 us for few chunks.  8 heads of 128 x 128, us walked and in chunks: one sequence of 128 rows: retention 52, 65,
+    # matrix memory 57, 50, delta rule 59, 66; of 160: 64, 68; 71, 51; 74, 74; of 200: 82, 68; 87, 47; 91, 81; four of 245 + 23 + 153 + 76: 116, 70;
+    # 136, 65; 147, 101.)  Where the caller does not say how long it is, the average decides.
     CHUNK_MIN_ROWS = 160
+    # In such a step, sequences of fewer rows than this are walked all the same, by a launch of their own: what a decoding sequence gets does not
+    # depend on whether a prompt is beside it.  (1000 rows beside 8 single ones, all walked, all in chunks, and so: retention 450 us, 75, 92; matrix memory
+    # 511, 72, 76; delta rule 542, 179, 158.)
+    CHUNK_SHORT_ROWS = 16
+
+    def _chunk_rule(self, n: int, n_seqs: int, max_new: Optional[int]) -> tuple:
+        """Whether a step of `n` rows goes in chunks, and below how many new rows a sequence of it is walked all the same (0: none is, or none may be)."""
+        if not self.chunked_recurrences or n_seqs < 1 or (n < self.CHUNK_MIN_ROWS * n_seqs if max_new is None else max_new < self.CHUNK_MIN_ROWS):
+            return False, 0
+        return True, 0 if max_new is None or n == n_seqs * max_new else self.CHUNK_SHORT_ROWS
+
     # What the chunks of a step may take beside the model, at most: 64 KB a chunk of 64 rows and head of 128 x 128 (retention, the matrix memory), 148 KB
     # (decays by channel).  Longer lists of chunks go in spans of equal length, one after another; a span of 128 MB keeps every SM busy (8 heads:
     # 113 chunks by channel, 1808 blocks of two an SM).
@@ -1187,12 +1199,13 @@ class Ops:
     # -- retention ------------------------------------------------------------------------
     def retention(self, q, k, v, out, state, seq_starts, kv_lens, seq_slots, n_seqs: int, decay, n_heads: int, *, inv_freq=None,
                   rot_dims: int = 0, interleaved: bool = False, k_scale: float = 1.0, gate=None, unit_norm_eps: Optional[float] = None,
-                  raw=None, silu_inputs: bool = False, raw_only: bool = False) -> None:
+                  raw=None, silu_inputs: bool = False, raw_only: bool = False, max_new: Optional[int] = None) -> None:
         """Per sequence and head, over the step's rows in order: S = decay_h S + k v^T, o = S^T q, with q and k turned by
         position first (`inv_freq`, `rot_dims`), k scaled by `k_scale`; `unit_norm_eps`: o over its root mean square per
         head; `gate`: times silu(gate).  `state` is `[slots, heads, dk, dv]` float32 and is carried on.  `raw`: float32
         scratch `[rows, heads x dv]`, needed where `retention_needs_raw` says so (a head's columns spread over blocks).
-        `silu_inputs`: q, k and v pass a silu first (32-bit).  `raw_only`: the 32-bit read-outs in `raw` are all that is
+        `max_new`: the longest run of new rows, which decides between the row by row walk and chunks (`CHUNK_MIN_ROWS`).  `silu_inputs`: q, k and v pass a silu
+        first (32-bit).  `raw_only`: the 32-bit read-outs in `raw` are all that is
         written (`out` may be None; no norm, no gate)."""
         _need_cuda(q, k, v, out, state, seq_starts, kv_lens, seq_slots, decay, inv_freq, gate)
         if raw_only:
@@ -1220,26 +1233,27 @@ class Ops:
         if raw is not None and (raw.dtype != torch.float32 or not raw.is_contiguous() or raw.numel() < n * n_heads * dv):
             raise KernelError("retention: the scratch must be contiguous float32 [rows, heads x dv]")
         E = 2 if self.dtype == torch.bfloat16 else 4          # bytes of an entry
-        if (self.chunked_recurrences and n >= self.CHUNK_MIN_ROWS * n_seqs and dk <= 128 and dv <= 128 and dk % 4 == 0 and dv % 4 == 0
-                and (ld_q | ld_k | ld_v | ld_g) % 4 == 0 and (q.data_ptr() | k.data_ptr() | v.data_ptr() | (gate.data_ptr() if gate is not None else 0)) % (4 * E) == 0
-                and state.data_ptr() % 16 == 0 and (not raw_only or raw.data_ptr() % 16 == 0)):
+        chunks, short = self._chunk_rule(n, n_seqs, max_new)
+        chunks = (chunks and dk <= 128 and dv <= 128 and dk % 4 == 0 and dv % 4 == 0 and (ld_q | ld_k | ld_v | ld_g) % 4 == 0
+                  and (q.data_ptr() | k.data_ptr() | v.data_ptr() | (gate.data_ptr() if gate is not None else 0)) % (4 * E) == 0
+                  and state.data_ptr() % 16 == 0 and (not raw_only or raw.data_ptr() % 16 == 0))
+        args = (self.code, _ptr(q), ld_q, _ptr(k), ld_k, _ptr(v), ld_v, _ptr(gate), ld_g, _ptr(out), ld_o, _ptr(raw), n, _ptr(state),
+                _ptr(seq_starts), _ptr(kv_lens), _ptr(seq_slots), _ptr(decay), _ptr(inv_freq), int(rot_dims),
+                int(bool(interleaved)), int(n_seqs), int(n_heads), dk, dv, float(k_scale),
+                float(unit_norm_eps or 0.0), 0 if unit_norm_eps is None else 1, int(bool(silu_inputs)), 0 if raw_only else 1)
+        if not chunks or (short > 0 and (raw is not None or not self.retention_needs_raw(dk, dv))):
+            # (first: where a head's columns are spread over blocks, it leaves something in every row of `out`)
+            h = lib("retention")
+            _check(h.kvad_retention(*args, short if chunks else 1 << 30, _stream()), h)
+        else:
+            short = 0
+        if chunks:
             global _launches
             h = lib("chunked_recurrence")
             span, spans = self._chunk_span(n, n_seqs, n_heads * dk * dv * 4)
             work = torch.empty(span * n_heads * dk * dv, dtype=torch.float32, device=q.device)
-            _check(h.kvad_retention_chunked(self.code, _ptr(q), ld_q, _ptr(k), ld_k, _ptr(v), ld_v, _ptr(gate), ld_g, _ptr(out), ld_o, _ptr(raw), n, _ptr(state),
-                                            _ptr(seq_starts), _ptr(kv_lens), _ptr(seq_slots), _ptr(decay), _ptr(inv_freq), int(rot_dims),
-                                            int(bool(interleaved)), int(n_seqs), int(n_heads), dk, dv, float(k_scale),
-                                            float(unit_norm_eps or 0.0), 0 if unit_norm_eps is None else 1, int(bool(silu_inputs)), 0 if raw_only else 1,
-                                            _ptr(work), span, _stream()), h)
+            _check(h.kvad_retention_chunked(*args, _ptr(work), span, max(short, 1), _stream()), h)
             _launches += 3 * spans - 1          # three kernels a span: the chunks' sums, the state from chunk to chunk, the read-outs
-            return
-        h = lib("retention")
-        _check(h.kvad_retention(self.code, _ptr(q), ld_q, _ptr(k), ld_k, _ptr(v), ld_v, _ptr(gate), ld_g, _ptr(out), ld_o, _ptr(raw), n, _ptr(state),
-                                _ptr(seq_starts), _ptr(kv_lens), _ptr(seq_slots), _ptr(decay), _ptr(inv_freq), int(rot_dims),
-                                int(bool(interleaved)), int(n_seqs), int(n_heads), dk, dv, float(k_scale),
-                                float(unit_norm_eps or 0.0), 0 if unit_norm_eps is None else 1, int(bool(silu_inputs)), 0 if raw_only else 1,
-                                _stream()), h)
 
     def row_norm_gate(self, raw, gate, weight, out, eps: float) -> None:
         """out = raw / sqrt(mean over the row (raw^2) + eps) * weight * sigmoid(gate): `raw` float32, `gate` (may be None) and
@@ -1275,8 +1289,8 @@ class Ops:
 
     def gated_recurrence(self, kind: str, q, k, v, gates, out, state, seq_starts, seq_slots, n_seqs: int, n_heads: int, n_kv_heads: int,
                          dk: int, dv: int, *, q_scale: float = 1.0, cap: float = 0.0, beta=None, a_log=None, dt_bias=None,
-                         gates_ready: bool = False, tau: float = 1.0) -> None:
-        """Per sequence and head over the step's rows in order; `state` is `[slots, floats]` (32-bit), carried on.
+                         gates_ready: bool = False, tau: float = 1.0, max_new: Optional[int] = None) -> None:
+        """Per sequence and head over the step's rows in order; `max_new`: the longest run of new rows, as in `retention`; `state` is `[slots, floats]` (32-bit), carried on.
         `matrix_memory`: S = exp(f + m' - m) S + exp(i - m) k v^T with the running maximum m, n likewise with k alone,
         o = S^T q / (max(|n.q|, exp(-m)) + 1e-6); `gates` float32 [rows, 2 heads] = raw input | forget projections, capped
         here (`cap` tanh(x / cap)), the forget gate through logsigmoid.  `delta_rule`: S = g * S per key channel,
@@ -1308,34 +1322,40 @@ class Ops:
             raise KernelError("gated_recurrence: tau must be positive")
         global _launches
         E = 2 if q.dtype == torch.bfloat16 else 4          # bytes of an entry
-        if (mode == 0 and self.chunked_recurrences and n >= self.CHUNK_MIN_ROWS * n_seqs and dk <= 128 and dv <= 128 and dk % 4 == 0 and dv % 4 == 0
-                and (ld_q | ld_k | ld_v | ld_o | state.stride(0)) % 4 == 0 and (q.data_ptr() | k.data_ptr() | v.data_ptr()) % (4 * E) == 0
-                and (state.data_ptr() | out.data_ptr()) % 16 == 0):
+        chunks, short = self._chunk_rule(n, n_seqs, max_new)
+        if mode == 0:
+            chunks = (chunks and dk <= 128 and dv <= 128 and dk % 4 == 0 and dv % 4 == 0 and (ld_q | ld_k | ld_v | ld_o | state.stride(0)) % 4 == 0
+                      and (q.data_ptr() | k.data_ptr() | v.data_ptr()) % (4 * E) == 0 and (state.data_ptr() | out.data_ptr()) % 16 == 0)
+        else:
+            chunks = (chunks and gates_ready and dk <= 128 and dk % 4 == 0 and (ld_q | ld_k | ld_g) % 4 == 0
+                      and (q.data_ptr() | k.data_ptr()) % (4 * E) == 0 and gates.data_ptr() % 16 == 0)
+        if not chunks or short > 0:
+            h = lib("gated_recurrence")
+            _check(h.kvad_gated_recurrence(mode, _code(q.dtype), _ptr(q), ld_q, _ptr(k), ld_k, _ptr(v), ld_v, _ptr(gates), ld_g, _ptr(beta), ld_b,
+                                           _ptr(a_log), _ptr(dt_bias), p_f32, _ptr(out), ld_o, _ptr(state), state.stride(0), _ptr(seq_starts),
+                                           _ptr(seq_slots), int(n_seqs), int(n_heads), int(n_kv_heads), int(dk), int(dv), float(q_scale),
+                                           float(cap), int(bool(gates_ready)), 1.0 / float(tau), short if chunks else 1 << 30, _stream()), h)
+        if not chunks:
+            return
+        short = max(short, 1)
+        if mode == 0:
             h = lib("chunked_recurrence")
             span, spans = self._chunk_span(n, n_seqs, n_heads * (dk * dv + dk + 3) * 4)
             work = torch.empty(span * n_heads * dk * dv, dtype=torch.float32, device=q.device)
             work_n = torch.empty(span * n_heads * (dk + 3), dtype=torch.float32, device=q.device)
             _check(h.kvad_matrix_memory_chunked(_code(q.dtype), _ptr(q), ld_q, _ptr(k), ld_k, _ptr(v), ld_v, _ptr(gates), ld_g, _ptr(out), ld_o, n, _ptr(state),
                                                 state.stride(0), _ptr(seq_starts), _ptr(seq_slots), int(n_seqs), int(n_heads), int(n_kv_heads), int(dk), int(dv),
-                                                float(q_scale), float(cap), _ptr(work), _ptr(work_n), span, _stream()), h)
+                                                float(q_scale), float(cap), _ptr(work), _ptr(work_n), span, short, _stream()), h)
             _launches += 4 * spans - 1          # four kernels a span: the chunks' sums, the state from chunk to chunk, the running maxima, the read-outs
-            return
-        if (mode != 0 and gates_ready and self.chunked_recurrences and n >= self.CHUNK_MIN_ROWS * n_seqs and dk <= 128 and dk % 4 == 0
-                and (ld_q | ld_k | ld_g) % 4 == 0 and (q.data_ptr() | k.data_ptr()) % (4 * E) == 0 and gates.data_ptr() % 16 == 0):
+        else:
             h = lib("chunked_channels")
             per_head = h.kvad_channels_work(int(dk), int(dv))
             span, spans = self._chunk_span(n, n_seqs, int(n_heads) * per_head * 4)
             work = torch.empty(span * int(n_heads) * per_head, dtype=torch.float32, device=q.device)
             _check(h.kvad_channels_chunked(_code(q.dtype), _ptr(q), ld_q, _ptr(k), ld_k, _ptr(v), ld_v, _ptr(gates), ld_g, _ptr(beta if mode == 1 else None), ld_b,
                                            _ptr(out), ld_o, n, _ptr(state), state.stride(0), _ptr(seq_starts), _ptr(seq_slots), int(n_seqs), int(n_heads),
-                                           int(n_kv_heads), int(dk), int(dv), float(q_scale), _ptr(work), span, _stream()), h)
+                                           int(n_kv_heads), int(dk), int(dv), float(q_scale), _ptr(work), span, short, _stream()), h)
             _launches += 2 * spans - 1          # two kernels a span: the chunks by themselves, the walk from chunk to chunk
-            return
-        h = lib("gated_recurrence")
-        _check(h.kvad_gated_recurrence(mode, _code(q.dtype), _ptr(q), ld_q, _ptr(k), ld_k, _ptr(v), ld_v, _ptr(gates), ld_g, _ptr(beta), ld_b,
-                                       _ptr(a_log), _ptr(dt_bias), p_f32, _ptr(out), ld_o, _ptr(state), state.stride(0), _ptr(seq_starts),
-                                       _ptr(seq_slots), int(n_seqs), int(n_heads), int(n_kv_heads), int(dk), int(dv), float(q_scale),
-                                       float(cap), int(bool(gates_ready)), 1.0 / float(tau), _stream()), h)
 
     def decay_gate(self, a, a_log, dt_bias, n_heads: int, dk: int) -> None:
         """In place on float32 `a` [rows, heads x dk]: g = exp(-exp(a_log_h) softplus(a + dt_bias))."""

@@ -96,7 +96,7 @@ class GatedDeltaRule(Mixer):
             ops.decay_gate(decay, self.a_log, self.dt_bias, H, dk)
         ops.gated_recurrence("delta_rule", y[:, :G * dk], y[:, G * dk:2 * G * dk], y[:, 2 * G * dk:C], decay, raw, state, ctx.seq_starts,
                              ctx.seq_slots, ctx.n_seqs, H, G, dk, self.value_dim, beta=y[:, C:C + H], a_log=self.a_log, dt_bias=self.dt_bias,
-                             gates_ready=ready)
+                             gates_ready=ready, max_new=ctx.batch.max_new)
         mixed = ctx.buffer((n, self.v_width))
         ops.head_norm_gate(raw, gate, self.norm_weight, mixed, H, self.norm_eps, weight_per_head=False)
         self.out.forward(ctx, mixed, residual, "residual")

@@ -67,7 +67,8 @@ class GatedLinearAttention(Mixer):
             ops.power_gate(decay, self.tau)
         raw = ctx.buffer((n, self.v_width), torch.float32)
         ops.gated_recurrence("gated_linear", q, k, v, decay, raw, ctx.state(call.cache), ctx.seq_starts, ctx.seq_slots, ctx.n_seqs, H, H,
-                             self.key_dim, self.value_dim, q_scale=self.key_dim ** -0.5, tau=self.tau, gates_ready=ready)
+                             self.key_dim, self.value_dim, q_scale=self.key_dim ** -0.5, tau=self.tau, gates_ready=ready,
+                             max_new=ctx.batch.max_new)
         mixed = ctx.buffer((n, self.v_width))
         ops.head_norm_gate(raw, gate, self.norm_weight, mixed, H, self.norm_eps, weight_per_head=False, act="silu")
         self.out.forward(ctx, mixed, residual, "residual")

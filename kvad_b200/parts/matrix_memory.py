@@ -68,7 +68,8 @@ class MatrixMemory(Mixer):
         q, k, v, g = (buf[:, self.proj.columns(i)] for i in range(4))
         raw = ctx.buffer((n, self.v_width), torch.float32)
         ops.gated_recurrence("matrix_memory", q, k, v, gates[:, :2 * H], raw, ctx.state(call.cache), ctx.seq_starts, ctx.seq_slots,
-                             ctx.n_seqs, H, H, self.key_dim, self.value_dim, q_scale=self.key_dim ** -0.5, cap=self.gate_cap)
+                             ctx.n_seqs, H, H, self.key_dim, self.value_dim, q_scale=self.key_dim ** -0.5, cap=self.gate_cap,
+                             max_new=ctx.batch.max_new)
         mixed = ctx.buffer((n, self.v_width))
         ops.head_norm_gate(raw, g, self.norm_weight, mixed, H, self.norm_eps, weight_per_head=True)
         self.out.forward(ctx, mixed, residual, "residual")

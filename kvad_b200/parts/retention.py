@@ -92,7 +92,7 @@ class Retention(Mixer):
             ctx.ops.retention(q, k, v, None, ctx.state(call.cache), ctx.seq_starts, ctx.kv_lens, ctx.seq_slots, ctx.n_seqs,
                               self.decay, self.n_heads, inv_freq=pos.inv_freq if pos is not None else None,
                               rot_dims=pos.dims if pos is not None else 0, interleaved=pos.interleaved if pos is not None else False,
-                              k_scale=self.key_scale, raw=raw, silu_inputs=self.silu_inputs, raw_only=True)
+                              k_scale=self.key_scale, raw=raw, silu_inputs=self.silu_inputs, raw_only=True, max_new=ctx.batch.max_new)
             ctx.ops.row_norm_gate(raw, gate, self.row_weight, mixed, float(self.row_norm["eps"]))
             self.out.forward(ctx, mixed, residual, "residual")
             return
@@ -100,7 +100,8 @@ class Retention(Mixer):
         ctx.ops.retention(q, k, v, mixed, ctx.state(call.cache), ctx.seq_starts, ctx.kv_lens, ctx.seq_slots, ctx.n_seqs,
                           self.decay, self.n_heads, inv_freq=pos.inv_freq if pos is not None else None,
                           rot_dims=pos.dims if pos is not None else 0, interleaved=pos.interleaved if pos is not None else False,
-                          k_scale=self.key_scale, gate=gate, unit_norm_eps=self.unit_norm_eps, raw=raw, silu_inputs=self.silu_inputs)
+                          k_scale=self.key_scale, gate=gate, unit_norm_eps=self.unit_norm_eps, raw=raw, silu_inputs=self.silu_inputs,
+                          max_new=ctx.batch.max_new)
         self.out.forward(ctx, mixed, residual, "residual")
 
 

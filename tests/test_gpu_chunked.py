@@ -336,3 +336,52 @@ def test_long_steps_go_in_spans_of_bounded_scratch(kind):
     out, state, peak = run([20000, 1, 300], budget)
     assert peak <= budget + (1 << 16), (peak, budget)
     assert out.isfinite().all()
+
+
+@pytest.mark.parametrize("kind", ["retention", "retention finished", "matrix_memory", "delta_rule", "gated_linear"])
+@pytest.mark.parametrize("dtype,dk,dv", [("float32", 64, 32), ("bfloat16", 128, 128)])
+def test_short_sequences_keep_their_bits_beside_a_prompt(kind, dtype, dk, dv):
+    """A prompt among decoding sequences goes in chunks, by the longest run; the sequences of fewer than 16 rows are walked and get what they get alone, to
+    the bit, and so does the prompt."""
+    if dtype == "bfloat16" and kind == "delta_rule":
+        dtype = "float32"
+    g = torch.Generator(device="cuda")
+    g.manual_seed(dk)
+    H, lens, t = 2, [1, 300, 1, 15, 16, 1], DT[dtype]
+    N, ops, slots = sum(lens), Ops(t), [3, 0, 5, 1, 4, 2]
+    q, k, v, gate = (torch.randn(N, H * d, generator=g, device="cuda").to(t) for d in (dk, dk, dv, dv))
+    memory, done = kind == "matrix_memory", kind.endswith("finished")
+    gates = torch.randn(N, 2 * H, generator=g, device="cuda") + 3.0 if memory else torch.sigmoid(torch.randn(N, H * dk, generator=g, device="cuda") + 3.0)
+    beta, decay = torch.sigmoid(torch.randn(N, H, generator=g, device="cuda")), torch.tensor([0.9, 0.97], device="cuda")
+    if kind == "delta_rule":
+        k = torch.nn.functional.normalize(k.view(N, H, dk), dim=-1).view(N, -1)
+    size = (H, dk, dv) if kind.startswith("retention") else (ops.recurrence_state_size(kind, H, dk, dv),)
+    first = torch.randn(6, *size, generator=g, device="cuda") if not memory else torch.zeros(6, *size, device="cuda")
+    at = [0] + list(np.cumsum(lens))
+
+    def run(which, told):
+        state, rows = first.clone(), torch.cat([torch.arange(at[i], at[i + 1], device="cuda") for i in which])
+        pick, ls = (lambda x: x[rows].contiguous()), [lens[i] for i in which]
+        raw, n = torch.full((len(rows), H * dv), float("nan"), device="cuda"), len(which)
+        out = torch.full((len(rows), H * dv), float("nan"), device="cuda", dtype=t)
+        more = dict(max_new=max(ls)) if told else {}
+        if kind.startswith("retention"):
+            ops.retention(pick(q), pick(k), pick(v), out if done else None, state, starts(ls), i32([x + 7 for x in ls]), i32([slots[i] for i in which]), n, decay, H,
+                          raw=raw, raw_only=not done, **(dict(gate=pick(gate), unit_norm_eps=1e-5) if done else {}), **more)
+        else:
+            kw = {"delta_rule": dict(beta=pick(beta), a_log=torch.zeros(H, device="cuda"), dt_bias=torch.zeros(H * dk, device="cuda"), gates_ready=True),
+                  "gated_linear": dict(gates_ready=True), "matrix_memory": dict(cap=15.0)}[kind]
+            ops.gated_recurrence(kind, pick(q), pick(k), pick(v), pick(gates), raw, state, starts(ls), i32([slots[i] for i in which]), n, H, H, dk, dv, **kw, **more)
+        return (out if done else raw), state
+
+    got, state = run(range(6), True)
+    assert got.isfinite().all()
+    for i in range(6):
+        alone, end = run([i], True)
+        if i == 4:                                         # 16 rows: in chunks here, walked alone
+            assert rel(got[at[4]:at[5]], alone.double()) < (5e-3 if done and dtype == "bfloat16" else 5e-5) and not torch.equal(state[slots[4]], end[slots[4]])
+        else:
+            assert torch.equal(got[at[i]:at[i + 1]], alone) and torch.equal(state[slots[i]], end[slots[i]]), i
+    ops.chunked_recurrences = False
+    walked, _ = run([1], True)
+    assert not torch.equal(walked, got[at[1]:at[2]])       # (the prompt did go in chunks)

@@ -17,3 +17,18 @@ def test_decode_key_ranges_keep_a_launch_one_wave():
     assert [Ops.decode_splits(r, 12, 16, n_sms=sms) for r in (1, 2, 4, 8, 12, 16, 20, 24, 64)] == [6, 6, 6, 4, 2, 2, 1, 1, 1]
     # it depends on the device's size, not on a constant
     assert Ops.decode_splits(8, 12, 16, n_sms=74) == 2
+
+
+def test_recurrences_go_in_chunks_by_the_longest_run():
+    import torch
+    ops = Ops(torch.float32)
+    ops.chunked_recurrences = True
+    rule = lambda lens, told=True: ops._chunk_rule(sum(lens), len(lens), max(lens) if told else None)          # noqa: E731
+    assert rule([1000]) == (True, 0) and rule([300, 300]) == (True, 0)          # nothing short can be beside them
+    assert rule([1000] + [1] * 8) == (True, 16)                                  # a prompt among decoding sequences: they keep to the walk
+    assert rule([245, 23, 153, 76]) == (True, 16)
+    assert rule([159, 159]) == (False, 0) and rule([1] * 2000) == (False, 0)
+    # without the longest run: the average, for all sequences alike
+    assert rule([1000, 517, 37], told=False) == (True, 0) and rule([1000] + [1] * 8, told=False) == (False, 0)
+    ops.chunked_recurrences = False
+    assert rule([1000]) == (False, 0)
