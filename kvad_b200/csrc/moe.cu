@@ -467,9 +467,35 @@ grouped_linear_kernel(const T* __restrict__ a, int64_t ld_a, const int* __restri
 // lanes take every 32nd 16-byte piece of the weight rows, from shared memory, and multiply them with the same pieces
 // of 1, 2, 4 or 8 of the tile's rows (which stay in the L1); a shuffle tree per (row, output) at the end.  A tile with more than
 // eight rows goes over its weights again per eight.  (With the weights fetched into registers piece by piece, 8 x 4 loads a warp, 64
-// pairs of 16 experts of 1408 x 1024 took 44 us: a block held its registers through three trips to memory one after another.)
+// pairs of 16 experts of 1408 x 1024 took 39 us: a block held its registers through three trips to memory one after another.)
 __device__ int g_rows_timeouts = 0;
 constexpr uint32_t ROWS_WAIT_LIMIT = 1u << 24;
+uint32_t g_rows_wait_limit = ROWS_WAIT_LIMIT;      // (tests: fewer polls, and a launch whose copies are left out)
+int g_rows_skip_copy = 0;
+struct RowsWait { uint32_t limit; int skip; };
+inline RowsWait rows_wait() {
+  const RowsWait w{g_rows_wait_limit, g_rows_skip_copy};
+  g_rows_skip_copy = 0;
+  return w;
+}
+
+// Whether the block's weights have come, for the warp as a whole.  Where they have not, that is counted, and the copy is waited for once more, so that it does not
+// land in the shared memory of a block that comes after this one.
+__device__ __forceinline__ bool rows_came(uint32_t bar, uint32_t limit) {
+  bool there = false;
+#pragma unroll 1
+  for (int turn = 0; turn < 2 && !there; ++turn) {
+    for (uint32_t i = 0; i < limit && !there; ++i) {
+      uint32_t ok;
+      asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar) : "memory");
+      there = ok != 0;
+    }
+    there = __all_sync(0xffffffffu, there);
+    if (turn == 0 && there) return true;
+    if (turn == 0 && (threadIdx.x & 31) == 0) atomicAdd(&g_rows_timeouts, 1);
+  }
+  return false;
+}
 
 template <typename T, typename TO, int R, int CU>
 __device__ __forceinline__ void rows_times(const T* __restrict__ a, int64_t ld_a, const int* rows_in, const int* rows_out, int n, const T* w,
@@ -514,7 +540,7 @@ template <typename T, typename TO, int CU>
 __global__ void __launch_bounds__(256, 3)
 grouped_rows_kernel(const T* __restrict__ a, int64_t ld_a, const int* __restrict__ in_rows, const T* __restrict__ w,
                     int64_t expert_stride, TO* __restrict__ out, int64_t ld_out, const int* __restrict__ out_rows,
-                    const int* __restrict__ valid, const int* __restrict__ tile_expert, int n_out, int k_dim) {
+                    const int* __restrict__ valid, const int* __restrict__ tile_expert, int n_out, int k_dim, RowsWait wait) {
   extern __shared__ __align__(128) uint8_t rows_smem[];
   T* ws = reinterpret_cast<T*>(rows_smem);      // [warps * CU][k_dim]
   __shared__ int rows_in[TM], rows_out[TM], n_valid;
@@ -534,8 +560,9 @@ grouped_rows_kernel(const T* __restrict__ a, int64_t ld_a, const int* __restrict
   if (tid == 0) {
     const uint32_t bytes = (uint32_t)min(per_block, n_out - first) * (uint32_t)k_dim * (uint32_t)sizeof(T);
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"((uint32_t)__cvta_generic_to_shared(ws)), "l"(w + (int64_t)expert * expert_stride + (int64_t)first * k_dim), "r"(bytes), "r"(bar) : "memory");
+    if (!wait.skip)
+      asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                   ::"r"((uint32_t)__cvta_generic_to_shared(ws)), "l"(w + (int64_t)expert * expert_stride + (int64_t)first * k_dim), "r"(bytes), "r"(bar) : "memory");
   }
   if (tid < TM) {                               // the tile's used positions, side by side
     const int p = tile * TM + tid;
@@ -549,16 +576,7 @@ grouped_rows_kernel(const T* __restrict__ a, int64_t ld_a, const int* __restrict
     if (tid == 0) n_valid = __popc(mask);
   }
   __syncthreads();
-  bool there = false;
-  for (uint32_t i = 0; i < ROWS_WAIT_LIMIT && !there; ++i) {
-    uint32_t ok;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar) : "memory");
-    there = ok != 0;
-  }
-  if (!there) {                                 // (the copy never came: say so, write nothing)
-    if (lane == 0) atomicAdd(&g_rows_timeouts, 1);
-    return;
-  }
+  if (!rows_came(bar, wait.limit)) return;      // (the copy never came: nothing is written)
   const int col0 = first + warp * CU;
   if (col0 >= n_out) return;
   const T* wr = ws + (int64_t)warp * CU * k_dim;      // (rows past the last output are not there: what they give is not written)
@@ -768,8 +786,8 @@ inline int flat_blocks(int64_t total, int threads) {
 // neighbouring k go to one lane - which is two m16n8k16.  The tensor core truncates where it accumulates, so a sum stays in it for those 32
 // of K only and then joins a register by a rounded addition; what those additions round away is carried beside the sum (`add_exactly`) and
 // joins it at the end, which pays for the truncation: the error against 64 bits
-// is 5.3e-8 at K = 704 .. 4096 (7.7e-8 without, 7.3e-8 the chain of fused multiply-adds).  64 pairs of 16 experts of 1408 x 1024: 38 us with the
-// weights fetched into registers, 27 with the bulk copy and that chain (more instructions than the copy costs time), 13.7 this way.
+// is 5.3e-8 at K = 704 .. 4096 (7.7e-8 without, 7.3e-8 the chain of fused multiply-adds).  64 pairs of 16 experts of 1408 x 1024: 39 us with the
+// weights fetched into registers, 27 with the bulk copy and that chain (more instructions than the copy costs time), 14 this way.
 __device__ __forceinline__ float add_exactly(float a, float b, float& lost) {      // a + b rounded; what the rounding lost is added to `lost` (Knuth's two-sum)
   const float s = __fadd_rn(a, b), of_b = __fsub_rn(s, a);
   lost = __fadd_rn(lost, __fadd_rn(__fsub_rn(a, __fsub_rn(s, of_b)), __fsub_rn(b, of_b)));
@@ -782,7 +800,7 @@ template <typename TO>
 __global__ void __launch_bounds__(256, 4)
 grouped_rows_mma_kernel(const __nv_bfloat16* __restrict__ a, int64_t ld_a, const int* __restrict__ in_rows, const __nv_bfloat16* __restrict__ w,
                         int64_t expert_stride, TO* __restrict__ out, int64_t ld_out, const int* __restrict__ out_rows,
-                        const int* __restrict__ valid, const int* __restrict__ tile_expert, int n_out, int k_dim) {
+                        const int* __restrict__ valid, const int* __restrict__ tile_expert, int n_out, int k_dim, RowsWait wait) {
   constexpr int OUTS = 16;
   extern __shared__ __align__(128) uint8_t rows_smem[];
   const __nv_bfloat16* ws = reinterpret_cast<const __nv_bfloat16*>(rows_smem);      // [16][k_dim]
@@ -804,8 +822,9 @@ grouped_rows_mma_kernel(const __nv_bfloat16* __restrict__ a, int64_t ld_a, const
   if (tid == 0) {
     const uint32_t bytes = (uint32_t)n_rows_w * (uint32_t)k_dim * 2u;
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"((uint32_t)__cvta_generic_to_shared(ws)), "l"(w + (int64_t)expert * expert_stride + (int64_t)first * k_dim), "r"(bytes), "r"(bar) : "memory");
+    if (!wait.skip)
+      asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                   ::"r"((uint32_t)__cvta_generic_to_shared(ws)), "l"(w + (int64_t)expert * expert_stride + (int64_t)first * k_dim), "r"(bytes), "r"(bar) : "memory");
   }
   if (tid < TM) {                               // the tile's used positions, side by side
     const int p = tile * TM + tid;
@@ -820,7 +839,7 @@ grouped_rows_mma_kernel(const __nv_bfloat16* __restrict__ a, int64_t ld_a, const
   }
   __syncthreads();
   const int g = lane >> 2, k_of = (lane & 3) * 8;
-  bool waited = false;
+  bool waited = false, lost_copy = false;
   for (int r0 = 0; r0 < max(n_valid, 1); r0 += 8) {      // (a tile without rows waits for its copy too)
     const int n = min(8, n_valid - r0);
     const __nv_bfloat16* ar = a + (g < n ? (int64_t)rows_in[r0 + g] * ld_a : 0) + k_of;
@@ -828,16 +847,8 @@ grouped_rows_mma_kernel(const __nv_bfloat16* __restrict__ a, int64_t ld_a, const
     uint4 next = make_uint4(0u, 0u, 0u, 0u);
     if (g < n && warp * 32 + k_of < k_dim) next = *reinterpret_cast<const uint4*>(ar + warp * 32);
     if (!waited) {                              // (the first rows are on their way meanwhile)
-      bool there = false;
-      for (uint32_t i = 0; i < ROWS_WAIT_LIMIT && !there; ++i) {
-        uint32_t ok;
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar) : "memory");
-        there = ok != 0;
-      }
+      lost_copy = !rows_came(bar, wait.limit);
       waited = true;
-      if (!there) {                             // (the copy never came: say so, write nothing that means anything)
-        if (lane == 0) atomicAdd(&g_rows_timeouts, 1);
-      }
     }
 #pragma unroll 2
     for (int k0 = warp * 32; k0 < k_dim; k0 += 256) {
@@ -861,7 +872,7 @@ grouped_rows_mma_kernel(const __nv_bfloat16* __restrict__ a, int64_t ld_a, const
     if (r0 > 0) __syncthreads();                // the sums before have been read
 #pragma unroll
     for (int e = 0; e < 4; ++e) sums[warp][(lane & 3) * 2 + (e & 1)][g + (e >> 1) * 8] = with_lost(acc[e], lost[e]);
-    __syncthreads();
+    if (__syncthreads_or(lost_copy)) return;    // (the copy never came: nothing is written)
     if (tid < 8 * OUTS) {
       const int r = tid / OUTS, o = tid % OUTS;
       if (r < n && first + o < n_out) {
@@ -884,7 +895,7 @@ int launch_rows_mma(int n_out, int max_tiles, size_t smem, cudaStream_t stream, 
     configured = smem;
   }
   kvad_launch(grouped_rows_mma_kernel<TO>, dim3((n_out + 15) / 16, max_tiles), dim3(256), smem, stream, a, ld_a, in_rows, w, expert_stride, out, ld_out, out_rows,
-              valid, tile_expert, n_out, k_dim);
+              valid, tile_expert, n_out, k_dim, rows_wait());
   KVAD_CHECK_LAUNCH("grouped_linear");
   return KVAD_OK;
 }
@@ -898,7 +909,8 @@ int launch_rows(dim3 grid, int warps, size_t smem, cudaStream_t stream, const T*
     if (e != cudaSuccess) KVAD_FAIL(KVAD_ERR_CUDA, "grouped_linear: cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
     configured = smem;
   }
-  kvad_launch(grouped_rows_kernel<T, TO, CU>, grid, dim3(32 * warps), smem, stream, a, ld_a, in_rows, w, expert_stride, out, ld_out, out_rows, valid, tile_expert, n_out, k_dim);
+  kvad_launch(grouped_rows_kernel<T, TO, CU>, grid, dim3(32 * warps), smem, stream, a, ld_a, in_rows, w, expert_stride, out, ld_out, out_rows, valid, tile_expert, n_out, k_dim,
+              rows_wait());
   return KVAD_OK;
 }
 
@@ -966,6 +978,13 @@ KVAD_EXPORT int kvad_moe_status() {
   cudaError_t e = cudaMemcpyFromSymbol(&n, g_rows_timeouts, sizeof(int));
   if (e != cudaSuccess) KVAD_FAIL(KVAD_ERR_CUDA, "moe_status: %s", cudaGetErrorString(e));
   return n;
+}
+
+// Tests of the bounded waits: `wait_limit` > 0 sets how many polls a wait makes before it gives up (0: the library's own limit); `skip_copies` makes the NEXT product
+// of few rows leave out its copies, so that the waits for them run out: its launch raises the counter, writes nothing and returns; those after it are ordinary.
+KVAD_EXPORT void kvad_moe_test_hooks(unsigned wait_limit, int skip_copies) {
+  g_rows_wait_limit = wait_limit > 0 ? wait_limit : ROWS_WAIT_LIMIT;
+  g_rows_skip_copy = skip_copies != 0;
 }
 
 // Position p reads row in_rows[p] of `a` (null: row p) and writes row out_rows[p] of `out` (null: row p); valid[p] < 0: padding.

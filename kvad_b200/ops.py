@@ -1811,6 +1811,31 @@ def tcgen05_wait_timeouts() -> int:
     return n
 
 
+def linear_split_wait_timeouts() -> int:
+    """How many bounded waits of the 32-bit product on the tensor cores have run out (0 in a healthy run)."""
+    h = lib("linear_split")
+    n = h.kvad_linear_split_status()
+    if n < 0:
+        raise KernelError(h.kvad_last_error().decode("utf-8", "replace"))
+    return n
+
+
+def moe_wait_timeouts() -> int:
+    """How many waits for experts' weights (products of few rows) have run out (0 in a healthy run)."""
+    h = lib("moe")
+    n = h.kvad_moe_status()
+    if n < 0:
+        raise KernelError(h.kvad_last_error().decode("utf-8", "replace"))
+    return n
+
+
+def moe_test_hooks(wait_limit: int = 0, skip_copies: bool = False) -> None:
+    """Tests of the experts' bounded waits: see kvad_moe_test_hooks."""
+    h = lib("moe")
+    h.kvad_moe_test_hooks.argtypes, h.kvad_moe_test_hooks.restype = [ctypes.c_uint, c_int], None
+    h.kvad_moe_test_hooks(int(wait_limit), int(bool(skip_copies)))
+
+
 def tcgen05_takes(a, weight, out, lda: int, ldo: int) -> bool:
     """Shapes the tensor-core linear kernel accepts: TMA wants 16-byte aligned
     bases and row strides (bfloat16: multiples of 8 elements)."""

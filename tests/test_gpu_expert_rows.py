@@ -53,3 +53,30 @@ def test_few_rows_of_experts_are_no_further_off_than_the_fmaf_chain(dtype, n_out
         few, chain = ((x - want).norm() / want.norm() for x in got)
         assert few <= 1.05 * chain + 2.0 ** -25               # (both are sums of rounding errors of a few hundred outputs)
     assert h.kvad_moe_status() == 0
+
+
+@pytest.mark.parametrize("dtype,k", [("bfloat16", 256), ("bfloat16", 6408), ("float32", 256), ("float32", 13000)])
+def test_a_copy_that_never_comes_is_reported_and_writes_nothing(dtype, k):
+    """The bounded wait for a block's weights, on the tensor cores and off: with the copies left out it gives up by counting, the counter rises and no output
+    is written; the launch after it is ordinary.  (The 32-bit product's counter has its reader too.)"""
+    from kvad_b200.ops import linear_split_wait_timeouts, moe_test_hooks, moe_wait_timeouts
+    g = torch.Generator(device="cuda")
+    g.manual_seed(k)
+    ops, TM, n_out = Ops(DT[dtype]), lib("moe").kvad_moe_tile_rows(), 20
+    a, w = torch.randn(TM, k, generator=g, device="cuda").to(DT[dtype]), torch.randn(1, n_out, k, generator=g, device="cuda").to(DT[dtype])
+    te, flat = torch.zeros(1, dtype=torch.int32, device="cuda"), torch.full((TM,), -1, dtype=torch.int32, device="cuda")
+    flat[:11] = 1
+    out = torch.full((TM, n_out), 7.0, dtype=DT[dtype], device="cuda")
+    before, split = moe_wait_timeouts(), linear_split_wait_timeouts()
+    try:
+        moe_test_hooks(wait_limit=200, skip_copies=True)
+        ops.grouped_linear(a, w, out, te, flat, few_rows=True)
+        torch.cuda.synchronize()
+        assert moe_wait_timeouts() > before and bool((out == 7.0).all())
+    finally:
+        moe_test_hooks()
+    again = moe_wait_timeouts()
+    ops.grouped_linear(a, w, out, te, flat, few_rows=True)
+    want = a[:11].double() @ w[0].double().t()
+    assert ((out[:11].double() - want).norm() / want.norm()).item() < (5e-3 if dtype == "bfloat16" else 1e-6) and bool((out[11:] == 7.0).all())
+    assert moe_wait_timeouts() == again and linear_split_wait_timeouts() == split
