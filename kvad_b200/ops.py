@@ -377,7 +377,9 @@ class Ops:
         """Everything on the host that decides which kernels a step of a given shape launches; part of
         the key under which a step's CUDA graph is kept."""
         return (_switch_epoch, self.tensor_core_linear, self.tensor_core_prefill, self.fast_decode,
-                self.rows_linear_max, self.qkv_sums, self.SUMS_MIN_K, self.tiled_prompt, self.split_linear, self.scored_prompt, self.chunked_recurrences)
+                self.rows_linear_max, self.qkv_sums, self.SUMS_MIN_K, self.tiled_prompt, self.split_linear, self.scored_prompt, self.chunked_recurrences,
+                self.SPLIT_MIN_ROWS, self.SCORED_PROMPT_MIN_NEW, self.CHUNK_MIN_ROWS, self.CHUNK_SHORT_ROWS, self.CHUNK_WORK_BYTES,
+                self.ROWS_LINEAR_MAX_OUT, self.ROWS_BLOCKS_MAX, self.HEADS_LINEAR_MAX_ROWS)
 
     def begin_step(self) -> None:
         """Called once before a step's first kernel (inside the capture, if the step is being captured)."""

@@ -32,3 +32,13 @@ def test_recurrences_go_in_chunks_by_the_longest_run():
     assert rule([1000, 517, 37], told=False) == (True, 0) and rule([1000] + [1] * 8, told=False) == (False, 0)
     ops.chunked_recurrences = False
     assert rule([1000]) == (False, 0)
+
+
+def test_a_constant_that_chooses_a_kernel_is_part_of_a_captured_step():
+    import torch
+    ops = Ops(torch.bfloat16)
+    for name in ("SPLIT_MIN_ROWS", "SCORED_PROMPT_MIN_NEW", "CHUNK_MIN_ROWS", "CHUNK_SHORT_ROWS", "CHUNK_WORK_BYTES", "SUMS_MIN_K", "ROWS_LINEAR_MAX_OUT",
+                 "ROWS_BLOCKS_MAX", "HEADS_LINEAR_MAX_ROWS", "split_linear", "scored_prompt", "chunked_recurrences"):
+        before = ops.path_key()
+        setattr(ops, name, getattr(ops, name) + 1)
+        assert ops.path_key() != before, name
