@@ -2,9 +2,9 @@
 // arithmetic: every product is an fmaf into a 32-bit accumulator and every
 // output element sums k = 0..K-1 in that order, whatever M is and wherever the
 // row sits in the batch.  This is the matrix kernel of the float32 engine for
-// 17 to 64 rows and for rows that are not in 16-byte pieces (more rows:
-// linear_split.cu), and the fallback of the bfloat16 engine for shapes its
-// tensor-core kernel refuses.  bisand/kvad's counterpart is its CPU gemm_bt / matvec_bt
+// rows that are not in 16-byte pieces and for up to 64 rows of K above 4096
+// (else: up to 64 rows linear_rows_f32.cu, more linear_split.cu), and the
+// fallback of the bfloat16 engine for shapes its tensor-core kernel refuses.  bisand/kvad's counterpart is its CPU gemm_bt / matvec_bt
 // (crates/llm/src/tensor.rs:56-193), bias added after the product
 // (crates/llm/src/quant.rs:849-857).
 #include "common.cuh"

@@ -118,10 +118,9 @@ def test_linear_cuda_cores(dtype):
 
 
 def test_linear_is_true_32_bit_and_row_independent():
-    """The 32-bit kernels sum with fused multiply-adds in an order that depends on K only: a row gives the same
-    bits whatever its company, on each of the two roads (at most 16 rows: the weight stream; more: the tiled
-    kernel, 64 x 64 or 128 x 128 tiles); the two roads agree to rounding; and values that a 19-bit (TF32)
-    product would lose survive on both."""
+    """The 32-bit products sum in an order that depends on K only: a row gives the same bits whatever its company, on each of the roads
+    that rows in whole 16-byte pieces take by themselves (at most 64 rows: the weight stream, in blocks of 16; more: the tensor cores on
+    exact pieces); the roads agree to rounding; and values that a 19-bit (TF32) product would lose survive on both."""
     ops = Ops(torch.float32)
     g = torch.Generator().manual_seed(4)
     a, w = torch.randn(300, 96, generator=g), torch.randn(6000, 96, generator=g)
@@ -131,8 +130,8 @@ def test_linear_is_true_32_bit_and_row_independent():
         ops.linear(dev(a[rows]), dev(w), None, out, "store_f32")
         return out
 
-    big = run(list(range(300)))                           # 128 x 128 tiles
-    mid = run(list(range(20, 90)))                        # 64 x 64 tiles
+    big = run(list(range(300)))                           # the tensor cores
+    mid = run(list(range(20, 90)))
     assert torch.equal(big[33:34], mid[13:14])
     few, one = run(list(range(30, 39))), run([33])        # the weight stream, 9 rows and 1
     assert torch.equal(few[3:4], one)
@@ -144,6 +143,33 @@ def test_linear_is_true_32_bit_and_row_independent():
         out = torch.empty(m, 1, device="cuda")
         ops.linear(dev(a1), dev(w1), None, out, "store_f32")
         assert abs(out[0, 0].item() - 8 * (1 + 2.0 ** -20) ** 2) < 2e-6        # TF32 would give exactly 8
+
+
+def test_tiled_32_bit_product_sums_in_one_order():
+    """The CUDA cores' tiled kernel, which takes rows that are not in 16-byte pieces, 17 to 64 rows of K above 4096, and shapes that the bfloat16 engine's
+    tensor-core product refuses: the same bits whatever the company and the tile (64 x 64 or 128 x 128), and no TF32."""
+    ops = Ops(torch.float32)
+    ops.split_linear, ops.rows_linear_max = False, 0
+    g = torch.Generator().manual_seed(4)
+    for k in (96, 97):
+        a, w = torch.randn(300, k, generator=g), torch.randn(6000, k, generator=g)
+
+        def run(rows):
+            out = torch.empty(len(rows), 6000, device="cuda")
+            ops.linear(dev(a[rows]), dev(w), None, out, "store_f32")
+            return out
+
+        big, mid, few, one = run(list(range(300))), run(list(range(20, 90))), run(list(range(30, 39))), run([33])
+        for other in (mid[13:14], few[3:4], one):
+            assert torch.equal(big[33:34], other)
+        if k == 97:                                       # by itself too: 97 is no whole number of pieces
+            by_itself = torch.empty(300, 6000, device="cuda")
+            Ops(torch.float32).linear(dev(a), dev(w), None, by_itself, "store_f32")
+            assert torch.equal(by_itself, big)
+    for m in (1, 40, 300):
+        out = torch.empty(m, 1, device="cuda")
+        ops.linear(dev(torch.full((m, 8), 1.0 + 2.0 ** -20)), dev(torch.full((1, 8), 1.0 + 2.0 ** -20)), None, out, "store_f32")
+        assert (out.double() - 8 * (1 + 2.0 ** -20) ** 2).abs().max().item() < 2e-6        # TF32 would give exactly 8
 
 
 @pytest.mark.parametrize("m", [1, 3, 8, 64, 127, 129, 300])
