@@ -11,7 +11,7 @@
 // A block works 64 (token, head) pairs that share a key head - 64 / hp consecutive tokens of one sequence times hp heads of the
 // group, a warp 16 of them - against the cache's pages of 64 keys, by two halves of four warps that take the pages the block sees in
 // turn and put their sums together at the end (`layout_of`: or by one half alone).  What bounds it is the chain through one
-// warp, ~1000 instructions and 5000 cycles a page with the products' latency; more warps at once and half as many pages a warp is what helps, and
+// warp, more than 1000 instructions and 5000 cycles a page with the products' latency; more warps at once and half as many pages a warp is what helps, and
 // four warps a barrier, so that halves and blocks are out of step and one's softmax runs under another's products.  A page comes into
 // shared memory by cp.async while the one before is worked on (values that are the keys' first entries come once).  Queries stay in shared
 // memory, all of the running output in registers.  Rows are padded to an odd number of 16-byte pieces, so ldmatrix meets no bank twice.
@@ -409,7 +409,7 @@ Layout layout_of(int dk, int dv, bool alias) {
   z.k_stride = (dk + 15) / 16 * 16 + 8;
   z.v_stride = alias ? z.k_stride : (dv + 15) / 16 * 16 + 8;
   // Two halves where two such blocks fit an SM (values of up to 64 entries: 128 registers a thread), else one: two halves that are the SM's
-  // only block leave it idle where they begin and end.  (Measured, 2 x 1024 rows, two halves against one: 12 heads of 64: 36 us and 50; 32 heads of
+  // only block leave it idle where they begin and end.  (Measured when weights went through in two pieces, 2 x 1024 rows, two halves against one: 12 heads of 64: 36 us and 50; 32 heads of
   // 128 on 8: 148 and 112; 16 heads over a latent of 256: 152 and 108.)
   auto need = [&](int halves) {
     return ((size_t)ROWS * z.k_stride + 2 * halves * ((size_t)PAGE * z.k_stride + (alias ? 0 : (size_t)PAGE * z.v_stride)) + 256 + 16) * 2;
