@@ -1,80 +1,127 @@
 // Softmax attention of prompt rows over the paged cache with shaped scores (`attention_scored.cu` says what a score can be
-// given), on the tensor cores: bfloat16 queries, keys and values, 32-bit scores, softmax weights and sums.
+// given), on the 5th-generation tensor cores: bfloat16 queries, keys and values, 32-bit scores, softmax weights and sums.
 //
-//   s = q . k        mma.sync m16n8k16, 32-bit accumulation (products of bfloat16 numbers are exact)
-//   p = exp(s - m)   32-bit, in the accumulators' own registers
-//   o += p v         p is cut into three bfloat16 pieces, p = h + m + l exactly: a weight keeps its 24 bits, the pieces are
-//                    multiplied one after another.  The tensor core's truncating accumulation is kept to 64 keys, whose sum
-//                    then joins the 32-bit running sum by a rounded addition: over all pages it left the sums of 8 k even weights
-//                    8e-5 short.
+//   S = Q K^T        tcgen05.mma, 128 (token, head) pairs x 64 keys of a page, in tensor memory
+//   p = exp(s - m)   32-bit, m the page's own largest score of the row: a page's weights wait for no other page
+//   T = P V          p is cut into three bfloat16 pieces, p = h + m + l exactly (a weight keeps its 24 bits), which lie in tensor memory as the
+//                    product's first operand, the smallest first.  The tensor core's truncating accumulation is kept to one page,
+//   O = a O + b T    whose sum joins the 32-bit running sum in registers by rounded operations (a, b: 2^(old maximum - new), 2^(m - new))
 //
-// A block works 64 (token, head) pairs that share a key head - 64 / hp consecutive tokens of one sequence times hp heads of the
-// group, a warp 16 of them - against the cache's pages of 64 keys, by two halves of four warps that take the pages the block sees in
-// turn and put their sums together at the end (`layout_of`: or by one half alone).  What bounds it is the chain through one
-// warp, more than 1000 instructions and 5000 cycles a page with the products' latency; more warps at once and half as many pages a warp is what helps, and
-// four warps a barrier, so that halves and blocks are out of step and one's softmax runs under another's products.  A page comes into
-// shared memory by cp.async while the one before is worked on (values that are the keys' first entries come once).  Queries stay in shared
-// memory, all of the running output in registers.  Rows are padded to an odd number of 16-byte pieces, so ldmatrix meets no bank twice.
-// Pages that no pair of the block sees are skipped.  Tiles are launched longest first.
+// A block works 128 (token, head) pairs that share a key head: 128 / hp consecutive tokens of one sequence times hp heads of the group.
+// Roles, so that the tensor core's queue never waits for one thread's chain: one warp brings the queries once and the pages' keys and
+// values by TMA into a ring; one thread issues the products, S of up to two pages ahead of P V; NS groups of four warps turn the pages' scores
+// into weights (a thread a row, pages in turn); NA groups of four warps keep the running output (a thread a row and up to 128 of its
+// columns).  NS = 2, NA = 1 for values of up to 128 entries, where softmax takes the time; NS = 1, NA = 2 above, where the products do.
+// P V goes in pieces of columns through two or three places of tensor memory, so that one can be read while the next is worked out.
+// Pages that no pair of the block sees are skipped; tiles are launched longest first.  Every wait is bounded (`kvad_attention_scored_prompt_status`).
 //
-// Why: on the CUDA cores (`attention_scored.cu`) 2 x 1024 rows of 16 heads over a latent of 256 took 1102 us (15.6 TFLOP/s) and take 127 here,
-// 16 heads of 64 on 4 key heads with capped scores, gates and a window of 512 took 358 us and take 64.
+// What bounds it.  Keys and values of 256: a page takes 16 products of 128 x 64 x 16 (48 cycles each: both operands in shared memory) and 24 of
+// 128 x 128 x 16 (64), 2300 cycles, and runs in 2850.  Values of up to 64: the weights, ~1000 instructions a row and page, 1400 cycles a page; then the
+// start of a block (~5 us with the first page's chain), of which two go one after another where there are more than 148 tiles.
+// Graph-replayed launches, us: 2 x 1024 rows of 16 heads over a latent of 256: 1100 on the CUDA cores, 127 by mma.sync, 40 here; 16 heads of 64 on 4 key heads, capped,
+// window 512: 358, 55, 27; without cap and window 46, 23.  64 new rows of 4 sequences with 300 cached positions: latent 47.6, 17.7; 16 heads of 64: 15.4, 10.4; 2 new rows:
+// 38.4, 14.7; 12.3, 9.5.  The mma.sync kernel was ahead nowhere and is gone.  (On the way: products issued by a branch of one lane 64, by the
+// whole warp 50, S and P V by warps of their own with wide P V 40.)
 #include <algorithm>
 
-#include "common.cuh"
+#include "tcgen05.cuh"
 
 using namespace kvad;
 
 namespace {
 
-constexpr int PAGE = 64, WARPS = 4, HALF = 32 * WARPS, THREADS = 2 * HALF, ROWS = 16 * WARPS;
-constexpr size_t SMEM_MOST = 220 * 1024, SMEM_HALF = 112 * 1024;      // (a block's; so that two fit an SM)
+constexpr int PAGE = 64, ROWS = 128, THREADS = 512, MAX_STAGES = 4;
+constexpr int STATS = 8;             // pages whose statistics are kept: weights run up to two pages ahead of P V, P V up to three of the output
 constexpr float LOG2E = 1.4426950408889634f, LN2 = 0.6931471805599453f;
+constexpr uint32_t TM_COLS = 512;
+constexpr uint32_t Q_BLOCK = ROWS * 128, PAGE_BLOCK = PAGE * 128;      // 64 entries (128 bytes, swizzled) of the queries, of a page
+constexpr size_t SMEM_MOST = 226 * 1024, SMEM_REST = STATS * ROWS * 8 + 320 + 1024;      // (statistics, barriers, alignment)
 
 struct PromptArgs {
-  const __nv_bfloat16* q; int64_t ld_q;
   void* out; int64_t ld_out;
   const __nv_bfloat16* gate; int64_t ld_gate; int gate_heads;    // gate_heads: one number per row and head
   const float* sinks;
   const int* seq_starts; const int* kv_lens; const int* page_table; int table_width;
-  const __nv_bfloat16* k_pages; const __nv_bfloat16* v_pages;
-  int64_t k_page_stride, v_page_stride;                           // in entries; a head's page is PAGE x dk (PAGE x dv)
-  int n_heads, n_kv_heads, dk, dv, hp, alias, key_maps, halves;
+  int n_heads, n_kv_heads, dk, dv, hp, alias, key_maps, stages, vec;
   int columns;                                                    // tiles of one place in their sequence: sequences x heads / hp (the grid is these, the last place first)
   float scale, softcap, slope_span;
   float cap_in, cap_out;                                          // a capped score: cap_out * tanh(cap_in * (q . k)), in units of log2
   int window, keep_first, chunk;
-  int k_steps, k_stride, v_stride;                                // 16-entry steps of a key; row strides in shared memory, in entries
 };
 
-__device__ __forceinline__ uint32_t smem_at(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void ldsm4(uint32_t at, uint32_t (&r)[4]) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(at) : "memory");
+__device__ __forceinline__ void fence_async_shared() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void regs_more() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> __device__ __forceinline__ void regs_fewer() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+
+__device__ __forceinline__ void tmem_ld32(uint32_t addr, uint32_t* r) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+        "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+        "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(addr) : "memory");
 }
-__device__ __forceinline__ void ldsm4_t(uint32_t at, uint32_t (&r)[4]) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(at) : "memory");
+__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_st8(uint32_t addr, const uint32_t (&r)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+               ::"r"(addr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
 }
-__device__ __forceinline__ void mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// D += A B with A in tensor memory (a lane a row, two neighbours along K a column)
+__device__ __forceinline__ void umma_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
-// 16 bytes to shared memory, zeros where `live` is false (places of the cache that no row sees yet may hold anything)
-__device__ __forceinline__ void copy16(uint32_t dst, const void* src, bool live) {
-  const int bytes = live ? 16 : 0;
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+// Values as the second operand of P V: rows are keys (the product's K), 128 contiguous bytes are 64 of its columns.
+__device__ __forceinline__ uint64_t sw128_mn_desc(uint32_t smem_addr) {
+  uint64_t d = 0;
+  d |= (uint64_t)((smem_addr & 0x3FFFFu) >> 4);
+  d |= (uint64_t)((PAGE_BLOCK >> 4) & 0x3FFFu) << 16;        // leading byte offset: between blocks of 64 columns (one at a time is used)
+  d |= (uint64_t)(1024 >> 4) << 32;                          // stride byte offset: between groups of 8 keys
+  d |= (uint64_t)1 << 46;
+  d |= (uint64_t)2 << 61;                                    // SWIZZLE_128B
+  return d;
 }
-// 2^x by the special-function unit (2 units in the last place; a weight below 2^-126 of its row's largest is zero).  With it a 32-bit output is off
-// by 1.4e-7 (16 heads of 64) to 1.8e-7 (a latent of 128) over 1024 rows, the CUDA-core kernel's by 2.6e-7 to 3.2e-7.
+
+// Two 32-bit numbers at once (an instruction for both).
+__device__ __forceinline__ uint64_t pair(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpair(uint64_t r, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(r)); }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+// 2^x by the special-function unit (2 units in the last place; a weight below 2^-126 of its row's largest is zero).
 __device__ __forceinline__ float exp2_fast(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+// 1 / (1 + 2^(-z log2 e)) by the special-function unit (3 units in the last place, before a rounding to bfloat16).
+__device__ __forceinline__ float sigmoid_fast(float z) { return __fdividef(1.0f, 1.0f + exp2_fast(-z * LOG2E)); }
 // The upper halves of two floats as a pair of bfloat16 (truncated), and what is left of each.
 __device__ __forceinline__ uint32_t cut(float& a, float& b) {
   const uint32_t x = __float_as_uint(a), y = __float_as_uint(b);
-  a -= __uint_as_float(x & 0xffff0000u);
-  b -= __uint_as_float(y & 0xffff0000u);
+  unpair(add2(pair(a, b), pair(-__uint_as_float(x & 0xffff0000u), -__uint_as_float(y & 0xffff0000u))), a, b);
   return __byte_perm(x, y, 0x7632);
 }
 __device__ __forceinline__ uint32_t pack(float a, float b) {
@@ -82,357 +129,458 @@ __device__ __forceinline__ uint32_t pack(float a, float b) {
   return *reinterpret_cast<const uint32_t*>(&v);
 }
 
-// NV: 16-entry groups of a value.
-template <int NV, bool F32OUT>
-__global__ void __launch_bounds__(NV <= 4 ? THREADS : HALF, 2) scored_prompt_kernel(const PromptArgs a) {
+// tanh(y) = y + y^3 P(y^2) up to |y| = 0.45 (P fitted to (tanh(y) / y - 1) / y^2 by reweighted least squares: off by 5e-9 of tanh).
+constexpr float TANH_NEAR = 0.45f, TANH0 = -0.3333325f, TANH1 = 0.13329249f, TANH2 = -0.05334366f, TANH3 = 0.01802476f;
+
+// NS: groups of four warps that turn scores into weights; CPW: 64-column pieces of the output that a group of four warps keeps.
+template <int NS, int CPW, bool F32OUT>
+__global__ void __launch_bounds__(THREADS, 1)
+scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const PromptArgs a) {
+  // Tensor-memory columns: the places of P V, S of two pages (64 each), the weights' pieces of two pages (32 columns each: two bfloat16 a column).  With values
+  // above 128 entries P V takes two places of 128 (products 128 wide leave the issuing warp time for its waits), and the third piece takes its page's S' place.
+  constexpr bool S_IS_P = NS == 1;
+  constexpr int CW = NS == 1 ? 128 : 64, SLOTS = NS == 1 ? 2 : 3;
+  constexpr uint32_t TM_T = 0, TM_S = SLOTS * CW, TM_P = TM_S + 128, P_STEP = S_IS_P ? 64 : 96;
+  static_assert(TM_P + 2 * P_STEP <= TM_COLS, "tensor memory");
   extern __shared__ uint8_t smem_raw[];
-  __nv_bfloat16* smem = reinterpret_cast<__nv_bfloat16*>(smem_raw);
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  const int k_blocks = (a.dk + 63) / 64, v_blocks = (a.dv + 63) / 64, n_chunks = (a.dv + CW - 1) / CW, stages = a.stages;
+  const uint32_t k_bytes = k_blocks * PAGE_BLOCK, stage_bytes = k_bytes + (a.alias ? 0 : v_blocks * PAGE_BLOCK);
+  uint8_t* q_tile = smem;
+  uint8_t* ring = smem + k_blocks * Q_BLOCK;                      // stage: keys, then values (or none: the keys)
+  float2* stats = reinterpret_cast<float2*>(ring + stages * stage_bytes);      // [STATS][ROWS] a page's largest score and sum of weights, per row
+  uint64_t* q_full = reinterpret_cast<uint64_t*>(stats + STATS * ROWS);
+  uint64_t* kv_full = q_full + 1;                                 // [stages] a page has come
+  uint64_t* kv_empty = kv_full + MAX_STAGES;                      // [stages] it has been used up
+  uint64_t* s_full = kv_empty + MAX_STAGES;                       // [2] S is in tensor memory
+  uint64_t* s_empty = s_full + 2;                                 // [2] S has been read
+  uint64_t* p_full = s_empty + 2;                                 // [2] the weights' pieces are in tensor memory
+  uint64_t* p_empty = p_full + 2;                                 // [2] P V has read them
+  uint64_t* st_full = p_empty + 2;                                // [STATS] a page's statistics are there
+  uint64_t* t_full = st_full + STATS;                                 // [3] a piece of P V is in tensor memory
+  uint64_t* t_empty = t_full + 3;                                 // [3] it has been read
+  uint64_t* drain = t_empty + 3;                                  // [2] the products that were issued before a wait ran out
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 2);
   const int hp = a.hp, tok = ROWS / hp, group = a.n_heads / a.n_kv_heads, chunks = group / hp;
   const int per_seq = a.n_kv_heads * chunks, from_end = blockIdx.x / a.columns, column = blockIdx.x - from_end * a.columns;
   const int s = column / per_seq, part = column - s * per_seq, kvh = part / chunks, h0 = kvh * group + (part - kvh * chunks) * hp;
-  const int half = threadIdx.x / HALF, tid = threadIdx.x - half * HALF, lane = tid & 31, warp = tid >> 5;      // (tid, warp: within the half)
-  const int kst = a.k_stride, vst = a.v_stride;
-  __nv_bfloat16* Qs = smem;                                     // [ROWS][kst]
-  const int stage_size = PAGE * kst + (a.alias ? 0 : PAGE * vst);
-  __nv_bfloat16* stages = Qs + ROWS * kst + half * 2 * stage_size;      // each half: two of: keys [PAGE][kst], values [PAGE][vst] (or none: the keys)
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   pdl_launch_dependents();
-  // The last step's entries past the key that no copy writes must not be NaN: zeros.  (Values past the last reach only outputs that are not written.)
-  if (a.dk % 16 != 0) {
-    for (int i = tid; i < ROWS + 2 * PAGE; i += HALF) {
-      __nv_bfloat16* at = i < ROWS ? Qs + i * kst : stages + ((i - ROWS) / PAGE) * stage_size + ((i - ROWS) % PAGE) * kst;
-      *reinterpret_cast<uint4*>(at + a.dk) = make_uint4(0u, 0u, 0u, 0u);
-    }
+  if (threadIdx.x == 0) {
+    prefetch_tensormap(&map_q);
+    prefetch_tensormap(&map_k);
+    prefetch_tensormap(&map_v);
+    mbar_init(q_full, 1);
+    for (int i = 0; i < MAX_STAGES; ++i) { mbar_init(&kv_full[i], 1); mbar_init(&kv_empty[i], 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&s_full[i], 1); mbar_init(&s_empty[i], 128); mbar_init(&p_full[i], 128); mbar_init(&p_empty[i], 1); }
+    for (int i = 0; i < STATS; ++i) mbar_init(&st_full[i], 128);
+    for (int i = 0; i < 3; ++i) { mbar_init(&t_full[i], 1); mbar_init(&t_empty[i], 128); }
+    for (int i = 0; i < 2; ++i) mbar_init(&drain[i], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    fence_async_shared();
   }
   pdl_wait();
   const int start = a.seq_starts[s], n_new = a.seq_starts[s + 1] - start, tok0 = ((int)gridDim.x / a.columns - 1 - from_end) * tok;
   if (tok0 >= n_new) return;
-  const int n_tok = min(tok, n_new - tok0), pos0 = a.kv_lens[s] - n_new + tok0, last_pos = pos0 + n_tok - 1;
-  const int* pages = a.page_table + (int64_t)s * a.table_width;
-  const int q_pieces = a.dk / 8, v_pieces = a.dv / 8;
-  for (int i = threadIdx.x; i < ROWS * q_pieces; i += blockDim.x) {
-    const int r = i / q_pieces, c = i - r * q_pieces, ti = r / hp, hi = r - ti * hp;
-    const bool live = ti < n_tok;
-    copy16(smem_at(Qs + r * kst + c * 8), a.q + (int64_t)(start + tok0 + (live ? ti : 0)) * a.ld_q + (int64_t)(h0 + hi) * a.dk + c * 8, live);
-  }
+  const int kv_len = a.kv_lens[s];
+  if (warp == 1) tmem_alloc(tmem_slot, TM_COLS);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  const int n_tok = min(tok, n_new - tok0), pos0 = kv_len - n_new + tok0, last_pos = pos0 + n_tok - 1;
   const int first_key = a.chunk > 0 ? pos0 - pos0 % a.chunk : ((a.window > 0 && pos0 - a.window + 1 > 0) ? pos0 - a.window + 1 : 0);   // of the block's first token
-  auto next_page = [&](int t) {                                 // the next page that a pair of the block sees (the same for every thread)
+  auto next_page = [&](int t) {                                   // the next page that a pair of the block sees (the same for every thread)
     while (t * PAGE <= last_pos && t * PAGE + PAGE <= first_key && t * PAGE >= a.keep_first) ++t;
     return t;
   };
-  // A thread steps from one of its pieces to the next by additions (a division a piece cost as much as the scores); where registers are to spare the
-  // first step is worked out once, not once a page.
-  struct Steps { int r, c, rows, rest; };
-  auto steps_of = [&](int pieces) {
-    const int rows = HALF / pieces, r = tid / pieces;
-    return Steps{r, tid - r * pieces, rows, HALF - rows * pieces};
-  };
-  constexpr bool ONCE = NV == 8;
-  const Steps k_once = ONCE ? steps_of(q_pieces) : Steps{}, v_once = ONCE ? steps_of(v_pieces) : Steps{};
-  auto bring_rows = [&](__nv_bfloat16* dst, int stride, const __nv_bfloat16* src, int pieces, const Steps& z, int n_live) {
-    int r = z.r, c = z.c;
-#pragma unroll 4
-    for (int i = tid; i < PAGE * pieces; i += HALF) {
-      copy16(smem_at(dst + r * stride + c * 8), src + (int64_t)i * 8, r < n_live);
-      r += z.rows;
-      c += z.rest;
-      if (c >= pieces) { c -= pieces; ++r; }
-    }
-  };
-  auto bring = [&](int t, int stage) {
-    const int page = pages[t], n_live = last_pos - t * PAGE + 1;
-    __nv_bfloat16* ks = stages + stage * stage_size;
-    const __nv_bfloat16* src = a.k_pages + (int64_t)page * a.k_page_stride + (int64_t)kvh * PAGE * a.dk;
-    bring_rows(ks, kst, src, q_pieces, ONCE ? k_once : steps_of(q_pieces), n_live);
-    if (!a.alias) {
-      __nv_bfloat16* vs = ks + PAGE * kst;
-      const __nv_bfloat16* vsrc = a.v_pages + (int64_t)page * a.v_page_stride + (int64_t)(kvh / a.key_maps) * PAGE * a.dv;
-      bring_rows(vs, vst, vsrc, v_pieces, ONCE ? v_once : steps_of(v_pieces), n_live);
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
 
-  // this thread's two rows of the warp's 16: lane / 4 and that plus 8
-  int pos[2], first[2], head[2];
-  bool live[2];
-  float slope[2], run_max[2] = {-INFINITY, -INFINITY}, run_sum[2] = {0.f, 0.f};      // (maxima in units of log2)
-#pragma unroll
-  for (int u = 0; u < 2; ++u) {
-    const int row = warp * 16 + (lane >> 2) + u * 8, ti = row / hp;
-    head[u] = h0 + row - ti * hp;
-    live[u] = ti < n_tok;
-    pos[u] = pos0 + ti;
-    first[u] = a.window > 0 ? pos[u] - a.window + 1 : (a.chunk > 0 ? pos[u] - pos[u] % a.chunk : 0);
-    slope[u] = a.slope_span > 0.f ? exp2f(-a.slope_span * (float)(head[u] + 1) / (float)a.n_heads) * LOG2E : 0.f;
-  }
-  // keys from `clear_from` up to `clear_to` (and the kept first ones) are seen by every live row of the warp
-  const int warp_ti0 = warp * 16 / hp, warp_ti1 = min((warp * 16 + 15) / hp, n_tok - 1);
-  const bool warp_live = warp_ti0 < n_tok;
-  const int clear_to = pos0 + warp_ti0;
-  const int far = pos0 + warp_ti1;
-  const int clear_from = a.window > 0 ? far - a.window + 1 : (a.chunk > 0 ? far - far % a.chunk : 0);
-  float o[2 * NV][4];
-#pragma unroll
-  for (int j = 0; j < 2 * NV; ++j)
-#pragma unroll
-    for (int e = 0; e < 4; ++e) o[j][e] = 0.f;
-  const float scale2 = a.scale * LOG2E;
-  const bool plain = !(a.softcap > 0.f) && !(a.slope_span > 0.f) && a.scale > 0.f;
-  const float unit = plain ? scale2 : 1.f;
-  const uint32_t q_at = smem_at(Qs + (warp * 16 + (lane & 15)) * kst + (lane >> 4) * 8);
-
-  // the pages that the block sees, dealt out to the halves in turn
-  int t = next_page(0), stage = 0;
-  if (half == 1) t = next_page(t + 1);
-  if (t * PAGE <= last_pos) bring(t, 0);
-  asm volatile("cp.async.wait_all;" ::: "memory");              // (a half without pages has queries on their way)
-  __syncthreads();                                              // the queries, brought by both halves, and each half's first page
-  bool first_page = true;
-  while (t * PAGE <= last_pos) {
-    if (!first_page) {
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
-      if (half == 0) asm volatile("bar.sync 1, %0;" ::"n"(HALF) : "memory");      // this page is there, and the one before has been used up
-      else asm volatile("bar.sync 2, %0;" ::"n"(HALF) : "memory");
-    }
-    first_page = false;
-    int t_next = next_page(t + 1);
-    if (a.halves == 2) t_next = next_page(t_next + 1);
-    if (t_next * PAGE <= last_pos) bring(t_next, stage ^ 1);
-    const int key0 = t * PAGE;
-    const __nv_bfloat16* ks = stages + stage * stage_size;
-    const __nv_bfloat16* vs = a.alias ? ks : ks + PAGE * kst;
-    t = t_next;
-    stage ^= 1;
-    if (!warp_live) continue;
-    float sc[8][4];
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) sc[j][e] = 0.f;
-    const uint32_t k_at = smem_at(ks + ((lane & 7) + (lane >> 4) * 8) * kst + ((lane >> 3) & 1) * 8);
-#pragma unroll 2
-    for (int kk = 0; kk < a.k_steps; ++kk) {
-      uint32_t qa[4];
-      ldsm4(q_at + kk * 32, qa);
-#pragma unroll
-      for (int ng = 0; ng < 4; ++ng) {
-        uint32_t kb[4];
-        ldsm4(k_at + kk * 32 + ng * 16 * kst * 2, kb);
-        mma(sc[2 * ng], qa, kb[0], kb[1]);
-        mma(sc[2 * ng + 1], qa, kb[2], kb[3]);
-      }
-    }
-    // Scores in units of log2, or, where nothing but a positive factor is on them, as they are with the factor `unit` still owed.
-    // (Whole passes over the 32 scores under tests that are the same for every thread: this part is bound by instructions.)
-    if (!plain) {
-      if (a.softcap > 0.f) {                                    // cap tanh(s / cap): by `tanhf`, whose error follows its result (1 - 2 / (exp(2 y) + 1): off by 2^-22 of the CAP)
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-#pragma unroll
-          for (int e = 0; e < 4; ++e)
-            sc[j][e] = a.cap_out * tanhf(sc[j][e] * a.cap_in);
-      } else {
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) sc[j][e] *= scale2;
-      }
-      if (a.slope_span > 0.f) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) sc[j][e] -= slope[e >> 1] * (float)(pos[e >> 1] - (key0 + j * 8 + (lane & 3) * 2 + (e & 1)));
-      }
-    }
-    if (!(key0 + PAGE - 1 <= clear_to && (key0 >= clear_from || key0 + PAGE <= a.keep_first))) {      // some pair does not see all of the page
-#pragma unroll
-      for (int j = 0; j < 8; ++j)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int u = e >> 1, key = key0 + j * 8 + (lane & 3) * 2 + (e & 1);
-          if (!(key <= pos[u] && (key >= first[u] || key < a.keep_first))) sc[j][e] = -INFINITY;
+  if (warp < 4) {
+    regs_fewer<40>();
+    if (warp == 0 && lane == 0) {
+      const int* pages = a.page_table + (int64_t)s * a.table_width;
+      int t = next_page(0), page_next = pages[t];
+      mbar_expect_tx(q_full, k_blocks * Q_BLOCK);
+      for (int b = 0; b < k_blocks; ++b) tma_load_3d(q_tile + b * Q_BLOCK, &map_q, q_full, b * 64, h0, start + tok0);
+      int j = 0, st = 0;
+      uint32_t turn = 0;
+      bool ok = true;
+      for (int t_next; t * PAGE <= last_pos; t = t_next, ++j) {
+        const int page = page_next;                               // (a page's place is looked up one page ahead)
+        t_next = next_page(t + 1);
+        if (t_next * PAGE <= last_pos) page_next = pages[t_next];
+        if (j >= stages && !mbar_wait(&kv_empty[st], turn ^ 1)) { ok = false; break; }
+        uint8_t* at = ring + st * stage_bytes;
+        mbar_expect_tx(&kv_full[st], stage_bytes);
+        const int y = (page * a.n_kv_heads + kvh) * PAGE;
+        for (int b = 0; b < k_blocks; ++b) tma_load_2d(at + b * PAGE_BLOCK, &map_k, &kv_full[st], b * 64, y);
+        if (!a.alias) {
+          const int yv = (page * (a.n_kv_heads / a.key_maps) + kvh / a.key_maps) * PAGE;
+          for (int b = 0; b < v_blocks; ++b) tma_load_2d(at + k_bytes + b * PAGE_BLOCK, &map_v, &kv_full[st], b * 64, yv);
         }
-    }
-    float top[2] = {-INFINITY, -INFINITY};
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) top[e >> 1] = fmaxf(top[e >> 1], sc[j][e]);
-    float base[2], keep[2], sum[2] = {0.f, 0.f};
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      top[u] = fmaxf(top[u], __shfl_xor_sync(0xffffffffu, top[u], 1));
-      top[u] = fmaxf(top[u], __shfl_xor_sync(0xffffffffu, top[u], 2));
-      const float new_max = fmaxf(run_max[u], top[u] * unit);
-      base[u] = new_max == -INFINITY ? 0.f : new_max;
-      keep[u] = run_max[u] == -INFINITY ? 0.f : exp2_fast(run_max[u] - base[u]);
-      run_max[u] = new_max;
-    }
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int u = e >> 1;
-        sc[j][e] = exp2_fast(fmaf(sc[j][e], unit, -base[u]));
-        sum[u] += sc[j][e];
+        if (++st == stages) { st = 0; turn ^= 1; }
       }
-#pragma unroll
-    for (int u = 0; u < 2; ++u) run_sum[u] = run_sum[u] * keep[u] + sum[u];      // (of this thread's keys; the row's four threads meet at the end)
-    const uint32_t v_at = smem_at(vs + ((lane & 7) + ((lane >> 3) & 1) * 8) * vst + (lane >> 4) * 8);
-    uint32_t ph[4][4], pm[4][4], pl[4][4];
-#pragma unroll
-    for (int kk = 0; kk < 4; ++kk)
-#pragma unroll
-      for (int f = 0; f < 4; ++f) {
-        float x = sc[2 * kk + (f >> 1)][(f & 1) * 2], y = sc[2 * kk + (f >> 1)][(f & 1) * 2 + 1];
-        ph[kk][f] = cut(x, y);
-        pm[kk][f] = cut(x, y);
-        pl[kk][f] = pack(x, y);
+      if (!ok) {                                                  // (copies in flight must not outlive the block)
+        mbar_wait(q_full, 0);
+        for (int i = 0; i < min(j, stages); ++i) mbar_wait(&kv_full[i], i < st ? turn : turn ^ 1);
       }
+    } else if (warp == 1) {                                       // S = Q K^T (the whole warp, its elected lane issues: see elect_one)
+      const int k_steps = (a.dk + 15) / 16;
+      const uint32_t idesc = umma_instr_desc(ROWS, PAGE);
+      const uint64_t q_desc = sw128_desc(smem_u32(q_tile)), k_desc = sw128_desc(smem_u32(ring));
+      const uint32_t stage_step = stage_bytes >> 4;               // (descriptors count sixteens of bytes)
+      const bool one = elect_one();
+      bool ok = mbar_wait(q_full, 0);
+      int j = 0, st = 0;
+      uint32_t turn = 0;
+      for (int t = next_page(0); t * PAGE <= last_pos && ok; t = next_page(t + 1), ++j) {
+        const int b = j & 1;
+        if (!mbar_wait(&kv_full[st], turn) || (j >= 2 && !mbar_wait(S_IS_P ? &p_empty[b] : &s_empty[b], ((j >> 1) & 1) ^ 1))) { ok = false; break; }
+        tc_fence_after();
+        const uint64_t k_at = k_desc + st * stage_step;
+        const uint32_t d = tmem_base + TM_S + b * 64;
+        if (one) {
+          int left = k_steps;
+          for (int kb = 0; kb < k_blocks; ++kb, left -= 4) {
+            const uint64_t qd = q_desc + kb * (Q_BLOCK >> 4), kd = k_at + kb * (PAGE_BLOCK >> 4);
+            if (left >= 4) {
 #pragma unroll
-    for (int ng = 0; ng < NV; ++ng) {
-      float low[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}}, page[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-#pragma unroll
-      for (int kk = 0; kk < 4; ++kk) {
-        uint32_t vb[4];
-        ldsm4_t(v_at + kk * 16 * vst * 2 + ng * 32, vb);
-#pragma unroll
-        for (int w = 0; w < 2; ++w) mma(low[w], pl[kk], vb[2 * w], vb[2 * w + 1]);
-#pragma unroll
-        for (int w = 0; w < 2; ++w) mma(page[w], ph[kk], vb[2 * w], vb[2 * w + 1]);
-#pragma unroll
-        for (int w = 0; w < 2; ++w) mma(low[w], pm[kk], vb[2 * w], vb[2 * w + 1]);
+              for (int k = 0; k < 4; ++k) umma(d, qd + k * 2, kd + k * 2, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+            } else {
+              for (int k = 0; k < left; ++k) umma(d, qd + k * 2, kd + k * 2, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+            }
+          }
+          umma_commit(&s_full[b]);
+        }
+        if (++st == stages) { st = 0; turn ^= 1; }
       }
-#pragma unroll
-      for (int w = 0; w < 2; ++w)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) o[2 * ng + w][e] = fmaf(o[2 * ng + w][e], keep[e >> 1], page[w][e] + low[w][e]);
-    }
-  }
-
-  // The second half's sums join the first's: its threads hold the same rows and entries.
-#pragma unroll
-  for (int u = 0; u < 2; ++u) {
-    run_sum[u] += __shfl_xor_sync(0xffffffffu, run_sum[u], 1);
-    run_sum[u] += __shfl_xor_sync(0xffffffffu, run_sum[u], 2);
-  }
-  if (a.halves == 2) {
-    float* meet = reinterpret_cast<float*>(smem_raw) + tid;
-    __syncthreads();                                              // nobody reads queries or pages any more
-    if (half == 1) {
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        meet[u * HALF] = run_max[u];
-        meet[(2 + u) * HALF] = run_sum[u];
+      if (!ok) {                                                  // (products in flight must not outlive the block's tensor memory)
+        if (one) umma_commit(&drain[0]);
+        mbar_wait(&drain[0], 0);
       }
+    } else if (warp == 2) {                                       // T = P V, by another warp: a wait takes a hundred cycles even when it is over
+      const uint64_t v_desc = sw128_mn_desc(smem_u32(ring) + (a.alias ? 0u : k_bytes));
+      const uint32_t stage_step = stage_bytes >> 4;
+      const bool one = elect_one();
+      bool ok = true;
+      int i = 0, st = 0, slot = 0, g = 0;
+      uint32_t slot_turn = 0;
+      for (int t = next_page(0); t * PAGE <= last_pos && ok; t = next_page(t + 1), ++i) {
+        const int b = i & 1;
+        if (!mbar_wait(&p_full[b], (i >> 1) & 1)) { ok = false; break; }
+        const uint32_t p_at = tmem_base + TM_P + b * P_STEP, low_at = tmem_base + (S_IS_P ? TM_S + b * 64 : TM_P + b * P_STEP + 64);
+        const uint64_t v_at = v_desc + st * stage_step;
+        for (int c = 0; c < n_chunks; ++c, ++g) {
+          if (g >= SLOTS && !mbar_wait(&t_empty[slot], slot_turn ^ 1)) { ok = false; break; }
+          tc_fence_after();
+          const uint32_t idesc = umma_instr_desc(ROWS, min(CW, (a.dv - c * CW + 15) & ~15), false, true), d = tmem_base + TM_T + slot * CW;
+          const uint64_t vd = v_at + c * (CW / 64) * (PAGE_BLOCK >> 4);
+          if (one) {
 #pragma unroll
-      for (int j = 0; j < 2 * NV; ++j)
+            for (int kk = 0; kk < 4; ++kk) umma_ta(d, low_at + kk * 8, vd + kk * (2048 >> 4), idesc, kk > 0 ? 1u : 0u);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) meet[(4 + j * 4 + e) * HALF] = o[j][e];
+            for (int kk = 0; kk < 4; ++kk) umma_ta(d, p_at + 32 + kk * 8, vd + kk * (2048 >> 4), idesc, 1u);
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk) umma_ta(d, p_at + kk * 8, vd + kk * (2048 >> 4), idesc, 1u);
+            umma_commit(&t_full[slot]);
+          }
+          if (++slot == SLOTS) { slot = 0; slot_turn ^= 1; }
+        }
+        if (!ok) break;
+        if (one) {
+          umma_commit(&p_empty[b]);
+          umma_commit(&kv_empty[st]);
+        }
+        if (++st == stages) st = 0;
+      }
+      if (!ok) {
+        if (one) umma_commit(&drain[1]);
+        mbar_wait(&drain[1], 0);
+      }
     }
-    __syncthreads();
-    if (half == 1) return;
-    float mine[2], theirs[2];
+  } else if (warp < 4 + 4 * NS) {
+    // ---- scores into weights: a thread a row
+    if (NS == 2) { if (CPW == 1) regs_more<176>(); else regs_more<152>(); } else regs_more<136>();
+    const int mine = (warp >> 2) - 1, quarter = warp & 3, row = quarter * 32 + lane;
+    const uint32_t lanes = tmem_base + ((uint32_t)(quarter * 32) << 16);
+    const int ti = row / hp, pos = pos0 + ti;
+    const int first = a.window > 0 ? pos - a.window + 1 : (a.chunk > 0 ? pos - pos % a.chunk : 0);
+    const float slope = a.slope_span > 0.f ? exp2f(-a.slope_span * (float)(h0 + row - ti * hp + 1) / (float)a.n_heads) * LOG2E : 0.f;
+    // keys from `clear_from` up to `clear_to` (and the kept first ones) are seen by every live row of the warp
+    const int clear_to = pos0 + quarter * 32 / hp, far = pos0 + min((quarter * 32 + 31) / hp, n_tok - 1);
+    const int clear_from = a.window > 0 ? far - a.window + 1 : (a.chunk > 0 ? far - far % a.chunk : 0);
+    const float scale2 = a.scale * LOG2E;
+    const bool plain = !(a.softcap > 0.f) && !(a.slope_span > 0.f) && a.scale > 0.f;
+    const float unit = plain ? scale2 : 1.f;
+    const uint64_t unit2 = pair(unit, unit);
+    int t = next_page(0), j = mine;
+    if (mine == 1) t = next_page(t + 1);
+    for (; t * PAGE <= last_pos; j += NS) {
+      const int b = j & 1, key0 = t * PAGE;
+      const uint32_t turn = (j >> 1) & 1;
+      if (!mbar_wait(&s_full[b], turn)) break;
+      tc_fence_after();
+      float sc[64];
+      {
+        uint32_t* raw = reinterpret_cast<uint32_t*>(sc);
+        tmem_ld32(lanes + TM_S + b * 64, raw);
+        tmem_ld32(lanes + TM_S + b * 64 + 32, raw + 32);
+        tmem_ld_wait();
+      }
+      tc_fence_before();
+      if (!S_IS_P) mbar_arrive_one(&s_empty[b]);
+      // Scores in units of log2, or, where nothing but a positive factor is on them, as they are with the factor `unit` still owed.
+      if (!plain) {
+        if (a.softcap > 0.f) {
+          float most = 0.f;
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const float their_max = meet[u * HALF], m = fmaxf(run_max[u], their_max), base = m == -INFINITY ? 0.f : m;
-      mine[u] = exp2_fast(run_max[u] - base);
-      theirs[u] = exp2_fast(their_max - base);
-      run_sum[u] = run_sum[u] * mine[u] + meet[(2 + u) * HALF] * theirs[u];
-      run_max[u] = m;
-    }
+          for (int c = 0; c < 64; ++c) most = fmaxf(most, fabsf(sc[c]));
+          if (__any_sync(0xffffffffu, most * fabsf(a.cap_in) > TANH_NEAR)) {
 #pragma unroll
-    for (int j = 0; j < 2 * NV; ++j)
+            for (int c = 0; c < 64; ++c) sc[c] = a.cap_out * tanhf(sc[c] * a.cap_in);
+          } else {
+            const uint64_t in2 = pair(a.cap_in, a.cap_in), out2 = pair(a.cap_out, a.cap_out);
 #pragma unroll
-      for (int e = 0; e < 4; ++e) o[j][e] = o[j][e] * mine[e >> 1] + meet[(4 + j * 4 + e) * HALF] * theirs[e >> 1];
-  }
-
-#pragma unroll
-  for (int u = 0; u < 2; ++u) {
-    if (!live[u]) continue;
-    const int row = warp * 16 + (lane >> 2) + u * 8, h = head[u];
-    const int64_t grow = start + tok0 + row / hp;
-    float inv;
-    if (a.sinks == nullptr) {
-      inv = 1.0f / run_sum[u];
-    } else {                                                    // a sink is one more term of the denominator
-      const float mine = run_max[u] * LN2, sink = a.sinks[h], m = fmaxf(mine, sink), f = expf(mine - m);
-      inv = f / fmaf(run_sum[u], f, expf(sink - m));
-    }
-    float head_factor = 1.f;
-    if (a.gate != nullptr && a.gate_heads) head_factor = 1.0f / (1.0f + expf(-__bfloat162float(a.gate[grow * a.ld_gate + h])));
-#pragma unroll
-    for (int j = 0; j < 2 * NV; ++j) {
-      const int d = j * 8 + (lane & 3) * 2;                     // (dv is a multiple of 8)
-      if (d >= a.dv) continue;
-      float x = o[j][2 * u] * inv, y = o[j][2 * u + 1] * inv;
-      if (F32OUT) {
-        *reinterpret_cast<float2*>(reinterpret_cast<float*>(a.out) + grow * a.ld_out + (int64_t)h * a.dv + d) = make_float2(x, y);
-      } else {
-        if (a.gate != nullptr && !a.gate_heads) {
-          const __nv_bfloat162 z = *reinterpret_cast<const __nv_bfloat162*>(a.gate + grow * a.ld_gate + (int64_t)h * a.dv + d);
-          x *= 1.0f / (1.0f + expf(-__bfloat162float(z.x)));
-          y *= 1.0f / (1.0f + expf(-__bfloat162float(z.y)));
+            for (int c = 0; c < 64; c += 2) {
+              const uint64_t y = mul2(pair(sc[c], sc[c + 1]), in2), z = mul2(y, y);
+              uint64_t p = fma2(z, pair(TANH3, TANH3), pair(TANH2, TANH2));
+              p = fma2(z, p, pair(TANH1, TANH1));
+              p = fma2(z, p, pair(TANH0, TANH0));
+              unpair(mul2(out2, fma2(mul2(y, z), p, y)), sc[c], sc[c + 1]);
+            }
+          }
         } else {
-          x *= head_factor;
-          y *= head_factor;
+#pragma unroll
+          for (int c = 0; c < 64; ++c) sc[c] *= scale2;
         }
-        *reinterpret_cast<uint32_t*>(reinterpret_cast<__nv_bfloat16*>(a.out) + grow * a.ld_out + (int64_t)h * a.dv + d) = pack(x, y);
+        if (a.slope_span > 0.f) {
+#pragma unroll
+          for (int c = 0; c < 64; ++c) sc[c] -= slope * (float)(pos - (key0 + c));
+        }
+      }
+      if (!(key0 + PAGE - 1 <= clear_to && (key0 >= clear_from || key0 + PAGE <= a.keep_first))) {      // some pair does not see all of the page
+        const int hi = pos - key0, lo = first - key0, kept = a.keep_first - key0;
+        uint64_t see = hi < 0 ? 0ull : (hi >= 63 ? ~0ull : (2ull << hi) - 1ull);
+        const uint64_t below = lo <= 0 ? 0ull : (lo >= 64 ? ~0ull : (1ull << lo) - 1ull);
+        const uint64_t held = kept <= 0 ? 0ull : (kept >= 64 ? ~0ull : (1ull << kept) - 1ull);
+        see &= ~below | held;
+        const uint32_t see0 = (uint32_t)see, see1 = (uint32_t)(see >> 32);
+#pragma unroll
+        for (int c = 0; c < 32; ++c) {
+          if (!(see0 >> c & 1)) sc[c] = -INFINITY;
+          if (!(see1 >> c & 1)) sc[32 + c] = -INFINITY;
+        }
+      }
+      float top[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+      for (int c = 0; c < 64; ++c) top[c & 3] = fmaxf(top[c & 3], sc[c]);
+      const float most = fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3])) * unit, base = most == -INFINITY ? 0.f : most;
+      if (j >= 2 && !mbar_wait(&p_empty[b], turn ^ 1)) break;
+      tc_fence_after();
+      const uint64_t less = pair(-base, -base);
+      uint64_t sum2[2] = {0ull, 0ull};
+      const uint32_t p_at = lanes + TM_P + b * P_STEP, low_at = S_IS_P ? lanes + TM_S + b * 64 : p_at + 64;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        uint32_t ph[8], pm[8], pl[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          float x, y;
+          unpair(fma2(pair(sc[q * 16 + 2 * e], sc[q * 16 + 2 * e + 1]), unit2, less), x, y);
+          x = exp2_fast(x);
+          y = exp2_fast(y);
+          sum2[e & 1] = add2(sum2[e & 1], pair(x, y));
+          ph[e] = cut(x, y);
+          pm[e] = cut(x, y);
+          pl[e] = pack(x, y);
+        }
+        tmem_st8(p_at + q * 8, ph);
+        tmem_st8(p_at + 32 + q * 8, pm);
+        tmem_st8(low_at + q * 8, pl);
+      }
+      float s0, s1;
+      unpair(add2(sum2[0], sum2[1]), s0, s1);
+      stats[(j % STATS) * ROWS + row] = make_float2(most, s0 + s1);
+      mbar_arrive_one(&st_full[j % STATS]);
+      // Places past the sequence's end may hold anything: no weight is on them, but their values must not be NaN.
+      const int valid = kv_len - key0;
+      if (valid < PAGE) {
+        const int st = j % stages;
+        if (!mbar_wait(&kv_full[st], (j / stages) & 1)) break;
+        uint8_t* v_tile = ring + st * stage_bytes + (a.alias ? 0 : k_bytes);
+        for (int vb = 0; vb < v_blocks; ++vb)
+          for (int x = row; x < (PAGE - valid) * 8; x += 128) *reinterpret_cast<uint4*>(v_tile + vb * PAGE_BLOCK + valid * 128 + x * 16) = make_uint4(0u, 0u, 0u, 0u);
+        fence_async_shared();
+      }
+      tmem_st_wait();
+      tc_fence_before();
+      mbar_arrive_one(&p_full[b]);
+      t = next_page(t + 1);
+      if (NS == 2) t = next_page(t + 1);
+    }
+  } else {
+    // ---- the running output: a thread a row and CPW x 64 of its columns
+    if (CPW == 1) regs_fewer<104>(); else regs_more<168>();
+    const int quarter = warp & 3, row = quarter * 32 + lane, c0 = ((warp >> 2) - 1 - NS) * CPW;
+    const uint32_t lanes = tmem_base + ((uint32_t)(quarter * 32) << 16) + TM_T;
+    const int ti = row / hp, h = h0 + row - ti * hp;
+    const int64_t grow = start + tok0 + ti;
+    const __nv_bfloat16* gate = a.gate == nullptr ? nullptr : (a.gate_heads ? a.gate + grow * a.ld_gate + h : a.gate + grow * a.ld_gate + (int64_t)h * a.dv + c0 * 64);
+    if (gate != nullptr && ti < n_tok) {                          // (the gate is asked for now: it is wanted after the last page)
+      const int bytes = a.gate_heads ? 2 : 2 * min(CPW * 64, a.dv - c0 * 64);
+      for (int at = 0; at < bytes; at += 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char*>(gate) + at));
+    }
+    float run_max = -INFINITY, run_sum = 0.f;
+    uint64_t o[CPW * 32];
+#pragma unroll
+    for (int c = 0; c < CPW * 32; ++c) o[c] = 0ull;
+    bool ok = true;
+    int j = 0;
+    for (int t = next_page(0); t * PAGE <= last_pos && ok; t = next_page(t + 1), ++j) {
+      if (!mbar_wait(&st_full[j % STATS], (j / STATS) & 1)) { ok = false; break; }
+      const float2 st = stats[(j % STATS) * ROWS + row];
+      const float new_max = fmaxf(run_max, st.x);
+      const float keep = run_max == -INFINITY ? 0.f : exp2_fast(run_max - new_max), take = st.x == -INFINITY ? 0.f : exp2_fast(st.x - new_max);
+      // (a page that the row sees nothing of has weights of zero and a sum of zero, or NaN, which stays)
+      run_sum = fmaf(run_sum, keep, st.y * (st.x == -INFINITY ? 1.f : take));
+      run_max = new_max;
+      const uint64_t keep2 = pair(keep, keep), take2 = pair(take, take);
+#pragma unroll
+      for (int c = 0; c < CPW * 64 / CW; ++c) {
+        if (c0 * 64 / CW + c >= n_chunks) continue;
+        const int g = j * n_chunks + c0 * 64 / CW + c, turns = g / SLOTS, slot = g - turns * SLOTS;
+        if (!mbar_wait(&t_full[slot], turns & 1)) { ok = false; break; }
+        tc_fence_after();
+#pragma unroll
+        for (int q = 0; q < CW / 16; ++q) {
+          float v[16];
+          tmem_ld16(lanes + slot * CW + q * 16, v);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            uint64_t& x = o[c * (CW / 2) + q * 8 + e];
+            x = fma2(x, keep2, mul2(pair(v[2 * e], v[2 * e + 1]), take2));
+          }
+        }
+        tc_fence_before();
+        mbar_arrive_one(&t_empty[slot]);
       }
     }
+    if (ok && ti < n_tok) {
+      float inv;
+      if (a.sinks == nullptr) {
+        inv = 1.0f / run_sum;
+      } else {                                                    // a sink is one more term of the denominator
+        const float most = run_max * LN2, sink = a.sinks[h], m = fmaxf(most, sink), f = expf(most - m);
+        inv = f / fmaf(run_sum, f, expf(sink - m));
+      }
+      if (gate != nullptr && a.gate_heads) inv *= sigmoid_fast(__bfloat162float(*gate));
+#pragma unroll
+      for (int c = 0; c < CPW * 8; ++c) {
+        const int d = c0 * 64 + c * 8;                            // (dv is a multiple of 8)
+        if (d >= a.dv) continue;
+        float x[8];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) unpair(o[c * 4 + e], x[2 * e], x[2 * e + 1]);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) x[e] *= inv;
+        if (F32OUT) {
+          float* dst = reinterpret_cast<float*>(a.out) + grow * a.ld_out + (int64_t)h * a.dv + d;
+          if (a.vec) {
+            reinterpret_cast<float4*>(dst)[0] = make_float4(x[0], x[1], x[2], x[3]);
+            reinterpret_cast<float4*>(dst)[1] = make_float4(x[4], x[5], x[6], x[7]);
+          } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) reinterpret_cast<float2*>(dst)[e] = make_float2(x[2 * e], x[2 * e + 1]);
+          }
+        } else {
+          __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(a.out) + grow * a.ld_out + (int64_t)h * a.dv + d;
+          if (gate != nullptr && !a.gate_heads) {
+            uint32_t z[4];
+            if (a.vec) {
+              const uint4 w = *reinterpret_cast<const uint4*>(gate + c * 8);
+              z[0] = w.x; z[1] = w.y; z[2] = w.z; z[3] = w.w;
+            } else {
+#pragma unroll
+              for (int e = 0; e < 4; ++e) z[e] = *reinterpret_cast<const uint32_t*>(gate + c * 8 + 2 * e);
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              x[2 * e] *= sigmoid_fast(__uint_as_float(z[e] << 16));
+              x[2 * e + 1] *= sigmoid_fast(__uint_as_float(z[e] & 0xffff0000u));
+            }
+          }
+          uint32_t w[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) w[e] = pack(x[2 * e], x[2 * e + 1]);
+          if (a.vec) {
+            *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+          } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) *reinterpret_cast<uint32_t*>(dst + 2 * e) = w[e];
+          }
+        }
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  if (warp == 1) {
+    __syncwarp();
+    tmem_dealloc(tmem_base, TM_COLS);
   }
 }
 
-template <int NV, bool F32OUT>
-int launch(const PromptArgs& a, int max_new, size_t smem, cudaStream_t stream) {
-  static size_t configured = 0;
-  if (smem > configured) {
-    cudaError_t e = cudaFuncSetAttribute(scored_prompt_kernel<NV, F32OUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) KVAD_FAIL(KVAD_ERR_CUDA, "attention (scored, prompts): cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
-    configured = smem;
+int make_map(CUtensorMap* map, const void* at, int rank, const cuuint64_t* dims, const cuuint64_t* strides, const cuuint32_t* box) {
+  EncodeTiledFn fn = encode_fn();
+  if (fn == nullptr) KVAD_FAIL(KVAD_ERR_CUDA, "attention (scored, prompts): the driver has no cuTensorMapEncodeTiled");
+  const cuuint32_t ones[3] = {1, 1, 1};
+  const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<void*>(at), dims, strides, box, ones, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) KVAD_FAIL(KVAD_ERR_CUDA, "attention (scored, prompts): cuTensorMapEncodeTiled failed (%d)", (int)r);
+  return KVAD_OK;
+}
+
+template <int NS, int CPW, bool F32OUT>
+int launch(const CUtensorMap& q, const CUtensorMap& k, const CUtensorMap& v, const PromptArgs& a, int max_new, size_t smem, cudaStream_t stream) {
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(scored_prompt_kernel<NS, CPW, F32OUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MOST);
+    if (e != cudaSuccess) KVAD_FAIL(KVAD_ERR_CUDA, "attention (scored, prompts): cannot reserve %zu bytes of shared memory: %s", SMEM_MOST, cudaGetErrorString(e));
+    configured = true;
   }
   const int tok = ROWS / a.hp;
   const int64_t tiles = (int64_t)a.columns * ((max_new + tok - 1) / tok);
   KVAD_REQUIRE(tiles < (1ll << 31), "attention (scored, prompts): %lld tiles are more than one launch takes", (long long)tiles);
-  kvad_launch(scored_prompt_kernel<NV, F32OUT>, dim3((unsigned)tiles), dim3(a.halves * HALF), smem, stream, a);
+  kvad_launch(scored_prompt_kernel<NS, CPW, F32OUT>, dim3((unsigned)tiles), dim3(THREADS), smem, stream, q, k, v, a);
   KVAD_CHECK_LAUNCH("attention_scored_prompt");
   return KVAD_OK;
 }
 
-// 16-entry groups of a value that the kernel is built for.
-int groups_of(int dv) { return dv <= 32 ? 2 : (dv <= 64 ? 4 : (dv <= 128 ? 8 : (dv <= 192 ? 12 : 16))); }
-
-struct Layout { int k_stride, v_stride, halves; size_t smem; };
-// Row strides of an odd number of 16-byte pieces over whole 16-entry steps; all of shared memory with the slack that the last row's unused
-// value columns may read (values are read in the kernel's groups of 16 entries), and room for the second half's sums at the end.
+struct Layout { int stages; size_t smem; };
+// As many pages on their way as fit (three keep all roles busy; one, for the longest keys, gives the same sums page by page).
 Layout layout_of(int dk, int dv, bool alias) {
+  const size_t kb = (dk + 63) / 64, vb = alias ? 0 : (dv + 63) / 64, fixed = kb * Q_BLOCK + SMEM_REST, stage = (kb + vb) * PAGE_BLOCK;
   Layout z;
-  z.k_stride = (dk + 15) / 16 * 16 + 8;
-  z.v_stride = alias ? z.k_stride : (dv + 15) / 16 * 16 + 8;
-  // Two halves where two such blocks fit an SM (values of up to 64 entries: 128 registers a thread), else one: two halves that are the SM's
-  // only block leave it idle where they begin and end.  (Measured when weights went through in two pieces, 2 x 1024 rows, two halves against one: 12 heads of 64: 36 us and 50; 32 heads of
-  // 128 on 8: 148 and 112; 16 heads over a latent of 256: 152 and 108.)
-  auto need = [&](int halves) {
-    return ((size_t)ROWS * z.k_stride + 2 * halves * ((size_t)PAGE * z.k_stride + (alias ? 0 : (size_t)PAGE * z.v_stride)) + 256 + 16) * 2;
-  };
-  z.halves = groups_of(dv) <= 4 && need(2) <= SMEM_HALF ? 2 : 1;
-  z.smem = need(z.halves);
-  if (z.halves == 2) z.smem = std::max(z.smem, (size_t)(8 * groups_of(dv) + 4) * HALF * sizeof(float));
+  z.stages = fixed >= SMEM_MOST ? 0 : (int)std::min<size_t>(MAX_STAGES, (SMEM_MOST - fixed) / stage);
+  z.smem = fixed + z.stages * stage;
   return z;
 }
 
 }  // namespace
 
-// 1 if prompts of these sizes run here: whole 16-byte pieces, values up to 256 entries (128 where the output is 32-bit), everything in shared memory.
-KVAD_EXPORT int kvad_attention_scored_prompt_takes(int dk, int dv, int alias, int out_f32) {
-  return dk > 0 && dv > 0 && dk % 8 == 0 && dv % 8 == 0 && dv <= (out_f32 ? 128 : 256) && layout_of(dk, dv, alias != 0).smem <= SMEM_MOST ? 1 : 0;
+// 1 if prompts of these sizes run here: whole 16-byte pieces, values up to 256 entries, the queries and a page in shared memory (whatever the output's type).
+KVAD_EXPORT int kvad_attention_scored_prompt_takes(int dk, int dv, int alias, int) {
+  return dk > 0 && dv > 0 && dk % 8 == 0 && dv % 8 == 0 && dv <= 256 && layout_of(dk, dv, alias != 0).stages >= 1 ? 1 : 0;
 }
 
-KVAD_EXPORT int kvad_attention_scored_prompt(const void* q, int64_t ld_q, void* out, int64_t ld_out, const void* gate, int64_t ld_gate, int gate_heads,
-                                             const float* sinks, const int* seq_starts, const int* kv_lens, const int* page_table, int table_width,
-                                             const void* k_pages, const void* v_pages, int n_seqs, int n_heads, int n_kv_heads, int dk, int dv,
-                                             int page_size, int max_new, float scale, float softcap, float slope_span, int window, int keep_first,
-                                             int chunk, int key_maps, int out_f32, cudaStream_t stream) {
-  KVAD_REQUIRE(n_seqs >= 0 && n_heads > 0 && n_kv_heads > 0 && dk > 0 && dv > 0 && table_width > 0 && max_new >= 0 && keep_first >= 0,
+// `n_rows`, `n_pages`: how many rows q has and how many pages the cache.
+KVAD_EXPORT int kvad_attention_scored_prompt(const void* q, int64_t ld_q, int n_rows, void* out, int64_t ld_out, const void* gate, int64_t ld_gate, int gate_heads,
+                                         const float* sinks, const int* seq_starts, const int* kv_lens, const int* page_table, int table_width,
+                                         const void* k_pages, const void* v_pages, int n_pages, int n_seqs, int n_heads, int n_kv_heads, int dk, int dv,
+                                         int page_size, int max_new, float scale, float softcap, float slope_span, int window, int keep_first,
+                                         int chunk, int key_maps, int out_f32, cudaStream_t stream) {
+  KVAD_REQUIRE(n_seqs >= 0 && n_heads > 0 && n_kv_heads > 0 && dk > 0 && dv > 0 && table_width > 0 && max_new >= 0 && keep_first >= 0 && n_rows >= 0 && n_pages > 0,
                "attention (scored, prompts): bad sizes seqs=%d heads=%d kv_heads=%d dk=%d dv=%d", n_seqs, n_heads, n_kv_heads, dk, dv);
   KVAD_REQUIRE(n_heads % n_kv_heads == 0, "attention (scored, prompts): %d heads do not divide into %d key/value heads", n_heads, n_kv_heads);
   KVAD_REQUIRE(chunk <= 0 || window <= 0, "attention (scored, prompts): a chunk goes without a window");
@@ -446,38 +594,54 @@ KVAD_EXPORT int kvad_attention_scored_prompt(const void* q, int64_t ld_q, void* 
   if ((all & 15) || ld_q % 8 != 0 || (reinterpret_cast<uintptr_t>(out) & 7) || ld_out % 2 != 0 ||
       (gate != nullptr && ((reinterpret_cast<uintptr_t>(gate) & 3) || ld_gate % 2 != 0)))
     KVAD_FAIL(KVAD_ERR_UNSUPPORTED, "attention (scored, prompts): rows must lie on 16-byte boundaries");
-  if (n_seqs == 0 || max_new == 0) return KVAD_OK;
+  KVAD_REQUIRE((int64_t)n_pages * n_kv_heads * PAGE < (1ll << 31), "attention (scored, prompts): %d pages of %d heads are more than a coordinate counts", n_pages, n_kv_heads);
+  if (n_seqs == 0 || max_new == 0 || n_rows == 0) return KVAD_OK;
   PromptArgs a;
-  a.q = (const __nv_bfloat16*)q; a.ld_q = ld_q; a.out = out; a.ld_out = ld_out; a.gate = (const __nv_bfloat16*)gate; a.ld_gate = ld_gate;
+  a.out = out; a.ld_out = ld_out; a.gate = (const __nv_bfloat16*)gate; a.ld_gate = ld_gate;
   a.gate_heads = gate_heads; a.sinks = sinks; a.seq_starts = seq_starts; a.kv_lens = kv_lens; a.page_table = page_table; a.table_width = table_width;
-  a.k_pages = (const __nv_bfloat16*)k_pages; a.v_pages = (const __nv_bfloat16*)v_pages;
-  a.k_page_stride = (int64_t)n_kv_heads * PAGE * dk; a.v_page_stride = (int64_t)(n_kv_heads / key_maps) * PAGE * dv;
   a.n_heads = n_heads; a.n_kv_heads = n_kv_heads; a.dk = dk; a.dv = dv; a.alias = alias ? 1 : 0; a.key_maps = key_maps;
   a.scale = scale; a.softcap = softcap; a.slope_span = slope_span; a.window = window > 0 ? window : 0; a.keep_first = window > 0 ? keep_first : 0;
   a.chunk = chunk > 0 ? chunk : 0;
   // (scale / cap stays an ordinary number: a cap above 2^100 moves no score below 2^87, one of nothing makes every score but 0 the cap)
   const float cap = std::min(softcap, 1.2676506e30f), ratio = scale / cap;
   a.cap_in = softcap > 0.f ? std::max(-3.402823466e38f, std::min(3.402823466e38f, ratio)) : 0.f; a.cap_out = cap * LOG2E;
-  // heads a tile: as many of the group as divide it, up to a warp's 16 rows (a tile then spans few tokens: little of its last page is masked)
+  // heads a tile: as many of the group as divide it, up to 16 (a tile then spans few tokens: little of its last page is masked)
   a.hp = 1;
   while (a.hp < 16 && (n_heads / n_kv_heads) % (a.hp * 2) == 0) a.hp *= 2;
   KVAD_REQUIRE((int64_t)n_seqs * (n_heads / a.hp) < (1ll << 31), "attention (scored, prompts): %d sequences x %d heads are more than one launch takes", n_seqs, n_heads);
   a.columns = n_seqs * (n_heads / a.hp);
+  const int item = out_f32 ? 4 : 2;
+  a.vec = (reinterpret_cast<uintptr_t>(out) & 15) == 0 && ld_out * item % 16 == 0 &&
+          (gate == nullptr || gate_heads || ((reinterpret_cast<uintptr_t>(gate) & 15) == 0 && ld_gate % 8 == 0)) ? 1 : 0;
   const Layout z = layout_of(dk, dv, alias);
-  a.halves = z.halves; a.k_steps = (dk + 15) / 16; a.k_stride = z.k_stride; a.v_stride = z.v_stride;
-#define KVAD_SP(N)                                                                          \
-  do {                                                                                      \
-    if (out_f32) return launch<(N > 8 ? 8 : N), true>(a, max_new, z.smem, stream);  \
-    return launch<N, false>(a, max_new, z.smem, stream);                            \
+  a.stages = z.stages;
+  CUtensorMap mq, mk, mv;
+  const cuuint64_t q_dims[3] = {(cuuint64_t)dk, (cuuint64_t)n_heads, (cuuint64_t)n_rows}, q_strides[2] = {(cuuint64_t)dk * 2, (cuuint64_t)ld_q * 2};
+  const cuuint32_t q_box[3] = {64, (cuuint32_t)a.hp, (cuuint32_t)(ROWS / a.hp)}, page_box[2] = {64, PAGE};
+  const cuuint64_t k_dims[2] = {(cuuint64_t)dk, (cuuint64_t)n_pages * n_kv_heads * PAGE}, k_strides[1] = {(cuuint64_t)dk * 2};
+  const cuuint64_t v_dims[2] = {(cuuint64_t)dv, (cuuint64_t)n_pages * (n_kv_heads / key_maps) * PAGE}, v_strides[1] = {(cuuint64_t)dv * 2};
+  int rc = make_map(&mq, q, 3, q_dims, q_strides, q_box);
+  if (rc == KVAD_OK) rc = make_map(&mk, k_pages, 2, k_dims, k_strides, page_box);
+  if (rc != KVAD_OK) return rc;
+  mv = mk;
+  if (!alias && (rc = make_map(&mv, v_pages, 2, v_dims, v_strides, page_box)) != KVAD_OK) return rc;
+#define KVAD_TC(NS, CPW)                                                                        \
+  do {                                                                                          \
+    if (out_f32) return launch<NS, CPW, true>(mq, mk, mv, a, max_new, z.smem, stream);          \
+    return launch<NS, CPW, false>(mq, mk, mv, a, max_new, z.smem, stream);                      \
   } while (0)
-  switch (groups_of(dv)) {
-    case 2: KVAD_SP(2);
-    case 4: KVAD_SP(4);
-    case 8: KVAD_SP(8);
-    case 12: KVAD_SP(12);
-    default: KVAD_SP(16);
-  }
-#undef KVAD_SP
+  if (dv <= 64) KVAD_TC(2, 1);
+  if (dv <= 128) KVAD_TC(2, 2);
+  KVAD_TC(1, 2);
+#undef KVAD_TC
+}
+
+// How many bounded waits have run out since the library was loaded (0 in a healthy run).  Synchronises the device.
+KVAD_EXPORT int kvad_attention_scored_prompt_status() {
+  int n = 0;
+  cudaError_t e = cudaMemcpyFromSymbol(&n, g_wait_timeouts, sizeof(int));
+  if (e != cudaSuccess) KVAD_FAIL(KVAD_ERR_CUDA, "attention_scored_prompt_status: %s", cudaGetErrorString(e));
+  return n;
 }
 
 KVAD_DEFINE_LAST_ERROR()

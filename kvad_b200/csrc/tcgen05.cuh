@@ -100,6 +100,15 @@ __device__ __forceinline__ uint64_t sw128_desc(uint32_t smem_addr) {
   return d;
 }
 
+// One lane of a converged warp (the same at every call).  A warp that issues products stays together and lets the elected lane do it: the operands
+// then live in uniform registers and an issue takes ~32 cycles; inside a branch that one lane took by itself it took 50 to 120, which is more than a
+// product of 128 x 64 x 16 runs (48 cycles with A in shared memory, 32 in tensor memory).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t yes;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(yes));
+  return yes != 0;
+}
+
 __device__ __forceinline__ void umma(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
   const uint32_t zero = 0;
   asm volatile(

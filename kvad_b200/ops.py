@@ -10,6 +10,7 @@ computes anything here, and nothing falls back to the CPU.
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 from ctypes import c_float, c_int, c_int64, c_void_p
 from typing import Optional
@@ -126,10 +127,11 @@ _SIGNATURES = {
                               c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int64, c_void_p, c_int, c_void_p, c_int64, c_int, c_void_p],
     },
     "attention_scored_prompt": {
-        "kvad_attention_scored_prompt": [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
-                                         c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_float, c_int, c_int,
+        "kvad_attention_scored_prompt": [c_void_p, c_int64, c_int, c_void_p, c_int64, c_void_p, c_int64, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
+                                         c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_float, c_int, c_int,
                                          c_int, c_int, c_int, c_void_p],
         "kvad_attention_scored_prompt_takes": [c_int, c_int, c_int, c_int],
+        "kvad_attention_scored_prompt_status": [],
     },
     "retention": {
         "kvad_retention": [c_int, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64,
@@ -333,6 +335,11 @@ def _rows_view(t: torch.Tensor, what: str) -> int:
     if t.dim() != 2 or t.stride(1) != 1:
         raise KernelError(f"{what}: needs a 2-D tensor with contiguous rows, got shape {tuple(t.shape)} strides {t.stride()}")
     return t.stride(0)
+
+
+@functools.lru_cache(maxsize=256)
+def _scored_prompt_takes(dk: int, dv: int, alias: bool, out_f32: bool) -> bool:
+    return lib("attention_scored_prompt").kvad_attention_scored_prompt_takes(dk, dv, int(alias), int(out_f32)) == 1
 
 
 class Ops:
@@ -1145,11 +1152,12 @@ class Ops:
         if (self.scored_prompt and max_new >= self.SCORED_PROMPT_MIN_NEW and n_splits == 1 and page == 64 and ld_q % 8 == 0 and ld_o % 2 == 0 and ld_g % 2 == 0
                 and (q.data_ptr() | k_pages.data_ptr() | v_ptr.data_ptr()) % 16 == 0 and out.data_ptr() % 8 == 0
                 and (gate is None or gate.data_ptr() % 4 == 0) and (v_pages is not None or dv <= dk) and n_seqs * n_heads * (max_new // 64 + 1) < 1 << 31
-                and lib("attention_scored_prompt").kvad_attention_scored_prompt_takes(dk, dv, int(v_pages is None), int(out_f32)) == 1):
+                and n_heads * dk <= ld_q < 1 << 36 and 0 < k_pages.shape[0] * n_kv * page < 1 << 31          # (what a tensor map takes)
+                and _scored_prompt_takes(dk, dv, v_pages is None, out_f32)):
             h = lib("attention_scored_prompt")
-            _check(h.kvad_attention_scored_prompt(_ptr(q), ld_q, _ptr(out), ld_o, _ptr(gate), ld_g, int(gate_heads), _ptr(sinks), _ptr(seq_starts),
-                                                  _ptr(kv_lens), _ptr(page_table), page_table.shape[1], _ptr(k_pages), _ptr(v_ptr), int(n_seqs),
-                                                  int(n_heads), n_kv, dk, dv, page, int(max_new), float(scale), float(softcap or 0.0),
+            _check(h.kvad_attention_scored_prompt(_ptr(q), ld_q, q.shape[0], _ptr(out), ld_o, _ptr(gate), ld_g, int(gate_heads), _ptr(sinks), _ptr(seq_starts),
+                                                  _ptr(kv_lens), _ptr(page_table), page_table.shape[1], _ptr(k_pages), _ptr(v_ptr), k_pages.shape[0],
+                                                  int(n_seqs), int(n_heads), n_kv, dk, dv, page, int(max_new), float(scale), float(softcap or 0.0),
                                                   float(slope_span or 0.0), int(window or 0), int(keep_first or 0), int(chunk or 0), int(key_maps),
                                                   int(out_f32), _stream()), h)
             return
@@ -1821,6 +1829,15 @@ def linear_split_wait_timeouts() -> int:
     """How many bounded waits of the 32-bit product on the tensor cores have run out (0 in a healthy run)."""
     h = lib("linear_split")
     n = h.kvad_linear_split_status()
+    if n < 0:
+        raise KernelError(h.kvad_last_error().decode("utf-8", "replace"))
+    return n
+
+
+def scored_prompt_wait_timeouts() -> int:
+    """How many bounded waits of the prompt attention with shaped scores have run out (0 in a healthy run)."""
+    h = lib("attention_scored_prompt")
+    n = h.kvad_attention_scored_prompt_status()
     if n < 0:
         raise KernelError(h.kvad_last_error().decode("utf-8", "replace"))
     return n

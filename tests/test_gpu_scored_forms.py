@@ -260,3 +260,20 @@ def test_a_prompt_of_more_tiles_than_a_grid_dimension_holds():
     first = torch.full((3000, H * dk), float("nan"), dtype=torch.bfloat16, device="cuda")
     ops.attention_scored(q[:3000], first, i32([0, 3000]), i32([3005]), 1, 3000, table, kp, None, H, 0.3, **kw)
     assert torch.equal(out[:3000], first) and out.isfinite().all()
+
+
+# tiles of 128 (token, head) pairs, products of 64 and 128 columns, one to four pages on their way; caps whose scores lie on both sides of the polynomial's range
+TILES = [
+    (4, 4, 64, 64, dict(cap=3.0)), (4, 4, 64, 64, dict(cap=300.0, gate="entry")), (2, 2, 128, 128, {}), (8, 1, 80, 72, {}), (8, 1, 136, 136, dict(window=64, keep=65)),
+    (16, 2, 200, 200, dict(sinks=True)), (16, 1, 288, 256, dict(alias=True)), (16, 1, 576, 256, dict(alias=True, chunk=64)), (2, 1, 384, 128, dict(span=8.0)), (32, 1, 64, 192, {}),
+]
+
+
+@pytest.mark.parametrize("H,G,dk,dv,form", TILES)
+def test_prompt_tiles(H, G, dk, dv, form):
+    from kvad_b200.ops import scored_prompt_wait_timeouts
+    assert lib("attention_scored_prompt").kvad_attention_scored_prompt_takes(dk, dv, int("alias" in form), 0) == 1
+    c = Case([(0, 128), (64, 64), (0, 257), (449, 31), (3, 2), (0, 1)], H, G, dk, dv, **form)
+    for out in [torch.bfloat16] if c.gate is not None else [torch.bfloat16, torch.float32]:
+        c.check(c.run(Ops(torch.bfloat16), out), out)
+    assert scored_prompt_wait_timeouts() == 0
