@@ -258,8 +258,10 @@ linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    {                                        // (the whole warp; its elected lane issues: see elect_one)
       constexpr uint32_t idesc = instr_desc<BN>();
+      const bool one = elect_one();
+      const uint64_t a_desc0 = sw128_desc(smem_u32(a_tiles)), b_desc0 = sw128_desc(smem_u32(b_tiles));
       uint32_t it = 0;
       int lt = 0;                            // tiles of this CTA so far
       bool ok = true;
@@ -282,17 +284,18 @@ linear_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
           ok = mbar_wait(&full_bar[s], (it / STAGES) & 1);
           if (!ok) break;
           tc_fence_after();
-          const uint64_t a_desc = sw128_desc(smem_u32(a_tiles + s * T::A_BYTES));
-          const uint64_t b_desc = sw128_desc(smem_u32(b_tiles + s * T::B_BYTES));
+          const uint64_t a_desc = a_desc0 + (uint32_t)s * (T::A_BYTES >> 4), b_desc = b_desc0 + (uint32_t)s * (T::B_BYTES >> 4);
+          if (one) {
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k) {
-            // 16 elements further along K: 32 bytes inside the swizzled row, i.e. 2 in units of 16 bytes
-            umma(acc, a_desc + (uint64_t)(k * 2), b_desc + (uint64_t)(k * 2), idesc, (i > 0 || k > 0) ? 1u : 0u);
+            for (int k = 0; k < BK / UMMA_K; ++k) {
+              // 16 elements further along K: 32 bytes inside the swizzled row, i.e. 2 in units of 16 bytes
+              umma(acc, a_desc + (uint64_t)(k * 2), b_desc + (uint64_t)(k * 2), idesc, (i > 0 || k > 0) ? 1u : 0u);
+            }
+            umma_commit(&empty_bar[s]);   // the stage is free again once these MMAs have read it
           }
-          umma_commit(&empty_bar[s]);     // the stage is free again once these MMAs have read it
         }
         if (!ok) break;
-        umma_commit(&tmem_full_bar[buf]); // the accumulator is complete once everything issued has run
+        if (one) umma_commit(&tmem_full_bar[buf]); // the accumulator is complete once everything issued has run
       }
     }
   } else {
@@ -496,21 +499,24 @@ linear_tcgen05_skinny_kernel(const __grid_constant__ CUtensorMap map_a, const __
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    {
+      const bool one = elect_one();
+      const uint64_t w_desc0 = sw128_desc(smem_u32(w_tiles)), a_desc0 = sw128_desc(smem_u32(a_tiles));
       constexpr uint32_t idesc = instr_desc<MB, TM>();
       for (int i = 0; i < num_kb; ++i) {
         const int s = i % STAGES;
         const uint32_t phase = (i / STAGES) & 1;
         if (!mbar_wait(&full_bar[s], phase)) break;
         tc_fence_after();
-        const uint64_t w_desc = sw128_desc(smem_u32(w_tiles + s * T::W_BYTES));
-        const uint64_t a_desc = sw128_desc(smem_u32(a_tiles + s * T::A_BYTES));
+        const uint64_t w_desc = w_desc0 + (uint32_t)s * (T::W_BYTES >> 4), a_desc = a_desc0 + (uint32_t)s * (T::A_BYTES >> 4);
+        if (one) {
 #pragma unroll
-        for (int k = 0; k < BK / UMMA_K; ++k)
-          umma(tmem_base, w_desc + (uint64_t)(k * 2), a_desc + (uint64_t)(k * 2), idesc, (i > 0 || k > 0) ? 1u : 0u);
-        umma_commit(&empty_bar[s]);
+          for (int k = 0; k < BK / UMMA_K; ++k)
+            umma(tmem_base, w_desc + (uint64_t)(k * 2), a_desc + (uint64_t)(k * 2), idesc, (i > 0 || k > 0) ? 1u : 0u);
+          umma_commit(&empty_bar[s]);
+        }
       }
-      umma_commit(tmem_full_bar);
+      if (one) umma_commit(tmem_full_bar);
     }
   } else {
     const int quarter = warp & 3;
@@ -649,7 +655,10 @@ linear_tcgen05_skinny3d_kernel(const __grid_constant__ CUtensorMap map_a, const 
     }
   } else if (warp == 1) {
     if (cluster_reduce) cluster_arrive();
-    if (lane == 0) {
+    __syncwarp();
+    {
+      const bool one = elect_one();
+      const uint64_t w_desc0 = sw128_desc(smem_u32(w_ring)), a_desc0 = sw128_desc(smem_u32(a_all));
       constexpr uint32_t idesc = instr_desc<MB>();
       bool ok = mbar_wait(a_full, 0);
       for (int g = 0; g < n_groups && ok; ++g) {
@@ -657,20 +666,21 @@ linear_tcgen05_skinny3d_kernel(const __grid_constant__ CUtensorMap map_a, const 
         ok = mbar_wait(&w_full[s], (g / stages) & 1);
         if (!ok) break;
         tc_fence_after();
+        if (one) {
 #pragma unroll
-        for (int j = 0; j < W_GROUP; ++j) {
-          const int kb = g * W_GROUP + j;
-          if (kb < num_kb) {
-            const uint64_t w_desc = sw128_desc(smem_u32(w_ring + ((size_t)s * W_GROUP + j) * W_BYTES));
-            const uint64_t a_desc = sw128_desc(smem_u32(a_all + (size_t)kb * A_BYTES));
+          for (int j = 0; j < W_GROUP; ++j) {
+            const int kb = g * W_GROUP + j;
+            if (kb < num_kb) {
+              const uint64_t w_desc = w_desc0 + (uint32_t)(s * W_GROUP + j) * (W_BYTES >> 4), a_desc = a_desc0 + (uint32_t)kb * (A_BYTES >> 4);
 #pragma unroll
-            for (int k = 0; k < BK / UMMA_K; ++k)
-              umma(tmem_base, w_desc + (uint64_t)(k * 2), a_desc + (uint64_t)(k * 2), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+              for (int k = 0; k < BK / UMMA_K; ++k)
+                umma(tmem_base, w_desc + (uint64_t)(k * 2), a_desc + (uint64_t)(k * 2), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+            }
           }
+          umma_commit(&w_empty[s]);
         }
-        umma_commit(&w_empty[s]);
       }
-      umma_commit(tmem_full_bar);
+      if (one) umma_commit(tmem_full_bar);
     }
   } else {
     const int quarter = warp & 3;
