@@ -7,7 +7,7 @@
 // the halves (unnormalised output, maximum, sum) meet through shared memory at the end; shorter
 // tiles go two to a CTA, a longer one paired with a shorter one.  Roles: warp 0 brings Q and a ring of
 // K/V pages by TMA (128-byte swizzle), in the order the slots use them (a page both slots read at the
-// same step is brought once); one thread of warp 1 issues tcgen05.mma; warps 2-5 are slot 0, warps 6-9
+// same step is brought once); warps 1 and 2 issue tcgen05.mma, one for each slot; warps 4-7 are slot 0, warps 8-11
 // slot 1.  (A kernel that allocates tensor memory gets one CTA per SM, whatever else it needs: the
 // second slot is what keeps the tensor core busy while the first one's softmax runs.)
 //
@@ -36,7 +36,8 @@ constexpr int ROWS = 128;         // query rows per tile
 constexpr int TILES = 2;          // slots of a CTA
 constexpr int SPLIT_ABOVE = 8;    // a tile that sees more pages than this is walked by both slots, half each (the launch may say otherwise)
 constexpr int KEYS = 64;          // keys per step = one cache page
-constexpr int THREADS = 64 + TILES * 128;
+constexpr int THREADS = 128 + TILES * 128;
+constexpr int REGS_FEW = 56, REGS_MANY = 224;     // of 168 a thread at launch: the warps that copy and issue, the softmax warps
 
 template <int HD> struct Layout {
   static constexpr int KB = HD / 64;                          // 64-wide blocks of the head dimension
@@ -209,7 +210,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     prefetch_tensormap(&map_k);
     prefetch_tensormap(&map_v);
     mbar_init(q_full, 1);
-    for (int st = 0; st < STAGES; ++st) { mbar_init(&kv_full[st], 1); mbar_init(&kv_empty[st], 1); }
+    for (int st = 0; st < STAGES; ++st) { mbar_init(&kv_full[st], 1); mbar_init(&kv_empty[st], TILES); }      // (both slots give a page back)
     for (int b = 0; b < TILES * 2; ++b) {
       mbar_init(&s_full[b], 1);
       mbar_init(&p_full[b], 128);
@@ -227,238 +228,221 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
 
   pdl_wait();                                      // everything below reads what earlier kernels of the step wrote
 
-  if (warp == 0) {
-    if (lane == 0) {
-      const int n_q = (tr[1].qt >= 0 && !split) ? 2 : 1;                   // both slots of a split tile read one copy of its rows
-      mbar_expect_tx(q_full, n_q * L::Q_BYTES);
+  if (warp < 4) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS_FEW));
+    if (warp == 0) {
+      if (lane == 0) {
+        const int n_q = (tr[1].qt >= 0 && !split) ? 2 : 1;                   // both slots of a split tile read one copy of its rows
+        mbar_expect_tx(q_full, n_q * L::Q_BYTES);
 #pragma unroll
-      for (int t = 0; t < TILES; ++t)
-        if (t < n_q)
-          for (int kb = 0; kb < L::KB; ++kb)
-            tma_load_2d(q_tiles + t * L::Q_BYTES + kb * (ROWS * 128), &map_q, q_full, h * HD + kb * 64, row0_seq + tr[t].qt * ROWS);
-      int li = 0;
-      bool ok = true;
-      for (int i = 0; i < n_steps_max && ok; ++i) {
-#pragma unroll
-        for (int t = 0; t < TILES; ++t) {
-          if (i >= (t == 0 ? n_steps0 : n_steps1) || (t == 1 && same_start)) continue;
-          const int st = li % STAGES;
-          if (li >= STAGES && !mbar_wait(&kv_empty[st], ((li / STAGES) & 1) ^ 1)) { ok = false; break; }
-          uint8_t* k_dst = kv_tiles + st * 2 * L::TILE_BYTES;
-          uint8_t* v_dst = k_dst + L::TILE_BYTES;
-          const int y = (pages[tr[t].j_lo + i] * n_kv_heads + kvh) * KEYS;
-          mbar_expect_tx(&kv_full[st], 2 * L::TILE_BYTES);
-#pragma unroll
-          for (int kb = 0; kb < L::KB; ++kb) {
-            tma_load_2d(k_dst + kb * (KEYS * 128), &map_k, &kv_full[st], kb * 64, y);
-            tma_load_2d(v_dst + kb * (KEYS * 128), &map_v, &kv_full[st], kb * 64, y);
-          }
-          ++li;
-        }
-      }
-    }
-  } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc_qk = umma_instr_desc(ROWS, KEYS);
-      constexpr uint32_t idesc_pv = umma_instr_desc(ROWS, HD, false, true);
-      bool ok = mbar_wait(q_full, 0);
-      // Per step: S of both slots, then P.V of the step before for both, so that the first product of a step is
-      // under way while the softmax threads are on the step before.  With a ring of fewer than four pages (head size
-      // 128) and two slots on pages of their own that order would need a fourth page: there each slot's S is followed
-      // at once by its P.V of the step before, which gives the page back.
-      constexpr bool INTERLEAVE = STAGES < 4;
-      auto product_s = [&](int t, int i) {
-        const int ld = load_of(t, i), st = ld % STAGES, b = i & 1;
-        if (!mbar_wait(&kv_full[st], (ld / STAGES) & 1)) { ok = false; return; }
-        tc_fence_after();
-        const uint32_t k_addr = smem_u32(kv_tiles + st * 2 * L::TILE_BYTES);
-        const uint32_t q_addr = smem_u32(q_tiles + (split ? 0 : t) * L::Q_BYTES);
-#pragma unroll
-        for (int k = 0; k < HD / 16; ++k) {
-          const uint64_t a_desc = sw128_desc(q_addr + (k / 4) * (ROWS * 128)) + (uint64_t)((k % 4) * 2);
-          const uint64_t b_desc = sw128_desc(k_addr + (k / 4) * (KEYS * 128)) + (uint64_t)((k % 4) * 2);
-          umma(tmem_base + t * L::TMEM_TILE + b * KEYS, a_desc, b_desc, idesc_qk, k > 0 ? 1u : 0u);
-        }
-        umma_commit(&s_full[t * 2 + b]);
-      };
-      auto product_pv = [&](int t, int ip) {
-        const int st = load_of(t, ip) % STAGES, b = ip & 1, tb = ip % T_BUFS;
-        const uint32_t v_addr = smem_u32(kv_tiles + st * 2 * L::TILE_BYTES + L::TILE_BYTES);
-        if (!(mbar_wait(&p_full[t * 2 + b], (ip >> 1) & 1) && mbar_wait(&t_empty[t * 2 + tb], ((ip / T_BUFS) & 1) ^ 1))) { ok = false; return; }
-        tc_fence_after();
-        const uint32_t p_addr = smem_u32(p_tiles + (t * 2 + b) * L::P_BYTES);
-#pragma unroll
-        for (int kk = 0; kk < KEYS / 16; ++kk) {
-          const uint64_t a_desc = sw128_desc(p_addr) + (uint64_t)(kk * 2);
-          const uint64_t b_desc = sw128_mn_desc(v_addr + kk * 2048, KEYS * 128);
-          umma(tmem_base + t * L::TMEM_TILE + L::TMEM_T + tb * HD, a_desc, b_desc, idesc_pv, kk > 0 ? 1u : 0u);
-        }
-        umma_commit(&t_full[t * 2 + tb]);
-      };
-      const int n_steps_of[TILES] = {n_steps0, n_steps1};
-      for (int i = 0; i <= n_steps_max && ok; ++i) {
-        if (INTERLEAVE && !same_start) {
+        for (int t = 0; t < TILES; ++t)
+          if (t < n_q)
+            for (int kb = 0; kb < L::KB; ++kb)
+              tma_load_2d(q_tiles + t * L::Q_BYTES + kb * (ROWS * 128), &map_q, q_full, h * HD + kb * 64, row0_seq + tr[t].qt * ROWS);
+        int li = 0;
+        bool ok = true;
+        for (int i = 0; i < n_steps_max && ok; ++i) {
 #pragma unroll
           for (int t = 0; t < TILES; ++t) {
-            if (i < n_steps_of[t] && ok) product_s(t, i);
-            if (i > 0 && i - 1 < n_steps_of[t] && ok) {
-              product_pv(t, i - 1);
-              if (ok) umma_commit(&kv_empty[load_of(t, i - 1) % STAGES]);      // the page has been read
+            if (i >= (t == 0 ? n_steps0 : n_steps1) || (t == 1 && same_start)) continue;
+            const int st = li % STAGES;
+            if (li >= STAGES && !mbar_wait(&kv_empty[st], ((li / STAGES) & 1) ^ 1)) { ok = false; break; }
+            uint8_t* k_dst = kv_tiles + st * 2 * L::TILE_BYTES;
+            uint8_t* v_dst = k_dst + L::TILE_BYTES;
+            const int y = (pages[tr[t].j_lo + i] * n_kv_heads + kvh) * KEYS;
+            mbar_expect_tx(&kv_full[st], 2 * L::TILE_BYTES);
+#pragma unroll
+            for (int kb = 0; kb < L::KB; ++kb) {
+              tma_load_2d(k_dst + kb * (KEYS * 128), &map_k, &kv_full[st], kb * 64, y);
+              tma_load_2d(v_dst + kb * (KEYS * 128), &map_v, &kv_full[st], kb * 64, y);
             }
+            ++li;
           }
-        } else {
+        }
+      }
+    } else if (warp < 1 + TILES) {
+      // ---- products: a warp per slot, converged, its elected lane issues (a wait takes a hundred cycles even when it is over, an issue from a branch of one
+      // lane 85: one thread for both slots was what the kernel's time went on).  Per step S, then P.V of the step before, which gives the page back.
+      const int t = warp - 1;
+      const int n_steps = t == 0 ? n_steps0 : n_steps1;
+      constexpr uint32_t idesc_qk = umma_instr_desc(ROWS, KEYS);
+      constexpr uint32_t idesc_pv = umma_instr_desc(ROWS, HD, false, true);
+      const bool one = elect_one();
+      const uint64_t q_desc = sw128_desc(smem_u32(q_tiles + (split ? 0 : t) * L::Q_BYTES)), k_desc = sw128_desc(smem_u32(kv_tiles));
+      const uint64_t v_desc = sw128_mn_desc(smem_u32(kv_tiles) + L::TILE_BYTES, KEYS * 128), p_desc = sw128_desc(smem_u32(p_tiles + t * 2 * L::P_BYTES));
+      const uint32_t tmem_t = tmem_base + t * L::TMEM_TILE;
+      bool ok = n_steps > 0 && mbar_wait(q_full, 0);
+      for (int i = 0; i <= n_steps && ok; ++i) {
+        if (i < n_steps) {
+          const int ld = load_of(t, i), st = ld % STAGES, b = i & 1;
+          if (!mbar_wait(&kv_full[st], (ld / STAGES) & 1)) { ok = false; break; }
+          tc_fence_after();
+          const uint64_t k_at = k_desc + (uint32_t)st * (2 * L::TILE_BYTES >> 4);
+          if (one) {
 #pragma unroll
-          for (int t = 0; t < TILES; ++t)
-            if (i < n_steps_of[t] && ok) product_s(t, i);
-          if (i > 0) {
+            for (int k = 0; k < HD / 16; ++k)
+              umma(tmem_t + b * KEYS, q_desc + (uint64_t)((k / 4) * (ROWS * 128 >> 4) + (k % 4) * 2), k_at + (uint64_t)((k / 4) * (KEYS * 128 >> 4) + (k % 4) * 2), idesc_qk,
+                   k > 0 ? 1u : 0u);
+            umma_commit(&s_full[t * 2 + b]);
+          }
+        }
+        if (i > 0) {
+          const int ip = i - 1, ld = load_of(t, ip), st = ld % STAGES, b = ip & 1, tb = ip % T_BUFS;
+          if (!(mbar_wait(&p_full[t * 2 + b], (ip >> 1) & 1) && mbar_wait(&t_empty[t * 2 + tb], ((ip / T_BUFS) & 1) ^ 1))) { ok = false; break; }
+          tc_fence_after();
+          const uint64_t v_at = v_desc + (uint32_t)st * (2 * L::TILE_BYTES >> 4), p_at = p_desc + (uint32_t)b * (L::P_BYTES >> 4);
+          const bool shared = same_start && ip < n_steps1;          // the other slot reads this page too and gives it back itself
+          if (one) {
 #pragma unroll
-            for (int t = 0; t < TILES; ++t)
-              if (i - 1 < n_steps_of[t] && ok) product_pv(t, i - 1);
-            // the step's pages have been read by all that use them
-#pragma unroll
-            for (int t = 0; t < TILES; ++t)
-              if (ok && i - 1 < n_steps_of[t] && !(t == 1 && same_start)) umma_commit(&kv_empty[load_of(t, i - 1) % STAGES]);
+            for (int kk = 0; kk < KEYS / 16; ++kk)
+              umma(tmem_t + L::TMEM_T + tb * HD, p_at + (uint64_t)(kk * 2), v_at + (uint64_t)(kk * (2048 >> 4)), idesc_pv, kk > 0 ? 1u : 0u);
+            umma_commit(&t_full[t * 2 + tb]);
+            umma_commit(&kv_empty[st]);
+            if (!shared) umma_commit(&kv_empty[st]);
           }
         }
       }
     }
-  } else if (tr[(warp - 2) >> 2].qt >= 0) {
-    // ---- softmax: warps 2-5 serve tile 0, warps 6-9 tile 1; thread -> row
-    const int t = (warp - 2) >> 2;
-    const TileRange me = tr[t];
-    const int quarter = warp & 3;
-    const int row = quarter * 32 + lane;
-    const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16) + t * L::TMEM_TILE;
-    const int pos = me.pos0 + row;
-    const int pos_last_row = me.pos0 + me.rows - 1;
-    const int n_steps = me.j_hi - me.j_lo + 1;
-    const float sl2 = scale * 1.4426950408889634f;
-    float run_max = -INFINITY, run_sum = 0.f, keep_prev = 0.f;
-    float o[HD];
+  } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REGS_MANY));
+    if (tr[(warp - 4) >> 2].qt >= 0) {
+      // ---- softmax: warps 4-7 serve slot 0, warps 8-11 slot 1; thread -> row
+      const int t = (warp - 4) >> 2;
+      const TileRange me = tr[t];
+      const int quarter = warp & 3;
+      const int row = quarter * 32 + lane;
+      const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16) + t * L::TMEM_TILE;
+      const int pos = me.pos0 + row;
+      const int pos_last_row = me.pos0 + me.rows - 1;
+      const int n_steps = me.j_hi - me.j_lo + 1;
+      const float sl2 = scale * 1.4426950408889634f;
+      float run_max = -INFINITY, run_sum = 0.f, keep_prev = 0.f;
+      float o[HD];
 #pragma unroll
-    for (int c = 0; c < HD; ++c) o[c] = 0.f;
-    bool ok = true;
+      for (int c = 0; c < HD; ++c) o[c] = 0.f;
+      bool ok = true;
 
-    // O = O * keep + P.V of step k
-    auto take_product = [&](int k, float keep) {
-      const int tb = k % T_BUFS;
-      if (!mbar_wait(&t_full[t * 2 + tb], (k / T_BUFS) & 1)) { ok = false; return; }
-      tc_fence_after();
+      // O = O * keep + P.V of step k
+      auto take_product = [&](int k, float keep) {
+        const int tb = k % T_BUFS;
+        if (!mbar_wait(&t_full[t * 2 + tb], (k / T_BUFS) & 1)) { ok = false; return; }
+        tc_fence_after();
 #pragma unroll
-      for (int c0 = 0; c0 < HD; c0 += 32) {
-        uint32_t r[32];
-        tmem_ld32_issue(lane_addr + L::TMEM_T + tb * HD + c0, r);
+        for (int c0 = 0; c0 < HD; c0 += 32) {
+          uint32_t r[32];
+          tmem_ld32_issue(lane_addr + L::TMEM_T + tb * HD + c0, r);
+          tmem_ld_wait();
+#pragma unroll
+          for (int c = 0; c < 32; ++c) o[c0 + c] = o[c0 + c] * keep + __uint_as_float(r[c]);
+        }
+        tc_fence_before();
+        mbar_arrive(&t_empty[t * 2 + tb]);
+      };
+
+      for (int k = 0; k < n_steps && ok; ++k) {
+        const int j = me.j_lo + k, b = k & 1;
+        if (!mbar_wait(&s_full[t * 2 + b], (k >> 1) & 1)) { ok = false; break; }
+        tc_fence_after();
+        uint32_t sr[KEYS];
+        tmem_ld32_issue(lane_addr + b * KEYS, sr);
+        tmem_ld32_issue(lane_addr + b * KEYS + 32, sr + 32);
         tmem_ld_wait();
+        const bool mask = (j * KEYS + KEYS - 1 > me.pos0) || (window > 0 && j * KEYS <= pos_last_row - window);
+        // (two loops, so that the pages every row sees whole carry no per-element test; four running maxima
+        // keep the chain of dependent instructions short.  The scale, which is positive, is applied to the
+        // maximum here and to each score inside the exponent's multiply-add below.)
+        float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+        if (!mask) {
 #pragma unroll
-        for (int c = 0; c < 32; ++c) o[c0 + c] = o[c0 + c] * keep + __uint_as_float(r[c]);
+          for (int c = 0; c < KEYS; ++c) mx[c & 3] = fmaxf(mx[c & 3], __uint_as_float(sr[c]));
+        } else {
+          const int lo_key = window > 0 ? pos - window + 1 : 0;       // the row sees keys lo_key .. pos
+#pragma unroll
+          for (int c = 0; c < KEYS; ++c) {
+            const int key = j * KEYS + c;
+            const float v = (key <= pos && key >= lo_key) ? __uint_as_float(sr[c]) : -INFINITY;
+            sr[c] = __float_as_uint(v);
+            mx[c & 3] = fmaxf(mx[c & 3], v);
+          }
+        }
+        const float tile_max = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * sl2;
+        const float new_max = fmaxf(run_max, tile_max);
+        const float base = new_max == -INFINITY ? 0.f : new_max;        // a row that has seen nothing yet
+        const float keep = run_max == -INFINITY ? 0.f : fast_exp2(run_max - base);
+        run_max = new_max;
+        float sum2[2] = {0.f, 0.f};
+        uint8_t* p_row = p_tiles + (t * 2 + b) * L::P_BYTES + row * 128;
+#pragma unroll
+        for (int ch = 0; ch < 8; ++ch) {
+          uint32_t w[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float p0 = fast_exp2(fmaf(__uint_as_float(sr[ch * 8 + 2 * e]), sl2, -base));
+            const float p1 = fast_exp2(fmaf(__uint_as_float(sr[ch * 8 + 2 * e + 1]), sl2, -base));
+            sum2[0] += p0;
+            sum2[1] += p1;
+            __nv_bfloat162 pk = __floats2bfloat162_rn(p0, p1);
+            w[e] = *reinterpret_cast<uint32_t*>(&pk);
+          }
+          *reinterpret_cast<uint4*>(p_row + ((ch ^ (row & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+        run_sum = run_sum * keep + (sum2[0] + sum2[1]);
+        // the last page may hold rows past the sequence's end: their V must not reach the product
+        // (both tiles may clear the same rows; they write the same zeros)
+        const int valid = kv_len - j * KEYS;
+        if (valid < KEYS) {
+          const int ld = load_of(t, k), st = ld % STAGES;
+          if (!mbar_wait(&kv_full[st], (ld / STAGES) & 1)) { ok = false; break; }
+          uint8_t* v_tile = kv_tiles + st * 2 * L::TILE_BYTES + L::TILE_BYTES;
+          const int first = valid < 0 ? 0 : valid;
+          const int n16 = (KEYS - first) * 8;                          // 16-byte pieces of the rows to clear, per 64-wide block
+          for (int kb = 0; kb < L::KB; ++kb)
+            for (int x = row; x < n16; x += 128)
+              *reinterpret_cast<uint4*>(v_tile + kb * (KEYS * 128) + first * 128 + x * 16) = make_uint4(0u, 0u, 0u, 0u);
+        }
+        tc_fence_before();
+        fence_async_shared();
+        mbar_arrive(&p_full[t * 2 + b]);
+        if (k >= 1) take_product(k - 1, keep_prev);
+        keep_prev = keep;
       }
-      tc_fence_before();
-      mbar_arrive(&t_empty[t * 2 + tb]);
-    };
-
-    for (int k = 0; k < n_steps && ok; ++k) {
-      const int j = me.j_lo + k, b = k & 1;
-      if (!mbar_wait(&s_full[t * 2 + b], (k >> 1) & 1)) { ok = false; break; }
-      tc_fence_after();
-      uint32_t sr[KEYS];
-      tmem_ld32_issue(lane_addr + b * KEYS, sr);
-      tmem_ld32_issue(lane_addr + b * KEYS + 32, sr + 32);
-      tmem_ld_wait();
-      const bool mask = (j * KEYS + KEYS - 1 > me.pos0) || (window > 0 && j * KEYS <= pos_last_row - window);
-      // (two loops, so that the pages every row sees whole carry no per-element test; four running maxima
-      // keep the chain of dependent instructions short.  The scale, which is positive, is applied to the
-      // maximum here and to each score inside the exponent's multiply-add below.)
-      float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-      if (!mask) {
+      if (ok && n_steps > 0) take_product(n_steps - 1, keep_prev);
+      if (split) {
+        // The two halves of the tile meet: all products of the CTA have been read (each slot has taken its last one),
+        // so the page ring is free; slot 1 leaves its rows' sums, maxima and unnormalised outputs there, slot 0 adds.
+        float* xch = reinterpret_cast<float*>(kv_tiles);                      // [ROWS][HD + 2]
+        asm volatile("bar.sync 2, 256;" ::: "memory");
+        if (t == 1) {
+          float* mine = xch + row * (HD + 2);
 #pragma unroll
-        for (int c = 0; c < KEYS; ++c) mx[c & 3] = fmaxf(mx[c & 3], __uint_as_float(sr[c]));
-      } else {
-        const int lo_key = window > 0 ? pos - window + 1 : 0;       // the row sees keys lo_key .. pos
+          for (int c = 0; c < HD; ++c) mine[c] = o[c];
+          mine[HD] = run_max;
+          mine[HD + 1] = run_sum;
+        }
+        asm volatile("bar.sync 2, 256;" ::: "memory");
+        if (t == 0) {
+          const float* other = xch + row * (HD + 2);
+          const float m1 = other[HD], l1 = other[HD + 1];
+          const float m = fmaxf(run_max, m1);
+          const float s0 = run_max == -INFINITY ? 0.f : fast_exp2(run_max - m), s1 = m1 == -INFINITY ? 0.f : fast_exp2(m1 - m);
+          run_sum = run_sum * s0 + l1 * s1;
 #pragma unroll
-        for (int c = 0; c < KEYS; ++c) {
-          const int key = j * KEYS + c;
-          const float v = (key <= pos && key >= lo_key) ? __uint_as_float(sr[c]) : -INFINITY;
-          sr[c] = __float_as_uint(v);
-          mx[c & 3] = fmaxf(mx[c & 3], v);
+          for (int c = 0; c < HD; ++c) o[c] = o[c] * s0 + other[c] * s1;
         }
       }
-      const float tile_max = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * sl2;
-      const float new_max = fmaxf(run_max, tile_max);
-      const float base = new_max == -INFINITY ? 0.f : new_max;        // a row that has seen nothing yet
-      const float keep = run_max == -INFINITY ? 0.f : fast_exp2(run_max - base);
-      run_max = new_max;
-      float sum2[2] = {0.f, 0.f};
-      uint8_t* p_row = p_tiles + (t * 2 + b) * L::P_BYTES + row * 128;
+      if (ok && row < me.rows && !(split && t == 1)) {
+        const float inv = 1.0f / run_sum;
+        __nv_bfloat16* dst = out + (int64_t)(row0_seq + me.qt * ROWS + row) * ld_out + (int64_t)h * HD;
 #pragma unroll
-      for (int ch = 0; ch < 8; ++ch) {
-        uint32_t w[4];
+        for (int c = 0; c < HD; c += 8) {
+          uint32_t w[4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float p0 = fast_exp2(fmaf(__uint_as_float(sr[ch * 8 + 2 * e]), sl2, -base));
-          const float p1 = fast_exp2(fmaf(__uint_as_float(sr[ch * 8 + 2 * e + 1]), sl2, -base));
-          sum2[0] += p0;
-          sum2[1] += p1;
-          __nv_bfloat162 pk = __floats2bfloat162_rn(p0, p1);
-          w[e] = *reinterpret_cast<uint32_t*>(&pk);
+          for (int e = 0; e < 4; ++e) {
+            __nv_bfloat162 pk = __floats2bfloat162_rn(o[c + 2 * e] * inv, o[c + 2 * e + 1] * inv);
+            w[e] = *reinterpret_cast<uint32_t*>(&pk);
+          }
+          *reinterpret_cast<uint4*>(dst + c) = make_uint4(w[0], w[1], w[2], w[3]);
         }
-        *reinterpret_cast<uint4*>(p_row + ((ch ^ (row & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
-      }
-      run_sum = run_sum * keep + (sum2[0] + sum2[1]);
-      // the last page may hold rows past the sequence's end: their V must not reach the product
-      // (both tiles may clear the same rows; they write the same zeros)
-      const int valid = kv_len - j * KEYS;
-      if (valid < KEYS) {
-        const int ld = load_of(t, k), st = ld % STAGES;
-        if (!mbar_wait(&kv_full[st], (ld / STAGES) & 1)) { ok = false; break; }
-        uint8_t* v_tile = kv_tiles + st * 2 * L::TILE_BYTES + L::TILE_BYTES;
-        const int first = valid < 0 ? 0 : valid;
-        const int n16 = (KEYS - first) * 8;                          // 16-byte pieces of the rows to clear, per 64-wide block
-        for (int kb = 0; kb < L::KB; ++kb)
-          for (int x = row; x < n16; x += 128)
-            *reinterpret_cast<uint4*>(v_tile + kb * (KEYS * 128) + first * 128 + x * 16) = make_uint4(0u, 0u, 0u, 0u);
-      }
-      tc_fence_before();
-      fence_async_shared();
-      mbar_arrive(&p_full[t * 2 + b]);
-      if (k >= 1) take_product(k - 1, keep_prev);
-      keep_prev = keep;
-    }
-    if (ok && n_steps > 0) take_product(n_steps - 1, keep_prev);
-    if (split) {
-      // The two halves of the tile meet: all products of the CTA have been read (each slot has taken its last one),
-      // so the page ring is free; slot 1 leaves its rows' sums, maxima and unnormalised outputs there, slot 0 adds.
-      float* xch = reinterpret_cast<float*>(kv_tiles);                      // [ROWS][HD + 2]
-      asm volatile("bar.sync 2, 256;" ::: "memory");
-      if (t == 1) {
-        float* mine = xch + row * (HD + 2);
-#pragma unroll
-        for (int c = 0; c < HD; ++c) mine[c] = o[c];
-        mine[HD] = run_max;
-        mine[HD + 1] = run_sum;
-      }
-      asm volatile("bar.sync 2, 256;" ::: "memory");
-      if (t == 0) {
-        const float* other = xch + row * (HD + 2);
-        const float m1 = other[HD], l1 = other[HD + 1];
-        const float m = fmaxf(run_max, m1);
-        const float s0 = run_max == -INFINITY ? 0.f : fast_exp2(run_max - m), s1 = m1 == -INFINITY ? 0.f : fast_exp2(m1 - m);
-        run_sum = run_sum * s0 + l1 * s1;
-#pragma unroll
-        for (int c = 0; c < HD; ++c) o[c] = o[c] * s0 + other[c] * s1;
-      }
-    }
-    if (ok && row < me.rows && !(split && t == 1)) {
-      const float inv = 1.0f / run_sum;
-      __nv_bfloat16* dst = out + (int64_t)(row0_seq + me.qt * ROWS + row) * ld_out + (int64_t)h * HD;
-#pragma unroll
-      for (int c = 0; c < HD; c += 8) {
-        uint32_t w[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          __nv_bfloat162 pk = __floats2bfloat162_rn(o[c + 2 * e] * inv, o[c + 2 * e + 1] * inv);
-          w[e] = *reinterpret_cast<uint32_t*>(&pk);
-        }
-        *reinterpret_cast<uint4*>(dst + c) = make_uint4(w[0], w[1], w[2], w[3]);
       }
     }
   }
