@@ -10,8 +10,10 @@
 //   2  S_(c+1) = (decay over chunk c) S_c + U_c                                 from chunk to chunk, entry by entry
 //   3  o_i = sum_(j <= i) (decay from j to i) w_j (q_i . k_j) v_j + (decay to i) S_c^T q_i      every chunk and head by itself
 //
-// All of it is 32-bit arithmetic on the CUDA cores (fmaf chains of 32 to 64 terms; 0.8 G multiply-adds for 2 x 1024 rows of 8
-// heads of 128 x 128, 22 us at their peak).  Decays are powers of the head's constant (retention), or exponentials of
+// The products run on mma.sync with 32-bit operands cut into bfloat16 pieces x = h + m + l (exact above about 2^-110; an operand that is bfloat16 as it
+// comes is one piece): the six products that reach 2^-24, or three, or one.  The tensor core truncates where it accumulates, so h h joins the 32-bit sums by
+// rounded additions after every 16 terms; the others, 2^-8 of it, have an accumulator of their own.  A thread cuts its fragments itself
+// from 32-bit rows in shared memory.  Numbers that are not finite have no pieces: a block that meets one leaves them out of the products and adds their terms by fmaf.  Decays are powers of the head's constant (retention), or exponentials of
 // differences of logarithms that are summed up in 64 bits within the chunk (matrix memory), so that a difference of two large sums
 // keeps its last places.  The matrix memory's running maximum goes along: a chunk's own maximum at its end, the maximum carried over
 // the chunks in step 2, and per row m_i = F_i + max(m_c, max_(j <= i) (i_j - F_j)); every weight is at most 1.
@@ -52,16 +54,134 @@ struct ChunkArgs {
   int tiles;
   // out: 32-bit read-outs, or finished rows
   float* raw; int64_t ld_raw;
-  void* out; int64_t ld_out; const void* gate; int64_t ld_gate; int unit_norm, finish;
+  void* out; int64_t ld_out; const void* gate; int64_t ld_gate; int unit_norm, finish, vec_out;      // vec_out: rows of `out` begin on whole quads
   float eps;
 };
 
-// Four neighbouring entries of a row as floats.
-__device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
-__device__ __forceinline__ float4 load4(const __nv_bfloat16* p) {
-  const uint2 raw = *reinterpret_cast<const uint2*>(p);
-  const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
-  return make_float4(a.x, a.y, b.x, b.y);
+// The upper halves of two floats as a pair of bfloat16 (truncated), and what is left of each.
+__device__ __forceinline__ uint32_t cut(float& a, float& b) {
+  const uint32_t x = __float_as_uint(a), y = __float_as_uint(b);
+  a -= __uint_as_float(x & 0xffff0000u);
+  b -= __uint_as_float(y & 0xffff0000u);
+  return __byte_perm(x, y, 0x7632);
+}
+__device__ __forceinline__ uint32_t upper(float a, float b) { return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632); }
+__device__ __forceinline__ void mma(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+__device__ __forceinline__ bool not_finite(float x) { return (__float_as_uint(x) & 0x7f800000u) == 0x7f800000u; }
+
+// acc[i][j] += sum over k in [0, n) of A[k][row0 + 16 i ..] B[k][col0 + 8 j ..] by a warp, in mma.sync's layout: entry e of a tile is row lane / 4 + 8 (e / 2),
+// column 2 (lane % 4) + e % 2.  PA, PB: pieces of the operands.  n in whole sixteens; row strides of 4 more than a multiple of 32 meet no bank twice.
+// CLEAN: entries that are not finite count as zeros (`leftover` adds what they give).
+template <int MT, int NT, int PA, int PB, bool CLEAN = false>
+__device__ __forceinline__ void product(float (&acc)[MT][NT][4], const float* A, int lda, const float* B, int ldb, int n) {
+  const int g = (threadIdx.x & 31) >> 2, t2 = (threadIdx.x & 3) * 2;
+  float low[MT][NT][4] = {};
+  A += t2 * lda + g;
+  B += t2 * ldb + g;
+#pragma unroll 1
+  for (int k = 0; k < n; k += 16, A += 16 * lda, B += 16 * ldb) {
+    uint32_t ap[PA][MT][4];
+#pragma unroll
+    for (int i = 0; i < MT; ++i)
+#pragma unroll
+      for (int f = 0; f < 4; ++f) {
+        const float* at = A + (f >> 1) * 8 * lda + i * 16 + (f & 1) * 8;
+        float x = at[0], y = at[lda];
+        if (CLEAN) x = not_finite(x) ? 0.f : x, y = not_finite(y) ? 0.f : y;
+        if (PA == 1) {
+          ap[0][i][f] = upper(x, y);
+        } else {
+          ap[0][i][f] = cut(x, y);
+          ap[PA > 1 ? 1 : 0][i][f] = cut(x, y);
+          ap[PA > 2 ? 2 : 0][i][f] = upper(x, y);
+        }
+      }
+    // (two columns of tiles at a time: a product follows three others before it meets its own accumulator again)
+    constexpr int W = NT < 2 ? NT : 2;
+#pragma unroll
+    for (int j0 = 0; j0 < NT; j0 += W) {
+      uint32_t bp[PB][W][2];
+#pragma unroll
+      for (int j = 0; j < W; ++j)
+#pragma unroll
+        for (int f = 0; f < 2; ++f) {
+          const float* at = B + f * 8 * ldb + (j0 + j) * 8;
+          float x = at[0], y = at[ldb];
+          if (CLEAN) x = not_finite(x) ? 0.f : x, y = not_finite(y) ? 0.f : y;
+          if (PB == 1) {
+            bp[0][j][f] = upper(x, y);
+          } else {
+            bp[0][j][f] = cut(x, y);
+            bp[PB > 1 ? 1 : 0][j][f] = cut(x, y);
+            bp[PB > 2 ? 2 : 0][j][f] = upper(x, y);
+          }
+        }
+      float high[MT][W][4] = {};
+      constexpr int PRODUCTS = PA == 3 && PB == 3 ? 6 : (PA == 3 || PB == 3 ? 3 : 1);
+      // which pieces meet: h h, then the small ones from the smallest on
+      constexpr int XA[6] = {0, PA == 3 ? 2 : 0, PA == 3 && PB == 3 ? 0 : (PA == 3 ? 1 : 0), 1, 1, 0}, XB[6] = {0, PA == 3 ? 0 : 2, PA == 3 && PB == 3 ? 2 : (PA == 3 ? 0 : 1), 1, 0, 1};
+#pragma unroll
+      for (int t = 0; t < PRODUCTS; ++t)
+#pragma unroll
+        for (int j = 0; j < W; ++j)
+#pragma unroll
+          for (int i = 0; i < MT; ++i) mma(t == 0 ? high[i][j] : low[i][j0 + j], ap[XA[t] % PA][i], bp[XB[t] % PB][j]);
+#pragma unroll
+      for (int j = 0; j < W; ++j)
+#pragma unroll
+        for (int i = 0; i < MT; ++i)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) acc[i][j0 + j][e] += high[i][j][e];
+    }
+  }
+  if (PA == 3 || PB == 3) {
+#pragma unroll
+    for (int i = 0; i < MT; ++i)
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[i][j][e] += low[i][j][e];
+  }
+}
+// The terms of which an operand is not finite, by fmaf: what they give is what 32-bit arithmetic gives, the other terms' sums keep their bits.  TRIANGLE: a row takes
+// the terms k <= row only (row0: its first row's number).
+template <int MT, int NT, bool TRIANGLE>
+__device__ __noinline__ void leftover_terms(float* acc, const float* A, int lda, const float* B, int ldb, int n, int row0) {
+  const int g = (threadIdx.x & 31) >> 2, t2 = (threadIdx.x & 3) * 2;
+  for (int at = 0; at < MT * NT * 4; ++at) {
+    const int e = at & 3, j = (at >> 2) % NT, i = (at >> 2) / NT;
+    const int r = i * 16 + g + (e >> 1) * 8, c = j * 8 + t2 + (e & 1), m = TRIANGLE ? min(n, row0 + r + 1) : n;
+    float sum = acc[at];
+    for (int k = 0; k < m; ++k) {
+      const float x = A[k * lda + r], y = B[k * ldb + c];
+      if (not_finite(x) || not_finite(y)) sum = fmaf(x, y, sum);
+    }
+    acc[at] = sum;
+  }
+}
+template <int MT, int NT, bool TRIANGLE>
+__device__ __forceinline__ void leftover(float (&acc)[MT][NT][4], const float* A, int lda, const float* B, int ldb, int n, int row0) {
+  float copy[MT * NT * 4];                  // (the accumulators themselves stay in registers)
+#pragma unroll
+  for (int at = 0; at < MT * NT * 4; ++at) copy[at] = acc[(at >> 2) / NT][(at >> 2) % NT][at & 3];
+  leftover_terms<MT, NT, TRIANGLE>(copy, A, lda, B, ldb, n, row0);
+#pragma unroll
+  for (int at = 0; at < MT * NT * 4; ++at) acc[(at >> 2) / NT][(at >> 2) % NT][at & 3] = copy[at];
+}
+// As many pieces as the operands need: PA, PB where rows are bfloat16 as they come (`as_is`), three and three elsewhere; `bad`: some operand is not finite.
+template <int MT, int NT, int PA, int PB, bool TRIANGLE, typename TI>
+__device__ __forceinline__ void product_of(float (&acc)[MT][NT][4], const float* A, int lda, const float* B, int ldb, int n, bool as_is, bool bad, int n_bad, int row0) {
+  if (!bad) {
+    if (sizeof(TI) == 2 && as_is) product<MT, NT, PA, PB>(acc, A, lda, B, ldb, n);
+    else product<MT, NT, 3, 3>(acc, A, lda, B, ldb, n);
+  } else {
+    if (sizeof(TI) == 2 && as_is) product<MT, NT, PA, PB, true>(acc, A, lda, B, ldb, n);
+    else product<MT, NT, 3, 3, true>(acc, A, lda, B, ldb, n);
+    leftover<MT, NT, TRIANGLE>(acc, A, lda, B, ldb, n_bad, row0);
+  }
 }
 
 struct Place { int s, row0, n, pos0; };      // sequence, first row, rows (0: no such chunk), position of the first row
@@ -139,32 +259,61 @@ __device__ __forceinline__ void chunk_gates(const ChunkArgs& a, const Place& p, 
   __syncthreads();
 }
 
-// A chunk's rows of one head into shared memory, `width_to` entries wide: transposed [entry][row] or plain [row][entry]; entries and rows that
-// do not exist are zeros.
-template <typename TI, bool TRANSPOSED>
-__device__ __forceinline__ void bring(float* dst, int ld, const TI* src, int64_t ld_src, const Place& p, int width, int width_to, bool act, float scale_from, int scaled_from) {
-  const int quads = width_to / 4;
-#pragma unroll 4
-  for (int i = threadIdx.x; i < C * quads; i += THREADS) {
-    // transposed: a warp takes 8 rows by 4 neighbouring quads (whole 32-byte sectors of bfloat16, and stores that meet a bank twice)
-    const int r = TRANSPOSED ? (i & 7) + (i >> 5) % (C / 8) * 8 : i / quads, c = (TRANSPOSED ? ((i >> 3) & 3) + (i >> 5) / (C / 8) * 4 : i % quads) * 4;
-    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (r < p.n && c < width) x = load4(src + (int64_t)(p.row0 + r) * ld_src + c);
-    float v[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      if (act) v[e] = silu_f(v[e]);
-      if (c + e >= scaled_from) v[e] *= scale_from;
-      if (TRANSPOSED) dst[(c + e) * ld + r] = v[e];
-    }
-    if (!TRANSPOSED) *reinterpret_cast<float4*>(dst + r * ld + c) = make_float4(v[0], v[1], v[2], v[3]);
-  }
+// A chunk's rows of one head on their way into shared memory, W entries wide: transposed [entry][row] or plain [row][entry]; entries and rows that
+// do not exist are zeros.  `ask` starts the loads (of several operands, before the first `put`), `put` says whether any of the thread's entries is not finite.
+__device__ __forceinline__ float4 widen(const float4& x) { return x; }
+__device__ __forceinline__ float4 widen(const uint2& raw) {
+  const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
+  return make_float4(a.x, a.y, b.x, b.y);
 }
+template <typename TI> struct Quad { using type = float4; };
+template <> struct Quad<__nv_bfloat16> { using type = uint2; };
+template <typename TI, int W, bool TRANSPOSED>
+struct Rows {
+  using Raw = typename Quad<TI>::type;
+  static constexpr int N = C * (W / 4) / THREADS;
+  Raw raw[N];
+  static __device__ __forceinline__ void place(int f, int& r, int& c) {
+    const int i = threadIdx.x + f * THREADS;
+    // transposed: a warp takes 8 rows by 4 neighbouring quads (whole 32-byte sectors of bfloat16, and stores that meet a bank twice)
+    r = TRANSPOSED ? (i & 7) + (i >> 5) % (C / 8) * 8 : i / (W / 4);
+    c = (TRANSPOSED ? ((i >> 3) & 3) + (i >> 5) / (C / 8) * 4 : i % (W / 4)) * 4;
+  }
+  __device__ __forceinline__ void ask(const TI* src, int64_t ld_src, const Place& p, int width) {
+#pragma unroll
+    for (int f = 0; f < N; ++f) {
+      int r, c;
+      place(f, r, c);
+      raw[f] = Raw{};
+      if (r < p.n && c < width) raw[f] = *reinterpret_cast<const Raw*>(src + (int64_t)(p.row0 + r) * ld_src + c);
+    }
+  }
+  __device__ __forceinline__ bool put(float* dst, int ld, bool act, float scale_from, int scaled_from) const {
+    bool bad = false;
+#pragma unroll
+    for (int f = 0; f < N; ++f) {
+      int r, c;
+      place(f, r, c);
+      const float4 x = widen(raw[f]);
+      float v[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        if (act) v[e] = silu_f(v[e]);
+        if (c + e >= scaled_from) v[e] *= scale_from;
+        bad |= not_finite(v[e]);
+        if (TRANSPOSED) dst[(c + e) * ld + r] = v[e];
+      }
+      if (!TRANSPOSED) *reinterpret_cast<float4*>(dst + r * ld + c) = make_float4(v[0], v[1], v[2], v[3]);
+    }
+    return bad;
+  }
+};
 
 // Pairs of q (or null) and k turned by the rows' positions where they lie, k scaled after turning.
 template <bool TRANSPOSED>
 __device__ __forceinline__ void turn(const ChunkArgs& a, const Place& p, float* q, float* k, int ld) {
   const int half = a.rot_dims / 2;
+#pragma unroll 4
   for (int i = threadIdx.x; i < C * half; i += THREADS) {
     const int r = TRANSPOSED ? i % C : i / half, pr = TRANSPOSED ? i / C : i % half;
     const int ea = a.interleaved ? 2 * pr : pr, eb = a.interleaved ? 2 * pr + 1 : pr + half;
@@ -182,29 +331,13 @@ __device__ __forceinline__ void turn(const ChunkArgs& a, const Place& p, float* 
   }
 }
 
-// acc[i][j] += sum over n of A[n][rows] B[n][cols], both read in quads; a thread's rows are ty * 4 .. + 3 (and the same 64 further), its columns likewise.
-template <int TR, int TC>
-__device__ __forceinline__ void outer(float (&acc)[TR][TC], const float* A, int lda, const float* B, int ldb, int n, int ty, int tx) {
-#pragma unroll 4
-  for (int t = 0; t < n; ++t) {
-    float x[TR], y[TC];
-#pragma unroll
-    for (int g = 0; g < TR; g += 4) *reinterpret_cast<float4*>(x + g) = *reinterpret_cast<const float4*>(A + t * lda + ty * 4 + g * 16);
-#pragma unroll
-    for (int g = 0; g < TC; g += 4) *reinterpret_cast<float4*>(y + g) = *reinterpret_cast<const float4*>(B + t * ldb + tx * 4 + g * 16);
-#pragma unroll
-    for (int i = 0; i < TR; ++i)
-#pragma unroll
-      for (int j = 0; j < TC; ++j) acc[i][j] = fmaf(x[i], y[j], acc[i][j]);
-  }
-}
-
 // ---- 1: what a chunk leaves in the state ---------------------------------------------------------------------------------
 template <int KIND, typename TI, int DK, int DV>
-__global__ void __launch_bounds__(THREADS) chunk_sum_kernel(const ChunkArgs a) {
+__global__ void __launch_bounds__(THREADS, 2) chunk_sum_kernel(const ChunkArgs a) {
+  constexpr int LDK = DK + 4, LDV = DV + 4;
   extern __shared__ float smem[];
-  float* ks = smem;                         // [C][DK]
-  float* vs = ks + C * DK;                  // [C][DV]
+  float* ks = smem;                         // [C][LDK]
+  float* vs = ks + C * LDK;                 // [C][LDV]
   __shared__ double F[KIND == MEMORY ? C : 1];
   __shared__ float in[C], best[C], weight[C], scratch;
   pdl_launch_dependents();
@@ -213,8 +346,15 @@ __global__ void __launch_bounds__(THREADS) chunk_sum_kernel(const ChunkArgs a) {
   const Place p = find(a, a.place0 + blockIdx.x);
   if (p.n == 0) return;
   const bool half = KIND == RETENTION && a.rot_dims > 0;
-  bring<TI, false>(ks, DK, (const TI*)a.k + qh * a.dk, a.ld_k, p, a.dk, DK, KIND == RETENTION && a.act, a.k_scale, a.rot_dims);
-  bring<TI, false>(vs, DV, (const TI*)a.v + h * a.dv, a.ld_v, p, a.dv, DV, KIND == RETENTION && a.act, 1.f, DV);
+  bool bad;
+  {
+    Rows<TI, DK, false> k;
+    Rows<TI, DV, false> v;
+    k.ask((const TI*)a.k + qh * a.dk, a.ld_k, p, a.dk);
+    v.ask((const TI*)a.v + h * a.dv, a.ld_v, p, a.dv);
+    k.put(ks, LDK, KIND == RETENTION && a.act, a.k_scale, a.rot_dims);
+    bad = v.put(vs, LDV, KIND == RETENTION && a.act, 1.f, DV);
+  }
   if (KIND == MEMORY) {
     chunk_gates(a, p, h, F, in, best, &scratch);
     if (threadIdx.x < C) {                  // weights at the chunk's end, against its own maximum there
@@ -224,40 +364,51 @@ __global__ void __launch_bounds__(THREADS) chunk_sum_kernel(const ChunkArgs a) {
   } else {
     if (half) {
       __syncthreads();
-      turn<false>(a, p, nullptr, ks, DK);
+      turn<false>(a, p, nullptr, ks, LDK);
     }
     if (threadIdx.x < C) weight[threadIdx.x] = powf(a.decay[h], (float)max(0, p.n - 1 - (int)threadIdx.x));
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < C * DK; i += THREADS) ks[i] *= weight[i / DK];
-  __syncthreads();
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  // (entries in the state's own order: retention [dk][dv], the matrix memory [dv][dk])
-  constexpr int TR = (KIND == MEMORY ? DV : DK) / 16, TC = (KIND == MEMORY ? DK : DV) / 16;
-  float acc[TR][TC];
-#pragma unroll
-  for (int i = 0; i < TR; ++i)
-#pragma unroll
-    for (int j = 0; j < TC; ++j) acc[i][j] = 0.f;
-  if (KIND == MEMORY) outer<TR, TC>(acc, vs, DV, ks, DK, p.n, ty, tx);
-  else outer<TR, TC>(acc, ks, DK, vs, DV, p.n, ty, tx);
+  for (int i = threadIdx.x; i < C * (DK / 4); i += THREADS) {
+    float4* at = reinterpret_cast<float4*>(ks + i / (DK / 4) * LDK + i % (DK / 4) * 4);
+    const float w = weight[i / (DK / 4)];
+    float4 x = *at;
+    x.x *= w; x.y *= w; x.z *= w; x.w *= w;
+    bad |= not_finite(x.x) || not_finite(x.y) || not_finite(x.z) || not_finite(x.w);
+    *at = x;
+  }
+  bad = __syncthreads_or(bad);
+  // (entries in the state's own order: retention [dk][dv], the matrix memory [dv][dk]; a warp has half of the rows, 32 at a time, and a quarter of the columns)
+  constexpr int NR = KIND == MEMORY ? DV : DK, NC = KIND == MEMORY ? DK : DV, NT = NC / 32;
+  const int warp = threadIdx.x >> 5, col0 = (warp >> 1) * (NC / 4), n16 = (p.n + 15) & ~15;
+  const float* A = KIND == MEMORY ? vs : ks;
+  const float* B = (KIND == MEMORY ? ks : vs) + col0;
+  constexpr int LDA = KIND == MEMORY ? LDV : LDK, LDB = KIND == MEMORY ? LDK : LDV, EA = KIND == MEMORY ? 1 : 3, EB = KIND == MEMORY ? 3 : 1;
   const int rows = KIND == MEMORY ? a.dv : a.dk, cols = KIND == MEMORY ? a.dk : a.dv;
   float* u = a.work + ((int64_t)blockIdx.x * a.heads + h) * a.dk * a.dv;
+  const int g = (threadIdx.x & 31) >> 2, t2 = (threadIdx.x & 3) * 2;
+#pragma unroll 1
+  for (int row0 = (warp & 1) * 32; row0 < NR; row0 += 64) {
+    float acc[2][NT][4] = {};
+    product_of<2, NT, EA, EB, false, TI>(acc, A + row0, LDA, B, LDB, n16, !(KIND == RETENTION && a.act), bad, p.n, 0);
 #pragma unroll
-  for (int i = 0; i < TR; ++i) {
-    const int r = ty * 4 + (i & 3) + (i >> 2) * 64;
-    if (r >= rows) continue;
+    for (int i = 0; i < 2; ++i)
 #pragma unroll
-    for (int j = 0; j < TC; j += 4) {
-      const int c = tx * 4 + (j >> 2) * 64;
-      if (c < cols) *reinterpret_cast<float4*>(u + r * cols + c) = make_float4(acc[i][j], acc[i][j + 1], acc[i][j + 2], acc[i][j + 3]);
-    }
+      for (int e = 0; e < 4; e += 2) {
+        const int r = row0 + i * 16 + g + e * 4;
+        if (r >= rows) continue;
+#pragma unroll
+        for (int j = 0; j < NT; ++j) {
+          const int c = col0 + j * 8 + t2;
+          if (c < cols) *reinterpret_cast<float2*>(u + r * cols + c) = make_float2(acc[i][j][e], acc[i][j][e + 1]);
+        }
+      }
   }
   if (KIND == MEMORY) {
     float* un = a.work_n + ((int64_t)blockIdx.x * a.heads + h) * (a.dk + 2);
     for (int d = threadIdx.x; d < a.dk; d += THREADS) {
       float sum = 0.f;
-      for (int t = 0; t < p.n; ++t) sum += ks[t * DK + d];
+      for (int t = 0; t < p.n; ++t) sum += ks[t * LDK + d];
       un[d] = sum;
     }
     if (threadIdx.x == 0) {
@@ -352,6 +503,7 @@ __global__ void chunk_max_kernel(const ChunkArgs a) {
 }
 
 // ---- 3: the read-outs ------------------------------------------------------------------------------------------------------
+// A warp has 32 of the chunk's rows and a quarter of the columns.
 template <int KIND, typename TI, int DK, int DV>
 __global__ void __launch_bounds__(THREADS, 2) chunk_read_kernel(const ChunkArgs a) {
   constexpr int PIECE = 32, LDS = DV + 4;                               // rows of the state that come at a time
@@ -359,21 +511,32 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_read_kernel(const ChunkArgs 
   extern __shared__ float smem[];
   float* qt = smem;                         // [DK][LDT]
   float* kt = qt + DK * LDT;                // [DK][LDT], later the weighted scores [j][i] and a piece of the state
-  float* vs = kt + REGION;                  // [C][DV]
+  float* vs = kt + REGION;                  // [C][LDS]
   float* pt = kt;
   float* ss = kt + C * LDT;
   __shared__ double F[KIND == MEMORY ? C : 1];
-  __shared__ float in[C], best[C], power[C + 1], carried[C], den[4][C], scratch, mx[C];
+  __shared__ float in[C], best[C], power[C + 1], carried[C], den[5][C], sq_sum[4][C], scratch, mx[C];
   pdl_launch_dependents();
   pdl_wait();
   const int h = blockIdx.y, qh = h / a.group;
   const Place p = find(a, a.place0 + blockIdx.x);
   if (p.n == 0) return;
   const bool act = KIND == RETENTION && a.act;
-  bring<TI, true>(qt, LDT, (const TI*)a.q + qh * a.dk, a.ld_q, p, a.dk, DK, act, a.q_scale, 0);
-  bring<TI, true>(kt, LDT, (const TI*)a.k + qh * a.dk, a.ld_k, p, a.dk, DK, act, a.k_scale, a.rot_dims);
-  bring<TI, false>(vs, DV, (const TI*)a.v + h * a.dv, a.ld_v, p, a.dv, DV, act, 1.f, DV);
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  // Rows that are bfloat16 as they come stay so (one piece); their factors go to the scores and to what the state gives.
+  const bool as_is = sizeof(TI) == 2 && !act && (KIND == MEMORY || a.rot_dims == 0);
+  bool bad;
+  {
+    Rows<TI, DK, true> q, k;
+    Rows<TI, DV, false> v;
+    q.ask((const TI*)a.q + qh * a.dk, a.ld_q, p, a.dk);
+    k.ask((const TI*)a.k + qh * a.dk, a.ld_k, p, a.dk);
+    v.ask((const TI*)a.v + h * a.dv, a.ld_v, p, a.dv);
+    bad = q.put(qt, LDT, act, a.q_scale, as_is ? DK : 0);
+    bad |= k.put(kt, LDT, act, a.k_scale, as_is ? DK : a.rot_dims);
+    bad |= v.put(vs, LDS, act, 1.f, DV);
+  }
+  const float owed_q = as_is ? a.q_scale : 1.f, owed_k = as_is ? a.k_scale : 1.f;
+  const int warp = threadIdx.x >> 5, wr = (warp & 1) * 32, wc = warp >> 1, g = (threadIdx.x & 31) >> 2, t2 = (threadIdx.x & 3) * 2;
   if (KIND == MEMORY) {
     const float m_c = a.work_m[(int64_t)blockIdx.x * a.heads + h];
     chunk_gates(a, p, h, F, in, best, &scratch);
@@ -390,7 +553,7 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_read_kernel(const ChunkArgs 
     }
     if (threadIdx.x <= C) power[threadIdx.x] = powf(a.decay[h], (float)threadIdx.x);
   }
-  __syncthreads();
+  bad = __syncthreads_or(bad);
 
   // The state before the chunk comes a piece at a time by way of registers, each piece asked for before the arithmetic that runs ahead of it.
   // (The matrix memory's is [dv][dk]: a thread takes four neighbours along dk of one column.)
@@ -409,57 +572,62 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_read_kernel(const ChunkArgs 
   };
   fetch(0);
 
-  float sc[4][4] = {};
-#pragma unroll 1
-  for (int d0 = 0; d0 < DK; d0 += PIECE) {              // (sums of 32 terms, added up: less rounding than one chain of 128)
-    float part[4][4] = {};
-    outer<4, 4>(part, qt + d0 * LDT, LDT, kt + d0 * LDT, LDT, PIECE, ty, tx);
+  float sc[2][2][4] = {};
+  if (wr + 31 >= wc * 16)                   // (tiles above the diagonal are not seen)
+    product_of<2, 2, 1, 1, false, TI>(sc, qt + wr, LDT, kt + wc * 16, LDT, DK, as_is, bad, a.dk, 0);
+  // weights; the matrix memory's sums of a row's weighted scores meet over its four threads and the four warps of its columns
+  bool wild = false;
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < 2; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) sc[i][j] += part[i][j];
-  }
-  // weights; the matrix memory's sums of a row's weighted scores meet over its 16 threads
+    for (int e2 = 0; e2 < 2; ++e2) {
+      const int r = wr + i * 16 + g + e2 * 8;
+      float sum = 0.f;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int r = ty * 4 + i;
-    float sum = 0.f;
+      for (int j = 0; j < 2; ++j)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int c = tx * 4 + j;
-      // (a row that is not seen counts for nothing, also where its score is no number)
-      if (c <= r && r < p.n) sc[i][j] *= KIND == MEMORY ? expf((float)((double)in[c] - F[c] - (double)mx[r])) : power[r - c];
-      else sc[i][j] = 0.f;
-      sum += sc[i][j];
+        for (int e1 = 0; e1 < 2; ++e1) {
+          const int c = wc * 16 + j * 8 + t2 + e1;
+          float& x = sc[i][j][e2 * 2 + e1];
+          // (a row that is not seen counts for nothing, also where its score is no number)
+          if (c <= r && r < p.n) x *= owed_q * owed_k * (KIND == MEMORY ? expf((float)((double)in[c] - F[c] - (double)mx[r])) : power[r - c]);
+          else x = 0.f;
+          wild |= not_finite(x);
+          sum += x;
+        }
+      if (KIND == MEMORY) {
+        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+        if (t2 == 0) den[wc][r] = sum;
+      }
     }
-    if (KIND == MEMORY) {
-#pragma unroll
-      for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-      if (tx == 0) den[0][r] = sum;
-    }
-  }
+  wild = __syncthreads_or(wild) || bad;     // (the keys have been used up)
   if (KIND == MEMORY) {                     // ... and the normaliser before the chunk along the row's query
     const float* n_c = a.work_n + ((int64_t)blockIdx.x * a.heads + h) * (a.dk + 2);
-    const int r = threadIdx.x & (C - 1), part = threadIdx.x / C;
+    const int r = threadIdx.x >> 2, part = threadIdx.x & 3;
     float sum = 0.f;
     for (int d = part; d < a.dk; d += 4) sum = fmaf(qt[d * LDT + r], n_c[d], sum);
-    __syncthreads();
-    if (part > 0) den[part][r] = sum;
-    __syncthreads();
-    if (part == 0) den[0][r] = fmaf(carried[r], (sum + den[1][r]) + (den[2][r] + den[3][r]), den[0][r]);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+    if (part == 0) den[4][r] = fmaf(carried[r], sum * owed_q, (den[0][r] + den[1][r]) + (den[2][r] + den[3][r]));
   }
-  __syncthreads();                          // the keys have been used up
 #pragma unroll
-  for (int j = 0; j < 4; ++j) *reinterpret_cast<float4*>(pt + (tx * 4 + j) * LDT + ty * 4) = make_float4(sc[0][j], sc[1][j], sc[2][j], sc[3][j]);
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) pt[(wc * 16 + j * 8 + t2 + (e & 1)) * LDT + wr + i * 16 + g + (e >> 1) * 8] = sc[i][j][e];
 
-  constexpr int TC = DV / 16;
-  float acc[4][TC] = {};
+  constexpr int NT = DV / 32;
+  const int col0 = wc * (DV / 4);
+  float acc[2][NT][4] = {};
   for (int d0 = 0; d0 < a.dk; d0 += PIECE) {
-    const int nd = min(PIECE, a.dk - d0);
     if (d0 > 0) __syncthreads();
+    bool odd = false;
 #pragma unroll
     for (int f = 0; f < FETCH; ++f) {
       const int i = threadIdx.x + f * THREADS;
+      odd |= not_finite(piece[f].x) || not_finite(piece[f].y) || not_finite(piece[f].z) || not_finite(piece[f].w);
       if (KIND == MEMORY) {
         const int c = i % DV, d = i / DV * 4;
         ss[d * LDS + c] = piece[f].x;
@@ -471,72 +639,89 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_read_kernel(const ChunkArgs 
       }
     }
     if (d0 + PIECE < a.dk) fetch(d0 + PIECE);
-    __syncthreads();
-    float part[4][TC] = {};
-    outer<4, TC>(part, qt + d0 * LDT, LDT, ss, LDS, nd, ty, tx);
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < TC; ++j) acc[i][j] += part[i][j];
+    odd = __syncthreads_or(odd) || bad;
+    product_of<2, NT, 1, 3, false, TI>(acc, qt + d0 * LDT + wr, LDT, ss + col0, LDS, PIECE, as_is, odd, min(PIECE, a.dk - d0), 0);
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float w = KIND == MEMORY ? carried[ty * 4 + i] : power[ty * 4 + i + 1];
+  for (int i = 0; i < 2; ++i)
 #pragma unroll
-    for (int j = 0; j < TC; ++j) acc[i][j] *= w;
-  }
-  // values of the rows that a row sees, and no others: a zero weight would make NaN of a value that is not finite
-  outer<4, TC>(acc, pt, LDT, vs, DV, min(p.n, ty * 4), ty, tx);
+    for (int e = 0; e < 4; ++e) {
+      const int r = wr + i * 16 + g + (e >> 1) * 8;
+      const float w = (KIND == MEMORY ? carried[r] : power[r + 1]) * owed_q;
 #pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    const int t = ty * 4 + e;
-    if (t >= p.n) break;
-    float y[TC];
-#pragma unroll
-    for (int g = 0; g < TC; g += 4) *reinterpret_cast<float4*>(y + g) = *reinterpret_cast<const float4*>(vs + t * DV + tx * 4 + g * 16);
-#pragma unroll
-    for (int i = e; i < 4; ++i) {
-      const float x = pt[t * LDT + ty * 4 + i];
-#pragma unroll
-      for (int j = 0; j < TC; ++j) acc[i][j] = fmaf(x, y[j], acc[i][j]);
+      for (int j = 0; j < NT; ++j) acc[i][j][e] *= w;
     }
-  }
+  // values of the rows that a row sees (the others' weights are zeros)
+  product_of<2, NT, 3, 1, true, TI>(acc, pt + wr, LDT, vs + col0, LDS, wr + 32, !act, wild, p.n, wr);
 
+  Rows<TI, DV, false> gate;                 // (asked for now, wanted with the rows)
+  if (KIND == RETENTION && a.finish && a.gate != nullptr) gate.ask((const TI*)a.gate + h * a.dv, a.ld_gate, p, a.dv);
+  float factor[2][2];
+  if (KIND == RETENTION && a.finish && a.unit_norm) {
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int r = ty * 4 + i;
-    float factor = 1.f;
-    if (KIND == MEMORY) factor = 1.f / (fmaxf(fabsf(den[0][r]), r < p.n ? expf(-(float)(F[r] + (double)mx[r])) : 1.f) + 1e-6f);
-    if (KIND == RETENTION && a.finish && a.unit_norm) {
-      float sq = 0.f;
+    for (int i = 0; i < 2; ++i)
 #pragma unroll
-      for (int j = 0; j < TC; ++j) sq = fmaf(acc[i][j], acc[i][j], sq);      // (columns beyond dv are zeros)
+      for (int e2 = 0; e2 < 2; ++e2) {
+        float sq = 0.f;
 #pragma unroll
-      for (int o = 8; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
-      factor = 1.0f / sqrtf(sq / (float)a.dv + a.eps);
+        for (int j = 0; j < NT; ++j)        // (columns beyond dv are zeros)
+          sq = fmaf(acc[i][j][e2 * 2], acc[i][j][e2 * 2], fmaf(acc[i][j][e2 * 2 + 1], acc[i][j][e2 * 2 + 1], sq));
+        sq += __shfl_xor_sync(0xffffffffu, sq, 1);
+        sq += __shfl_xor_sync(0xffffffffu, sq, 2);
+        if (t2 == 0) sq_sum[wc][wr + i * 16 + g + e2 * 8] = sq;
+      }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int e2 = 0; e2 < 2; ++e2) {
+      const int r = wr + i * 16 + g + e2 * 8;
+      factor[i][e2] = 1.f;
+      if (KIND == MEMORY) factor[i][e2] = 1.f / (fmaxf(fabsf(den[4][r]), r < p.n ? expf(-(float)(F[r] + (double)mx[r])) : 1.f) + 1e-6f);
+      if (KIND == RETENTION && a.finish && a.unit_norm)
+        factor[i][e2] = 1.0f / sqrtf(((sq_sum[0][r] + sq_sum[1][r]) + (sq_sum[2][r] + sq_sum[3][r])) / (float)a.dv + a.eps);
     }
-    if (r >= p.n) continue;
+  // rows leave by way of shared memory, whole quads side by side (a thread's own entries are pairs)
+  __syncthreads();                          // nobody reads queries, scores or pieces any more
+  float* os = smem;                         // [C][LDS]
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int e2 = 0; e2 < 2; ++e2)
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
+        *reinterpret_cast<float2*>(os + (wr + i * 16 + g + e2 * 8) * LDS + col0 + j * 8 + t2) =
+            make_float2(acc[i][j][e2 * 2] * factor[i][e2], acc[i][j][e2 * 2 + 1] * factor[i][e2]);
+  __syncthreads();
+#pragma unroll
+  for (int f = 0; f < gate.N; ++f) {
+    int r, c;
+    gate.place(f, r, c);
+    if (r >= p.n || c >= a.dv) continue;
     const int64_t row = p.row0 + r;
+    const float4 x = *reinterpret_cast<const float4*>(os + r * LDS + c);
+    if (KIND == RETENTION && a.finish) {
+      float y[4] = {x.x, x.y, x.z, x.w};
+      if (a.gate != nullptr) {
+        const float4 g4 = widen(gate.raw[f]);
+        const float gt[4] = {g4.x, g4.y, g4.z, g4.w};
 #pragma unroll
-    for (int j = 0; j < TC; j += 4) {
-      const int c = tx * 4 + (j >> 2) * 64;
-      if (c >= a.dv) continue;
-      float y[4];
+        for (int e = 0; e < 4; ++e) y[e] *= sizeof(TI) == 2 ? __fdividef(gt[e], 1.0f + __expf(-gt[e])) : gt[e] / (1.0f + expf(-gt[e]));
+      }
+      TI* o = (TI*)a.out + row * a.ld_out + h * a.dv + c;
+      if (a.vec_out) {
+        typename Quad<TI>::type w;
+        TI* parts = reinterpret_cast<TI*>(&w);
 #pragma unroll
-      for (int e = 0; e < 4; ++e) y[e] = acc[i][j + e] * factor;
-      if (KIND == RETENTION && a.finish) {
-        if (a.gate != nullptr) {
-          const float4 g4 = load4((const TI*)a.gate + row * a.ld_gate + h * a.dv + c);
-          const float g[4] = {g4.x, g4.y, g4.z, g4.w};
-#pragma unroll
-          for (int e = 0; e < 4; ++e) y[e] *= g[e] / (1.0f + expf(-g[e]));
-        }
-        TI* o = (TI*)a.out + row * a.ld_out + h * a.dv + c;
+        for (int e = 0; e < 4; ++e) parts[e] = from_f32<TI>(y[e]);
+        *reinterpret_cast<typename Quad<TI>::type*>(o) = w;
+      } else {
 #pragma unroll
         for (int e = 0; e < 4; ++e) o[e] = from_f32<TI>(y[e]);
-      } else {
-        *reinterpret_cast<float4*>(a.raw + row * a.ld_raw + h * a.dv + c) = make_float4(y[0], y[1], y[2], y[3]);
       }
+    } else {
+      *reinterpret_cast<float4*>(a.raw + row * a.ld_raw + h * a.dv + c) = x;
     }
   }
 }
@@ -550,9 +735,10 @@ int room(K kernel, size_t smem) {
 
 template <int KIND, typename TI, int DK, int DV>
 int launch(ChunkArgs a, int span, cudaStream_t stream) {
-  constexpr size_t sum_smem = (size_t)C * (DK + DV) * 4;
+  constexpr size_t sum_smem = (size_t)C * (DK + DV + 8) * 4;
   constexpr int LDS = DV + 4, region = DK * LDT > C * LDT + 32 * LDS ? DK * LDT : C * LDT + 32 * LDS;
-  constexpr size_t read_smem = ((size_t)DK * LDT + region + C * DV) * 4;
+  constexpr size_t read_smem = ((size_t)DK * LDT + region + C * LDS) * 4;
+  static_assert((size_t)C * LDS * 4 <= read_smem, "the rows leave through shared memory");
   static bool configured = false;
   if (!configured) {
     int rc = room(chunk_sum_kernel<KIND, TI, DK, DV>, sum_smem);
@@ -618,6 +804,7 @@ KVAD_EXPORT int kvad_retention_chunked(int dtype, const void* q, int64_t ld_q, c
   const uintptr_t unit = dtype == KVAD_DTYPE_F32 ? 15 : 7;
   if (gate != nullptr && (ld_gate % 4 || (reinterpret_cast<uintptr_t>(gate) & unit)))
     KVAD_FAIL(KVAD_ERR_UNSUPPORTED, "retention (chunked): the gate comes in whole quads");
+  a.vec_out = ld_out % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & unit) == 0 ? 1 : 0;
   if (dtype == KVAD_DTYPE_F32) return dispatch<RETENTION, float>(a, span, stream);
   if (dtype == KVAD_DTYPE_BF16) return dispatch<RETENTION, __nv_bfloat16>(a, span, stream);
   KVAD_FAIL(KVAD_ERR_UNSUPPORTED, "retention (chunked): unknown dtype %d", dtype);
