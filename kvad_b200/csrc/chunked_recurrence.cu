@@ -70,6 +70,11 @@ __device__ __forceinline__ void mma(float (&c)[4], const uint32_t (&a)[4], const
   asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
+// the same into zeros
+__device__ __forceinline__ void mma_first(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+      : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]), "f"(0.f));
+}
 __device__ __forceinline__ bool not_finite(float x) { return (__float_as_uint(x) & 0x7f800000u) == 0x7f800000u; }
 
 // acc[i][j] += sum over k in [0, n) of A[k][row0 + 16 i ..] B[k][col0 + 8 j ..] by a warp, in mma.sync's layout: entry e of a tile is row lane / 4 + 8 (e / 2),
@@ -119,7 +124,7 @@ __device__ __forceinline__ void product(float (&acc)[MT][NT][4], const float* A,
             bp[PB > 2 ? 2 : 0][j][f] = upper(x, y);
           }
         }
-      float high[MT][W][4] = {};
+      float high[MT][W][4];
       constexpr int PRODUCTS = PA == 3 && PB == 3 ? 6 : (PA == 3 || PB == 3 ? 3 : 1);
       // which pieces meet: h h, then the small ones from the smallest on
       constexpr int XA[6] = {0, PA == 3 ? 2 : 0, PA == 3 && PB == 3 ? 0 : (PA == 3 ? 1 : 0), 1, 1, 0}, XB[6] = {0, PA == 3 ? 0 : 2, PA == 3 && PB == 3 ? 2 : (PA == 3 ? 0 : 1), 1, 0, 1};
@@ -128,7 +133,10 @@ __device__ __forceinline__ void product(float (&acc)[MT][NT][4], const float* A,
 #pragma unroll
         for (int j = 0; j < W; ++j)
 #pragma unroll
-          for (int i = 0; i < MT; ++i) mma(t == 0 ? high[i][j] : low[i][j0 + j], ap[XA[t] % PA][i], bp[XB[t] % PB][j]);
+          for (int i = 0; i < MT; ++i) {
+            if (t == 0) mma_first(high[i][j], ap[0][i], bp[0][j]);
+            else mma(low[i][j0 + j], ap[XA[t] % PA][i], bp[XB[t] % PB][j]);
+          }
 #pragma unroll
       for (int j = 0; j < W; ++j)
 #pragma unroll

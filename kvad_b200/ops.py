@@ -56,6 +56,10 @@ _SIGNATURES = {
         "kvad_linear_split_heads": [c_void_p, c_int64, c_int64, c_void_p, c_void_p, c_int64, c_int64, c_int, c_int, c_int, c_int, c_void_p],
         "kvad_linear_split_status": [],
     },
+    "linear_pieces": {
+        "kvad_linear_pieces": [c_void_p, c_int64, c_void_p, c_void_p, c_int, c_void_p, c_int64, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int64, c_void_p],
+        "kvad_linear_pieces_status": [],
+    },
     "linear_tcgen05": {
         "kvad_linear_tcgen05": [c_void_p, c_int64, c_void_p, c_void_p, c_int, c_void_p, c_int64, c_int, c_int, c_int,
                                 c_int, c_int, c_void_p],
@@ -258,7 +262,7 @@ def lib(name: str) -> ctypes.CDLL:
 
 #: kernel libraries by what needs them: every model ("base"), and the families a part names in `Part.kernel_families`
 _FAMILY_LIBRARIES = {
-    "base": {"any": ("rows", "linear_simt", "sampling"), torch.bfloat16: ("linear_rows", "linear_tcgen05"), torch.float32: ("linear_rows_f32", "linear_split")},
+    "base": {"any": ("rows", "linear_simt", "sampling"), torch.bfloat16: ("linear_rows", "linear_tcgen05"), torch.float32: ("linear_rows_f32", "linear_split", "linear_pieces")},
     "causal_attention": {"any": ("attention_simt", "attention_decode"), torch.bfloat16: ("attention_prefill",), torch.float32: ()},
     "norm_rotary": {"any": ("norm_rotary",)},
     "scored_attention": {"any": ("attention_scored",), torch.bfloat16: ("attention_scored_prompt",)},
@@ -370,6 +374,7 @@ class Ops:
         self.rows_linear_max = (2 if dtype == torch.bfloat16 else 16) if self._rows_lib in have else 0
         # 32-bit products of many rows on the tensor cores, their operands cut into bfloat16 pieces (linear_split.cu)
         self.split_linear = dtype == torch.float32 and "linear_split" in have
+        self.pieces_linear = self.split_linear and "linear_pieces" in have      # the same with the pieces cut by a pass before (linear_pieces.cu)
         self.scored_prompt = dtype == torch.bfloat16 and "attention_scored_prompt" in have     # shaped scores of prompt rows on the tensor cores
         self.chunked_recurrences = "chunked_recurrence" in have     # recurrences of prompts: products of 64 rows, not a walk
         self.tiled_prompt = True    # prompts that the tensor-core kernel does not take: the tiled CUDA-core kernel, not the row-by-row one
@@ -388,8 +393,8 @@ class Ops:
         """Everything on the host that decides which kernels a step of a given shape launches; part of
         the key under which a step's CUDA graph is kept."""
         return (_switch_epoch, self.tensor_core_linear, self.tensor_core_prefill, self.fast_decode,
-                self.rows_linear_max, self.qkv_sums, self.SUMS_MIN_K, self.tiled_prompt, self.split_linear, self.scored_prompt, self.chunked_recurrences,
-                self.SPLIT_MIN_ROWS, self.SCORED_PROMPT_MIN_NEW, self.CHUNK_MIN_ROWS, self.CHUNK_SHORT_ROWS, self.CHUNK_WORK_BYTES,
+                self.rows_linear_max, self.qkv_sums, self.SUMS_MIN_K, self.tiled_prompt, self.split_linear, self.pieces_linear, self.scored_prompt, self.chunked_recurrences,
+                self.SPLIT_MIN_ROWS, self.PIECES_MIN_ROWS, self.PIECES_MIN_K, self.PIECES_WORK_BYTES, self.SCORED_PROMPT_MIN_NEW, self.CHUNK_MIN_ROWS, self.CHUNK_SHORT_ROWS, self.CHUNK_WORK_BYTES,
                 self.ROWS_LINEAR_MAX_OUT, self.ROWS_BLOCKS_MAX, self.HEADS_LINEAR_MAX_ROWS)
 
     def begin_step(self) -> None:
@@ -450,6 +455,10 @@ class Ops:
     # for few rows: at 33 rows a layer of GPT-2 small's sizes takes 147 us this way and about 100 us as weights streamed in blocks of
     # 16 rows (a generation from a 33-token prompt: 8.99 ms against 8.25 ms); at 65 rows of 768 x 3072 it is 78 us against the CUDA cores' 165.
     SPLIT_MIN_ROWS = 65
+    # The same with the weights cut by a pass of their own (linear_pieces.cu), where K is long enough to pay for the pass.  (us of that and of linear_split.cu: 70 rows of
+    # 128 x 128: 7.2, 6.5; 256 x 256: 9.0, 9.6; 512 x 512: 12.6, 15.8; 768 x 3072: 55, 78; 1510 rows of 768 x 2304: 36, 61; 768 x 768: 23, 26; 768 x 3072: 55, 68; 3072 x 768: 53, 80.)
+    PIECES_MIN_ROWS, PIECES_MIN_K = 65, 256
+    PIECES_WORK_BYTES = 1 << 29      # scratch of a product, at most (a head of 50257 x 1600: 482 MB)
     ROWS_BLOCKS_MAX = 64           # 32-bit: up to so many rows go through the weight-streaming form in blocks of 16
 
     def linear(self, a, weight, bias, out, epilogue: str = "store", *, tile: int = 0, splits: int = 0,
@@ -498,6 +507,15 @@ class Ops:
             raise KernelError("linear: the weight-streaming form takes at most 16 rows and K a multiple of a 16-byte piece, at most 1024 pieces")
         if (form == "auto" and self.split_linear and m >= self.SPLIT_MIN_ROWS and k % 4 == 0 and lda % 4 == 0 and a.data_ptr() % 16 == 0
                 and weight.data_ptr() % 16 == 0):
+            need = 192 * (n + 191) * ((k + 31) // 32)          # (three pieces of the weights, rows up to a tile's end, K to a block's)
+            if self.pieces_linear and m >= self.PIECES_MIN_ROWS and k >= self.PIECES_MIN_K and need <= self.PIECES_WORK_BYTES:
+                h = lib("linear_pieces")
+                work = torch.empty(need, dtype=torch.uint8, device=a.device)
+                width = int(tile) if tile in (64, 128, 192) else 0
+                _check(h.kvad_linear_pieces(_ptr(a), lda, _ptr(weight), _ptr(bias), bias_f32, _ptr(out), ldo, m, n, k, epi, width, _ptr(work), need, _stream()), h)
+                global _launches
+                _launches += 1          # the pass that cuts
+                return
             h = lib("linear_split")
             width = int(tile) if tile in (64, 128) else 0          # (its own widths; the bfloat16 kernel's others say nothing to it)
             _check(h.kvad_linear_split(_ptr(a), lda, _ptr(weight), _ptr(bias), bias_f32, _ptr(out), ldo, m, n, k, epi, width, _stream()), h)
@@ -1833,6 +1851,15 @@ def linear_split_wait_timeouts() -> int:
     """How many bounded waits of the 32-bit product on the tensor cores have run out (0 in a healthy run)."""
     h = lib("linear_split")
     n = h.kvad_linear_split_status()
+    if n < 0:
+        raise KernelError(h.kvad_last_error().decode("utf-8", "replace"))
+    return n
+
+
+def linear_pieces_wait_timeouts() -> int:
+    """How many bounded waits of the 32-bit product of cut operands have run out (0 in a healthy run)."""
+    h = lib("linear_pieces")
+    n = h.kvad_linear_pieces_status()
     if n < 0:
         raise KernelError(h.kvad_last_error().decode("utf-8", "replace"))
     return n

@@ -101,3 +101,27 @@ def test_a_tile_width_of_the_other_kernels_is_the_split_products_own_choice(tile
     ops.linear(a, w, None, want)
     ops.linear(a, w, None, got, tile=tile)
     assert torch.equal(got, want)
+
+
+# one row past a tile, ends of tiles of every width, K that ends within a block of 32 and within an odd one, more tiles than SMs (a CTA's rings run on)
+@pytest.mark.parametrize("m,n,k", [(65, 1, 256), (128, 193, 260), (129, 64, 300), (257, 385, 512), (1500, 2309, 292), (70, 130, 772)])
+@pytest.mark.parametrize("tile", [64, 128, 192])
+def test_product_of_cut_weights_has_the_split_products_bits(m, n, k, tile):
+    from kvad_b200.ops import linear_pieces_wait_timeouts
+    g = torch.Generator(device="cuda")
+    g.manual_seed(m + n * k)
+    ops, split = Ops(torch.float32), Ops(torch.float32)
+    split.pieces_linear, ops.PIECES_MIN_K = False, 1
+    a, w, b, old = randn(g, m, k + 8)[:, 4:4 + k], randn(g, n, k) * 0.3, randn(g, n), randn(g, m, n + 3)[:, :n]
+    strange = a.clone()
+    strange[m // 2, 3], strange[m - 1, k - 1] = float("inf"), float("nan")
+    for x, epi in ((a, "store"), (a, "gelu_tanh"), (a, "gelu_erf"), (a, "residual"), (strange, "store")):
+        outs = []
+        for o, t in ((ops, tile), (split, 0)):
+            out = torch.full((m, n + 3), float("nan"), device="cuda")
+            out[:, :n] = old
+            o.linear(x, w, b, out[:, :n], epi, tile=t)
+            assert torch.isnan(out[:, n:]).all()
+            outs.append(out[:, :n].clone())
+        assert torch.equal(outs[0].nan_to_num(7.0), outs[1].nan_to_num(7.0)) and torch.equal(outs[0].isnan(), outs[1].isnan())
+    assert linear_pieces_wait_timeouts() == 0
