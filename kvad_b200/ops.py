@@ -137,6 +137,13 @@ _SIGNATURES = {
         "kvad_attention_scored_prompt_takes": [c_int, c_int, c_int, c_int],
         "kvad_attention_scored_prompt_status": [],
     },
+    "attention_scored_wide": {
+        "kvad_attention_scored_wide": [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
+                                       c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_float, c_int, c_int,
+                                       c_int, c_int, c_void_p],
+        "kvad_attention_scored_wide_takes": [c_int, c_int, c_int],
+        "kvad_attention_scored_wide_status": [],
+    },
     "retention": {
         "kvad_retention": [c_int, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64,
                            c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
@@ -263,9 +270,9 @@ def lib(name: str) -> ctypes.CDLL:
 #: kernel libraries by what needs them: every model ("base"), and the families a part names in `Part.kernel_families`
 _FAMILY_LIBRARIES = {
     "base": {"any": ("rows", "linear_simt", "sampling"), torch.bfloat16: ("linear_rows", "linear_tcgen05"), torch.float32: ("linear_rows_f32", "linear_split", "linear_pieces")},
-    "causal_attention": {"any": ("attention_simt", "attention_decode"), torch.bfloat16: ("attention_prefill",), torch.float32: ()},
+    "causal_attention": {"any": ("attention_simt", "attention_decode"), torch.bfloat16: ("attention_prefill",), torch.float32: ("attention_scored_wide",)},
     "norm_rotary": {"any": ("norm_rotary",)},
-    "scored_attention": {"any": ("attention_scored",), torch.bfloat16: ("attention_scored_prompt",)},
+    "scored_attention": {"any": ("attention_scored",), torch.bfloat16: ("attention_scored_prompt",), torch.float32: ("attention_scored_wide",)},
     "prompt_attention": {torch.bfloat16: ("attention_prefill",)},
     "retention": {"any": ("retention", "chunked_recurrence")},
     "gated_recurrence": {"any": ("gated_recurrence", "chunked_recurrence", "chunked_channels")},
@@ -350,6 +357,11 @@ def _scored_prompt_takes(dk: int, dv: int, alias: bool, out_f32: bool) -> bool:
     return lib("attention_scored_prompt").kvad_attention_scored_prompt_takes(dk, dv, int(alias), int(out_f32)) == 1
 
 
+@functools.lru_cache(maxsize=256)
+def _scored_wide_takes(dk: int, dv: int, alias: bool) -> bool:
+    return lib("attention_scored_wide").kvad_attention_scored_wide_takes(dk, dv, int(alias)) == 1
+
+
 class Ops:
     """Kernels bound to one compute dtype."""
 
@@ -376,6 +388,7 @@ class Ops:
         self.split_linear = dtype == torch.float32 and "linear_split" in have
         self.pieces_linear = self.split_linear and "linear_pieces" in have      # the same with the pieces cut by a pass before (linear_pieces.cu)
         self.scored_prompt = dtype == torch.bfloat16 and "attention_scored_prompt" in have     # shaped scores of prompt rows on the tensor cores
+        self.scored_wide = dtype == torch.float32 and "attention_scored_wide" in have          # prompt rows of 32-bit attention there too, in pieces
         self.chunked_recurrences = "chunked_recurrence" in have     # recurrences of prompts: products of 64 rows, not a walk
         self.tiled_prompt = True    # prompts that the tensor-core kernel does not take: the tiled CUDA-core kernel, not the row-by-row one
         self._counters = None       # zeroed ints the decode kernel counts finished splits in (left zeroed by it)
@@ -393,7 +406,7 @@ class Ops:
         """Everything on the host that decides which kernels a step of a given shape launches; part of
         the key under which a step's CUDA graph is kept."""
         return (_switch_epoch, self.tensor_core_linear, self.tensor_core_prefill, self.fast_decode,
-                self.rows_linear_max, self.qkv_sums, self.SUMS_MIN_K, self.tiled_prompt, self.split_linear, self.pieces_linear, self.scored_prompt, self.chunked_recurrences,
+                self.rows_linear_max, self.qkv_sums, self.SUMS_MIN_K, self.tiled_prompt, self.split_linear, self.pieces_linear, self.scored_prompt, self.scored_wide, self.chunked_recurrences,
                 self.SPLIT_MIN_ROWS, self.PIECES_MIN_ROWS, self.PIECES_MIN_K, self.PIECES_WORK_BYTES, self.SCORED_PROMPT_MIN_NEW, self.CHUNK_MIN_ROWS, self.CHUNK_SHORT_ROWS, self.CHUNK_WORK_BYTES,
                 self.ROWS_LINEAR_MAX_OUT, self.ROWS_BLOCKS_MAX, self.HEADS_LINEAR_MAX_ROWS)
 
@@ -645,9 +658,9 @@ class Ops:
     def attention_prompt(self, q, out, seq_starts, kv_lens, n_seqs: int, max_new: int, page_table, k_pages, v_pages,
                          n_heads: int, scale: float, window: int = 0) -> None:
         """Rows of sequences packed one after another (`seq_starts`), each sequence's rows being its last positions
-        (`kv_lens` is its length after the step): causal attention on the CUDA cores in 32-bit arithmetic, a page of
-        keys brought into shared memory once for 32 rows (the float32 engine's prompts; in bfloat16 the head sizes
-        the tensor-core kernel refuses)."""
+        (`kv_lens` is its length after the step): causal attention in 32-bit arithmetic (the float32 engine's prompts; in bfloat16 the
+        head sizes the tensor-core kernel refuses).  32-bit heads of up to 128 entries in eights run on the tensor cores in pieces, the others
+        on the CUDA cores, a page of keys brought into shared memory once for 32 rows."""
         _need_cuda(q, out, seq_starts, kv_lens, page_table, k_pages, v_pages)
         ld_q, ld_o = _rows_view(q, "attention queries"), _rows_view(out, "attention output")
         _, n_kv, page, hd = k_pages.shape
@@ -655,6 +668,12 @@ class Ops:
             raise KernelError("attention_prompt: queries/output do not match heads x head size")
         if q.dtype != self.dtype or out.dtype != self.dtype or k_pages.dtype != self.dtype:
             raise KernelError(f"attention_prompt: tensors must be {self.dtype}")
+        if self.scored_wide and max_new >= self.SCORED_PROMPT_MIN_NEW and self._wide_takes(q, out, k_pages, v_pages, hd, hd, page, ld_q, ld_o, n_seqs, n_heads, max_new):
+            h = lib("attention_scored_wide")
+            _check(h.kvad_attention_scored_wide(_ptr(q), ld_q, _ptr(out), ld_o, None, 0, 0, None, _ptr(seq_starts), _ptr(kv_lens), _ptr(page_table),
+                                                page_table.shape[1], _ptr(k_pages), _ptr(v_pages), int(n_seqs), n_heads, n_kv, hd, hd, page, int(max_new),
+                                                float(scale), 0.0, 0.0, int(window or 0), 0, 0, 1, _stream()), h)
+            return
         h = lib("attention_simt")
         _check(h.kvad_attention_tiled(self.code, _ptr(q), ld_q, _ptr(out), ld_o, _ptr(seq_starts), _ptr(kv_lens), _ptr(page_table),
                                       page_table.shape[1], _ptr(k_pages), _ptr(v_pages), int(n_seqs), n_heads, n_kv, hd, page,
@@ -1183,6 +1202,15 @@ class Ops:
                                                   float(slope_span or 0.0), int(window or 0), int(keep_first or 0), int(chunk or 0), int(key_maps),
                                                   int(out_f32), _stream()), h)
             return
+        if (self.scored_wide and max_new >= self.SCORED_PROMPT_MIN_NEW and n_splits == 1
+                and self._wide_takes(q, out, k_pages, v_pages, dk, dv, page, ld_q, ld_o, n_seqs, n_heads, max_new)
+                and (gate is None or gate_heads or (ld_g % 4 == 0 and gate.data_ptr() % 16 == 0))):
+            h = lib("attention_scored_wide")
+            _check(h.kvad_attention_scored_wide(_ptr(q), ld_q, _ptr(out), ld_o, _ptr(gate), ld_g, int(gate_heads), _ptr(sinks), _ptr(seq_starts), _ptr(kv_lens),
+                                                _ptr(page_table), page_table.shape[1], _ptr(k_pages), _ptr(v_ptr), int(n_seqs), int(n_heads), n_kv, dk, dv,
+                                                page, int(max_new), float(scale), float(softcap or 0.0), float(slope_span or 0.0), int(window or 0),
+                                                int(keep_first or 0), int(chunk or 0), int(key_maps), _stream()), h)
+            return
         h = lib("attention_scored")
         _check(h.kvad_attention_scored(self.code, _ptr(q), ld_q, _ptr(out), ld_o, _ptr(gate), ld_g, _ptr(seq_starts), _ptr(kv_lens),
                                        _ptr(page_table), page_table.shape[1], _ptr(k_pages), _ptr(v_ptr), int(n_seqs), int(n_heads), n_kv,
@@ -1193,6 +1221,12 @@ class Ops:
         if n_splits > 1 and merge:
             global _launches
             _launches += 1          # the merge kernel
+
+    def _wide_takes(self, q, out, k_pages, v_pages, dk, dv, page, ld_q, ld_o, n_seqs, n_heads, max_new) -> bool:
+        """Whether 32-bit prompt rows go to attention_scored_wide.cu: whole 16-byte pieces, sizes whose pieces fit an SM."""
+        v = k_pages if v_pages is None else v_pages
+        return (page == 64 and ld_q % 4 == 0 and ld_o % 4 == 0 and (q.data_ptr() | out.data_ptr() | k_pages.data_ptr() | v.data_ptr()) % 16 == 0
+                and (v_pages is not None or dv <= dk) and n_seqs * n_heads * (max_new // 64 + 1) < 1 << 31 and _scored_wide_takes(dk, dv, v_pages is None))
 
     @staticmethod
     def scored_splits(n_rows: int, n_kv_heads: int, group: int, reach: int, n_sms: Optional[int] = None, per_sm: int = 2) -> int:
@@ -1860,6 +1894,15 @@ def linear_pieces_wait_timeouts() -> int:
     """How many bounded waits of the 32-bit product of cut operands have run out (0 in a healthy run)."""
     h = lib("linear_pieces")
     n = h.kvad_linear_pieces_status()
+    if n < 0:
+        raise KernelError(h.kvad_last_error().decode("utf-8", "replace"))
+    return n
+
+
+def scored_wide_wait_timeouts() -> int:
+    """How many bounded waits of the 32-bit prompt attention have run out (0 in a healthy run)."""
+    h = lib("attention_scored_wide")
+    n = h.kvad_attention_scored_wide_status()
     if n < 0:
         raise KernelError(h.kvad_last_error().decode("utf-8", "replace"))
     return n
