@@ -20,8 +20,12 @@
 // This header holds the kernel; linear_rows.cu builds it for bfloat16 and linear_rows_f32.cu for float32 - two
 // libraries, compiled side by side, of which a model loads the one of its compute dtype.
 //
+// Few outputs of long K (a down projection) are too few warps that way, each a long chain: there four warps take a quarter of a column's K each
+// and meet in shared memory (768 outputs of K = 3072, one row, back to back on weights of their own: 32-bit 4.28 -> 3.03 us, bfloat16 3.31 -> 2.91).
+//
 // Sums are 32-bit; the order of additions for an output depends on K only, so a row's bits do not
-// depend on its company.  (It is another order than the tiled kernel's: the two agree to rounding.)
+// depend on its company: a lane's sums of each quarter of K are added in their order, whoever summed them up, then the lanes meet.  (It is another order than
+// the tiled kernel's: the two agree to rounding.)
 #pragma once
 #include "common.cuh"
 
@@ -62,8 +66,12 @@ template <> struct Piece<float> {
   }
 };
 
-// MR: activation rows handled (M <= MR); NI: 16-byte pieces of a weight row per lane (K <= NI * 32 * VE).
-template <typename T, int MR, int NI, int EPI>
+// Pieces a lane has of a row, and of a quarter of it where there are enough to sum quarters up by themselves.
+__host__ __device__ inline int lane_pieces(int K, int ve) { return (K / ve + 31) / 32; }
+__host__ __device__ inline int quarter_pieces(int K, int ve) { return lane_pieces(K, ve) >= 12 ? (lane_pieces(K, ve) + 3) / 4 : lane_pieces(K, ve); }
+
+// MR: activation rows handled (M <= MR); NI: 16-byte pieces of a weight row per lane (K <= NI * 32 * VE; where SHARE warps share a column: of its quarter).
+template <typename T, int MR, int NI, int EPI, int SHARE>
 __global__ void __launch_bounds__(ROWS_THREADS)
 linear_rows_kernel(const T* __restrict__ A, int64_t lda, const T* __restrict__ W,
                    const void* __restrict__ bias, int bias_f32, void* __restrict__ out, int64_t ldo,
@@ -71,17 +79,19 @@ linear_rows_kernel(const T* __restrict__ A, int64_t lda, const T* __restrict__ W
   constexpr int VE = Piece<T>::VE;
   extern __shared__ __align__(16) unsigned char rows_smem[];
   T* As = reinterpret_cast<T*>(rows_smem);      // [MR][K]
+  __shared__ float quarters[SHARE > 1 ? ROWS_WARPS : 1][MR][32];
   pdl_launch_dependents();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int col0 = (blockIdx.x * ROWS_WARPS + warp) * cols_per_warp;
+  const int quarter = quarter_pieces(K, VE), part = SHARE > 1 ? warp % SHARE : 0, i0 = part * quarter;
+  const int col0 = SHARE > 1 ? blockIdx.x * (ROWS_WARPS / SHARE) + warp / SHARE : (blockIdx.x * ROWS_WARPS + warp) * cols_per_warp;
 
   // the first column's weights, before the wait
   uint4 w[NI];
   auto fetch = [&](int n) {
 #pragma unroll
     for (int i = 0; i < NI; ++i) {
-      const int k0 = (lane + 32 * i) * VE;
-      w[i] = (n < N && k0 < K) ? *reinterpret_cast<const uint4*>(W + (int64_t)n * K + k0) : make_uint4(0u, 0u, 0u, 0u);
+      const int k0 = (lane + 32 * (i0 + i)) * VE;
+      w[i] = (n < N && k0 < K && (SHARE == 1 || i < quarter)) ? *reinterpret_cast<const uint4*>(W + (int64_t)n * K + k0) : make_uint4(0u, 0u, 0u, 0u);
     }
   };
   fetch(col0);
@@ -99,14 +109,23 @@ linear_rows_kernel(const T* __restrict__ A, int64_t lda, const T* __restrict__ W
 
   for (int c = 0; c < cols_per_warp; ++c) {
     const int n = col0 + c;
-    if (n >= N) break;
-    float acc[MR];
+    if (SHARE == 1 && n >= N) break;
+    float acc[MR], total[MR];
 #pragma unroll
-    for (int m = 0; m < MR; ++m) acc[m] = 0.f;
+    for (int m = 0; m < MR; ++m) acc[m] = total[m] = 0.f;
+    int whole = quarter;                     // where the next quarter begins
 #pragma unroll
     for (int i = 0; i < NI; ++i) {
-      const int k0 = (lane + 32 * i) * VE;
-      if (k0 < K) {
+      const int k0 = (lane + 32 * (i0 + i)) * VE;
+      if (SHARE == 1 && NI >= 12 && i == whole) {
+        whole += quarter;
+#pragma unroll
+        for (int m = 0; m < MR; ++m) {
+          total[m] += acc[m];
+          acc[m] = 0.f;
+        }
+      }
+      if (k0 < K && (SHARE == 1 || i < quarter)) {
         float wf[VE];
         Piece<T>::unpack(w[i], wf);
 #pragma unroll
@@ -120,6 +139,21 @@ linear_rows_kernel(const T* __restrict__ A, int64_t lda, const T* __restrict__ W
           acc[m] = s;
         }
       }
+    }
+    if (SHARE > 1) {
+#pragma unroll
+      for (int m = 0; m < MR; ++m) quarters[warp][m][lane] = acc[m];
+      __syncthreads();
+      if (part != 0 || n >= N) return;
+#pragma unroll
+      for (int m = 0; m < MR; ++m) {
+#pragma unroll
+        for (int q = 0; q < SHARE; ++q) total[m] += quarters[warp + q][m][lane];
+        acc[m] = total[m];
+      }
+    } else {
+#pragma unroll
+      for (int m = 0; m < MR; ++m) acc[m] = total[m] + acc[m];
     }
     const float b = b0;
     if (c + 1 < cols_per_warp) {             // the next column's weights are on their way during the reduction
@@ -148,25 +182,25 @@ linear_rows_kernel(const T* __restrict__ A, int64_t lda, const T* __restrict__ W
   }
 }
 
-template <typename T, int MR, int NI>
+template <typename T, int MR, int NI, int SHARE>
 int launch_epi(int epilogue, const void* A, int64_t lda, const void* W, const void* bias, int bias_f32, void* out,
                int64_t ldo, int M, int N, int K, cudaStream_t stream) {
   // columns per warp: enough CTAs to fill every SM with four, not more
   int cpw = (N + ROWS_WARPS * KVAD_ROWS_TARGET_CTAS - 1) / (ROWS_WARPS * KVAD_ROWS_TARGET_CTAS);
-  if (cpw < 1) cpw = 1;
-  const int grid = (N + ROWS_WARPS * cpw - 1) / (ROWS_WARPS * cpw);
+  if (cpw < 1 || SHARE > 1) cpw = 1;
+  const int grid = (N + ROWS_WARPS * cpw / SHARE - 1) / (ROWS_WARPS * cpw / SHARE);
   const size_t smem = (size_t)MR * K * sizeof(T);
   if (smem > 200 * 1024)
     KVAD_FAIL(KVAD_ERR_UNSUPPORTED, "linear_rows: %d rows of %d columns do not fit shared memory", MR, K);
 #define KVAD_ROWS(E)                                                                                                \
   {                                                                                                                 \
     static size_t configured = 0;                                                                                   \
-    if (smem > 48 * 1024 && smem > configured) {                                                                    \
-      cudaError_t e = cudaFuncSetAttribute(linear_rows_kernel<T, MR, NI, E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+    if (smem > 40 * 1024 && smem > configured) {                                                                    \
+      cudaError_t e = cudaFuncSetAttribute(linear_rows_kernel<T, MR, NI, E, SHARE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
       if (e != cudaSuccess) KVAD_FAIL(KVAD_ERR_CUDA, "linear_rows: cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(e)); \
       configured = smem;                                                                                            \
     }                                                                                                               \
-    kvad_launch(linear_rows_kernel<T, MR, NI, E>, dim3(grid), dim3(ROWS_THREADS), smem, stream, (const T*)A,        \
+    kvad_launch(linear_rows_kernel<T, MR, NI, E, SHARE>, dim3(grid), dim3(ROWS_THREADS), smem, stream, (const T*)A,        \
                 lda, (const T*)W, bias, bias_f32, out, ldo, M, N, K, cpw);                                          \
   }
   switch (epilogue) {
@@ -185,11 +219,17 @@ int launch_epi(int epilogue, const void* A, int64_t lda, const void* W, const vo
 template <typename T, int MR>
 int launch_ni(int epilogue, const void* A, int64_t lda, const void* W, const void* bias, int bias_f32, void* out,
               int64_t ldo, int M, int N, int K, cudaStream_t stream) {
-  constexpr int PER = 32 * Piece<T>::VE;          // columns of K one piece per lane covers
-  if (K <= 4 * PER) return launch_epi<T, MR, 4>(epilogue, A, lda, W, bias, bias_f32, out, ldo, M, N, K, stream);
-  if (K <= 8 * PER) return launch_epi<T, MR, 8>(epilogue, A, lda, W, bias, bias_f32, out, ldo, M, N, K, stream);
-  if (K <= 16 * PER) return launch_epi<T, MR, 16>(epilogue, A, lda, W, bias, bias_f32, out, ldo, M, N, K, stream);
-  return launch_epi<T, MR, 32>(epilogue, A, lda, W, bias, bias_f32, out, ldo, M, N, K, stream);
+  const int pieces = lane_pieces(K, Piece<T>::VE), quarter = quarter_pieces(K, Piece<T>::VE);
+  // Four warps a column where K is long, the columns are few enough for a launch of four CTAs an SM, and a block's rows leave room for those CTAs.
+  if constexpr (MR <= 4) {
+    if (quarter < pieces && N * 4 <= ROWS_WARPS * KVAD_ROWS_TARGET_CTAS && (size_t)MR * K * sizeof(T) <= 50 * 1024)
+      return quarter <= 4 ? launch_epi<T, MR, 4, 4>(epilogue, A, lda, W, bias, bias_f32, out, ldo, M, N, K, stream)
+                          : launch_epi<T, MR, 8, 4>(epilogue, A, lda, W, bias, bias_f32, out, ldo, M, N, K, stream);
+  }
+  if (pieces <= 4) return launch_epi<T, MR, 4, 1>(epilogue, A, lda, W, bias, bias_f32, out, ldo, M, N, K, stream);
+  if (pieces <= 8) return launch_epi<T, MR, 8, 1>(epilogue, A, lda, W, bias, bias_f32, out, ldo, M, N, K, stream);
+  if (pieces <= 16) return launch_epi<T, MR, 16, 1>(epilogue, A, lda, W, bias, bias_f32, out, ldo, M, N, K, stream);
+  return launch_epi<T, MR, 32, 1>(epilogue, A, lda, W, bias, bias_f32, out, ldo, M, N, K, stream);
 }
 
 template <typename T>

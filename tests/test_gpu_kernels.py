@@ -723,3 +723,21 @@ def test_a_bounded_wait_that_runs_out_is_reported_and_harmless():
     assert linear_case(ops, "bfloat16", 32, 128, 128, "store", g, form="swapped") < KTOL["bfloat16"]
     assert linear_case(ops, "bfloat16", 300, 200, 256, "gelu_tanh", g) < KTOL["bfloat16"]
     assert tcgen05_wait_timeouts() == again
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("n,k", [(1, 1536), (766, 3072), (1184, 2000), (1185, 3072), (100, 4096)])
+def test_linear_of_few_rows_and_long_k_keeps_a_rows_bits(dtype, n, k):
+    """Four warps a column at one to four rows and few outputs, one warp elsewhere: the same sums in the same order, whatever a row's company."""
+    g = torch.Generator().manual_seed(n + k)
+    ops = Ops(DT[dtype])
+    a, w = dev(torch.randn(16, k, generator=g).to(DT[dtype])), dev((torch.randn(n, k, generator=g) * 0.1).to(DT[dtype]))
+    want = a.double().cpu() @ w.double().cpu().t()
+    whole = None
+    for m in (16, 8, 5, 4, 3, 2, 1):
+        out = torch.full((m, n), float("nan"), device="cuda")
+        if m * k * a.element_size() <= 200 * 1024:
+            ops.linear(a[:m], w, None, out, "store_f32", form="rows")
+            whole = out if whole is None else whole
+            assert torch.equal(out, whole[:m])
+            assert rel(out, want[:m]) < 1e-6
