@@ -2,7 +2,7 @@
 //
 // A CTA has two SLOTS, each a group of four softmax warps (a thread per row) with its own S, P and P.V
 // buffers, that walk cache pages (64 keys each) side by side.  What limits the kernel is the chain
-// through one softmax thread - ~0.9 us a page - so the work is cut to keep every chain short: a tile of
+// of waits through one slot - ~1.1 us a page - so the work is cut to keep every chain short: a tile of
 // 128 rows that sees more than 8 pages is given to BOTH slots, each walking half of its pages, and
 // the halves (unnormalised output, maximum, sum) meet through shared memory at the end; shorter
 // tiles go two to a CTA, a longer one paired with a shorter one.  Roles: warp 0 brings Q and a ring of

@@ -6,8 +6,8 @@
 // sum, so the order of operations for a row depends on nothing but its own
 // keys.  It takes what the faster kernels do not: head sizes and page sizes
 // that the decode kernel or the tiled kernel below refuse, in either dtype.
-// The float32 engine's prompts (and the bfloat16 engine's, at head sizes its
-// tensor-core kernel refuses) run the tiled kernel further down.
+// Prompts at head sizes that the tensor-core kernels refuse (bfloat16: attention_prefill.cu;
+// 32-bit heads above 128 entries or not in eights: attention_scored_wide.cu) run the tiled kernel further down.
 //
 // bisand/kvad: attend(), crates/llm/src/model/mod.rs:769-819 - score =
 // dot(q,k) * (1/sqrt(head_dim)), softmax with the maximum subtracted

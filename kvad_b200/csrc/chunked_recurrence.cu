@@ -18,8 +18,10 @@
 // keeps its last places.  The matrix memory's running maximum goes along: a chunk's own maximum at its end, the maximum carried over
 // the chunks in step 2, and per row m_i = F_i + max(m_c, max_(j <= i) (i_j - F_j)); every weight is at most 1.
 //
-// Measured: 2 x 1024 rows of 8 heads of 128 x 128 (rotated, normed, gated, bfloat16) 387 -> 85 us; the matrix memory over 1000 + 517 + 37 rows of 8
-// heads of 64 x 128 334 -> 50 us.  (92 and 53 before the state came a piece ahead by way of registers and rows by whole sectors.)
+// Measured: 2 x 1024 rows of 8 heads of 128 x 128 (rotated, normed, gated, bfloat16) 387 us walked, 84 with fmaf chains, 68 so; the matrix memory over
+// 1000 + 517 + 37 rows of 8 heads of 64 x 128 334, 48 and 39.  Of the 68: kernel 1 15 (rows 4, turning and weights 4, product 6), kernel 2 6, kernel 3 42 (rows 5,
+// turning 4, scores 7, state 17, values 1, norm, gate and rows out 6), the rest between them.  At six products mma.sync is no faster than the CUDA cores' peak; what it
+// saves is the shared-memory traffic that kept them at a fifth of it.
 //
 // Chunks of all sequences lie in one list: chunk c of sequence s is place seq_starts[s] / 64 + s + c, which never collides.  The list is taken in
 // spans of as many places as the scratch holds, one after another: the sequences' own states carry over from one to the next.

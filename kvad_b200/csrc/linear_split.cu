@@ -1,5 +1,5 @@
 // out[M,N] = epilogue(A[M,K] . W[N,K]^T + bias) of 32-bit operands on the 5th-generation tensor cores, without giving up
-// 32-bit accuracy: the product of the float32 engine's prompts.
+// 32-bit accuracy: the float32 engine's products of many rows and short K, and its head-wise maps (longer K: linear_pieces.cu, which cuts the weights once a product).
 //
 // Every operand x is cut into three bfloat16 pieces by truncation, x = h + m + l exactly (24 bits of significand = 3 x 8), and
 //   a.w = h_a h_w + (h_a m_w + m_a h_w) + (h_a l_w + m_a m_w + l_a h_w)       (what is left out is below 2^-24 of |a||w|)
