@@ -1202,8 +1202,8 @@ class Ops:
                                                   float(slope_span or 0.0), int(window or 0), int(keep_first or 0), int(chunk or 0), int(key_maps),
                                                   int(out_f32), _stream()), h)
             return
-        if (self.scored_wide and max_new >= self.SCORED_PROMPT_MIN_NEW and n_splits == 1
-                and self._wide_takes(q, out, k_pages, v_pages, dk, dv, page, ld_q, ld_o, n_seqs, n_heads, max_new)
+        if (self.scored_wide and max_new >= self.SCORED_PROMPT_MIN_NEW and n_splits == 1 and 1 <= heads_per_block <= 32 and (sinks is None or merge)
+                and n_seqs <= 65535 and self._wide_takes(q, out, k_pages, v_pages, dk, dv, page, ld_q, ld_o, n_seqs, n_heads, max_new)
                 and (gate is None or gate_heads or (ld_g % 4 == 0 and gate.data_ptr() % 16 == 0))):
             h = lib("attention_scored_wide")
             _check(h.kvad_attention_scored_wide(_ptr(q), ld_q, _ptr(out), ld_o, _ptr(gate), ld_g, int(gate_heads), _ptr(sinks), _ptr(seq_starts), _ptr(kv_lens),
