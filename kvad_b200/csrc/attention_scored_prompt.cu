@@ -36,6 +36,7 @@ constexpr uint32_t TM_COLS = 512;
 constexpr size_t SMEM_MOST = 226 * 1024, SMEM_REST = STATS * ROWS * 8 + 320 + 1024;      // (statistics, barriers, alignment)
 
 struct PromptArgs {
+  const __nv_bfloat16* q; int64_t ld_q; const __nv_bfloat16* k_pages; const __nv_bfloat16* v_pages;      // (read by `row_again` alone: the products' operands come by TMA)
   void* out; int64_t ld_out;
   const __nv_bfloat16* gate; int64_t ld_gate; int gate_heads;    // gate_heads: one number per row and head
   const float* sinks;
@@ -279,8 +280,9 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
       unpair(add2(sum2[0], sum2[1]), s0, s1);
       stats[(j % STATS) * ROWS + row] = make_float2(most, s0 + s1);
       mbar_arrive_one(&st_full[j % STATS]);
-      // Places past the sequence's end may hold anything: no weight is on them, but their values must not be NaN.
-      const int valid = kv_len - key0;
+      // Places past the block's last position may hold anything: no weight is on them, but their values must not be NaN.  (Those past the sequence's end always, so that
+      // no row is worked out twice for what the cache held before; S of the page is done, so shared keys and values can go.)
+      const int valid = last_pos + 1 - key0;
       if (valid < PAGE) {
         const int st = j % stages;
         if (!mbar_wait(&kv_full[st], (j / stages) & 1)) break;
@@ -342,6 +344,7 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         mbar_arrive_one(&t_empty[slot]);
       }
     }
+    float odd = 0.f;                                              // no number as soon as an entry is not finite
     if (ok && ti < n_tok) {
       float inv;
       if (a.sinks == nullptr) {
@@ -359,7 +362,10 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
 #pragma unroll
         for (int e = 0; e < 4; ++e) unpair(o[c * 4 + e], x[2 * e], x[2 * e + 1]);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) x[e] *= inv;
+        for (int e = 0; e < 8; ++e) {
+          x[e] *= inv;
+          odd = fmaf(x[e], 0.f, odd);
+        }
         if (F32OUT) {
           float* dst = reinterpret_cast<float*>(a.out) + grow * a.ld_out + (int64_t)h * a.dv + d;
           if (a.vec) {
@@ -397,6 +403,31 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
           }
         }
       }
+    }
+    __syncwarp();                                                 // (a lane's entries are read by the others)
+    for (uint32_t rows = __ballot_sync(0xffffffffu, ok && ti < n_tok && !(odd == 0.f)); rows != 0; rows &= rows - 1) {
+      const int r = quarter * 32 + __ffs(rows) - 1, tr = r / hp, hr = h0 + r - tr * hp;
+      const int64_t at = start + tok0 + tr;
+      RowAgain<__nv_bfloat16> z;
+      z.q = a.q + at * a.ld_q + (int64_t)hr * a.dk;
+      z.k = a.k_pages + (int64_t)kvh * PAGE * a.dk;
+      z.v = a.alias ? z.k : a.v_pages + (int64_t)(kvh / a.key_maps) * PAGE * a.dv;
+      z.pages = a.page_table + (int64_t)s * a.table_width;
+      z.k_step = (int64_t)a.n_kv_heads * PAGE * a.dk;
+      z.v_step = a.alias ? z.k_step : (int64_t)(a.n_kv_heads / a.key_maps) * PAGE * a.dv;
+      z.dk = a.dk; z.ld_v = a.alias ? a.dk : a.dv;
+      z.pos = pos0 + tr;
+      z.first = a.window > 0 ? z.pos - a.window + 1 : (a.chunk > 0 ? z.pos - z.pos % a.chunk : 0);
+      z.kept = a.keep_first;
+      z.scale2 = a.scale * LOG2E; z.cap_in = a.cap_in; z.cap_out = a.cap_out; z.capped = a.softcap > 0.f;
+      z.slope = a.slope_span > 0.f ? exp2f(-a.slope_span * (float)(hr + 1) / (float)a.n_heads) * LOG2E : 0.f;
+      z.sink = a.sinks == nullptr ? nullptr : a.sinks + hr;
+      z.gate = a.gate == nullptr ? nullptr : (a.gate_heads ? a.gate + at * a.ld_gate + hr : a.gate + at * a.ld_gate + (int64_t)hr * a.dv);
+      z.gate_step = a.gate_heads ? 0 : 1;
+      const int64_t to = at * a.ld_out + (int64_t)hr * a.dv;
+      const int c1 = min(a.dv, (c0 + CPW) * 64);
+      if (F32OUT) row_again(z, reinterpret_cast<float*>(a.out) + to, c0 * 64, c1);
+      else row_again(z, reinterpret_cast<__nv_bfloat16*>(a.out) + to, c0 * 64, c1);
     }
   }
   tc_fence_before();
@@ -474,6 +505,7 @@ KVAD_EXPORT int kvad_attention_scored_prompt(const void* q, int64_t ld_q, int n_
   KVAD_REQUIRE((int64_t)n_pages * n_kv_heads * PAGE < (1ll << 31), "attention (scored, prompts): %d pages of %d heads are more than a coordinate counts", n_pages, n_kv_heads);
   if (n_seqs == 0 || max_new == 0 || n_rows == 0) return KVAD_OK;
   PromptArgs a;
+  a.q = (const __nv_bfloat16*)q; a.ld_q = ld_q; a.k_pages = (const __nv_bfloat16*)k_pages; a.v_pages = (const __nv_bfloat16*)v_pages;
   a.out = out; a.ld_out = ld_out; a.gate = (const __nv_bfloat16*)gate; a.ld_gate = ld_gate;
   a.gate_heads = gate_heads; a.sinks = sinks; a.seq_starts = seq_starts; a.kv_lens = kv_lens; a.page_table = page_table; a.table_width = table_width;
   a.n_heads = n_heads; a.n_kv_heads = n_kv_heads; a.dk = dk; a.dv = dv; a.alias = alias ? 1 : 0; a.key_maps = key_maps;

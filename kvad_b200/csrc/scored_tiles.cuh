@@ -136,4 +136,91 @@ __device__ __forceinline__ void hide_scores(float (&sc)[64], int hi, int lo, int
   }
 }
 
+// A row worked out once more by a whole warp, key by key, from what it sees alone.  In the products a key that a row does not see has weight 0, and 0 times a
+// value that is not a finite number is none: where such a number is in a tile's pages, rows that do not see it lose the entries it meets.  So every entry that came
+// out as no finite number is worked out here again (a lane a key for the scores, a lane a column for the output), and is one only if the row sees the cause.
+// Nothing of it runs otherwise.  A prompt that is all NaN takes as long as this: see the kernels for figures.
+template <typename T> struct RowAgain {
+  const T* q;                                     // the row's query
+  const T* k; const T* v;                         // the head's keys and values in page 0
+  const int* pages;
+  int64_t k_step, v_step;                         // from page to page
+  int dk, ld_v, pos, first, kept;
+  float scale2, cap_in, cap_out, slope;
+  int capped;
+  const float* sink;                              // or null
+  const T* gate; int gate_step;                   // or null; gate_step 0: one number for all entries
+};
+__device__ __forceinline__ void load8(const float* p, float (&x)[8]) {
+  const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
+  x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w; x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
+}
+__device__ __forceinline__ void load8(const __nv_bfloat16* p, float (&x)[8]) {
+  const uint4 raw = *reinterpret_cast<const uint4*>(p);
+  const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    x[2 * i] = __uint_as_float(w[i] << 16);
+    x[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+  }
+}
+__device__ __forceinline__ bool not_finite(float x) { return (__float_as_uint(x) & 0x7f800000u) == 0x7f800000u; }
+// `out`: the row's entries of this head, of which those from c0 up to c1 (256 at most) that are not finite are written again.
+template <typename T, typename TO>
+__device__ __noinline__ void row_again(const RowAgain<T>& z, TO* out, int c0, int c1) {
+  const int lane = threadIdx.x & 31;
+  float o[8], most = -INFINITY, sum = 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) o[i] = 0.f;
+  for (int j0 = 0; j0 <= z.pos; j0 += 32) {       // (half a page)
+    if (j0 + 32 <= z.first && j0 >= z.kept) continue;
+    const int64_t page = z.pages[j0 / PAGE];
+    const int j = j0 + lane, place = j % PAGE;
+    const bool seen = j <= z.pos && (j >= z.first || j < z.kept);
+    float s = 0.f;
+    if (seen) {
+      const T* k = z.k + page * z.k_step + (int64_t)place * z.dk;
+#pragma unroll 1
+      for (int d = 0; d < z.dk; d += 8) {
+        float a[8], b[8];
+        load8(z.q + d, a);
+        load8(k + d, b);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) s = fmaf(a[e], b[e], s);
+      }
+      s = z.capped ? z.cap_out * tanhf(s * z.cap_in) : s * z.scale2;
+      s -= z.slope * (float)(z.pos - j);
+    }
+    const float top = fmaxf(most, warp_max(seen ? s : -INFINITY)), base = top == -INFINITY ? 0.f : top, keep = most == -INFINITY ? 0.f : exp2f(most - base);
+    const float p = seen ? exp2f(s - base) : 0.f;
+    most = top;
+    sum = fmaf(sum, keep, warp_sum(p));
+#pragma unroll
+    for (int i = 0; i < 8; ++i) o[i] *= keep;
+    uint32_t live = __ballot_sync(0xffffffffu, seen);
+    const T* v = z.v + page * z.v_step + (int64_t)(j0 % PAGE) * z.ld_v + c0 + lane;
+#pragma unroll 1
+    for (; live != 0; live &= live - 1) {
+      const int at = __ffs(live) - 1;
+      const float w = __shfl_sync(0xffffffffu, p, at);
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (c0 + lane + 32 * i < c1) o[i] = fmaf(w, to_f32(v[(int64_t)at * z.ld_v + 32 * i]), o[i]);
+    }
+  }
+  float inv = 1.f / sum;
+  if (z.sink != nullptr) {
+    const float sink = *z.sink * LOG2E, m = fmaxf(most, sink), f = exp2f(most - m);
+    inv = f / fmaf(sum, f, exp2f(sink - m));
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int d = c0 + lane + 32 * i;
+    if (d >= c1 || !not_finite(to_f32(out[d]))) continue;
+    float y = o[i] * inv;
+    if (z.gate != nullptr) y *= 1.f / (1.f + expf(-to_f32(z.gate[(int64_t)d * z.gate_step])));
+    out[d] = from_f32<TO>(y);
+  }
+}
+
 }  // namespace kvad

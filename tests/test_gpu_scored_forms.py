@@ -277,3 +277,60 @@ def test_prompt_tiles(H, G, dk, dv, form):
     for out in [torch.bfloat16] if c.gate is not None else [torch.bfloat16, torch.float32]:
         c.check(c.run(Ops(torch.bfloat16), out), out)
     assert scored_prompt_wait_timeouts() == 0
+
+
+def rows_by_formula(c, s=0):
+    """The rows of sequence `s` in 64 bits, each from the keys and values that it sees and nothing else."""
+    cached, new = c.seqs[s]
+    kw, H, L = c.kw, c.H, cached + new
+    first = int(c.starts[s])
+    take = lambda p, width: p[c.table[s].long()].double().permute(1, 0, 2, 3).reshape(p.shape[1], -1, p.shape[3])[:, :L, :width]
+    k = take(c.kp, c.kp.shape[3])
+    v = (k[:, :, :c.dv] if c.vp is None else take(c.vp, c.dv)).repeat_interleave(kw["key_maps"], 0)
+    k, v = k.repeat_interleave(H // k.shape[0], 0), v.repeat_interleave(H // v.shape[0], 0)
+    q = c.q[first:first + new].double().reshape(new, H, -1)
+    out = torch.empty(new, H, c.dv, dtype=torch.float64, device="cuda")
+    for i in range(new):
+        pos, key = cached + i, torch.arange(cached + i + 1, device="cuda")
+        seen = torch.ones_like(key, dtype=torch.bool)
+        if kw["window"]:
+            seen = (key > pos - kw["window"]) | (key < kw["keep_first"])
+        if kw["chunk"]:
+            seen = key >= pos - pos % kw["chunk"]
+        at = key[seen]
+        x = (k[:, at] * q[i][:, None, :]).sum(2) * c.scale
+        if kw["softcap"]:
+            x = kw["softcap"] * torch.tanh(x / kw["softcap"])
+        if kw["slope_span"]:
+            x = x - (2.0 ** (-kw["slope_span"] * torch.arange(1, H + 1, device="cuda").double() / H))[:, None] * (pos - at)[None]
+        if c.sinks is not None:
+            x = torch.cat([x, c.sinks.double()[:, None]], 1)
+        o = (torch.softmax(x, 1)[:, :len(at), None] * v[:, at]).sum(1)
+        if c.gate is not None:
+            o = o * torch.sigmoid(c.gate[first + i].double().reshape(H, -1))
+        out[i] = o
+    return out.reshape(new, -1)
+
+
+# the number lies at position 104 of the first sequence: in the middle of a tile, and (one head a group) of a page that other tiles' rows end in
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+@pytest.mark.parametrize("where", ["q", "k", "v"])
+@pytest.mark.parametrize("H,G,dk,dv,form", [
+    (4, 4, 64, 64, {}), (16, 1, 64, 64, dict(span=8.0)), (8, 2, 128, 128, dict(window=20, keep=4, gate="entry")), (16, 1, 256, 256, dict(alias=True, gate="head")),
+    (4, 2, 200, 200, dict(sinks=True)), (2, 1, 72, 136, dict(chunk=96, cap=5.0)), (8, 8, 64, 64, dict(key_maps=2, window=40))])
+def test_a_number_that_is_not_finite_stays_with_the_rows_that_see_it(H, G, dk, dv, form, where, bad):
+    c = Case([(70, 150), (3, 40)], H, G, dk, dv, **form)
+    if where == "q":
+        c.q[34, dk + 5] = bad                             # head 1 of position 104
+    else:
+        (c.kp if where == "k" or c.vp is None else c.vp)[c.table[0, 1].long(), 0, 40, 5] = bad
+    want = c.want.clone()
+    want[:150] = rows_by_formula(c)
+    assert want[150:].isfinite().all() and (not want[:150].isfinite().all() or (where != "v" and bad == float("inf")))      # (a score of minus infinity hides a key, a cap makes it finite)
+    for out in [torch.bfloat16] if c.gate is not None else [torch.bfloat16, torch.float32]:
+        got = c.run(Ops(torch.bfloat16), out)
+        assert torch.equal(got.isfinite(), want.isfinite())
+        ok = want.isfinite()
+        # (a row that loses a key's weight keeps its bound's order: twice it is generous)
+        bound = 2 * c.slack + (2.0 ** -8 if out == torch.bfloat16 else 2.0 ** -22) * want.abs() + 1e-30
+        assert float(((got - want).abs() / bound)[ok].max()) <= 1.0
