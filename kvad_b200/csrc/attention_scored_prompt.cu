@@ -51,7 +51,7 @@ struct PromptArgs {
 // NS: groups of four warps that turn scores into weights; CPW: 64-column pieces of the output that a group of four warps keeps.
 template <int NS, int CPW, bool F32OUT>
 __global__ void __launch_bounds__(THREADS, 1)
-scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const PromptArgs a) {
+scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const __grid_constant__ PromptArgs a) {
   // Tensor-memory columns: the places of P V, S of two pages (64 each), the weights' pieces of two pages (32 columns each: two bfloat16 a column).  With values
   // above 128 entries P V takes two places of 128 (products 128 wide leave the issuing warp time for its waits), and the third piece takes its page's S' place.
   constexpr bool S_IS_P = NS == 1;
@@ -77,6 +77,7 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
   uint64_t* t_empty = t_full + 3;                                 // [3] it has been read
   uint64_t* drain = t_empty + 3;                                  // [2] the products that were issued before a wait ran out
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 2);
+  uint32_t* again = tmem_slot + 1;                                // [4] rows with an entry that is not finite, a bit a row
   const int hp = a.hp, tok = ROWS / hp, group = a.n_heads / a.n_kv_heads, chunks = group / hp;
   const int per_seq = a.n_kv_heads * chunks, from_end = blockIdx.x / a.columns, column = blockIdx.x - from_end * a.columns;
   const int s = column / per_seq, part = column - s * per_seq, kvh = part / chunks, h0 = kvh * group + (part - kvh * chunks) * hp;
@@ -92,6 +93,7 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
     for (int i = 0; i < STATS; ++i) mbar_init(&st_full[i], 128);
     for (int i = 0; i < 3; ++i) { mbar_init(&t_full[i], 1); mbar_init(&t_empty[i], 128); }
     for (int i = 0; i < 2; ++i) mbar_init(&drain[i], 1);
+    for (int i = 0; i < 4; ++i) again[i] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     fence_async_shared();
   }
@@ -280,9 +282,9 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
       unpair(add2(sum2[0], sum2[1]), s0, s1);
       stats[(j % STATS) * ROWS + row] = make_float2(most, s0 + s1);
       mbar_arrive_one(&st_full[j % STATS]);
-      // Places past the block's last position may hold anything: no weight is on them, but their values must not be NaN.  (Those past the sequence's end always, so that
-      // no row is worked out twice for what the cache held before; S of the page is done, so shared keys and values can go.)
-      const int valid = last_pos + 1 - key0;
+      // Places past the sequence's end may hold anything: no weight is on them, but their values must not be NaN.  (Hidden places before the end hold numbers in earnest;
+      // where one is not finite, `rows_again` sees to it.  Clearing those too took 2 x 1024 rows of 16 heads of 64 from 23.6 to 24.6 us, a latent of 256 from 40.1 to 42.0.)
+      const int valid = kv_len - key0;
       if (valid < PAGE) {
         const int st = j % stages;
         if (!mbar_wait(&kv_full[st], (j / stages) & 1)) break;
@@ -344,8 +346,9 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         mbar_arrive_one(&t_empty[slot]);
       }
     }
-    float odd = 0.f;                                              // no number as soon as an entry is not finite
+    bool bad = false;                                             // some entry is not finite (0 times it is none)
     if (ok && ti < n_tok) {
+      uint64_t odd = 0ull;
       float inv;
       if (a.sinks == nullptr) {
         inv = 1.0f / run_sum;
@@ -360,12 +363,12 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         if (d >= a.dv) continue;
         float x[8];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) unpair(o[c * 4 + e], x[2 * e], x[2 * e + 1]);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          x[e] *= inv;
-          odd = fmaf(x[e], 0.f, odd);
+        for (int e = 0; e < 4; ++e) {
+          unpair(o[c * 4 + e], x[2 * e], x[2 * e + 1]);
+          odd = fma2(o[c * 4 + e], 0ull, odd);
         }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) x[e] *= inv;
         if (F32OUT) {
           float* dst = reinterpret_cast<float*>(a.out) + grow * a.ld_out + (int64_t)h * a.dv + d;
           if (a.vec) {
@@ -403,32 +406,11 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
           }
         }
       }
+      float odd0, odd1;
+      unpair(odd, odd0, odd1);
+      bad = !(odd0 + odd1 == 0.f) || not_finite(inv);
     }
-    __syncwarp();                                                 // (a lane's entries are read by the others)
-    for (uint32_t rows = __ballot_sync(0xffffffffu, ok && ti < n_tok && !(odd == 0.f)); rows != 0; rows &= rows - 1) {
-      const int r = quarter * 32 + __ffs(rows) - 1, tr = r / hp, hr = h0 + r - tr * hp;
-      const int64_t at = start + tok0 + tr;
-      RowAgain<__nv_bfloat16> z;
-      z.q = a.q + at * a.ld_q + (int64_t)hr * a.dk;
-      z.k = a.k_pages + (int64_t)kvh * PAGE * a.dk;
-      z.v = a.alias ? z.k : a.v_pages + (int64_t)(kvh / a.key_maps) * PAGE * a.dv;
-      z.pages = a.page_table + (int64_t)s * a.table_width;
-      z.k_step = (int64_t)a.n_kv_heads * PAGE * a.dk;
-      z.v_step = a.alias ? z.k_step : (int64_t)(a.n_kv_heads / a.key_maps) * PAGE * a.dv;
-      z.dk = a.dk; z.ld_v = a.alias ? a.dk : a.dv;
-      z.pos = pos0 + tr;
-      z.first = a.window > 0 ? z.pos - a.window + 1 : (a.chunk > 0 ? z.pos - z.pos % a.chunk : 0);
-      z.kept = a.keep_first;
-      z.scale2 = a.scale * LOG2E; z.cap_in = a.cap_in; z.cap_out = a.cap_out; z.capped = a.softcap > 0.f;
-      z.slope = a.slope_span > 0.f ? exp2f(-a.slope_span * (float)(hr + 1) / (float)a.n_heads) * LOG2E : 0.f;
-      z.sink = a.sinks == nullptr ? nullptr : a.sinks + hr;
-      z.gate = a.gate == nullptr ? nullptr : (a.gate_heads ? a.gate + at * a.ld_gate + hr : a.gate + at * a.ld_gate + (int64_t)hr * a.dv);
-      z.gate_step = a.gate_heads ? 0 : 1;
-      const int64_t to = at * a.ld_out + (int64_t)hr * a.dv;
-      const int c1 = min(a.dv, (c0 + CPW) * 64);
-      if (F32OUT) row_again(z, reinterpret_cast<float*>(a.out) + to, c0 * 64, c1);
-      else row_again(z, reinterpret_cast<__nv_bfloat16*>(a.out) + to, c0 * 64, c1);
-    }
+    note_again(again, quarter, bad);
   }
   tc_fence_before();
   __syncthreads();
@@ -436,6 +418,11 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
   if (warp == 1) {
     __syncwarp();
     tmem_dealloc(tmem_base, TM_COLS);
+  }
+  constexpr int NI = NS == 1 ? 8 : 2 * CPW, AGAIN = CPW == 1 ? 4 * NS : THREADS / 32 - 4;      // (of values of up to 64 entries the output's warps have given registers away)
+  if (warp >= 4 && warp < 4 + AGAIN && (again[0] | again[1] | again[2] | again[3]) != 0) {
+    if (F32OUT) rows_again<NI, __nv_bfloat16, float>(a, again, 4, AGAIN);
+    else rows_again<NI, __nv_bfloat16, __nv_bfloat16>(a, again, 4, AGAIN);
   }
 }
 

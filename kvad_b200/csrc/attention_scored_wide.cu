@@ -12,7 +12,7 @@
 // two new rows of four sequences behind 300 positions: 17.7 against 56; one prompt of 17: 9.8 against 16.6; 12 heads of 64, prompts of 64 .. 540: 33 against 108
 // (the tiled kernel of `attention_simt.cu`).  (With one group of warps cutting a batch ahead by way of registers: 90 where it is 54.)
 //
-// A block that meets a number that is not finite (it has no pieces) works its rows out again by fmaf, key by key.  Every wait is bounded.
+// A number that is not finite has no pieces: rows whose outputs it reaches are worked out again by fmaf (`row_again`).  Every wait is bounded.
 #include <algorithm>
 
 #include "scored_tiles.cuh"
@@ -41,8 +41,8 @@ struct WideArgs {
   int window, keep_first, chunk;
 };
 
-// Eight neighbours into three pieces of 16 bytes, `step` bytes apart; whether one is not finite (its last piece then is no number).
-__device__ __forceinline__ bool put8(uint8_t* dst, uint32_t step, const float4& a, const float4& b) {
+// Eight neighbours into three pieces of 16 bytes, `step` bytes apart.  (Of a number that is not finite the last pieces are no number.)
+__device__ __forceinline__ void put8(uint8_t* dst, uint32_t step, const float4& a, const float4& b) {
   float x[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
   for (int piece = 0; piece < 2; ++piece) {
@@ -55,48 +55,11 @@ __device__ __forceinline__ bool put8(uint8_t* dst, uint32_t step, const float4& 
 #pragma unroll
   for (int i = 0; i < 4; ++i) w[i] = __byte_perm(__float_as_uint(x[2 * i]), __float_as_uint(x[2 * i + 1]), 0x7632);
   *reinterpret_cast<uint4*>(dst + 2 * step) = make_uint4(w[0], w[1], w[2], w[3]);
-  const float all = ((x[0] + x[1]) + (x[2] + x[3])) + ((x[4] + x[5]) + (x[6] + x[7]));
-  return all != all;
-}
-
-// A row by fmaf, key by key, 16 columns of the output at a time.
-__device__ __noinline__ void plain_row(const WideArgs& a, const int* pages, const float* q, int kvh, int h, int pos, int first, float slope, int64_t grow) {
-  const int64_t k_step = (int64_t)a.n_kv_heads * PAGE * a.dk, v_step = (int64_t)(a.n_kv_heads / a.key_maps) * PAGE * a.dv;
-  auto key_at = [&](int j) { return a.k_pages + (int64_t)pages[j / PAGE] * k_step + ((int64_t)kvh * PAGE + j % PAGE) * a.dk; };
-  auto seen = [&](int j) { return j >= first || j < a.keep_first; };
-  auto score = [&](int j) {
-    const float* k = key_at(j);
-    float s = 0.f;
-    for (int d = 0; d < a.dk; ++d) s = fmaf(q[d], k[d], s);
-    s = a.softcap > 0.f ? a.cap_out * tanhf(s * a.cap_in) : s * (a.scale * LOG2E);
-    return s - slope * (float)(pos - j);
-  };
-  float most = -INFINITY;
-  for (int j = 0; j <= pos; ++j)
-    if (seen(j)) most = fmaxf(most, score(j));
-  const float base = most == -INFINITY ? 0.f : most;
-  for (int d0 = 0; d0 < a.dv; d0 += 16) {
-    float o[16], sum = 0.f;
-    for (int e = 0; e < 16; ++e) o[e] = 0.f;
-    for (int j = 0; j <= pos; ++j) {
-      if (!seen(j)) continue;
-      const float p = exp2f(score(j) - base);
-      const float* v = a.alias ? key_at(j) : a.v_pages + (int64_t)pages[j / PAGE] * v_step + ((int64_t)(kvh / a.key_maps) * PAGE + j % PAGE) * a.dv;
-      sum += p;
-      for (int e = 0; e < 16 && d0 + e < a.dv; ++e) o[e] = fmaf(p, v[d0 + e], o[e]);
-    }
-    if (a.sinks != nullptr) sum += exp2f(a.sinks[h] * LOG2E - base);
-    for (int e = 0; e < 16 && d0 + e < a.dv; ++e) {
-      float y = o[e] / sum;
-      if (a.gate != nullptr) y *= 1.0f / (1.0f + expf(-(a.gate_heads ? a.gate[grow * a.ld_gate + h] : a.gate[grow * a.ld_gate + (int64_t)h * a.dv + d0 + e])));
-      a.out[grow * a.ld_out + (int64_t)h * a.dv + d0 + e] = y;
-    }
-  }
 }
 
 // CPW: 64-column pieces of the output.
 template <int CPW>
-__global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const WideArgs a) {
+__global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const __grid_constant__ WideArgs a) {
   constexpr int PA[6] = {2, 0, 1, 1, 0, 0}, PB[6] = {0, 2, 1, 0, 1, 0};      // which pieces meet, the smallest products first
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -117,7 +80,7 @@ __global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const WideArgs 
   uint64_t* t_empty = t_full + 3;                                 // [3] it has been read
   uint64_t* drain = t_empty + 3;                                  // [2] the products that were issued before a wait ran out
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 2);
-  volatile int* strange = reinterpret_cast<volatile int*>(tmem_slot + 1);      // some operand is not finite
+  uint32_t* again = tmem_slot + 1;                                // [4] rows with an entry that is not finite, a bit a row
   const int hp = a.hp, tok = ROWS / hp, group = a.n_heads / a.n_kv_heads, chunks = group / hp;
   const int per_seq = a.n_kv_heads * chunks, from_end = blockIdx.x / a.columns, column = blockIdx.x - from_end * a.columns;
   const int s = column / per_seq, part = column - s * per_seq, kvh = part / chunks, h0 = kvh * group + (part - kvh * chunks) * hp;
@@ -129,7 +92,7 @@ __global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const WideArgs 
     for (int i = 0; i < STATS; ++i) mbar_init(&st_full[i], 128);
     for (int i = 0; i < 3; ++i) { mbar_init(&t_full[i], 1); mbar_init(&t_empty[i], 128); }
     for (int i = 0; i < 2; ++i) mbar_init(&drain[i], 1);
-    *strange = 0;
+    for (int i = 0; i < 4; ++i) again[i] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     fence_async_shared();
   }
@@ -146,9 +109,7 @@ __global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const WideArgs 
   };
   const int* pages = a.page_table + (int64_t)s * a.table_width;
   const int k_eights = (a.dk + 15) / 16 * 2, v_eights = a.alias ? 0 : (a.dv + 15) / 16 * 2;      // pieces of eight entries of a row, up to whole sixteens (zeros)
-  __syncthreads();                                                // (`strange` is zero)
   {                                                               // the queries, by all
-    bool bad = false;
 #pragma unroll 2
     for (int i = threadIdx.x; i < ROWS * k_eights; i += THREADS) {
       const int r = i / k_eights, c = i - r * k_eights, ti = r / hp;
@@ -158,9 +119,8 @@ __global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const WideArgs 
         x = src[0];
         y = src[1];
       }
-      bad |= put8(q_tile + (c >> 3) * Q_BLOCK + r * 128 + (((c & 7) ^ (r & 7)) << 4), q_piece, x, y);
+      put8(q_tile + (c >> 3) * Q_BLOCK + r * 128 + (((c & 7) ^ (r & 7)) << 4), q_piece, x, y);
     }
-    if (bad) *strange = 1;
     fence_async_shared();
   }
   tc_fence_before();
@@ -252,7 +212,6 @@ __global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const WideArgs 
     auto bring = [&](uint8_t* dst, uint32_t step, const float* src, int width, int eights, int n_live) {
       const int rows = 128 / eights, rest = 128 - rows * eights;  // (from one of a thread's places to the next)
       int r = tid / eights, c = tid - r * eights;
-      bool bad = false;
       for (int i = tid; i < PAGE * eights; i += 512) {
         float4 x[4], y[4];
         int at[4];
@@ -260,7 +219,7 @@ __global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const WideArgs 
         for (int f = 0; f < 4; ++f) {
           x[f] = y[f] = make_float4(0.f, 0.f, 0.f, 0.f);
           at[f] = r < PAGE ? (c >> 3) * (int)PAGE_BLOCK + r * 128 + (((c & 7) ^ (r & 7)) << 4) : -1;
-          if (r < n_live && c * 8 < width) {                      // (places past the sequence's end may hold anything)
+          if (r < n_live && c * 8 < width) {                      // (places past the block's last position may hold anything)
             const float4* from = reinterpret_cast<const float4*>(src + r * width + c * 8);
             x[f] = from[0];
             y[f] = from[1];
@@ -271,16 +230,15 @@ __global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const WideArgs 
         }
 #pragma unroll
         for (int f = 0; f < 4; ++f)
-          if (at[f] >= 0) bad |= put8(dst + at[f], step, x[f], y[f]);
+          if (at[f] >= 0) put8(dst + at[f], step, x[f], y[f]);
       }
-      if (bad) *strange = 1;
     };
     // (with room for one page only the first group works: a group that waits for a place to be given back must not be two givings behind)
     const int takers = stages > 1 ? 2 : 1;
     int j = mine, t = next_page(0);
     if (mine == 1) t = next_page(t + 1);
     for (; mine < takers && t * PAGE <= last_pos && ok; j += takers) {
-      const int page = pages[t], st = j % stages, n_live = min(PAGE, kv_len - t * PAGE);
+      const int page = pages[t], st = j % stages, n_live = min(PAGE, last_pos + 1 - t * PAGE);
       if (j >= stages && !mbar_wait(&kv_empty[st], ((j / stages) & 1) ^ 1)) { ok = false; break; }
       uint8_t* at = ring + st * stage_bytes;
       bring(at, k_piece, a.k_pages + (int64_t)page * k_step + (int64_t)kvh * PAGE * a.dk, a.dk, k_eights, n_live);
@@ -407,11 +365,9 @@ __global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const WideArgs 
         mbar_arrive_one(&t_empty[slot]);
       }
     }
-    if (ok && ti < n_tok && *strange != 0) {
-      const float slope = a.slope_span > 0.f ? exp2f(-a.slope_span * (float)(h + 1) / (float)a.n_heads) * LOG2E : 0.f;
-      const int pos = pos0 + ti, first = a.window > 0 ? pos - a.window + 1 : (a.chunk > 0 ? pos - pos % a.chunk : 0);
-      plain_row(a, pages, a.q + grow * a.ld_q + (int64_t)h * a.dk, kvh, h, pos, first, slope, grow);
-    } else if (ok && ti < n_tok) {
+    bool bad = false;                                             // some entry is not finite (0 times it is none)
+    if (ok && ti < n_tok) {
+      uint64_t odd = 0ull;
       float inv;
       if (a.sinks == nullptr) {
         inv = 1.0f / run_sum;
@@ -427,6 +383,7 @@ __global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const WideArgs 
         float x[4];
         unpair(o[d / 2], x[0], x[1]);
         unpair(o[d / 2 + 1], x[2], x[3]);
+        odd = fma2(o[d / 2 + 1], 0ull, fma2(o[d / 2], 0ull, odd));
 #pragma unroll
         for (int e = 0; e < 4; ++e) x[e] *= inv;
         if (gate != nullptr && !a.gate_heads) {
@@ -435,7 +392,11 @@ __global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const WideArgs 
         }
         *reinterpret_cast<float4*>(dst + d) = make_float4(x[0], x[1], x[2], x[3]);
       }
+      float odd0, odd1;
+      unpair(odd, odd0, odd1);
+      bad = !(odd0 + odd1 == 0.f) || not_finite(inv);
     }
+    note_again(again, quarter, bad);
   }
   tc_fence_before();
   __syncthreads();
@@ -444,6 +405,7 @@ __global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const WideArgs 
     __syncwarp();
     tmem_dealloc(tmem_base, TM_COLS);
   }
+  if (warp >= 12 && (again[0] | again[1] | again[2] | again[3]) != 0) rows_again<2 * CPW, float, float>(a, again, 12, THREADS / 32 - 12);
 }
 
 struct Layout { int stages; size_t smem; };

@@ -139,13 +139,14 @@ __device__ __forceinline__ void hide_scores(float (&sc)[64], int hi, int lo, int
 // A row worked out once more by a whole warp, key by key, from what it sees alone.  In the products a key that a row does not see has weight 0, and 0 times a
 // value that is not a finite number is none: where such a number is in a tile's pages, rows that do not see it lose the entries it meets.  So every entry that came
 // out as no finite number is worked out here again (a lane a key for the scores, a lane a column for the output), and is one only if the row sees the cause.
-// Nothing of it runs otherwise.  A prompt that is all NaN takes as long as this: see the kernels for figures.
+// A block's rows are noted (`note_again`) and shared out over its warps at its end.  Nothing of it runs otherwise.  (2 x 1024 rows of 16 heads of 64 on 4 key heads, ms:
+// all keys NaN, 0.25 where finite ones take 0.024 in bfloat16, 0.60 for 0.048 in 32 bits; one NaN value 0.12 and 3.2; a thread a row, all rows of a tile: 24 in 32 bits.)
 template <typename T> struct RowAgain {
   const T* q;                                     // the row's query
   const T* k; const T* v;                         // the head's keys and values in page 0
   const int* pages;
   int64_t k_step, v_step;                         // from page to page
-  int dk, ld_v, pos, first, kept;
+  int dk, dv, ld_v, pos, first, kept;
   float scale2, cap_in, cap_out, slope;
   int capped;
   const float* sink;                              // or null
@@ -165,13 +166,18 @@ __device__ __forceinline__ void load8(const __nv_bfloat16* p, float (&x)[8]) {
   }
 }
 __device__ __forceinline__ bool not_finite(float x) { return (__float_as_uint(x) & 0x7f800000u) == 0x7f800000u; }
-// `out`: the row's entries of this head, of which those from c0 up to c1 (256 at most) that are not finite are written again.
-template <typename T, typename TO>
-__device__ __noinline__ void row_again(const RowAgain<T>& z, TO* out, int c0, int c1) {
+// `out`: the row's entries of this head, of which those that are not finite are written again.
+// NI: 32s of entries.  An entry that has become NaN stays so: the row is left as it is as soon as all that are worked out again have.
+template <int NI, typename T, typename TO>
+__device__ __forceinline__ void row_again(const RowAgain<T>& z, TO* out) {
   const int lane = threadIdx.x & 31;
-  float o[8], most = -INFINITY, sum = 0.f;
+  float o[NI], most = -INFINITY, sum = 0.f;
+  uint32_t need = 0;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) o[i] = 0.f;
+  for (int i = 0; i < NI; ++i) {
+    o[i] = 0.f;
+    if (lane + 32 * i < z.dv && not_finite(to_f32(out[lane + 32 * i]))) need |= 1u << i;
+  }
   for (int j0 = 0; j0 <= z.pos; j0 += 32) {       // (half a page)
     if (j0 + 32 <= z.first && j0 >= z.kept) continue;
     const int64_t page = z.pages[j0 / PAGE];
@@ -180,7 +186,7 @@ __device__ __noinline__ void row_again(const RowAgain<T>& z, TO* out, int c0, in
     float s = 0.f;
     if (seen) {
       const T* k = z.k + page * z.k_step + (int64_t)place * z.dk;
-#pragma unroll 1
+#pragma unroll 2
       for (int d = 0; d < z.dk; d += 8) {
         float a[8], b[8];
         load8(z.q + d, a);
@@ -196,17 +202,21 @@ __device__ __noinline__ void row_again(const RowAgain<T>& z, TO* out, int c0, in
     most = top;
     sum = fmaf(sum, keep, warp_sum(p));
 #pragma unroll
-    for (int i = 0; i < 8; ++i) o[i] *= keep;
-    uint32_t live = __ballot_sync(0xffffffffu, seen);
-    const T* v = z.v + page * z.v_step + (int64_t)(j0 % PAGE) * z.ld_v + c0 + lane;
-#pragma unroll 1
-    for (; live != 0; live &= live - 1) {
-      const int at = __ffs(live) - 1;
+    for (int i = 0; i < NI; ++i) o[i] *= keep;
+    const uint32_t live = __ballot_sync(0xffffffffu, seen);
+    const T* v = z.v + page * z.v_step + (int64_t)(j0 % PAGE) * z.ld_v + lane;
+#pragma unroll 4
+    for (int at = 0; at < 32; ++at, v += z.ld_v) {
       const float w = __shfl_sync(0xffffffffu, p, at);
+      if (!(live >> at & 1)) continue;
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
-        if (c0 + lane + 32 * i < c1) o[i] = fmaf(w, to_f32(v[(int64_t)at * z.ld_v + 32 * i]), o[i]);
+      for (int i = 0; i < NI; ++i)
+        if (need >> i & 1) o[i] = fmaf(w, to_f32(v[32 * i]), o[i]);
     }
+    bool settled = true;
+#pragma unroll
+    for (int i = 0; i < NI; ++i) settled = settled && (!(need >> i & 1) || o[i] != o[i]);
+    if (__all_sync(0xffffffffu, settled)) return;
   }
   float inv = 1.f / sum;
   if (z.sink != nullptr) {
@@ -214,12 +224,49 @@ __device__ __noinline__ void row_again(const RowAgain<T>& z, TO* out, int c0, in
     inv = f / fmaf(sum, f, exp2f(sink - m));
   }
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int d = c0 + lane + 32 * i;
-    if (d >= c1 || !not_finite(to_f32(out[d]))) continue;
+  for (int i = 0; i < NI; ++i) {
+    const int d = lane + 32 * i;
+    if (!(need >> i & 1)) continue;
     float y = o[i] * inv;
     if (z.gate != nullptr) y *= 1.f / (1.f + expf(-to_f32(z.gate[(int64_t)d * z.gate_step])));
     out[d] = from_f32<TO>(y);
+  }
+}
+
+// The 32 rows of a warp: which have an entry that is not finite.  `again`: a bit a row.
+__device__ __forceinline__ void note_again(uint32_t* again, int quarter, bool bad) {
+  const uint32_t rows = __ballot_sync(0xffffffffu, bad);
+  if (rows != 0 && (threadIdx.x & 31) == 0) atomicOr(again + quarter, rows);
+}
+// The noted rows of a block, by `warps` of its warps from `first` on (those that have given no registers away: a function may take as many as the kernel was launched
+// with); after a barrier of the whole block.  Args: the kernels' arguments (in constant memory).  It finds the block's place again: nothing of it is kept in the kernels' registers.
+template <int NI, typename T, typename TO, typename Args>
+__device__ __noinline__ void rows_again(const Args& a, const uint32_t* again, int first, int warps) {
+  const int hp = a.hp, tok = ROWS / hp, group = a.n_heads / a.n_kv_heads, chunks = group / hp, per_seq = a.n_kv_heads * chunks;
+  const int from_end = blockIdx.x / a.columns, column = blockIdx.x - from_end * a.columns, s = column / per_seq, part = column - s * per_seq, kvh = part / chunks;
+  const int h0 = kvh * group + (part - kvh * chunks) * hp, start = a.seq_starts[s], n_new = a.seq_starts[s + 1] - start;
+  const int tok0 = ((int)gridDim.x / a.columns - 1 - from_end) * tok, pos0 = a.kv_lens[s] - n_new + tok0, n_tok = min(tok, n_new - tok0);
+  for (int r = (threadIdx.x >> 5) - first; r < ROWS; r += warps) {
+    const int ti = r / hp, h = h0 + r - ti * hp;
+    if (!(again[r >> 5] >> (r & 31) & 1) || ti >= n_tok) continue;
+    const int64_t at = start + tok0 + ti;
+    RowAgain<T> z;
+    z.q = a.q + at * a.ld_q + (int64_t)h * a.dk;
+    z.k = a.k_pages + (int64_t)kvh * PAGE * a.dk;
+    z.v = a.alias ? z.k : a.v_pages + (int64_t)(kvh / a.key_maps) * PAGE * a.dv;
+    z.pages = a.page_table + (int64_t)s * a.table_width;
+    z.k_step = (int64_t)a.n_kv_heads * PAGE * a.dk;
+    z.v_step = a.alias ? z.k_step : (int64_t)(a.n_kv_heads / a.key_maps) * PAGE * a.dv;
+    z.dk = a.dk; z.dv = a.dv; z.ld_v = a.alias ? a.dk : a.dv;
+    z.pos = pos0 + ti;
+    z.first = a.window > 0 ? z.pos - a.window + 1 : (a.chunk > 0 ? z.pos - z.pos % a.chunk : 0);
+    z.kept = a.keep_first;
+    z.scale2 = a.scale * LOG2E; z.cap_in = a.cap_in; z.cap_out = a.cap_out; z.capped = a.softcap > 0.f;
+    z.slope = a.slope_span > 0.f ? exp2f(-a.slope_span * (float)(h + 1) / (float)a.n_heads) * LOG2E : 0.f;
+    z.sink = a.sinks == nullptr ? nullptr : a.sinks + h;
+    z.gate = a.gate == nullptr ? nullptr : (a.gate_heads ? a.gate + at * a.ld_gate + h : a.gate + at * a.ld_gate + (int64_t)h * a.dv);
+    z.gate_step = a.gate_heads ? 0 : 1;
+    row_again<NI>(z, reinterpret_cast<TO*>(a.out) + at * a.ld_out + (int64_t)h * a.dv);
   }
 }
 

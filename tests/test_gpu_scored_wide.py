@@ -4,6 +4,7 @@ import pytest
 import torch
 
 from kvad_b200.ops import Ops, lib, scored_wide_wait_timeouts
+from tests.test_gpu_scored_forms import rows_by_formula
 
 pytestmark = pytest.mark.gpu
 PAGE = 64
@@ -20,6 +21,7 @@ class Case:
         rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
         self.seqs, self.H, self.scale, self.key_maps = seqs, H, 1.5 / dk ** 0.5, key_maps
         self.cap, self.span, self.window, self.keep, self.chunk = cap, span, window, keep, chunk
+        self.kw = dict(softcap=cap, slope_span=span, window=window, keep_first=keep, chunk=chunk, key_maps=key_maps)
         width = -(-max(c + n for c, n in seqs) // PAGE)
         order = torch.randperm(width * len(seqs) + 2, generator=torch.Generator().manual_seed(3))
         self.table = order[:width * len(seqs)].reshape(len(seqs), width).to(torch.int32).cuda().contiguous()
@@ -120,3 +122,24 @@ def test_numbers_that_are_not_finite(where, bad):
     assert got[others].isfinite().all() and (got.isfinite() | ~want.isfinite()).all()
     ok = want.isfinite()
     assert float((got[ok] - want[ok]).abs().max()) < 2e-6
+
+
+# position 104 of the first sequence: in the middle of a tile, and (one head a group) of a page that other tiles' rows end in
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+@pytest.mark.parametrize("where", ["q", "k", "v"])
+@pytest.mark.parametrize("H,G,dk,dv,form", [(4, 4, 64, 64, {}), (16, 1, 96, 64, dict(alias=True, sinks=True)), (8, 2, 128, 128, dict(window=20, keep=4, gate="entry")),
+                                            (6, 2, 72, 40, dict(cap=3.0)), (8, 8, 64, 64, dict(key_maps=2, chunk=40, gate="head"))])
+def test_a_number_that_is_not_finite_stays_with_the_rows_that_see_it(H, G, dk, dv, form, where, bad):
+    c = Case([(70, 150), (3, 40)], H, G, dk, dv, **form)
+    clean = c.want()
+    if where == "q":
+        c.q[34, dk + 5] = bad                             # head 1 of position 104
+    else:
+        (c.kp if where == "k" or c.vp is None else c.vp)[c.table[0, 1].long(), 0, 40, 5] = bad
+    want = torch.cat([rows_by_formula(c), clean[150:]])
+    assert want[150:].isfinite().all() and (not want[:150].isfinite().all() or (where != "v" and bad == float("inf")))      # (a score of minus infinity hides a key, a cap makes it finite)
+    got = c.run(Ops(torch.float32))
+    assert torch.equal(got.isfinite(), want.isfinite())
+    ok = want.isfinite()
+    assert float((got - want)[ok].abs().max()) < 1e-5      # (scores of up to 2^4 with errors of 2^-21: a weight's of 2^-17)
+    assert scored_wide_wait_timeouts() == 0
