@@ -23,6 +23,7 @@
 // 38.4, 14.7; 12.3, 9.5.  The mma.sync kernel was ahead nowhere and is gone.  (On the way: products issued by a branch of one lane 64, by the
 // whole warp 50, S and P V by warps of their own with wide P V 40.)
 #include <algorithm>
+#include <type_traits>
 
 #include "scored_tiles.cuh"
 
@@ -55,6 +56,7 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
   // Tensor-memory columns: the places of P V, S of two pages (64 each), the weights' pieces of two pages (32 columns each: two bfloat16 a column).  With values
   // above 128 entries P V takes two places of 128 (products 128 wide leave the issuing warp time for its waits), and the third piece takes its page's S' place.
   constexpr bool S_IS_P = NS == 1;
+  constexpr int NI = NS == 1 ? 8 : 2 * CPW, FINISHERS = THREADS / 32 - 4;      // 32s of a value's entries; warps that finish a block together
   constexpr int CW = NS == 1 ? 128 : 64, SLOTS = NS == 1 ? 2 : 3;
   constexpr uint32_t TM_T = 0, TM_S = SLOTS * CW, TM_P = TM_S + 128, P_STEP = S_IS_P ? 64 : 96;
   static_assert(TM_P + 2 * P_STEP <= TM_COLS, "tensor memory");
@@ -108,15 +110,23 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
   const uint32_t tmem_base = *tmem_slot;
   const int n_tok = min(tok, n_new - tok0), pos0 = kv_len - n_new + tok0, last_pos = pos0 + n_tok - 1;
   const int first_key = a.chunk > 0 ? pos0 - pos0 % a.chunk : ((a.window > 0 && pos0 - a.window + 1 > 0) ? pos0 - a.window + 1 : 0);   // of the block's first token
+  const int keep_first = a.keep_first;                            // (arguments that a loop over pages wants are read before it: every wait in it would have them read again)
   auto next_page = [&](int t) {                                   // the next page that a pair of the block sees (the same for every thread)
-    while (t * PAGE <= last_pos && t * PAGE + PAGE <= first_key && t * PAGE >= a.keep_first) ++t;
+    while (t * PAGE <= last_pos && t * PAGE + PAGE <= first_key && t * PAGE >= keep_first) ++t;
     return t;
+  };
+  // after a role's last page: the rows that have to be worked out again, by all warps that have the registers
+  auto finish = [&]() {
+    asm volatile("bar.sync 1, %0;" ::"n"(FINISHERS * 32) : "memory");
+    if ((again[0] | again[1] | again[2] | again[3]) != 0) rows_again<NI, __nv_bfloat16, typename std::conditional<F32OUT, float, __nv_bfloat16>::type>(a, again, 4, FINISHERS);
   };
 
   if (warp < 4) {
     regs_fewer<40>();
     if (warp == 0 && lane == 0) {
       const int* pages = a.page_table + (int64_t)s * a.table_width;
+      const int n_kv = a.n_kv_heads, n_v = n_kv / a.key_maps, v_head = kvh / a.key_maps;
+      const bool alias = a.alias;
       int t = next_page(0), page_next = pages[t];
       mbar_expect_tx(q_full, k_blocks * Q_BLOCK);
       for (int b = 0; b < k_blocks; ++b) tma_load_3d(q_tile + b * Q_BLOCK, &map_q, q_full, b * 64, h0, start + tok0);
@@ -130,10 +140,10 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         if (j >= stages && !mbar_wait(&kv_empty[st], turn ^ 1)) { ok = false; break; }
         uint8_t* at = ring + st * stage_bytes;
         mbar_expect_tx(&kv_full[st], stage_bytes);
-        const int y = (page * a.n_kv_heads + kvh) * PAGE;
+        const int y = (page * n_kv + kvh) * PAGE;
         for (int b = 0; b < k_blocks; ++b) tma_load_2d(at + b * PAGE_BLOCK, &map_k, &kv_full[st], b * 64, y);
-        if (!a.alias) {
-          const int yv = (page * (a.n_kv_heads / a.key_maps) + kvh / a.key_maps) * PAGE;
+        if (!alias) {
+          const int yv = (page * n_v + v_head) * PAGE;
           for (int b = 0; b < v_blocks; ++b) tma_load_2d(at + k_bytes + b * PAGE_BLOCK, &map_v, &kv_full[st], b * 64, yv);
         }
         if (++st == stages) { st = 0; turn ^= 1; }
@@ -180,6 +190,7 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
       const uint64_t v_desc = sw128_mn_desc(smem_u32(ring) + (a.alias ? 0u : k_bytes));
       const uint32_t stage_step = stage_bytes >> 4;
       const bool one = elect_one();
+      const int dv = a.dv;
       bool ok = true;
       int i = 0, st = 0, slot = 0, g = 0;
       uint32_t slot_turn = 0;
@@ -191,7 +202,7 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         for (int c = 0; c < n_chunks; ++c, ++g) {
           if (g >= SLOTS && !mbar_wait(&t_empty[slot], slot_turn ^ 1)) { ok = false; break; }
           tc_fence_after();
-          const uint32_t idesc = umma_instr_desc(ROWS, min(CW, (a.dv - c * CW + 15) & ~15), false, true), d = tmem_base + TM_T + slot * CW;
+          const uint32_t idesc = umma_instr_desc(ROWS, min(CW, (dv - c * CW + 15) & ~15), false, true), d = tmem_base + TM_T + slot * CW;
           const uint64_t vd = v_at + c * (CW / 64) * (PAGE_BLOCK >> 4);
           if (one) {
 #pragma unroll
@@ -228,7 +239,8 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
     const int clear_to = pos0 + quarter * 32 / hp, far = pos0 + min((quarter * 32 + 31) / hp, n_tok - 1);
     const int clear_from = a.window > 0 ? far - a.window + 1 : (a.chunk > 0 ? far - far % a.chunk : 0);
     const float scale2 = a.scale * LOG2E;
-    const bool plain = !(a.softcap > 0.f) && !(a.slope_span > 0.f) && a.scale > 0.f;
+    const bool capped = a.softcap > 0.f, sloped = a.slope_span > 0.f, plain = !capped && !sloped && a.scale > 0.f;
+    const float cap_in = a.cap_in, cap_out = a.cap_out;
     const float unit = plain ? scale2 : 1.f;
     const uint64_t unit2 = pair(unit, unit);
     int t = next_page(0), j = mine;
@@ -248,9 +260,9 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
       tc_fence_before();
       if (!S_IS_P) mbar_arrive_one(&s_empty[b]);
       // Scores in units of log2, or, where nothing but a positive factor is on them, as they are with the factor `unit` still owed.
-      if (!plain) shape_scores(sc, a.softcap > 0.f, a.cap_in, a.cap_out, scale2, a.slope_span > 0.f, slope, pos - key0);
-      if (!(key0 + PAGE - 1 <= clear_to && (key0 >= clear_from || key0 + PAGE <= a.keep_first)))      // some pair does not see all of the page
-        hide_scores(sc, pos - key0, first - key0, a.keep_first - key0);
+      if (!plain) shape_scores(sc, capped, cap_in, cap_out, scale2, sloped, slope, pos - key0);
+      if (!(key0 + PAGE - 1 <= clear_to && (key0 >= clear_from || key0 + PAGE <= keep_first)))      // some pair does not see all of the page
+        hide_scores(sc, pos - key0, first - key0, keep_first - key0);
       float top[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
       for (int c = 0; c < 64; ++c) top[c & 3] = fmaxf(top[c & 3], sc[c]);
@@ -299,6 +311,7 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
       t = next_page(t + 1);
       if (NS == 2) t = next_page(t + 1);
     }
+    finish();
   } else {
     // ---- the running output: a thread a row and CPW x 64 of its columns
     if (CPW == 1) regs_fewer<104>(); else regs_more<168>();
@@ -411,6 +424,7 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
       bad = !(odd0 + odd1 == 0.f) || not_finite(inv);
     }
     note_again(again, quarter, bad);
+    finish();
   }
   tc_fence_before();
   __syncthreads();
@@ -418,11 +432,6 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
   if (warp == 1) {
     __syncwarp();
     tmem_dealloc(tmem_base, TM_COLS);
-  }
-  constexpr int NI = NS == 1 ? 8 : 2 * CPW, AGAIN = CPW == 1 ? 4 * NS : THREADS / 32 - 4;      // (of values of up to 64 entries the output's warps have given registers away)
-  if (warp >= 4 && warp < 4 + AGAIN && (again[0] | again[1] | again[2] | again[3]) != 0) {
-    if (F32OUT) rows_again<NI, __nv_bfloat16, float>(a, again, 4, AGAIN);
-    else rows_again<NI, __nv_bfloat16, __nv_bfloat16>(a, again, 4, AGAIN);
   }
 }
 

@@ -103,8 +103,9 @@ __global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const __grid_co
   if (warp == 1) tmem_alloc(tmem_slot, TM_COLS);
   const int n_tok = min(tok, n_new - tok0), pos0 = kv_len - n_new + tok0, last_pos = pos0 + n_tok - 1;
   const int first_key = a.chunk > 0 ? pos0 - pos0 % a.chunk : ((a.window > 0 && pos0 - a.window + 1 > 0) ? pos0 - a.window + 1 : 0);   // of the block's first token
+  const int keep_first = a.keep_first;                            // (arguments that a loop over pages wants are read before it: every wait in it would have them read again)
   auto next_page = [&](int t) {                                   // the next page that a pair of the block sees (the same for every thread)
-    while (t * PAGE <= last_pos && t * PAGE + PAGE <= first_key && t * PAGE >= a.keep_first) ++t;
+    while (t * PAGE <= last_pos && t * PAGE + PAGE <= first_key && t * PAGE >= keep_first) ++t;
     return t;
   };
   const int* pages = a.page_table + (int64_t)s * a.table_width;
@@ -127,6 +128,11 @@ __global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const __grid_co
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  // after a role's last page: the rows that have to be worked out again, by all warps that have the registers
+  auto finish = [&]() {
+    asm volatile("bar.sync 1, 256;" ::: "memory");
+    if ((again[0] | again[1] | again[2] | again[3]) != 0) rows_again<2 * CPW, float, float>(a, again, 12, 8);
+  };
 
   if (warp < 4) {
     regs_fewer<32>();
@@ -169,6 +175,7 @@ __global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const __grid_co
     } else if (warp == 2) {                                       // T = P V, by another warp
       const uint64_t v_desc = sw128_mn_desc(smem_u32(ring) + v_off);
       const bool one = elect_one();
+      const int dv = a.dv;
       bool ok = true;
       int i = 0, st = 0, slot = 0, g = 0;
       uint32_t slot_turn = 0;
@@ -180,7 +187,7 @@ __global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const __grid_co
         for (int c = 0; c < v_blocks; ++c, ++g) {
           if (g >= SLOTS && !mbar_wait(&t_empty[slot], slot_turn ^ 1)) { ok = false; break; }
           tc_fence_after();
-          const uint32_t idesc = umma_instr_desc(ROWS, min(CW, (a.dv - c * CW + 15) & ~15), false, true), d = tmem_base + TM_T + slot * CW;
+          const uint32_t idesc = umma_instr_desc(ROWS, min(CW, (dv - c * CW + 15) & ~15), false, true), d = tmem_base + TM_T + slot * CW;
           const uint64_t vd = v_at + c * (PAGE_BLOCK >> 4);
           if (one) {
 #pragma unroll
@@ -261,7 +268,8 @@ __global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const __grid_co
     const int clear_to = pos0 + quarter * 32 / hp, far = pos0 + min((quarter * 32 + 31) / hp, n_tok - 1);
     const int clear_from = a.window > 0 ? far - a.window + 1 : (a.chunk > 0 ? far - far % a.chunk : 0);
     const float scale2 = a.scale * LOG2E;
-    const bool plain = !(a.softcap > 0.f) && !(a.slope_span > 0.f) && a.scale > 0.f;
+    const bool capped = a.softcap > 0.f, sloped = a.slope_span > 0.f, plain = !capped && !sloped && a.scale > 0.f;
+    const float cap_in = a.cap_in, cap_out = a.cap_out;
     const float unit = plain ? scale2 : 1.f;
     const uint64_t unit2 = pair(unit, unit);
     int j = 0;
@@ -280,9 +288,9 @@ __global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const __grid_co
       tc_fence_before();
       mbar_arrive_one(&s_empty[b]);
       // Scores in units of log2, or, where nothing but a positive factor is on them, as they are with the factor `unit` still owed.
-      if (!plain) shape_scores(sc, a.softcap > 0.f, a.cap_in, a.cap_out, scale2, a.slope_span > 0.f, slope, pos - key0);
-      if (!(key0 + PAGE - 1 <= clear_to && (key0 >= clear_from || key0 + PAGE <= a.keep_first)))      // some pair does not see all of the page
-        hide_scores(sc, pos - key0, first - key0, a.keep_first - key0);
+      if (!plain) shape_scores(sc, capped, cap_in, cap_out, scale2, sloped, slope, pos - key0);
+      if (!(key0 + PAGE - 1 <= clear_to && (key0 >= clear_from || key0 + PAGE <= keep_first)))      // some pair does not see all of the page
+        hide_scores(sc, pos - key0, first - key0, keep_first - key0);
       float top[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
       for (int c = 0; c < 64; ++c) top[c & 3] = fmaxf(top[c & 3], sc[c]);
@@ -318,6 +326,7 @@ __global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const __grid_co
       tc_fence_before();
       mbar_arrive_one(&p_full[b]);
     }
+    finish();
   } else {
     // ---- the running output: a thread a row and CPW x 64 of its columns
     if (CPW == 1) regs_more<120>(); else regs_more<152>();
@@ -397,6 +406,7 @@ __global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const __grid_co
       bad = !(odd0 + odd1 == 0.f) || not_finite(inv);
     }
     note_again(again, quarter, bad);
+    finish();
   }
   tc_fence_before();
   __syncthreads();
@@ -405,7 +415,6 @@ __global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const __grid_co
     __syncwarp();
     tmem_dealloc(tmem_base, TM_COLS);
   }
-  if (warp >= 12 && (again[0] | again[1] | again[2] | again[3]) != 0) rows_again<2 * CPW, float, float>(a, again, 12, THREADS / 32 - 12);
 }
 
 struct Layout { int stages; size_t smem; };

@@ -89,29 +89,36 @@ __device__ __forceinline__ uint32_t pack(float a, float b) {
   return *reinterpret_cast<const uint32_t*>(&v);
 }
 
-// tanh(y) = y + y^3 P(y^2) up to |y| = 0.45 (P fitted to (tanh(y) / y - 1) / y^2 by reweighted least squares: off by 5e-9 of tanh).
+// tanh(y) = y + y^3 P(y^2) up to |y| = 0.45 (P fitted to (tanh(y) / y - 1) / y^2 by reweighted least squares: off by 7.8e-9 of tanh with these coefficients).
 constexpr float TANH_NEAR = 0.45f, TANH0 = -0.3333325f, TANH1 = 0.13329249f, TANH2 = -0.05334366f, TANH3 = 0.01802476f;
 
 // A row's 64 scores of a page, in units of log2: capped or scaled, less the slope times the distance (`ahead`: the row's position less the page's first).
 // (Whole passes under tests that are the same for every thread: this part is bound by instructions.)
 __device__ __forceinline__ void shape_scores(float (&sc)[64], bool capped, float cap_in, float cap_out, float scale2, bool sloped, float slope, int ahead) {
-  if (capped) {                             // cap tanh(s / cap): by `tanhf` where some score is far out, whose error follows its result too
+  if (capped) {                             // cap tanh(s / cap): which formula a score takes is its own affair (by `tanhf`, whose error follows its result too, far out)
+    const uint64_t in2 = pair(cap_in, cap_in), out2 = pair(cap_out, cap_out);
+    auto near2 = [&](int c) {
+      const uint64_t y = mul2(pair(sc[c], sc[c + 1]), in2), z = mul2(y, y);
+      uint64_t p = fma2(z, pair(TANH3, TANH3), pair(TANH2, TANH2));
+      p = fma2(z, p, pair(TANH1, TANH1));
+      p = fma2(z, p, pair(TANH0, TANH0));
+      return mul2(out2, fma2(mul2(y, z), p, y));
+    };
     float most = 0.f;
 #pragma unroll
     for (int c = 0; c < 64; ++c) most = fmaxf(most, fabsf(sc[c]));
-    if (__any_sync(0xffffffffu, most * fabsf(cap_in) > TANH_NEAR)) {
-#pragma unroll
-      for (int c = 0; c < 64; ++c) sc[c] = cap_out * tanhf(sc[c] * cap_in);
-    } else {
-      const uint64_t in2 = pair(cap_in, cap_in), out2 = pair(cap_out, cap_out);
+    if (__any_sync(0xffffffffu, most * fabsf(cap_in) > TANH_NEAR)) {      // (the vote only saves work: whoever is not far out has the polynomial's result either way)
 #pragma unroll
       for (int c = 0; c < 64; c += 2) {
-        const uint64_t y = mul2(pair(sc[c], sc[c + 1]), in2), z = mul2(y, y);
-        uint64_t p = fma2(z, pair(TANH3, TANH3), pair(TANH2, TANH2));
-        p = fma2(z, p, pair(TANH1, TANH1));
-        p = fma2(z, p, pair(TANH0, TANH0));
-        unpair(mul2(out2, fma2(mul2(y, z), p, y)), sc[c], sc[c + 1]);
+        float n0, n1;
+        unpair(near2(c), n0, n1);
+        const float y0 = sc[c] * cap_in, y1 = sc[c + 1] * cap_in, f0 = cap_out * tanhf(y0), f1 = cap_out * tanhf(y1);
+        asm("{\n\t.reg .pred p;\n\tsetp.gt.f32 p, %1, %2;\n\tselp.f32 %0, %3, %4, p;\n\t}" : "=f"(sc[c]) : "f"(fabsf(y0)), "f"(TANH_NEAR), "f"(f0), "f"(n0));      // (no branch an entry)
+        asm("{\n\t.reg .pred p;\n\tsetp.gt.f32 p, %1, %2;\n\tselp.f32 %0, %3, %4, p;\n\t}" : "=f"(sc[c + 1]) : "f"(fabsf(y1)), "f"(TANH_NEAR), "f"(f1), "f"(n1));
       }
+    } else {
+#pragma unroll
+      for (int c = 0; c < 64; c += 2) unpair(near2(c), sc[c], sc[c + 1]);
     }
   } else {
 #pragma unroll
@@ -238,8 +245,8 @@ __device__ __forceinline__ void note_again(uint32_t* again, int quarter, bool ba
   const uint32_t rows = __ballot_sync(0xffffffffu, bad);
   if (rows != 0 && (threadIdx.x & 31) == 0) atomicOr(again + quarter, rows);
 }
-// The noted rows of a block, by `warps` of its warps from `first` on (those that have given no registers away: a function may take as many as the kernel was launched
-// with); after a barrier of the whole block.  Args: the kernels' arguments (in constant memory).  It finds the block's place again: nothing of it is kept in the kernels' registers.
+// The noted rows of a block, by `warps` of its warps from `first` on, which all call it at the end of their roles (where they still have the registers that they took).
+// Args: the kernels' arguments (in constant memory).  It finds the block's place again: nothing of it is kept in the kernels' registers.
 template <int NI, typename T, typename TO, typename Args>
 __device__ __noinline__ void rows_again(const Args& a, const uint32_t* again, int first, int warps) {
   const int hp = a.hp, tok = ROWS / hp, group = a.n_heads / a.n_kv_heads, chunks = group / hp, per_seq = a.n_kv_heads * chunks;

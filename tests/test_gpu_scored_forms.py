@@ -334,3 +334,29 @@ def test_a_number_that_is_not_finite_stays_with_the_rows_that_see_it(H, G, dk, d
         # (a row that loses a key's weight keeps its bound's order: twice it is generous)
         bound = 2 * c.slack + (2.0 ** -8 if out == torch.bfloat16 else 2.0 ** -22) * want.abs() + 1e-30
         assert float(((got - want).abs() / bound)[ok].max()) <= 1.0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_a_capped_rows_bits_are_its_own(dtype):
+    """Scores far out, where the cap takes another formula, in later rows of the tile, in another sequence and in places of the cache that hold nothing yet."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(5)
+    ops, H, G, d = Ops(dtype), 4, 2, 64
+    kp, vp, q = (torch.randn(*s, generator=g, device="cuda").to(dtype) for s in ((5, G, PAGE, d), (5, G, PAGE, d), (50, H * d)))
+    table = i32([[3, 1], [0, 4]])
+
+    def run(q, kp, n_seqs):
+        out = torch.full((50 if n_seqs == 2 else 20, H * d), float("nan"), device="cuda")      # (32-bit: a rounding to 16 would hide it)
+        ops.attention_scored(q[:len(out)], out, i32([0, 20, 50][:n_seqs + 1]), i32([90, 35][:n_seqs]), n_seqs, 30 if n_seqs == 2 else 20, table[:n_seqs], kp, vp, H, 0.125, softcap=30.0)
+        return out
+    want = run(q, kp, 1)
+    assert want.isfinite().all()
+    far = q.clone()
+    far[10:] *= 1000
+    assert torch.equal(run(far, kp, 1)[:10], want[:10])
+    far = q.clone()
+    far[20:] *= 1000
+    assert torch.equal(run(far, kp, 2)[:20], want)
+    stale = kp.clone()
+    stale[1, :, 90 - PAGE:] *= 1000                      # places past the first sequence's end
+    assert torch.equal(run(q, stale, 1), want)
