@@ -369,7 +369,7 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         const float most = run_max * LN2, sink = a.sinks[h], m = fmaxf(most, sink), f = expf(most - m);
         inv = f / fmaf(run_sum, f, expf(sink - m));
       }
-      if (gate != nullptr && a.gate_heads) inv *= sigmoid_fast(__bfloat162float(*gate));
+      if (gate != nullptr && a.gate_heads) inv *= sigmoid(__bfloat162float(*gate));
 #pragma unroll
       for (int c = 0; c < CPW * 8; ++c) {
         const int d = c0 * 64 + c * 8;                            // (dv is a multiple of 8)
@@ -404,8 +404,8 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
             }
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-              x[2 * e] *= sigmoid_fast(__uint_as_float(z[e] << 16));
-              x[2 * e + 1] *= sigmoid_fast(__uint_as_float(z[e] & 0xffff0000u));
+              x[2 * e] *= sigmoid(__uint_as_float(z[e] << 16));
+              x[2 * e + 1] *= sigmoid(__uint_as_float(z[e] & 0xffff0000u));
             }
           }
           uint32_t w[4];

@@ -717,7 +717,7 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_read_kernel(const ChunkArgs 
         const float4 g4 = widen(gate.raw[f]);
         const float gt[4] = {g4.x, g4.y, g4.z, g4.w};
 #pragma unroll
-        for (int e = 0; e < 4; ++e) y[e] *= sizeof(TI) == 2 ? __fdividef(gt[e], 1.0f + __expf(-gt[e])) : gt[e] / (1.0f + expf(-gt[e]));
+        for (int e = 0; e < 4; ++e) y[e] *= silu_f(gt[e]);
       }
       TI* o = (TI*)a.out + row * a.ld_out + h * a.dv + c;
       if (a.vec_out) {

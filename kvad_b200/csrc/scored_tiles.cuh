@@ -76,8 +76,8 @@ __device__ __forceinline__ float exp2_fast(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-// 1 / (1 + 2^(-z log2 e)) by the special-function unit (3 units in the last place, before a rounding to bfloat16).
-__device__ __forceinline__ float sigmoid_fast(float z) { return __fdividef(1.0f, 1.0f + exp2_fast(-z * LOG2E)); }
+// (a full division: the fast one gives 0 for gates below -87.3, where 1 + e^(-z) is beyond 2^126)
+__device__ __forceinline__ float sigmoid(float z) { return 1.0f / (1.0f + expf(-z)); }
 // The upper halves of two floats as a pair of bfloat16 (truncated), and what is left of each.
 __device__ __forceinline__ uint32_t cut(float& a, float& b) {
   const uint32_t x = __float_as_uint(a), y = __float_as_uint(b);

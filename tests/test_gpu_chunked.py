@@ -385,3 +385,18 @@ def test_short_sequences_keep_their_bits_beside_a_prompt(kind, dtype, dk, dv):
     ops.chunked_recurrences = False
     walked, _ = run([1], True)
     assert not torch.equal(walked, got[at[1]:at[2]])       # (the prompt did go in chunks)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_gates_far_below_zero_of_chunked_retention(dtype):
+    """silu(-88) is -5e-37: 1 + e^88 lies where a fast division gives 0."""
+    g, ops = torch.Generator(device="cuda"), Ops(DT[dtype])
+    g.manual_seed(3)
+    q, k, v = (torch.randn(200, 2 * 64, generator=g, device="cuda").to(DT[dtype]) for _ in range(3))
+    outs = []
+    for z in (-88.0, 2.0):
+        out, gate = (torch.full((200, 128), x, device="cuda", dtype=DT[dtype]) for x in (float("nan"), z))
+        ops.retention(q, k, v, out, torch.zeros(1, 2, 64, 64, device="cuda"), i32([0, 200]), i32([200]), i32([0]), 1, torch.tensor([0.9, 1.0], device="cuda"), 2, gate=gate,
+                      unit_norm_eps=1e-5, raw=torch.empty(200, 128, device="cuda"), max_new=200)
+        outs.append(out.double() / (z * torch.sigmoid(torch.tensor(z, dtype=torch.float64))).item())
+    assert rel(outs[0], outs[1]) < (6e-3 if dtype == "bfloat16" else 1e-6)      # (both rounded to the output's type; 32-bit exponentials and divisions)

@@ -360,3 +360,18 @@ def test_a_capped_rows_bits_are_its_own(dtype):
     stale = kp.clone()
     stale[1, :, 90 - PAGE:] *= 1000                      # places past the first sequence's end
     assert torch.equal(run(q, stale, 1), want)
+
+
+@pytest.mark.parametrize("H,G,dk,dv", [(4, 2, 64, 64), (16, 1, 256, 256)])
+@pytest.mark.parametrize("gate", ["entry", "head"])
+def test_gates_far_below_zero(H, G, dk, dv, gate):
+    """sigmoid(-88) is 6e-39: 1 + e^88 lies where a fast division gives 0."""
+    c = Case([(3, 70)], H, G, dk, dv, gate=gate)
+    f = torch.sigmoid(c.gate.double())
+    c.gate.fill_(-88.0)
+    c.vp.mul_(2.0 ** 100)
+    wide = (lambda x: x.repeat_interleave(dv, 1)) if gate == "head" else (lambda x: x)
+    change = wide(torch.sigmoid(c.gate.double()) / f) * 2.0 ** 100
+    got, want, slack = c.run(Ops(torch.bfloat16)), c.want * change, c.slack * change
+    assert ((got - want).abs() <= slack + 2.0 ** -8 * want.abs() + 1e-30).all()
+    assert float(want.abs().max()) > 1e-9
