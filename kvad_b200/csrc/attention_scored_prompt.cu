@@ -2,14 +2,14 @@
 // given), on the 5th-generation tensor cores: bfloat16 queries, keys and values, 32-bit scores, softmax weights and sums.
 //
 //   S = Q K^T        tcgen05.mma, 128 (token, head) pairs x 64 keys of a page, in tensor memory
-//   p = exp(s - m)   32-bit, m the page's own largest score of the row: a page's weights wait for no other page
+//   p = exp(s - m)   32-bit, m the page's own largest score of the row (a whole power of two): a page's weights wait for no other page
 //   T = P V          p is cut into three bfloat16 pieces, p = h + m + l exactly (a weight keeps its 24 bits), which lie in tensor memory as the
 //                    product's first operand, the smallest first.  The tensor core's truncating accumulation is kept to one page,
-//   O = a O + b T    whose sum joins the 32-bit running sum in registers by rounded operations (a, b: 2^(old maximum - new), 2^(m - new))
+//   O = a O + b T    whose sum joins the 32-bit running sum in registers by rounded operations (a, b: 2^(old maximum - new), 2^(m - new), both exact)
 //
 // A block works 128 (token, head) pairs that share a key head: 128 / hp consecutive tokens of one sequence times hp heads of the group.
 // Roles, so that the tensor core's queue never waits for one thread's chain: one warp brings the queries once and the pages' keys and
-// values by TMA into a ring; one thread issues the products, S of up to two pages ahead of P V; NS groups of four warps turn the pages' scores
+// values by TMA into a ring; one warp issues S = Q K^T, up to two pages ahead of P V, which another issues; NS groups of four warps turn the pages' scores
 // into weights (a thread a row, pages in turn); NA groups of four warps keep the running output (a thread a row and up to 128 of its
 // columns).  NS = 2, NA = 1 for values of up to 128 entries, where softmax takes the time; NS = 1, NA = 2 above, where the products do.
 // P V goes in pieces of columns through two or three places of tensor memory, so that one can be read while the next is worked out.
@@ -58,6 +58,9 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
   constexpr bool S_IS_P = NS == 1;
   constexpr int NI = NS == 1 ? 8 : 2 * CPW, FINISHERS = THREADS / 32 - 4;      // 32s of a value's entries; warps that finish a block together
   constexpr int CW = NS == 1 ? 128 : 64, SLOTS = NS == 1 ? 2 : 3;
+  // With a 32-bit output the small pieces' products have an accumulator of their own, so that nothing truncates what is small once it is large; a rounding to bfloat16 hides it.
+  constexpr int PARTS = F32OUT ? 2 : 1;
+  constexpr bool TOGETHER = PARTS == 2 && NS == 2;      // the two meet before they join the running output (where two groups of warps share the places, a group has one of its own)
   constexpr uint32_t TM_T = 0, TM_S = SLOTS * CW, TM_P = TM_S + 128, P_STEP = S_IS_P ? 64 : 96;
   static_assert(TM_P + 2 * P_STEP <= TM_COLS, "tensor memory");
   extern __shared__ uint8_t smem_raw[];
@@ -199,18 +202,24 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         if (!mbar_wait(&p_full[b], (i >> 1) & 1)) { ok = false; break; }
         const uint32_t p_at = tmem_base + TM_P + b * P_STEP, low_at = tmem_base + (S_IS_P ? TM_S + b * 64 : TM_P + b * P_STEP + 64);
         const uint64_t v_at = v_desc + st * stage_step;
-        for (int c = 0; c < n_chunks; ++c, ++g) {
+        for (int c = 0; c < n_chunks * PARTS; ++c, ++g) {
           if (g >= SLOTS && !mbar_wait(&t_empty[slot], slot_turn ^ 1)) { ok = false; break; }
           tc_fence_after();
-          const uint32_t idesc = umma_instr_desc(ROWS, min(CW, (dv - c * CW + 15) & ~15), false, true), d = tmem_base + TM_T + slot * CW;
-          const uint64_t vd = v_at + c * (CW / 64) * (PAGE_BLOCK >> 4);
+          // (where two groups of warps share the places: all chunks' small products, then all their h h, so that each meets every turn of its own place)
+          const int part = TOGETHER ? c & 1 : (c >= n_chunks ? 1 : 0), chunk = TOGETHER ? c >> 1 : c - part * n_chunks;
+          const uint32_t idesc = umma_instr_desc(ROWS, min(CW, (dv - chunk * CW + 15) & ~15), false, true), d = tmem_base + TM_T + slot * CW;
+          const uint64_t vd = v_at + chunk * (CW / 64) * (PAGE_BLOCK >> 4);
           if (one) {
+            if (part == 0) {
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk) umma_ta(d, low_at + kk * 8, vd + kk * (2048 >> 4), idesc, kk > 0 ? 1u : 0u);
+              for (int kk = 0; kk < 4; ++kk) umma_ta(d, low_at + kk * 8, vd + kk * (2048 >> 4), idesc, kk > 0 ? 1u : 0u);
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk) umma_ta(d, p_at + 32 + kk * 8, vd + kk * (2048 >> 4), idesc, 1u);
+              for (int kk = 0; kk < 4; ++kk) umma_ta(d, p_at + 32 + kk * 8, vd + kk * (2048 >> 4), idesc, 1u);
+            }
+            if (part == PARTS - 1) {
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk) umma_ta(d, p_at + kk * 8, vd + kk * (2048 >> 4), idesc, 1u);
+              for (int kk = 0; kk < 4; ++kk) umma_ta(d, p_at + kk * 8, vd + kk * (2048 >> 4), idesc, (PARTS == 1 || kk > 0) ? 1u : 0u);
+            }
             umma_commit(&t_full[slot]);
           }
           if (++slot == SLOTS) { slot = 0; slot_turn ^= 1; }
@@ -266,7 +275,7 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
       float top[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
       for (int c = 0; c < 64; ++c) top[c & 3] = fmaxf(top[c & 3], sc[c]);
-      const float most = fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3])) * unit, base = most == -INFINITY ? 0.f : most;
+      const float most = ceilf(fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3])) * unit), base = most == -INFINITY ? 0.f : most;
       if (j >= 2 && !mbar_wait(&p_empty[b], turn ^ 1)) break;
       tc_fence_after();
       const uint64_t less = pair(-base, -base);
@@ -334,29 +343,46 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
       if (!mbar_wait(&st_full[j % STATS], (j / STATS) & 1)) { ok = false; break; }
       const float2 st = stats[(j % STATS) * ROWS + row];
       const float new_max = fmaxf(run_max, st.x);
-      const float keep = run_max == -INFINITY ? 0.f : exp2_fast(run_max - new_max), take = st.x == -INFINITY ? 0.f : exp2_fast(st.x - new_max);
+      const float keep = run_max == -INFINITY ? 0.f : exp2_whole(run_max - new_max), take = st.x == -INFINITY ? 0.f : exp2_whole(st.x - new_max);
       // (a page that the row sees nothing of has weights of zero and a sum of zero, or NaN, which stays)
       run_sum = fmaf(run_sum, keep, st.y * (st.x == -INFINITY ? 1.f : take));
       run_max = new_max;
       const uint64_t keep2 = pair(keep, keep), take2 = pair(take, take);
+      auto take_page = [&](int part, uint64_t stay) {             // this group's chunks of P V, one part of them
 #pragma unroll
-      for (int c = 0; c < CPW * 64 / CW; ++c) {
-        if (c0 * 64 / CW + c >= n_chunks) continue;
-        const int g = j * n_chunks + c0 * 64 / CW + c, turns = g / SLOTS, slot = g - turns * SLOTS;
-        if (!mbar_wait(&t_full[slot], turns & 1)) { ok = false; break; }
-        tc_fence_after();
+        for (int c = 0; c < CPW * 64 / CW; ++c) {
+          if (c0 * 64 / CW + c >= n_chunks) continue;
+          const int g = TOGETHER ? (j * n_chunks + c) * 2 : (j * PARTS + part) * n_chunks + c0 * 64 / CW + c, turns = g / SLOTS, slot = g - turns * SLOTS;
+          const int slot2 = slot + 1 == SLOTS ? 0 : slot + 1;
+          if (!mbar_wait(&t_full[slot], turns & 1) || (TOGETHER && !mbar_wait(&t_full[slot2], (slot2 == 0 ? turns + 1 : turns) & 1))) { ok = false; break; }
+          tc_fence_after();
 #pragma unroll
-        for (int q = 0; q < CW / 16; ++q) {
-          float v[16];
-          tmem_ld16(lanes + slot * CW + q * 16, v);
+          for (int q = 0; q < CW / 16; ++q) {
+            uint64_t v[8];
+            if (TOGETHER) {
+              tmem_ld_sum<16>(lanes + slot * CW + q * 16, lanes + slot2 * CW + q * 16, v);
+            } else {
+              float one[16];
+              tmem_ld16(lanes + slot * CW + q * 16, one);
 #pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            uint64_t& x = o[c * (CW / 2) + q * 8 + e];
-            x = fma2(x, keep2, mul2(pair(v[2 * e], v[2 * e + 1]), take2));
+              for (int e = 0; e < 8; ++e) v[e] = pair(one[2 * e], one[2 * e + 1]);
+            }
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              uint64_t& x = o[c * (CW / 2) + q * 8 + e];
+              x = fma2(x, stay, mul2(v[e], take2));
+            }
           }
+          tc_fence_before();
+          mbar_arrive_one(&t_empty[slot]);
+          if (TOGETHER) mbar_arrive_one(&t_empty[slot2]);
         }
-        tc_fence_before();
-        mbar_arrive_one(&t_empty[slot]);
+      };
+      if (PARTS == 1 || TOGETHER) {
+        take_page(0, keep2);
+      } else {
+#pragma unroll 1
+        for (int part = 0; part < 2 && ok; ++part) take_page(part, part == 0 ? keep2 : pair(1.f, 1.f));
       }
     }
     bool bad = false;                                             // some entry is not finite (0 times it is none)
@@ -370,55 +396,59 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         inv = f / fmaf(run_sum, f, expf(sink - m));
       }
       if (gate != nullptr && a.gate_heads) inv *= sigmoid(__bfloat162float(*gate));
+      auto leave = [&](auto gated) {                              // (apart: what gates take makes the way of those without any longer by fetching it: 8 us for 9.8, 17 rows of 8 heads of 128)
 #pragma unroll
-      for (int c = 0; c < CPW * 8; ++c) {
-        const int d = c0 * 64 + c * 8;                            // (dv is a multiple of 8)
-        if (d >= a.dv) continue;
-        float x[8];
+        for (int c = 0; c < CPW * 8; ++c) {
+          const int d = c0 * 64 + c * 8;                            // (dv is a multiple of 8)
+          if (d >= a.dv) continue;
+          float x[8];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          unpair(o[c * 4 + e], x[2 * e], x[2 * e + 1]);
-          odd = fma2(o[c * 4 + e], 0ull, odd);
-        }
-#pragma unroll
-        for (int e = 0; e < 8; ++e) x[e] *= inv;
-        if (F32OUT) {
-          float* dst = reinterpret_cast<float*>(a.out) + grow * a.ld_out + (int64_t)h * a.dv + d;
-          if (a.vec) {
-            reinterpret_cast<float4*>(dst)[0] = make_float4(x[0], x[1], x[2], x[3]);
-            reinterpret_cast<float4*>(dst)[1] = make_float4(x[4], x[5], x[6], x[7]);
-          } else {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) reinterpret_cast<float2*>(dst)[e] = make_float2(x[2 * e], x[2 * e + 1]);
+          for (int e = 0; e < 4; ++e) {
+            unpair(o[c * 4 + e], x[2 * e], x[2 * e + 1]);
+            odd = fma2(o[c * 4 + e], 0ull, odd);
           }
-        } else {
-          __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(a.out) + grow * a.ld_out + (int64_t)h * a.dv + d;
-          if (gate != nullptr && !a.gate_heads) {
-            uint32_t z[4];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) x[e] *= inv;
+          if (F32OUT) {
+            float* dst = reinterpret_cast<float*>(a.out) + grow * a.ld_out + (int64_t)h * a.dv + d;
             if (a.vec) {
-              const uint4 w = *reinterpret_cast<const uint4*>(gate + c * 8);
-              z[0] = w.x; z[1] = w.y; z[2] = w.z; z[3] = w.w;
+              reinterpret_cast<float4*>(dst)[0] = make_float4(x[0], x[1], x[2], x[3]);
+              reinterpret_cast<float4*>(dst)[1] = make_float4(x[4], x[5], x[6], x[7]);
             } else {
 #pragma unroll
-              for (int e = 0; e < 4; ++e) z[e] = *reinterpret_cast<const uint32_t*>(gate + c * 8 + 2 * e);
+              for (int e = 0; e < 4; ++e) reinterpret_cast<float2*>(dst)[e] = make_float2(x[2 * e], x[2 * e + 1]);
             }
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              x[2 * e] *= sigmoid(__uint_as_float(z[e] << 16));
-              x[2 * e + 1] *= sigmoid(__uint_as_float(z[e] & 0xffff0000u));
-            }
-          }
-          uint32_t w[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) w[e] = pack(x[2 * e], x[2 * e + 1]);
-          if (a.vec) {
-            *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
           } else {
+            __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(a.out) + grow * a.ld_out + (int64_t)h * a.dv + d;
+            if (gated.value) {
+              uint32_t z[4];
+              if (a.vec) {
+                const uint4 w = *reinterpret_cast<const uint4*>(gate + c * 8);
+                z[0] = w.x; z[1] = w.y; z[2] = w.z; z[3] = w.w;
+              } else {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) *reinterpret_cast<uint32_t*>(dst + 2 * e) = w[e];
+                for (int e = 0; e < 4; ++e) z[e] = *reinterpret_cast<const uint32_t*>(gate + c * 8 + 2 * e);
+              }
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                x[2 * e] *= sigmoid(__uint_as_float(z[e] << 16));
+                x[2 * e + 1] *= sigmoid(__uint_as_float(z[e] & 0xffff0000u));
+              }
+            }
+            uint32_t w[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) w[e] = pack(x[2 * e], x[2 * e + 1]);
+            if (a.vec) {
+              *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+            } else {
+#pragma unroll
+              for (int e = 0; e < 4; ++e) *reinterpret_cast<uint32_t*>(dst + 2 * e) = w[e];
+            }
           }
         }
-      }
+      };
+      if (!F32OUT && gate != nullptr && !a.gate_heads) leave(std::true_type());
+      else leave(std::false_type());
       float odd0, odd1;
       unpair(odd, odd0, odd1);
       bad = !(odd0 + odd1 == 0.f) || not_finite(inv);

@@ -4,16 +4,20 @@
 // As `attention_scored_prompt.cu` (128 (token, head) pairs a block, pages of 64 keys, a page's weights against its own maximum, sums of one page in the
 // tensor core, 32-bit registers beyond), with every operand cut into bfloat16 pieces x = h + m + l (exact above about 2^-110) and the six products of
 // pieces that reach 2^-24 (h h, h m, m h, h l, m m, l h, the smallest first): S takes 24 products of 128 x 64 x 16 for keys of 64, P V as many.
-// Queries are cut once; a page's keys and values are cut by four warps (of eight that take pages in turn) into the ring that the tensor core reads.
+// The tensor core truncates where it accumulates, so S leaves it after 64 entries of a key, P V after 64 keys with its h h in an accumulator of their own; all
+// joins are rounded.  Queries are cut once; a page's keys and values are cut by four warps (of eight that take pages in turn) into the ring that the tensor core reads.
 //
 // What bounds it: cutting a page (1000 instructions a thread of four warps) about as much as its 48 products (1150 + 770 cycles for 64 + 64 entries); one page at a time
-// where keys and values are above 64 entries.  us against the CUDA cores, relative error against 64 bits: 2 x 1024 rows of 16 heads of 64 on 4 key heads: 54 against 387,
-// 2.1e-7 against 3.3e-7; capped, gated, window 512: 81 against 347; heads of 128: 136 against 739; a latent of 128 with 32 more key entries: 125 against 752;
-// two new rows of four sequences behind 300 positions: 17.7 against 56; one prompt of 17: 9.8 against 16.6; 12 heads of 64, prompts of 64 .. 540: 33 against 108
-// (the tiled kernel of `attention_simt.cu`).  (With one group of warps cutting a batch ahead by way of registers: 90 where it is 54.)
+// where keys and values are above 64 entries.  us against the CUDA cores: 2 x 1024 rows of 16 heads of 64 on 4 key heads: 56 against 381; capped, window 512: 63 against 313
+// (scores beyond 0.45 caps among them: 87); heads of 128: 132 against 472; a latent of 96 with 32 more key entries: 78 against 640; two new rows of four sequences behind 300
+// positions: 17 against 54; one prompt of 17: 9.6 against 15.6.  (With one group of warps cutting a batch ahead by way of registers: 90 where it was 54.  One accumulator for all
+// of S and one for all of P V: 53, 64, 130, 71.)
+// Relative error against 64 bits, here and there (heads of 64; of 128): 2 x 1024 rows 2.2e-7, 3.3e-7; 2.0e-7, 3.9e-7; operands of one sign 1.3e-7, 3.4e-7 in both; 2000 cached positions
+// 3.1e-7, 8.5e-7; one prompt of 17 1.2e-7, 1.2e-7; 1.3e-7, 1.8e-7.  It is larger only where the weights of few keys are nearly even (17 rows, scores below 0.1: 8.8e-8 for 6.0e-8).
 //
 // A number that is not finite has no pieces: rows whose outputs it reaches are worked out again by fmaf (`row_again`).  Every wait is bounded.
 #include <algorithm>
+#include <type_traits>
 
 #include "scored_tiles.cuh"
 
@@ -142,29 +146,30 @@ __global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const __grid_co
       const uint64_t q_desc = sw128_desc(smem_u32(q_tile)), k_desc = sw128_desc(smem_u32(ring));
       const bool one = elect_one();
       bool ok = true;
-      int j = 0, st = 0;
+      int u = 0, st = 0;                                          // u: blocks of 64 entries so far, each an accumulator of its own (the tensor core truncates where it accumulates)
       uint32_t turn = 0;
-      for (int t = next_page(0); t * PAGE <= last_pos && ok; t = next_page(t + 1), ++j) {
-        const int b = j & 1;
-        if (!mbar_wait(&kv_full[st], turn) || (j >= 2 && !mbar_wait(&s_empty[b], ((j >> 1) & 1) ^ 1))) { ok = false; break; }
-        tc_fence_after();
+      for (int t = next_page(0); t * PAGE <= last_pos && ok; t = next_page(t + 1)) {
+        if (!mbar_wait(&kv_full[st], turn)) { ok = false; break; }
         const uint64_t k_at = k_desc + st * (stage_bytes >> 4);
-        const uint32_t d = tmem_base + TM_S + b * 64;
-        if (one) {
+        int left = k_steps;
+        for (int kb = 0; kb < k_blocks; ++kb, ++u, left -= 4) {
+          const int b = u & 1;
+          if (u >= 2 && !mbar_wait(&s_empty[b], ((u >> 1) & 1) ^ 1)) { ok = false; break; }
+          tc_fence_after();
+          const uint32_t d = tmem_base + TM_S + b * 64;
+          if (one) {
 #pragma unroll
-          for (int x = 0; x < 6; ++x) {
-            int left = k_steps;
-            for (int kb = 0; kb < k_blocks; ++kb, left -= 4) {
+            for (int x = 0; x < 6; ++x) {
               const uint64_t qd = q_desc + PA[x] * (q_piece >> 4) + kb * (Q_BLOCK >> 4), kd = k_at + PB[x] * (k_piece >> 4) + kb * (PAGE_BLOCK >> 4);
               if (left >= 4) {
 #pragma unroll
-                for (int k = 0; k < 4; ++k) umma(d, qd + k * 2, kd + k * 2, idesc, (x > 0 || kb > 0 || k > 0) ? 1u : 0u);
+                for (int k = 0; k < 4; ++k) umma(d, qd + k * 2, kd + k * 2, idesc, (x > 0 || k > 0) ? 1u : 0u);
               } else {
-                for (int k = 0; k < left; ++k) umma(d, qd + k * 2, kd + k * 2, idesc, (x > 0 || kb > 0 || k > 0) ? 1u : 0u);
+                for (int k = 0; k < left; ++k) umma(d, qd + k * 2, kd + k * 2, idesc, (x > 0 || k > 0) ? 1u : 0u);
               }
             }
+            umma_commit(&s_full[b]);
           }
-          umma_commit(&s_full[b]);
         }
         if (++st == stages) { st = 0; turn ^= 1; }
       }
@@ -184,16 +189,21 @@ __global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const __grid_co
         if (!mbar_wait(&p_full[b], (i >> 1) & 1)) { ok = false; break; }
         const uint32_t p_at = tmem_base + TM_P + b * P_STEP;
         const uint64_t v_at = v_desc + st * (stage_bytes >> 4);
-        for (int c = 0; c < v_blocks; ++c, ++g) {
+        for (int c = 0; c < 2 * v_blocks; ++c, ++g) {             // 64 columns' small products, then their h h: apart, so that nothing truncates what is small once it is large
           if (g >= SLOTS && !mbar_wait(&t_empty[slot], slot_turn ^ 1)) { ok = false; break; }
           tc_fence_after();
-          const uint32_t idesc = umma_instr_desc(ROWS, min(CW, (dv - c * CW + 15) & ~15), false, true), d = tmem_base + TM_T + slot * CW;
-          const uint64_t vd = v_at + c * (PAGE_BLOCK >> 4);
+          const uint32_t idesc = umma_instr_desc(ROWS, min(CW, (dv - (c >> 1) * CW + 15) & ~15), false, true), d = tmem_base + TM_T + slot * CW;
+          const uint64_t vd = v_at + (c >> 1) * (PAGE_BLOCK >> 4);
           if (one) {
+            if ((c & 1) == 0) {
 #pragma unroll
-            for (int x = 0; x < 6; ++x)
+              for (int x = 0; x < 5; ++x)
 #pragma unroll
-              for (int kk = 0; kk < 4; ++kk) umma_ta(d, p_at + PA[x] * 32 + kk * 8, vd + PB[x] * (v_piece >> 4) + kk * (2048 >> 4), idesc, (x > 0 || kk > 0) ? 1u : 0u);
+                for (int kk = 0; kk < 4; ++kk) umma_ta(d, p_at + PA[x] * 32 + kk * 8, vd + PB[x] * (v_piece >> 4) + kk * (2048 >> 4), idesc, (x > 0 || kk > 0) ? 1u : 0u);
+            } else {
+#pragma unroll
+              for (int kk = 0; kk < 4; ++kk) umma_ta(d, p_at + kk * 8, vd + kk * (2048 >> 4), idesc, kk > 0 ? 1u : 0u);
+            }
             umma_commit(&t_full[slot]);
           }
           if (++slot == SLOTS) { slot = 0; slot_turn ^= 1; }
@@ -258,7 +268,7 @@ __global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const __grid_co
     }
   } else if (warp < 16) {
     // ---- scores into weights: a thread a row
-    if (CPW == 1) regs_more<152>(); else regs_more<136>();
+    if (CPW == 1) regs_more<152>(); else regs_more<112>();
     const int quarter = warp & 3, row = quarter * 32 + lane;
     const uint32_t lanes = tmem_base + ((uint32_t)(quarter * 32) << 16);
     const int ti = row / hp, pos = pos0 + ti;
@@ -272,21 +282,33 @@ __global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const __grid_co
     const float cap_in = a.cap_in, cap_out = a.cap_out;
     const float unit = plain ? scale2 : 1.f;
     const uint64_t unit2 = pair(unit, unit);
-    int j = 0;
+    int j = 0, u = 0;
     for (int t = next_page(0); t * PAGE <= last_pos; t = next_page(t + 1), ++j) {
       const int b = j & 1, key0 = t * PAGE;
       const uint32_t turn = (j >> 1) & 1;
-      if (!mbar_wait(&s_full[b], turn)) break;
-      tc_fence_after();
       float sc[64];
-      {
-        uint32_t* raw = reinterpret_cast<uint32_t*>(sc);
-        tmem_ld32(lanes + TM_S + b * 64, raw);
-        tmem_ld32(lanes + TM_S + b * 64 + 32, raw + 32);
-        tmem_ld_wait();
+      bool come = true;
+      for (int kb = 0; kb < k_blocks; ++kb, ++u) {
+        if (!mbar_wait(&s_full[u & 1], (u >> 1) & 1)) { come = false; break; }
+        tc_fence_after();
+        if (kb == 0) {
+          uint32_t* raw = reinterpret_cast<uint32_t*>(sc);
+          tmem_ld32(lanes + TM_S + (u & 1) * 64, raw);
+          tmem_ld32(lanes + TM_S + (u & 1) * 64 + 32, raw + 32);
+          tmem_ld_wait();
+        } else {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            float more[16];
+            tmem_ld16(lanes + TM_S + (u & 1) * 64 + q * 16, more);
+#pragma unroll
+            for (int e = 0; e < 16; ++e) sc[q * 16 + e] += more[e];
+          }
+        }
+        tc_fence_before();
+        mbar_arrive_one(&s_empty[u & 1]);
       }
-      tc_fence_before();
-      mbar_arrive_one(&s_empty[b]);
+      if (!come) break;
       // Scores in units of log2, or, where nothing but a positive factor is on them, as they are with the factor `unit` still owed.
       if (!plain) shape_scores(sc, capped, cap_in, cap_out, scale2, sloped, slope, pos - key0);
       if (!(key0 + PAGE - 1 <= clear_to && (key0 >= clear_from || key0 + PAGE <= keep_first)))      // some pair does not see all of the page
@@ -294,7 +316,7 @@ __global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const __grid_co
       float top[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
       for (int c = 0; c < 64; ++c) top[c & 3] = fmaxf(top[c & 3], sc[c]);
-      const float most = fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3])) * unit, base = most == -INFINITY ? 0.f : most;
+      const float most = ceilf(fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3])) * unit), base = most == -INFINITY ? 0.f : most;
       if (j >= 2 && !mbar_wait(&p_empty[b], turn ^ 1)) break;
       tc_fence_after();
       const uint64_t less = pair(-base, -base);
@@ -329,7 +351,7 @@ __global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const __grid_co
     finish();
   } else {
     // ---- the running output: a thread a row and CPW x 64 of its columns
-    if (CPW == 1) regs_more<120>(); else regs_more<152>();
+    if (CPW == 1) regs_more<120>(); else regs_more<176>();
     const int quarter = warp & 3, row = quarter * 32 + lane;
     const uint32_t lanes = tmem_base + ((uint32_t)(quarter * 32) << 16) + TM_T;
     const int ti = row / hp, h = h0 + row - ti * hp;
@@ -349,7 +371,7 @@ __global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const __grid_co
       if (!mbar_wait(&st_full[j % STATS], (j / STATS) & 1)) { ok = false; break; }
       const float2 st = stats[(j % STATS) * ROWS + row];
       const float new_max = fmaxf(run_max, st.x);
-      const float keep = run_max == -INFINITY ? 0.f : exp2_fast(run_max - new_max), take = st.x == -INFINITY ? 0.f : exp2_fast(st.x - new_max);
+      const float keep = run_max == -INFINITY ? 0.f : exp2_whole(run_max - new_max), take = st.x == -INFINITY ? 0.f : exp2_whole(st.x - new_max);
       // (a page that the row sees nothing of has weights of zero and a sum of zero, or NaN, which stays)
       run_sum = fmaf(run_sum, keep, st.y * (st.x == -INFINITY ? 1.f : take));
       run_max = new_max;
@@ -357,21 +379,23 @@ __global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const __grid_co
 #pragma unroll
       for (int c = 0; c < CPW; ++c) {
         if (c >= v_blocks) continue;
-        const int g = j * v_blocks + c, turns = g / SLOTS, slot = g - turns * SLOTS;
-        if (!mbar_wait(&t_full[slot], turns & 1)) { ok = false; break; }
+        const int g = (j * v_blocks + c) * 2, turns = g / SLOTS, slot = g - turns * SLOTS, slot2 = slot + 1 == SLOTS ? 0 : slot + 1;
+        if (!mbar_wait(&t_full[slot], turns & 1) || !mbar_wait(&t_full[slot2], (slot2 == 0 ? turns + 1 : turns) & 1)) { ok = false; break; }
         tc_fence_after();
+        constexpr int Q = CPW == 1 ? 16 : 8;                      // columns at a time, as registers allow
 #pragma unroll
-        for (int q = 0; q < CW / 16; ++q) {
-          float v[16];
-          tmem_ld16(lanes + slot * CW + q * 16, v);
+        for (int q = 0; q < CW / Q; ++q) {
+          uint64_t v[Q / 2];
+          tmem_ld_sum<Q>(lanes + slot * CW + q * Q, lanes + slot2 * CW + q * Q, v);
 #pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            uint64_t& x = o[c * (CW / 2) + q * 8 + e];
-            x = fma2(x, keep2, mul2(pair(v[2 * e], v[2 * e + 1]), take2));
+          for (int e = 0; e < Q / 2; ++e) {
+            uint64_t& x = o[c * (CW / 2) + q * (Q / 2) + e];
+            x = fma2(x, keep2, mul2(v[e], take2));
           }
         }
         tc_fence_before();
         mbar_arrive_one(&t_empty[slot]);
+        mbar_arrive_one(&t_empty[slot2]);
       }
     }
     bool bad = false;                                             // some entry is not finite (0 times it is none)
@@ -384,23 +408,27 @@ __global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const __grid_co
         const float most = run_max * LN2, sink = a.sinks[h], m = fmaxf(most, sink), f = expf(most - m);
         inv = f / fmaf(run_sum, f, expf(sink - m));
       }
-      if (gate != nullptr && a.gate_heads) inv *= 1.0f / (1.0f + expf(-*gate));
+      if (gate != nullptr && a.gate_heads) inv *= sigmoid(*gate);
       float* dst = a.out + grow * a.ld_out + (int64_t)h * a.dv;
+      auto leave = [&](auto gated) {                              // (apart: what gates take makes the way of those without any longer by fetching it)
 #pragma unroll
-      for (int d = 0; d < CPW * 64; d += 4) {                     // (dv is a multiple of 8)
-        if (d >= a.dv) continue;
-        float x[4];
-        unpair(o[d / 2], x[0], x[1]);
-        unpair(o[d / 2 + 1], x[2], x[3]);
-        odd = fma2(o[d / 2 + 1], 0ull, fma2(o[d / 2], 0ull, odd));
+        for (int d = 0; d < CPW * 64; d += 4) {                   // (dv is a multiple of 8)
+          if (d >= a.dv) continue;
+          float x[4];
+          unpair(o[d / 2], x[0], x[1]);
+          unpair(o[d / 2 + 1], x[2], x[3]);
+          odd = fma2(o[d / 2 + 1], 0ull, fma2(o[d / 2], 0ull, odd));
 #pragma unroll
-        for (int e = 0; e < 4; ++e) x[e] *= inv;
-        if (gate != nullptr && !a.gate_heads) {
-          const float4 z = *reinterpret_cast<const float4*>(gate + d);
-          x[0] *= 1.0f / (1.0f + expf(-z.x)); x[1] *= 1.0f / (1.0f + expf(-z.y)); x[2] *= 1.0f / (1.0f + expf(-z.z)); x[3] *= 1.0f / (1.0f + expf(-z.w));
+          for (int e = 0; e < 4; ++e) x[e] *= inv;
+          if (gated.value) {
+            const float4 z = *reinterpret_cast<const float4*>(gate + d);
+            x[0] *= sigmoid(z.x); x[1] *= sigmoid(z.y); x[2] *= sigmoid(z.z); x[3] *= sigmoid(z.w);
+          }
+          *reinterpret_cast<float4*>(dst + d) = make_float4(x[0], x[1], x[2], x[3]);
         }
-        *reinterpret_cast<float4*>(dst + d) = make_float4(x[0], x[1], x[2], x[3]);
-      }
+      };
+      if (gate != nullptr && !a.gate_heads) leave(std::true_type());
+      else leave(std::false_type());
       float odd0, odd1;
       unpair(odd, odd0, odd1);
       bad = !(odd0 + odd1 == 0.f) || not_finite(inv);

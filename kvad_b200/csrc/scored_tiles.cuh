@@ -41,11 +41,23 @@ __device__ __forceinline__ void umma_ta(uint32_t tmem_d, uint32_t tmem_a, uint64
 __device__ __forceinline__ uint64_t sw128_mn_desc(uint32_t smem_addr) {
   uint64_t d = 0;
   d |= (uint64_t)((smem_addr & 0x3FFFFu) >> 4);
-  d |= (uint64_t)((PAGE_BLOCK >> 4) & 0x3FFFu) << 16;        // leading byte offset: between blocks of 64 columns (one at a time is used)
+  d |= (uint64_t)((PAGE_BLOCK >> 4) & 0x3FFFu) << 16;        // leading byte offset: between blocks of 64 columns (products of 128 step over two)
   d |= (uint64_t)(1024 >> 4) << 32;                          // stride byte offset: between groups of 8 keys
   d |= (uint64_t)1 << 46;
   d |= (uint64_t)2 << 61;                                    // SWIZZLE_128B
   return d;
+}
+
+__device__ __forceinline__ void tmem_ld_issue(uint32_t addr, uint32_t (&r)[16]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]),
+                 "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+               : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void tmem_ld_issue(uint32_t addr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(addr) : "memory");
 }
 
 // Two 32-bit numbers at once (an instruction for both).
@@ -70,12 +82,26 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
+// What two places of N (8 or 16) columns hold, added up, two columns a number.
+template <int N>
+__device__ __forceinline__ void tmem_ld_sum(uint32_t at, uint32_t and_at, uint64_t (&v)[N / 2]) {
+  uint32_t x[N], y[N];
+  tmem_ld_issue(at, x);
+  tmem_ld_issue(and_at, y);
+  tmem_ld_wait();
+#pragma unroll
+  for (int i = 0; i < N / 2; ++i)
+    v[i] = add2(pair(__uint_as_float(x[2 * i]), __uint_as_float(x[2 * i + 1])), pair(__uint_as_float(y[2 * i]), __uint_as_float(y[2 * i + 1])));
+}
 // 2^x by the special-function unit (2 units in the last place; a weight below 2^-126 of its row's largest is zero).
 __device__ __forceinline__ float exp2_fast(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+// 2^x of a whole number x <= 0 (exactly; 0 below -126).  Pages are brought to whole powers of two of one another, so that joining them rounds nothing but the sums: with each
+// page's own largest score as its unit, factors of exp2_fast's errors went into every page's share (2000 keys, values of one sign: 1.4e-7 off, so 1.0e-7).
+__device__ __forceinline__ float exp2_whole(float x) { return __int_as_float((int)(fmaxf(x, -127.f) + 127.f) << 23); }
 // (a full division: the fast one gives 0 for gates below -87.3, where 1 + e^(-z) is beyond 2^126)
 __device__ __forceinline__ float sigmoid(float z) { return 1.0f / (1.0f + expf(-z)); }
 // The upper halves of two floats as a pair of bfloat16 (truncated), and what is left of each.

@@ -143,3 +143,19 @@ def test_a_number_that_is_not_finite_stays_with_the_rows_that_see_it(H, G, dk, d
     ok = want.isfinite()
     assert float((got - want)[ok].abs().max()) < 1e-5      # (scores of up to 2^4 with errors of 2^-21: a weight's of 2^-17)
     assert scored_wide_wait_timeouts() == 0
+
+
+@pytest.mark.parametrize("scale", [0.01, 0.3])
+@pytest.mark.parametrize("H,G,dk,dv,alias", [(4, 2, 64, 64, False), (4, 1, 160, 128, True), (4, 2, 128, 128, False)])
+def test_numbers_of_one_sign(H, G, dk, dv, alias, scale):
+    """Sums to which every term adds, where an accumulator that truncates falls behind: no further off than the CUDA cores' chains of fmaf, from one page to many."""
+    ops, cores = Ops(torch.float32), Ops(torch.float32)
+    cores.scored_wide = False
+    for seqs in ([(0, 17), (3, 70)], [(0, 300)], [(1500, 60)]):
+        c = Case(seqs, H, G, dk, dv, alias=alias, sinks=True)
+        c.q, c.kp, c.scale, c.sinks = c.q.abs(), c.kp.abs(), scale / dk ** 0.5, c.sinks + scale * dk ** 0.5 * 2 / 3.14
+        c.vp = None if alias else c.vp.abs()
+        want = c.want()
+        far, bias = zip(*[(float((x - want).norm() / want.norm()), float(((x - want) / want).mean())) for x in (c.run(ops), c.run(cores))])
+        # 2^-23: exponentials good to 2 units in the last place; a page's sums truncate at their last four steps, 2^-25 of the sum each on the average
+        assert far[0] < max(1.1 * far[1], 2.0 ** -23) and abs(bias[0]) < 2.0 ** -23, (far, bias)
