@@ -47,7 +47,10 @@ struct PromptArgs {
   float scale, softcap, slope_span;
   float cap_in, cap_out;                                          // a capped score: cap_out * tanh(cap_in * (q . k)), in units of log2
   int window, keep_first, chunk;
+  int skip_copy;                                                  // (tests: a block's first page is left out, so that the wait for it runs out)
 };
+
+int g_skip_copy = 0;
 
 // NS: groups of four warps that turn scores into weights; CPW: 64-column pieces of the output that a group of four warps keeps.
 template <int NS, int CPW, bool F32OUT>
@@ -80,9 +83,9 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
   uint64_t* st_full = p_empty + 2;                                // [STATS] a page's statistics are there
   uint64_t* t_full = st_full + STATS;                                 // [3] a piece of P V is in tensor memory
   uint64_t* t_empty = t_full + 3;                                 // [3] it has been read
-  uint64_t* drain = t_empty + 3;                                  // [2] the products that were issued before a wait ran out
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 2);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(t_empty + 3);
   uint32_t* again = tmem_slot + 1;                                // [4] rows with an entry that is not finite, a bit a row
+  volatile uint32_t* failed = again + 4;                          // a wait of the block has run out
   const int hp = a.hp, tok = ROWS / hp, group = a.n_heads / a.n_kv_heads, chunks = group / hp;
   const int per_seq = a.n_kv_heads * chunks, from_end = blockIdx.x / a.columns, column = blockIdx.x - from_end * a.columns;
   const int s = column / per_seq, part = column - s * per_seq, kvh = part / chunks, h0 = kvh * group + (part - kvh * chunks) * hp;
@@ -97,8 +100,8 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
     for (int i = 0; i < 2; ++i) { mbar_init(&s_full[i], 1); mbar_init(&s_empty[i], 128); mbar_init(&p_full[i], 128); mbar_init(&p_empty[i], 1); }
     for (int i = 0; i < STATS; ++i) mbar_init(&st_full[i], 128);
     for (int i = 0; i < 3; ++i) { mbar_init(&t_full[i], 1); mbar_init(&t_empty[i], 128); }
-    for (int i = 0; i < 2; ++i) mbar_init(&drain[i], 1);
     for (int i = 0; i < 4; ++i) again[i] = 0;
+    *failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     fence_async_shared();
   }
@@ -118,6 +121,11 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
     while (t * PAGE <= last_pos && t * PAGE + PAGE <= first_key && t * PAGE >= keep_first) ++t;
     return t;
   };
+  auto wait = [&](uint64_t* bar, uint32_t parity) {
+    if (mbar_wait(bar, parity)) return true;
+    *failed = 1;
+    return false;
+  };
   // after a role's last page: the rows that have to be worked out again, by all warps that have the registers
   auto finish = [&]() {
     asm volatile("bar.sync 1, %0;" ::"n"(FINISHERS * 32) : "memory");
@@ -135,25 +143,22 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
       for (int b = 0; b < k_blocks; ++b) tma_load_3d(q_tile + b * Q_BLOCK, &map_q, q_full, b * 64, h0, start + tok0);
       int j = 0, st = 0;
       uint32_t turn = 0;
-      bool ok = true;
       for (int t_next; t * PAGE <= last_pos; t = t_next, ++j) {
         const int page = page_next;                               // (a page's place is looked up one page ahead)
         t_next = next_page(t + 1);
         if (t_next * PAGE <= last_pos) page_next = pages[t_next];
-        if (j >= stages && !mbar_wait(&kv_empty[st], turn ^ 1)) { ok = false; break; }
+        if (j >= stages && !wait(&kv_empty[st], turn ^ 1)) break;
         uint8_t* at = ring + st * stage_bytes;
-        mbar_expect_tx(&kv_full[st], stage_bytes);
-        const int y = (page * n_kv + kvh) * PAGE;
-        for (int b = 0; b < k_blocks; ++b) tma_load_2d(at + b * PAGE_BLOCK, &map_k, &kv_full[st], b * 64, y);
-        if (!alias) {
-          const int yv = (page * n_v + v_head) * PAGE;
-          for (int b = 0; b < v_blocks; ++b) tma_load_2d(at + k_bytes + b * PAGE_BLOCK, &map_v, &kv_full[st], b * 64, yv);
+        if (!(a.skip_copy && j == 0)) {
+          mbar_expect_tx(&kv_full[st], stage_bytes);
+          const int y = (page * n_kv + kvh) * PAGE;
+          for (int b = 0; b < k_blocks; ++b) tma_load_2d(at + b * PAGE_BLOCK, &map_k, &kv_full[st], b * 64, y);
+          if (!alias) {
+            const int yv = (page * n_v + v_head) * PAGE;
+            for (int b = 0; b < v_blocks; ++b) tma_load_2d(at + k_bytes + b * PAGE_BLOCK, &map_v, &kv_full[st], b * 64, yv);
+          }
         }
         if (++st == stages) { st = 0; turn ^= 1; }
-      }
-      if (!ok) {                                                  // (copies in flight must not outlive the block)
-        mbar_wait(q_full, 0);
-        for (int i = 0; i < min(j, stages); ++i) mbar_wait(&kv_full[i], i < st ? turn : turn ^ 1);
       }
     } else if (warp == 1) {                                       // S = Q K^T (the whole warp, its elected lane issues: see elect_one)
       const int k_steps = (a.dk + 15) / 16;
@@ -161,12 +166,12 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
       const uint64_t q_desc = sw128_desc(smem_u32(q_tile)), k_desc = sw128_desc(smem_u32(ring));
       const uint32_t stage_step = stage_bytes >> 4;               // (descriptors count sixteens of bytes)
       const bool one = elect_one();
-      bool ok = mbar_wait(q_full, 0);
+      bool ok = wait(q_full, 0);
       int j = 0, st = 0;
       uint32_t turn = 0;
       for (int t = next_page(0); t * PAGE <= last_pos && ok; t = next_page(t + 1), ++j) {
         const int b = j & 1;
-        if (!mbar_wait(&kv_full[st], turn) || (j >= 2 && !mbar_wait(S_IS_P ? &p_empty[b] : &s_empty[b], ((j >> 1) & 1) ^ 1))) { ok = false; break; }
+        if (!wait(&kv_full[st], turn) || (j >= 2 && !wait(S_IS_P ? &p_empty[b] : &s_empty[b], ((j >> 1) & 1) ^ 1))) { ok = false; break; }
         tc_fence_after();
         const uint64_t k_at = k_desc + st * stage_step;
         const uint32_t d = tmem_base + TM_S + b * 64;
@@ -185,10 +190,6 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         }
         if (++st == stages) { st = 0; turn ^= 1; }
       }
-      if (!ok) {                                                  // (products in flight must not outlive the block's tensor memory)
-        if (one) umma_commit(&drain[0]);
-        mbar_wait(&drain[0], 0);
-      }
     } else if (warp == 2) {                                       // T = P V, by another warp: a wait takes a hundred cycles even when it is over
       const uint64_t v_desc = sw128_mn_desc(smem_u32(ring) + (a.alias ? 0u : k_bytes));
       const uint32_t stage_step = stage_bytes >> 4;
@@ -199,11 +200,11 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
       uint32_t slot_turn = 0;
       for (int t = next_page(0); t * PAGE <= last_pos && ok; t = next_page(t + 1), ++i) {
         const int b = i & 1;
-        if (!mbar_wait(&p_full[b], (i >> 1) & 1)) { ok = false; break; }
+        if (!wait(&p_full[b], (i >> 1) & 1)) { ok = false; break; }
         const uint32_t p_at = tmem_base + TM_P + b * P_STEP, low_at = tmem_base + (S_IS_P ? TM_S + b * 64 : TM_P + b * P_STEP + 64);
         const uint64_t v_at = v_desc + st * stage_step;
         for (int c = 0; c < n_chunks * PARTS; ++c, ++g) {
-          if (g >= SLOTS && !mbar_wait(&t_empty[slot], slot_turn ^ 1)) { ok = false; break; }
+          if (g >= SLOTS && !wait(&t_empty[slot], slot_turn ^ 1)) { ok = false; break; }
           tc_fence_after();
           // (where two groups of warps share the places: all chunks' small products, then all their h h, so that each meets every turn of its own place)
           const int part = TOGETHER ? c & 1 : (c >= n_chunks ? 1 : 0), chunk = TOGETHER ? c >> 1 : c - part * n_chunks;
@@ -231,10 +232,6 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         }
         if (++st == stages) st = 0;
       }
-      if (!ok) {
-        if (one) umma_commit(&drain[1]);
-        mbar_wait(&drain[1], 0);
-      }
     }
   } else if (warp < 4 + 4 * NS) {
     // ---- scores into weights: a thread a row
@@ -257,7 +254,7 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
     for (; t * PAGE <= last_pos; j += NS) {
       const int b = j & 1, key0 = t * PAGE;
       const uint32_t turn = (j >> 1) & 1;
-      if (!mbar_wait(&s_full[b], turn)) break;
+      if (!wait(&s_full[b], turn)) break;
       tc_fence_after();
       float sc[64];
       {
@@ -276,7 +273,7 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
 #pragma unroll
       for (int c = 0; c < 64; ++c) top[c & 3] = fmaxf(top[c & 3], sc[c]);
       const float most = ceilf(fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3])) * unit), base = most == -INFINITY ? 0.f : most;
-      if (j >= 2 && !mbar_wait(&p_empty[b], turn ^ 1)) break;
+      if (j >= 2 && !wait(&p_empty[b], turn ^ 1)) break;
       tc_fence_after();
       const uint64_t less = pair(-base, -base);
       uint64_t sum2[2] = {0ull, 0ull};
@@ -308,7 +305,7 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
       const int valid = kv_len - key0;
       if (valid < PAGE) {
         const int st = j % stages;
-        if (!mbar_wait(&kv_full[st], (j / stages) & 1)) break;
+        if (!wait(&kv_full[st], (j / stages) & 1)) break;
         uint8_t* v_tile = ring + st * stage_bytes + (a.alias ? 0 : k_bytes);
         for (int vb = 0; vb < v_blocks; ++vb)
           for (int x = row; x < (PAGE - valid) * 8; x += 128) *reinterpret_cast<uint4*>(v_tile + vb * PAGE_BLOCK + valid * 128 + x * 16) = make_uint4(0u, 0u, 0u, 0u);
@@ -340,7 +337,7 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
     bool ok = true;
     int j = 0;
     for (int t = next_page(0); t * PAGE <= last_pos && ok; t = next_page(t + 1), ++j) {
-      if (!mbar_wait(&st_full[j % STATS], (j / STATS) & 1)) { ok = false; break; }
+      if (!wait(&st_full[j % STATS], (j / STATS) & 1)) { ok = false; break; }
       const float2 st = stats[(j % STATS) * ROWS + row];
       const float new_max = fmaxf(run_max, st.x);
       const float keep = run_max == -INFINITY ? 0.f : exp2_whole(run_max - new_max), take = st.x == -INFINITY ? 0.f : exp2_whole(st.x - new_max);
@@ -354,7 +351,7 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
           if (c0 * 64 / CW + c >= n_chunks) continue;
           const int g = TOGETHER ? (j * n_chunks + c) * 2 : (j * PARTS + part) * n_chunks + c0 * 64 / CW + c, turns = g / SLOTS, slot = g - turns * SLOTS;
           const int slot2 = slot + 1 == SLOTS ? 0 : slot + 1;
-          if (!mbar_wait(&t_full[slot], turns & 1) || (TOGETHER && !mbar_wait(&t_full[slot2], (slot2 == 0 ? turns + 1 : turns) & 1))) { ok = false; break; }
+          if (!wait(&t_full[slot], turns & 1) || (TOGETHER && !wait(&t_full[slot2], (slot2 == 0 ? turns + 1 : turns) & 1))) { ok = false; break; }
           tc_fence_after();
 #pragma unroll
           for (int q = 0; q < CW / 16; ++q) {
@@ -459,6 +456,7 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  if (*failed != 0) outlast_what_is_in_flight();
   if (warp == 1) {
     __syncwarp();
     tmem_dealloc(tmem_base, TM_COLS);
@@ -545,6 +543,8 @@ KVAD_EXPORT int kvad_attention_scored_prompt(const void* q, int64_t ld_q, int n_
   while (a.hp < 16 && (n_heads / n_kv_heads) % (a.hp * 2) == 0) a.hp *= 2;
   KVAD_REQUIRE((int64_t)n_seqs * (n_heads / a.hp) < (1ll << 31), "attention (scored, prompts): %d sequences x %d heads are more than one launch takes", n_seqs, n_heads);
   a.columns = n_seqs * (n_heads / a.hp);
+  a.skip_copy = g_skip_copy;
+  g_skip_copy = 0;
   const int item = out_f32 ? 4 : 2;
   a.vec = (reinterpret_cast<uintptr_t>(out) & 15) == 0 && ld_out * item % 16 == 0 &&
           (gate == nullptr || gate_heads || ((reinterpret_cast<uintptr_t>(gate) & 15) == 0 && ld_gate % 8 == 0)) ? 1 : 0;
@@ -577,6 +577,13 @@ KVAD_EXPORT int kvad_attention_scored_prompt_status() {
   cudaError_t e = cudaMemcpyFromSymbol(&n, g_wait_timeouts, sizeof(int));
   if (e != cudaSuccess) KVAD_FAIL(KVAD_ERR_CUDA, "attention_scored_prompt_status: %s", cudaGetErrorString(e));
   return n;
+}
+
+// Tests of the bounded waits: `wait_limit` > 0 sets how many polls a wait makes before it gives up (0: the library's own limit); `skip_copy` leaves the first page out of
+// the NEXT launch's blocks, so that the wait for it runs out.  Synchronises the device.
+KVAD_EXPORT int kvad_attention_scored_prompt_test_hooks(unsigned wait_limit, int skip_copy) {
+  g_skip_copy = skip_copy;
+  return set_wait_limit(wait_limit);
 }
 
 KVAD_DEFINE_LAST_ERROR()

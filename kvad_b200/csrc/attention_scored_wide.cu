@@ -43,7 +43,10 @@ struct WideArgs {
   float scale, softcap, slope_span;
   float cap_in, cap_out;                                          // a capped score: cap_out * tanh(cap_in * (q . k)), in units of log2
   int window, keep_first, chunk;
+  int skip_copy;                                                  // (tests: a block's first page is not said to be there, so that the wait for it runs out)
 };
+
+int g_skip_copy = 0;
 
 // Eight neighbours into three pieces of 16 bytes, `step` bytes apart.  (Of a number that is not finite the last pieces are no number.)
 __device__ __forceinline__ void put8(uint8_t* dst, uint32_t step, const float4& a, const float4& b) {
@@ -82,9 +85,9 @@ __global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const __grid_co
   uint64_t* st_full = p_empty + 2;                                // [STATS] a page's statistics are there
   uint64_t* t_full = st_full + STATS;                             // [3] a piece of P V is in tensor memory
   uint64_t* t_empty = t_full + 3;                                 // [3] it has been read
-  uint64_t* drain = t_empty + 3;                                  // [2] the products that were issued before a wait ran out
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 2);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(t_empty + 3);
   uint32_t* again = tmem_slot + 1;                                // [4] rows with an entry that is not finite, a bit a row
+  volatile uint32_t* failed = again + 4;                          // a wait of the block has run out
   const int hp = a.hp, tok = ROWS / hp, group = a.n_heads / a.n_kv_heads, chunks = group / hp;
   const int per_seq = a.n_kv_heads * chunks, from_end = blockIdx.x / a.columns, column = blockIdx.x - from_end * a.columns;
   const int s = column / per_seq, part = column - s * per_seq, kvh = part / chunks, h0 = kvh * group + (part - kvh * chunks) * hp;
@@ -95,8 +98,8 @@ __global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const __grid_co
     for (int i = 0; i < 2; ++i) { mbar_init(&s_full[i], 1); mbar_init(&s_empty[i], 128); mbar_init(&p_full[i], 128); mbar_init(&p_empty[i], 1); }
     for (int i = 0; i < STATS; ++i) mbar_init(&st_full[i], 128);
     for (int i = 0; i < 3; ++i) { mbar_init(&t_full[i], 1); mbar_init(&t_empty[i], 128); }
-    for (int i = 0; i < 2; ++i) mbar_init(&drain[i], 1);
     for (int i = 0; i < 4; ++i) again[i] = 0;
+    *failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     fence_async_shared();
   }
@@ -132,6 +135,11 @@ __global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const __grid_co
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  auto wait = [&](uint64_t* bar, uint32_t parity) {
+    if (mbar_wait(bar, parity)) return true;
+    *failed = 1;
+    return false;
+  };
   // after a role's last page: the rows that have to be worked out again, by all warps that have the registers
   auto finish = [&]() {
     asm volatile("bar.sync 1, 256;" ::: "memory");
@@ -149,12 +157,12 @@ __global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const __grid_co
       int u = 0, st = 0;                                          // u: blocks of 64 entries so far, each an accumulator of its own (the tensor core truncates where it accumulates)
       uint32_t turn = 0;
       for (int t = next_page(0); t * PAGE <= last_pos && ok; t = next_page(t + 1)) {
-        if (!mbar_wait(&kv_full[st], turn)) { ok = false; break; }
+        if (!wait(&kv_full[st], turn)) { ok = false; break; }
         const uint64_t k_at = k_desc + st * (stage_bytes >> 4);
         int left = k_steps;
         for (int kb = 0; kb < k_blocks; ++kb, ++u, left -= 4) {
           const int b = u & 1;
-          if (u >= 2 && !mbar_wait(&s_empty[b], ((u >> 1) & 1) ^ 1)) { ok = false; break; }
+          if (u >= 2 && !wait(&s_empty[b], ((u >> 1) & 1) ^ 1)) { ok = false; break; }
           tc_fence_after();
           const uint32_t d = tmem_base + TM_S + b * 64;
           if (one) {
@@ -173,10 +181,6 @@ __global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const __grid_co
         }
         if (++st == stages) { st = 0; turn ^= 1; }
       }
-      if (!ok) {                                                  // (products in flight must not outlive the block's tensor memory)
-        if (one) umma_commit(&drain[0]);
-        mbar_wait(&drain[0], 0);
-      }
     } else if (warp == 2) {                                       // T = P V, by another warp
       const uint64_t v_desc = sw128_mn_desc(smem_u32(ring) + v_off);
       const bool one = elect_one();
@@ -186,11 +190,11 @@ __global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const __grid_co
       uint32_t slot_turn = 0;
       for (int t = next_page(0); t * PAGE <= last_pos && ok; t = next_page(t + 1), ++i) {
         const int b = i & 1;
-        if (!mbar_wait(&p_full[b], (i >> 1) & 1)) { ok = false; break; }
+        if (!wait(&p_full[b], (i >> 1) & 1)) { ok = false; break; }
         const uint32_t p_at = tmem_base + TM_P + b * P_STEP;
         const uint64_t v_at = v_desc + st * (stage_bytes >> 4);
         for (int c = 0; c < 2 * v_blocks; ++c, ++g) {             // 64 columns' small products, then their h h: apart, so that nothing truncates what is small once it is large
-          if (g >= SLOTS && !mbar_wait(&t_empty[slot], slot_turn ^ 1)) { ok = false; break; }
+          if (g >= SLOTS && !wait(&t_empty[slot], slot_turn ^ 1)) { ok = false; break; }
           tc_fence_after();
           const uint32_t idesc = umma_instr_desc(ROWS, min(CW, (dv - (c >> 1) * CW + 15) & ~15), false, true), d = tmem_base + TM_T + slot * CW;
           const uint64_t vd = v_at + (c >> 1) * (PAGE_BLOCK >> 4);
@@ -214,10 +218,6 @@ __global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const __grid_co
           umma_commit(&kv_empty[st]);
         }
         if (++st == stages) st = 0;
-      }
-      if (!ok) {
-        if (one) umma_commit(&drain[1]);
-        mbar_wait(&drain[1], 0);
       }
     }
   } else if (warp < 12) {
@@ -256,13 +256,13 @@ __global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const __grid_co
     if (mine == 1) t = next_page(t + 1);
     for (; mine < takers && t * PAGE <= last_pos && ok; j += takers) {
       const int page = pages[t], st = j % stages, n_live = min(PAGE, last_pos + 1 - t * PAGE);
-      if (j >= stages && !mbar_wait(&kv_empty[st], ((j / stages) & 1) ^ 1)) { ok = false; break; }
+      if (j >= stages && !wait(&kv_empty[st], ((j / stages) & 1) ^ 1)) { ok = false; break; }
       uint8_t* at = ring + st * stage_bytes;
       bring(at, k_piece, a.k_pages + (int64_t)page * k_step + (int64_t)kvh * PAGE * a.dk, a.dk, k_eights, n_live);
       if (v_eights > 0) bring(at + v_off, v_piece, a.v_pages + (int64_t)page * v_step + (int64_t)(kvh / a.key_maps) * PAGE * a.dv, a.dv, v_eights, n_live);
       fence_async_shared();
       __syncwarp();
-      if (lane == 0) mbar_arrive_one(&kv_full[st]);
+      if (lane == 0 && !(a.skip_copy && j == 0)) mbar_arrive_one(&kv_full[st]);
       t = next_page(t + 1);
       if (takers == 2) t = next_page(t + 1);
     }
@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const __grid_co
       float sc[64];
       bool come = true;
       for (int kb = 0; kb < k_blocks; ++kb, ++u) {
-        if (!mbar_wait(&s_full[u & 1], (u >> 1) & 1)) { come = false; break; }
+        if (!wait(&s_full[u & 1], (u >> 1) & 1)) { come = false; break; }
         tc_fence_after();
         if (kb == 0) {
           uint32_t* raw = reinterpret_cast<uint32_t*>(sc);
@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const __grid_co
 #pragma unroll
       for (int c = 0; c < 64; ++c) top[c & 3] = fmaxf(top[c & 3], sc[c]);
       const float most = ceilf(fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3])) * unit), base = most == -INFINITY ? 0.f : most;
-      if (j >= 2 && !mbar_wait(&p_empty[b], turn ^ 1)) break;
+      if (j >= 2 && !wait(&p_empty[b], turn ^ 1)) break;
       tc_fence_after();
       const uint64_t less = pair(-base, -base);
       uint64_t sum2[2] = {0ull, 0ull};
@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const __grid_co
     bool ok = true;
     int j = 0;
     for (int t = next_page(0); t * PAGE <= last_pos && ok; t = next_page(t + 1), ++j) {
-      if (!mbar_wait(&st_full[j % STATS], (j / STATS) & 1)) { ok = false; break; }
+      if (!wait(&st_full[j % STATS], (j / STATS) & 1)) { ok = false; break; }
       const float2 st = stats[(j % STATS) * ROWS + row];
       const float new_max = fmaxf(run_max, st.x);
       const float keep = run_max == -INFINITY ? 0.f : exp2_whole(run_max - new_max), take = st.x == -INFINITY ? 0.f : exp2_whole(st.x - new_max);
@@ -380,7 +380,7 @@ __global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const __grid_co
       for (int c = 0; c < CPW; ++c) {
         if (c >= v_blocks) continue;
         const int g = (j * v_blocks + c) * 2, turns = g / SLOTS, slot = g - turns * SLOTS, slot2 = slot + 1 == SLOTS ? 0 : slot + 1;
-        if (!mbar_wait(&t_full[slot], turns & 1) || !mbar_wait(&t_full[slot2], (slot2 == 0 ? turns + 1 : turns) & 1)) { ok = false; break; }
+        if (!wait(&t_full[slot], turns & 1) || !wait(&t_full[slot2], (slot2 == 0 ? turns + 1 : turns) & 1)) { ok = false; break; }
         tc_fence_after();
         constexpr int Q = CPW == 1 ? 16 : 8;                      // columns at a time, as registers allow
 #pragma unroll
@@ -439,6 +439,7 @@ __global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const __grid_co
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  if (*failed != 0) outlast_what_is_in_flight();
   if (warp == 1) {
     __syncwarp();
     tmem_dealloc(tmem_base, TM_COLS);
@@ -507,6 +508,8 @@ KVAD_EXPORT int kvad_attention_scored_wide(const float* q, int64_t ld_q, float* 
   while (a.hp < 16 && (n_heads / n_kv_heads) % (a.hp * 2) == 0) a.hp *= 2;
   KVAD_REQUIRE((int64_t)n_seqs * (n_heads / a.hp) < (1ll << 31), "attention (scored, 32-bit prompts): %d sequences x %d heads are more than one launch takes", n_seqs, n_heads);
   a.columns = n_seqs * (n_heads / a.hp);
+  a.skip_copy = g_skip_copy;
+  g_skip_copy = 0;
   const Layout z = layout_of(dk, dv, alias);
   a.stages = z.stages;
   return dv <= 64 ? launch<1>(a, max_new, z.smem, stream) : launch<2>(a, max_new, z.smem, stream);
@@ -518,6 +521,13 @@ KVAD_EXPORT int kvad_attention_scored_wide_status() {
   cudaError_t e = cudaMemcpyFromSymbol(&n, g_wait_timeouts, sizeof(int));
   if (e != cudaSuccess) KVAD_FAIL(KVAD_ERR_CUDA, "attention_scored_wide_status: %s", cudaGetErrorString(e));
   return n;
+}
+
+// Tests of the bounded waits: `wait_limit` > 0 sets how many polls a wait makes before it gives up (0: the library's own limit); `skip_copy` leaves the first page out of
+// the NEXT launch's blocks, so that the wait for it runs out.  Synchronises the device.
+KVAD_EXPORT int kvad_attention_scored_wide_test_hooks(unsigned wait_limit, int skip_copy) {
+  g_skip_copy = skip_copy;
+  return set_wait_limit(wait_limit);
 }
 
 KVAD_DEFINE_LAST_ERROR()

@@ -34,7 +34,10 @@ struct PieceArgs {
   const void* bias; int bias_f32;
   float* out; int64_t ldo;
   int M, N, K, vec_out;
+  int skip_copy;                                // (tests: the first copy is left out, so that the wait for it runs out)
 };
+
+int g_skip_copy = 0;
 
 // The upper halves of two floats as a pair of bfloat16 (truncated), and what is left of each.
 __device__ __forceinline__ uint32_t cut(float& a, float& b) {
@@ -132,9 +135,11 @@ __global__ void __launch_bounds__(THREADS, 1) linear_pieces_kernel(const uint8_t
   uint64_t* ready = reinterpret_cast<uint64_t*>(smem + RING * T::STAGE);           // [RING]
   uint64_t* done = ready + RING;                                                    // [RING]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + RING);
+  volatile uint32_t* failed = tmem_slot + 1;                                        // a wait of the block has run out
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   pdl_launch_dependents();
   if (threadIdx.x == 0) {
+    *failed = 0;
     for (int s = 0; s < RING; ++s) { mbar_init(&ready[s], 1 + 4 + 8); mbar_init(&done[s], 1); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -148,6 +153,11 @@ __global__ void __launch_bounds__(THREADS, 1) linear_pieces_kernel(const uint8_t
   const int mine = (int)blockIdx.x < tiles ? (tiles - (int)blockIdx.x - 1) / (int)gridDim.x + 1 : 0, blocks = mine * num_kb;      // of this CTA
   pdl_wait();
 
+  auto wait = [&](uint64_t* bar, uint32_t parity) {
+    if (mbar_wait(bar, parity)) return true;
+    *failed = 1;
+    return false;
+  };
   if (warp < 4) {
     regs_fewer<32>();
     if (warp == 0 && lane == 0) {
@@ -157,14 +167,14 @@ __global__ void __launch_bounds__(THREADS, 1) linear_pieces_kernel(const uint8_t
       for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
         const uint8_t* w_at = w_pieces + (int64_t)(t % tiles_n) * num_kb * T::STAGE;
         for (int kb = 0; kb < num_kb; ++kb, ++j, w_at += T::STAGE) {
-          if (j >= RING && !mbar_wait(&done[s], turn ^ 1)) { ok = false; break; }
-          mbar_expect_tx(&ready[s], T::STAGE);
-          bulk_load(smem + s * T::STAGE, w_at, T::STAGE, &ready[s]);
+          if (j >= RING && !wait(&done[s], turn ^ 1)) { ok = false; break; }
+          if (!(p.skip_copy && j == 0)) {
+            mbar_expect_tx(&ready[s], T::STAGE);
+            bulk_load(smem + s * T::STAGE, w_at, T::STAGE, &ready[s]);
+          }
           if (++s == RING) { s = 0; turn ^= 1; }
         }
       }
-      if (!ok)                                  // (copies in flight must not outlive the block)
-        for (int i = 0; i < min(j, RING); ++i) mbar_wait(&ready[i], i < s ? turn : turn ^ 1);
     } else if (warp == 1) {
       constexpr uint32_t idesc = umma_instr_desc(BM, BN);
       const uint64_t w0 = sw64_desc(smem_u32(smem));
@@ -172,10 +182,7 @@ __global__ void __launch_bounds__(THREADS, 1) linear_pieces_kernel(const uint8_t
       int s = 0, acc = 0;
       uint32_t turn = 0;
       for (int j = 0; j < blocks; ++j) {
-        if (!mbar_wait(&ready[s], turn)) {
-          if (j > 0) mbar_wait(&done[(j - 1) % RING], ((j - 1) / RING) & 1);      // (products in flight must not outlive the block's tensor memory)
-          break;
-        }
+        if (!wait(&ready[s], turn)) break;
         tc_fence_after();
         const uint64_t w = w0 + (uint32_t)s * (T::STAGE >> 4);
         const uint32_t d = tmem_base + (uint32_t)(acc * BN), a = tmem_a + (uint32_t)(s * A_COLS);
@@ -217,7 +224,7 @@ __global__ void __launch_bounds__(THREADS, 1) linear_pieces_kernel(const uint8_t
     fetch();
     for (int j = group; j < blocks; j += 2) {
       const int ring = j % RING;
-      if (j >= RING && !mbar_wait(&done[ring], ((j / RING) & 1) ^ 1)) break;
+      if (j >= RING && !wait(&done[ring], ((j / RING) & 1) ^ 1)) break;
       tc_fence_after();
 #pragma unroll
       for (int pair = 0; pair < 2; ++pair) {    // 16 rows: i = 2 pair and 2 pair + 1
@@ -259,7 +266,7 @@ __global__ void __launch_bounds__(THREADS, 1) linear_pieces_kernel(const uint8_t
 #pragma unroll
       for (int i = 0; i < SHARE; ++i) sum[i] = 0.f;
       for (int kb = 0; kb < num_kb; ++kb, ++j) {
-        if (!mbar_wait(&done[j % RING], (j / RING) & 1)) { ok = false; break; }
+        if (!wait(&done[j % RING], (j / RING) & 1)) { ok = false; break; }
         tc_fence_after();
         {
           uint32_t v[32];
@@ -313,6 +320,7 @@ __global__ void __launch_bounds__(THREADS, 1) linear_pieces_kernel(const uint8_t
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  if (*failed != 0) outlast_what_is_in_flight();
   if (warp == 1) {
     __syncwarp();
     tmem_dealloc(tmem_base, 512);
@@ -370,6 +378,8 @@ KVAD_EXPORT int kvad_linear_pieces(const float* A, int64_t lda, const float* W, 
   KVAD_REQUIRE(work != nullptr, "linear_pieces: needs scratch");
   PieceArgs a;
   a.A = A; a.lda = lda; a.W = W; a.bias = bias; a.bias_f32 = bias_f32; a.out = out; a.ldo = ldo; a.M = M; a.N = N; a.K = K;
+  a.skip_copy = g_skip_copy;
+  g_skip_copy = 0;
   a.vec_out = (ldo % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0) ? 1 : 0;
   int bn = force_bn;
   if (bn == 0) {        // waves of one tile an SM times a block's products (half a cycle a column each; a narrow tile's cutting takes longer than its products)
@@ -398,6 +408,13 @@ KVAD_EXPORT int kvad_linear_pieces_status() {
   cudaError_t e = cudaMemcpyFromSymbol(&n, g_wait_timeouts, sizeof(int));
   if (e != cudaSuccess) KVAD_FAIL(KVAD_ERR_CUDA, "linear_pieces_status: %s", cudaGetErrorString(e));
   return n;
+}
+
+// Tests of the bounded waits: `wait_limit` > 0 sets how many polls a wait makes before it gives up (0: the library's own limit); `skip_copy` leaves the first copy out of
+// the NEXT launch's blocks, so that the wait for it runs out.  Synchronises the device.
+KVAD_EXPORT int kvad_linear_pieces_test_hooks(unsigned wait_limit, int skip_copy) {
+  g_skip_copy = skip_copy;
+  return set_wait_limit(wait_limit);
 }
 
 KVAD_DEFINE_LAST_ERROR()

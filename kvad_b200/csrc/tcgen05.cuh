@@ -47,6 +47,15 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
   return false;
 }
 
+// Where a wait has run out, copies and products that some role has issued may still be in flight when the block gives its memory back: the block then stays for 10 ms, which
+// nothing in flight takes.  (To wait for each of them at the end of its role, always, took 1.7 us of 24 from the attention kernels, whose other warps it holds up.)
+__device__ __forceinline__ void outlast_what_is_in_flight() {
+  uint64_t begun, now;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(begun));
+  do asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+  while (now - begun < 10000000ull);
+}
+
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
@@ -138,6 +147,12 @@ __device__ __forceinline__ void tmem_ld16(uint32_t addr, float* v) {
 __host__ __device__ constexpr uint32_t umma_instr_desc(int m, int n, bool a_mn_major = false, bool b_mn_major = false) {
   return (1u << 4) | (1u << 7) | (1u << 10) | (a_mn_major ? (1u << 15) : 0u) | (b_mn_major ? (1u << 16) : 0u) |
          ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
+}
+
+// Tests of the bounded waits: how many polls a wait makes before it gives up (0: the library's own limit).  0, or a CUDA error code.
+static inline int set_wait_limit(unsigned polls) {
+  const uint32_t limit = polls > 0 ? polls : WAIT_LIMIT;
+  return (int)cudaMemcpyToSymbol(g_wait_limit, &limit, sizeof(limit));
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,

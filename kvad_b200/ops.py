@@ -12,7 +12,7 @@ from __future__ import annotations
 import ctypes
 import functools
 import os
-from ctypes import c_float, c_int, c_int64, c_void_p
+from ctypes import c_float, c_int, c_int64, c_uint, c_void_p
 from typing import Optional
 
 import torch
@@ -59,6 +59,7 @@ _SIGNATURES = {
     "linear_pieces": {
         "kvad_linear_pieces": [c_void_p, c_int64, c_void_p, c_void_p, c_int, c_void_p, c_int64, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int64, c_void_p],
         "kvad_linear_pieces_status": [],
+        "kvad_linear_pieces_test_hooks": [c_uint, c_int],
     },
     "linear_tcgen05": {
         "kvad_linear_tcgen05": [c_void_p, c_int64, c_void_p, c_void_p, c_int, c_void_p, c_int64, c_int, c_int, c_int,
@@ -136,6 +137,7 @@ _SIGNATURES = {
                                          c_int, c_int, c_int, c_void_p],
         "kvad_attention_scored_prompt_takes": [c_int, c_int, c_int, c_int],
         "kvad_attention_scored_prompt_status": [],
+        "kvad_attention_scored_prompt_test_hooks": [c_uint, c_int],
     },
     "attention_scored_wide": {
         "kvad_attention_scored_wide": [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
@@ -143,6 +145,7 @@ _SIGNATURES = {
                                        c_int, c_int, c_void_p],
         "kvad_attention_scored_wide_takes": [c_int, c_int, c_int],
         "kvad_attention_scored_wide_status": [],
+        "kvad_attention_scored_wide_test_hooks": [c_uint, c_int],
     },
     "retention": {
         "kvad_retention": [c_int, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64,
@@ -1915,6 +1918,14 @@ def scored_prompt_wait_timeouts() -> int:
     if n < 0:
         raise KernelError(h.kvad_last_error().decode("utf-8", "replace"))
     return n
+
+
+def wait_test_hooks(library: str, wait_limit: int = 0, skip_copy: bool = False) -> None:
+    """Tests of the bounded waits of "linear_pieces", "attention_scored_prompt" and "attention_scored_wide": `wait_limit` polls before a wait gives up
+    (0: the library's own limit), and a copy that the next launch's blocks leave out."""
+    h = lib(library)
+    if getattr(h, f"kvad_{library}_test_hooks")(int(wait_limit), int(bool(skip_copy))) != 0:
+        raise KernelError(f"{library}: the wait limit cannot be set")
 
 
 def moe_wait_timeouts() -> int:
