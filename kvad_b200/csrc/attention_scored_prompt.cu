@@ -52,8 +52,9 @@ struct PromptArgs {
 
 int g_skip_copy = 0;
 
-// NS: groups of four warps that turn scores into weights; CPW: 64-column pieces of the output that a group of four warps keeps.
-template <int NS, int CPW, bool F32OUT>
+// NS: groups of four warps that turn scores into weights; CPW: 64-column pieces of the output that a group of four warps keeps.  IN_TURN: there is room for a page's keys or
+// its values only, which come into the same place one after the other.
+template <int NS, int CPW, bool F32OUT, bool IN_TURN>
 __global__ void __launch_bounds__(THREADS, 1)
 scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const __grid_constant__ PromptArgs a) {
   // Tensor-memory columns: the places of P V, S of two pages (64 each), the weights' pieces of two pages (32 columns each: two bfloat16 a column).  With values
@@ -69,12 +70,13 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const int k_blocks = (a.dk + 63) / 64, v_blocks = (a.dv + 63) / 64, n_chunks = (a.dv + CW - 1) / CW, stages = a.stages;
-  const uint32_t k_bytes = k_blocks * PAGE_BLOCK, stage_bytes = k_bytes + (a.alias ? 0 : v_blocks * PAGE_BLOCK);
+  const uint32_t k_bytes = k_blocks * PAGE_BLOCK, v_bytes = a.alias ? 0 : v_blocks * PAGE_BLOCK, v_off = a.alias || IN_TURN ? 0 : k_bytes;
+  const uint32_t stage_bytes = IN_TURN ? max(k_bytes, v_bytes) : k_bytes + v_bytes;
   uint8_t* q_tile = smem;
   uint8_t* ring = smem + k_blocks * Q_BLOCK;                      // stage: keys, then values (or none: the keys)
   float2* stats = reinterpret_cast<float2*>(ring + stages * stage_bytes);      // [STATS][ROWS] a page's largest score and sum of weights, per row
   uint64_t* q_full = reinterpret_cast<uint64_t*>(stats + STATS * ROWS);
-  uint64_t* kv_full = q_full + 1;                                 // [stages] a page has come
+  uint64_t* kv_full = q_full + 1;                                 // [stages] a page has come (in turn: its keys, and [1] its values)
   uint64_t* kv_empty = kv_full + MAX_STAGES;                      // [stages] it has been used up
   uint64_t* s_full = kv_empty + MAX_STAGES;                       // [2] S is in tensor memory
   uint64_t* s_empty = s_full + 2;                                 // [2] S has been read
@@ -150,12 +152,17 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         if (j >= stages && !wait(&kv_empty[st], turn ^ 1)) break;
         uint8_t* at = ring + st * stage_bytes;
         if (!(a.skip_copy && j == 0)) {
-          mbar_expect_tx(&kv_full[st], stage_bytes);
+          mbar_expect_tx(&kv_full[st], IN_TURN ? k_bytes : stage_bytes);
           const int y = (page * n_kv + kvh) * PAGE;
           for (int b = 0; b < k_blocks; ++b) tma_load_2d(at + b * PAGE_BLOCK, &map_k, &kv_full[st], b * 64, y);
           if (!alias) {
+            uint64_t* come = IN_TURN ? &kv_full[1] : &kv_full[st];
+            if (IN_TURN) {
+              if (!wait(&s_full[j & 1], (j >> 1) & 1)) break;     // (the keys have been read)
+              mbar_expect_tx(come, v_bytes);
+            }
             const int yv = (page * n_v + v_head) * PAGE;
-            for (int b = 0; b < v_blocks; ++b) tma_load_2d(at + k_bytes + b * PAGE_BLOCK, &map_v, &kv_full[st], b * 64, yv);
+            for (int b = 0; b < v_blocks; ++b) tma_load_2d(at + v_off + b * PAGE_BLOCK, &map_v, come, b * 64, yv);
           }
         }
         if (++st == stages) { st = 0; turn ^= 1; }
@@ -191,7 +198,7 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
         if (++st == stages) { st = 0; turn ^= 1; }
       }
     } else if (warp == 2) {                                       // T = P V, by another warp: a wait takes a hundred cycles even when it is over
-      const uint64_t v_desc = sw128_mn_desc(smem_u32(ring) + (a.alias ? 0u : k_bytes));
+      const uint64_t v_desc = sw128_mn_desc(smem_u32(ring) + v_off);
       const uint32_t stage_step = stage_bytes >> 4;
       const bool one = elect_one();
       const int dv = a.dv;
@@ -200,7 +207,7 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
       uint32_t slot_turn = 0;
       for (int t = next_page(0); t * PAGE <= last_pos && ok; t = next_page(t + 1), ++i) {
         const int b = i & 1;
-        if (!wait(&p_full[b], (i >> 1) & 1)) { ok = false; break; }
+        if (!wait(&p_full[b], (i >> 1) & 1) || (IN_TURN && !wait(&kv_full[1], i & 1))) { ok = false; break; }
         const uint32_t p_at = tmem_base + TM_P + b * P_STEP, low_at = tmem_base + (S_IS_P ? TM_S + b * 64 : TM_P + b * P_STEP + 64);
         const uint64_t v_at = v_desc + st * stage_step;
         for (int c = 0; c < n_chunks * PARTS; ++c, ++g) {
@@ -305,8 +312,8 @@ scored_prompt_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
       const int valid = kv_len - key0;
       if (valid < PAGE) {
         const int st = j % stages;
-        if (!wait(&kv_full[st], (j / stages) & 1)) break;
-        uint8_t* v_tile = ring + st * stage_bytes + (a.alias ? 0 : k_bytes);
+        if (IN_TURN ? !wait(&kv_full[1], j & 1) : !wait(&kv_full[st], (j / stages) & 1)) break;
+        uint8_t* v_tile = ring + st * stage_bytes + v_off;
         for (int vb = 0; vb < v_blocks; ++vb)
           for (int x = row; x < (PAGE - valid) * 8; x += 128) *reinterpret_cast<uint4*>(v_tile + vb * PAGE_BLOCK + valid * 128 + x * 16) = make_uint4(0u, 0u, 0u, 0u);
         fence_async_shared();
@@ -473,29 +480,35 @@ int make_map(CUtensorMap* map, const void* at, int rank, const cuuint64_t* dims,
   return KVAD_OK;
 }
 
-template <int NS, int CPW, bool F32OUT>
+template <int NS, int CPW, bool F32OUT, bool IN_TURN>
 int launch(const CUtensorMap& q, const CUtensorMap& k, const CUtensorMap& v, const PromptArgs& a, int max_new, size_t smem, cudaStream_t stream) {
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(scored_prompt_kernel<NS, CPW, F32OUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MOST);
+    cudaError_t e = cudaFuncSetAttribute(scored_prompt_kernel<NS, CPW, F32OUT, IN_TURN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MOST);
     if (e != cudaSuccess) KVAD_FAIL(KVAD_ERR_CUDA, "attention (scored, prompts): cannot reserve %zu bytes of shared memory: %s", SMEM_MOST, cudaGetErrorString(e));
     configured = true;
   }
   const int tok = ROWS / a.hp;
   const int64_t tiles = (int64_t)a.columns * ((max_new + tok - 1) / tok);
   KVAD_REQUIRE(tiles < (1ll << 31), "attention (scored, prompts): %lld tiles are more than one launch takes", (long long)tiles);
-  kvad_launch(scored_prompt_kernel<NS, CPW, F32OUT>, dim3((unsigned)tiles), dim3(THREADS), smem, stream, q, k, v, a);
+  kvad_launch(scored_prompt_kernel<NS, CPW, F32OUT, IN_TURN>, dim3((unsigned)tiles), dim3(THREADS), smem, stream, q, k, v, a);
   KVAD_CHECK_LAUNCH("attention_scored_prompt");
   return KVAD_OK;
 }
 
-struct Layout { int stages; size_t smem; };
-// As many pages on their way as fit (three keep all roles busy; one, for the longest keys, gives the same sums page by page).
+struct Layout { int stages, in_turn; size_t smem; };
+// As many pages on their way as fit (three keep all roles busy; one, for the longest keys, gives the same sums page by page; of keys above 512 entries, and above 448 with
+// values above 192, a page's keys and values come in turn).
 Layout layout_of(int dk, int dv, bool alias) {
   const size_t kb = (dk + 63) / 64, vb = alias ? 0 : (dv + 63) / 64, fixed = kb * Q_BLOCK + SMEM_REST, stage = (kb + vb) * PAGE_BLOCK;
   Layout z;
   z.stages = fixed >= SMEM_MOST ? 0 : (int)std::min<size_t>(MAX_STAGES, (SMEM_MOST - fixed) / stage);
+  z.in_turn = 0;
   z.smem = fixed + z.stages * stage;
+  if (z.stages == 0 && !alias && fixed + std::max(kb, vb) * PAGE_BLOCK <= SMEM_MOST) {
+    z.stages = z.in_turn = 1;
+    z.smem = fixed + std::max(kb, vb) * PAGE_BLOCK;
+  }
   return z;
 }
 
@@ -560,10 +573,12 @@ KVAD_EXPORT int kvad_attention_scored_prompt(const void* q, int64_t ld_q, int n_
   if (rc != KVAD_OK) return rc;
   mv = mk;
   if (!alias && (rc = make_map(&mv, v_pages, 2, v_dims, v_strides, page_box)) != KVAD_OK) return rc;
-#define KVAD_TC(NS, CPW)                                                                        \
-  do {                                                                                          \
-    if (out_f32) return launch<NS, CPW, true>(mq, mk, mv, a, max_new, z.smem, stream);          \
-    return launch<NS, CPW, false>(mq, mk, mv, a, max_new, z.smem, stream);                      \
+#define KVAD_TC(NS, CPW)                                                                                                      \
+  do {                                                                                                                        \
+    if (z.in_turn && out_f32) return launch<NS, CPW, true, true>(mq, mk, mv, a, max_new, z.smem, stream);                     \
+    if (z.in_turn) return launch<NS, CPW, false, true>(mq, mk, mv, a, max_new, z.smem, stream);                               \
+    if (out_f32) return launch<NS, CPW, true, false>(mq, mk, mv, a, max_new, z.smem, stream);                                 \
+    return launch<NS, CPW, false, false>(mq, mk, mv, a, max_new, z.smem, stream);                                             \
   } while (0)
   if (dv <= 64) KVAD_TC(2, 1);
   if (dv <= 128) KVAD_TC(2, 2);

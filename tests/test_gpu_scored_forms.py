@@ -375,3 +375,14 @@ def test_gates_far_below_zero(H, G, dk, dv, gate):
     got, want, slack = c.run(Ops(torch.bfloat16)), c.want * change, c.slack * change
     assert ((got - want).abs() <= slack + 2.0 ** -8 * want.abs() + 1e-30).all()
     assert float(want.abs().max()) > 1e-9
+
+
+@pytest.mark.parametrize("H,G,dk,dv,form", [(8, 2, 520, 64, {}), (4, 1, 528, 8, dict(cap=3.0, sinks=True)), (2, 2, 576, 256, dict(window=70, keep=65)), (4, 2, 512, 256, dict(gate="entry")),
+                                            (4, 1, 528, 72, dict(chunk=96))])
+def test_keys_so_long_that_keys_and_values_of_a_page_come_in_turn(H, G, dk, dv, form):
+    from kvad_b200.ops import scored_prompt_wait_timeouts
+    assert lib("attention_scored_prompt").kvad_attention_scored_prompt_takes(dk, dv, 0, 0) == 1
+    c = Case([(0, 128), (64, 64), (449, 31), (3, 2), (0, 1)], H, G, dk, dv, **form)
+    for out in [torch.bfloat16] if c.gate is not None else [torch.bfloat16, torch.float32]:
+        c.check(c.run(Ops(torch.bfloat16), out), out)
+    assert scored_prompt_wait_timeouts() == 0
