@@ -410,7 +410,7 @@ class Ops:
         the key under which a step's CUDA graph is kept."""
         return (_switch_epoch, self.tensor_core_linear, self.tensor_core_prefill, self.fast_decode,
                 self.rows_linear_max, self.qkv_sums, self.SUMS_MIN_K, self.tiled_prompt, self.split_linear, self.pieces_linear, self.scored_prompt, self.scored_wide, self.chunked_recurrences,
-                self.SPLIT_MIN_ROWS, self.PIECES_MIN_ROWS, self.PIECES_MIN_K, self.PIECES_WORK_BYTES, self.SCORED_PROMPT_MIN_NEW, self.CHUNK_MIN_ROWS, self.CHUNK_SHORT_ROWS, self.CHUNK_WORK_BYTES,
+                self.SPLIT_MIN_ROWS, self.PIECES_MIN_ROWS, self.PIECES_MIN_K, self.PIECES_ONE_TILE, self.PIECES_WORK_BYTES, self.SCORED_PROMPT_MIN_NEW, self.CHUNK_MIN_ROWS, self.CHUNK_SHORT_ROWS, self.CHUNK_WORK_BYTES,
                 self.ROWS_LINEAR_MAX_OUT, self.ROWS_BLOCKS_MAX, self.HEADS_LINEAR_MAX_ROWS)
 
     def begin_step(self) -> None:
@@ -474,7 +474,11 @@ class Ops:
     # The same with the weights cut by a pass of their own (linear_pieces.cu), where K is long enough to pay for the pass.  (us of that and of linear_split.cu: 70 rows of
     # 128 x 128: 7.2, 6.5; 256 x 256: 9.0, 9.6; 512 x 512: 12.6, 15.8; 768 x 3072: 55, 78; 1510 rows of 768 x 2304: 36, 61; 768 x 768: 23, 26; 768 x 3072: 55, 68; 3072 x 768: 53, 80.)
     PIECES_MIN_ROWS, PIECES_MIN_K = 65, 256
-    PIECES_WORK_BYTES = 1 << 29      # scratch of a product, at most (a head of 50257 x 1600: 482 MB)
+    # One tile of rows (128) reads every piece once: many outputs then cost more to cut than the tiles gain.  (us of that and of linear_split.cu, 65 rows: 50257 x 768: 138, 104; 50257 x 1600: 275, 197;
+    # 12288 x 768: 34, 29; 8192 x 1600: 54, 44; 6400 x 1600: 47, 44; 4800 x 1600: 40, 44; 4800 x 4096: 109, 103; 4096 x 4096: 112, 103; 3072 x 4096: 96, 103.  Two tiles, 129 rows: 50257 x 768:
+    # 209, 205; 12288 x 4096: 213, 297; 512 rows of 50257 x 768: 351, 450.)
+    PIECES_ONE_TILE = (128, 3072, 4800, 8 << 20)      # rows; outputs always, outputs at most and weights of those
+    PIECES_WORK_BYTES = 1 << 29      # scratch of a product, at most: 6 bytes an entry of the weights while the call runs (a head of 50257 x 1600: 482 MB)
     ROWS_BLOCKS_MAX = 64           # 32-bit: up to so many rows go through the weight-streaming form in blocks of 16
 
     def linear(self, a, weight, bias, out, epilogue: str = "store", *, tile: int = 0, splits: int = 0,
@@ -524,9 +528,16 @@ class Ops:
         if (form == "auto" and self.split_linear and m >= self.SPLIT_MIN_ROWS and k % 4 == 0 and lda % 4 == 0 and a.data_ptr() % 16 == 0
                 and weight.data_ptr() % 16 == 0):
             need = 192 * (n + 191) * ((k + 31) // 32)          # (three pieces of the weights, rows up to a tile's end, K to a block's)
-            if self.pieces_linear and m >= self.PIECES_MIN_ROWS and k >= self.PIECES_MIN_K and need <= self.PIECES_WORK_BYTES:
+            rows, always, most, weights = self.PIECES_ONE_TILE
+            work = None
+            if (self.pieces_linear and m >= self.PIECES_MIN_ROWS and k >= self.PIECES_MIN_K and need <= self.PIECES_WORK_BYTES
+                    and (m > rows or n <= always or (n <= most and n * k <= weights))):
+                try:
+                    work = torch.empty(need, dtype=torch.uint8, device=a.device)
+                except torch.cuda.OutOfMemoryError:
+                    pass                    # linear_split needs no scratch and gives the same bits
+            if work is not None:
                 h = lib("linear_pieces")
-                work = torch.empty(need, dtype=torch.uint8, device=a.device)
                 width = int(tile) if tile in (64, 128, 192) else 0
                 _check(h.kvad_linear_pieces(_ptr(a), lda, _ptr(weight), _ptr(bias), bias_f32, _ptr(out), ldo, m, n, k, epi, width, _ptr(work), need, _stream()), h)
                 global _launches

@@ -125,3 +125,47 @@ def test_product_of_cut_weights_has_the_split_products_bits(m, n, k, tile):
             outs.append(out[:, :n].clone())
         assert torch.equal(outs[0].nan_to_num(7.0), outs[1].nan_to_num(7.0)) and torch.equal(outs[0].isnan(), outs[1].isnan())
     assert linear_pieces_wait_timeouts() == 0
+
+
+def roads(monkeypatch, call):
+    """Which of the two libraries the products of `call` went to."""
+    import kvad_b200.ops as module
+    seen, real = [], module.lib
+    monkeypatch.setattr(module, "lib", lambda name: (seen.append(name), real(name))[1])
+    call()
+    return [x for x in seen if x in ("linear_split", "linear_pieces")]
+
+
+@pytest.mark.parametrize("m,n,k,road", [(65, 4804, 256, "split"), (128, 4800, 256, "pieces"), (128, 4096, 2052, "split"), (128, 3072, 4096, "pieces"), (129, 4804, 256, "pieces"),
+                                        (64, 300, 256, ""), (70, 300, 252, "split")])
+def test_which_road_a_product_takes(monkeypatch, m, n, k, road):
+    """One tile of rows and many outputs: the weights are cut where they are used; either way the same bits."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n)
+    ops, split = Ops(torch.float32), Ops(torch.float32)
+    split.pieces_linear = False
+    a, w = randn(g, m, k), randn(g, n, k)
+    outs = [torch.full((m, n), float("nan"), device="cuda") for _ in range(2)]
+    assert roads(monkeypatch, lambda: ops.linear(a, w, None, outs[0])) == (["linear_" + road] if road else [])
+    split.linear(a, w, None, outs[1])
+    assert torch.equal(*outs) and outs[0].isfinite().all()
+
+
+def test_a_product_without_room_for_its_scratch_runs_all_the_same(monkeypatch):
+    g = torch.Generator(device="cuda")
+    g.manual_seed(5)
+    ops = Ops(torch.float32)
+    a, w, real = randn(g, 200, 512), randn(g, 700, 512), torch.empty
+    want, got = (torch.full((200, 700), float("nan"), device="cuda") for _ in range(2))
+    assert roads(monkeypatch, lambda: ops.linear(a, w, None, want)) == ["linear_pieces"]
+
+    def none_left(*args, **kw):
+        if kw.get("dtype") == torch.uint8:
+            raise torch.cuda.OutOfMemoryError("no room")
+        return real(*args, **kw)
+    monkeypatch.setattr(torch, "empty", none_left)
+    assert roads(monkeypatch, lambda: ops.linear(a, w, None, got)) == ["linear_split"]
+    assert torch.equal(got, want)
+    ops.PIECES_WORK_BYTES = 1 << 16
+    monkeypatch.setattr(torch, "empty", real)
+    assert roads(monkeypatch, lambda: ops.linear(a, w, None, got)) == ["linear_split"]
