@@ -43,6 +43,7 @@ struct WideArgs {
   float scale, softcap, slope_span;
   float cap_in, cap_out;                                          // a capped score: cap_out * tanh(cap_in * (q . k)), in units of log2
   int window, keep_first, chunk;
+  int shorter;                                                    // sequences of up to so many positions are left alone (attention_simt.cu takes them)
   int skip_copy;                                                  // (tests: a block's first page is not said to be there, so that the wait for it runs out)
 };
 
@@ -105,8 +106,8 @@ __global__ void __launch_bounds__(THREADS, 1) scored_wide_kernel(const __grid_co
   }
   pdl_wait();
   const int start = a.seq_starts[s], n_new = a.seq_starts[s + 1] - start, tok0 = ((int)gridDim.x / a.columns - 1 - from_end) * tok;
-  if (tok0 >= n_new) return;
   const int kv_len = a.kv_lens[s];
+  if (tok0 >= n_new || kv_len <= a.shorter) return;
   if (warp == 1) tmem_alloc(tmem_slot, TM_COLS);
   const int n_tok = min(tok, n_new - tok0), pos0 = kv_len - n_new + tok0, last_pos = pos0 + n_tok - 1;
   const int first_key = a.chunk > 0 ? pos0 - pos0 % a.chunk : ((a.window > 0 && pos0 - a.window + 1 > 0) ? pos0 - a.window + 1 : 0);   // of the block's first token
@@ -478,11 +479,12 @@ KVAD_EXPORT int kvad_attention_scored_wide_takes(int dk, int dv, int alias) {
   return dk > 0 && dv > 0 && dk % 8 == 0 && dv % 8 == 0 && dv <= 128 && layout_of(dk, dv, alias != 0).stages >= 1 ? 1 : 0;
 }
 
+// `shorter`: sequences of up to so many positions are left alone.
 KVAD_EXPORT int kvad_attention_scored_wide(const float* q, int64_t ld_q, float* out, int64_t ld_out, const float* gate, int64_t ld_gate, int gate_heads,
                                            const float* sinks, const int* seq_starts, const int* kv_lens, const int* page_table, int table_width,
                                            const float* k_pages, const float* v_pages, int n_seqs, int n_heads, int n_kv_heads, int dk, int dv,
                                            int page_size, int max_new, float scale, float softcap, float slope_span, int window, int keep_first,
-                                           int chunk, int key_maps, cudaStream_t stream) {
+                                           int chunk, int key_maps, int shorter, cudaStream_t stream) {
   KVAD_REQUIRE(n_seqs >= 0 && n_heads > 0 && n_kv_heads > 0 && dk > 0 && dv > 0 && table_width > 0 && max_new >= 0 && keep_first >= 0,
                "attention (scored, 32-bit prompts): bad sizes seqs=%d heads=%d kv_heads=%d dk=%d dv=%d", n_seqs, n_heads, n_kv_heads, dk, dv);
   KVAD_REQUIRE(n_heads % n_kv_heads == 0, "attention (scored, 32-bit prompts): %d heads do not divide into %d key/value heads", n_heads, n_kv_heads);
@@ -508,6 +510,7 @@ KVAD_EXPORT int kvad_attention_scored_wide(const float* q, int64_t ld_q, float* 
   while (a.hp < 16 && (n_heads / n_kv_heads) % (a.hp * 2) == 0) a.hp *= 2;
   KVAD_REQUIRE((int64_t)n_seqs * (n_heads / a.hp) < (1ll << 31), "attention (scored, 32-bit prompts): %d sequences x %d heads are more than one launch takes", n_seqs, n_heads);
   a.columns = n_seqs * (n_heads / a.hp);
+  a.shorter = shorter;
   a.skip_copy = g_skip_copy;
   g_skip_copy = 0;
   const Layout z = layout_of(dk, dv, alias);

@@ -110,7 +110,7 @@ attention_tiled_kernel(const T* __restrict__ q, int64_t ld_q, T* __restrict__ ou
                        const int* __restrict__ seq_starts, const int* __restrict__ kv_lens,
                        const int* __restrict__ page_table, int table_width,
                        const T* __restrict__ k_pages, const T* __restrict__ v_pages,
-                       int n_heads, int n_kv_heads, int hd, float scale, int window) {
+                       int n_heads, int n_kv_heads, int hd, float scale, int window, int longest) {
   extern __shared__ float tiled_smem[];
   float* Qs = tiled_smem;                         // [TR][hd]
   float* Ks = Qs + TR * hd;                       // [TK][hd + 1]
@@ -118,7 +118,7 @@ attention_tiled_kernel(const T* __restrict__ q, int64_t ld_q, T* __restrict__ ou
   float* Ps = Vs + TK * hd;                       // [TR][TK]
   const int s = blockIdx.y, h = blockIdx.z, row0 = blockIdx.x * TR;
   const int start = seq_starts[s], n_new = seq_starts[s + 1] - start;
-  if (row0 >= n_new) return;
+  if (row0 >= n_new || (longest > 0 && kv_lens[s] > longest)) return;
   const int n_rows = n_new - row0 < TR ? n_new - row0 : TR;
   const int pos0 = kv_lens[s] - n_new + row0;                     // position of the block's first row
   const int kvh = h / (n_heads / n_kv_heads);
@@ -225,7 +225,7 @@ attention_tiled_kernel(const T* __restrict__ q, int64_t ld_q, T* __restrict__ ou
 template <typename T, int DPL>
 int launch_tiled(const void* q, int64_t ld_q, void* out, int64_t ld_out, const int* seq_starts, const int* kv_lens,
                  const int* page_table, int table_width, const void* k_pages, const void* v_pages, int n_seqs, int n_heads,
-                 int n_kv_heads, int hd, int max_new, float scale, int window, cudaStream_t stream) {
+                 int n_kv_heads, int hd, int max_new, float scale, int window, int longest, cudaStream_t stream) {
   const size_t smem = ((size_t)TR * hd + (size_t)TK * (hd + 1) + (size_t)TK * hd + (size_t)TR * TK) * sizeof(float);
   static size_t configured = 0;
   if (smem > 48 * 1024 && smem > configured) {
@@ -236,7 +236,7 @@ int launch_tiled(const void* q, int64_t ld_q, void* out, int64_t ld_out, const i
   dim3 grid((max_new + TR - 1) / TR, n_seqs, n_heads);
   attention_tiled_kernel<T, DPL><<<grid, TILED_THREADS, smem, stream>>>((const T*)q, ld_q, (T*)out, ld_out, seq_starts, kv_lens, page_table,
                                                                          table_width, (const T*)k_pages, (const T*)v_pages, n_heads,
-                                                                         n_kv_heads, hd, scale, window);
+                                                                         n_kv_heads, hd, scale, window, longest);
   KVAD_CHECK_LAUNCH("attention_tiled");
   return KVAD_OK;
 }
@@ -244,11 +244,12 @@ int launch_tiled(const void* q, int64_t ld_q, void* out, int64_t ld_out, const i
 }  // namespace
 
 // Prompts (rows of sequences packed one after another, each sequence's rows being its last positions): head sizes that
-// are multiples of 4 up to 256, pages of 64 positions; otherwise KVAD_ERR_UNSUPPORTED and the caller takes kvad_attention_simt.
+// are multiples of 4 up to 256, pages of 64 positions; otherwise KVAD_ERR_UNSUPPORTED and the caller takes kvad_attention_simt.  `longest` > 0: only sequences of up to so
+// many positions (the others: attention_scored_wide.cu).
 KVAD_EXPORT int kvad_attention_tiled(int dtype, const void* q, int64_t ld_q, void* out, int64_t ld_out, const int* seq_starts,
                                      const int* kv_lens, const int* page_table, int table_width, const void* k_pages,
                                      const void* v_pages, int n_seqs, int n_heads, int n_kv_heads, int head_dim, int page_size,
-                                     int max_new, float scale, int window, cudaStream_t stream) {
+                                     int max_new, float scale, int window, int longest, cudaStream_t stream) {
   KVAD_REQUIRE(n_seqs >= 0 && n_heads > 0 && n_kv_heads > 0 && head_dim > 0 && table_width > 0 && max_new >= 0,
                "attention (tiled): bad sizes seqs=%d heads=%d kv_heads=%d head_dim=%d", n_seqs, n_heads, n_kv_heads, head_dim);
   KVAD_REQUIRE(n_heads % n_kv_heads == 0, "attention (tiled): %d heads do not divide into %d key/value heads", n_heads, n_kv_heads);
@@ -261,10 +262,10 @@ KVAD_EXPORT int kvad_attention_tiled(int dtype, const void* q, int64_t ld_q, voi
   case D:                                                                                                                       \
     if (dtype == KVAD_DTYPE_F32)                                                                                                \
       return launch_tiled<float, D>(q, ld_q, out, ld_out, seq_starts, kv_lens, page_table, table_width, k_pages, v_pages, n_seqs, \
-                                    n_heads, n_kv_heads, head_dim, max_new, scale, window, stream);                             \
+                                    n_heads, n_kv_heads, head_dim, max_new, scale, window, longest, stream);                             \
     if (dtype == KVAD_DTYPE_BF16)                                                                                               \
       return launch_tiled<__nv_bfloat16, D>(q, ld_q, out, ld_out, seq_starts, kv_lens, page_table, table_width, k_pages, v_pages, \
-                                            n_seqs, n_heads, n_kv_heads, head_dim, max_new, scale, window, stream);             \
+                                            n_seqs, n_heads, n_kv_heads, head_dim, max_new, scale, window, longest, stream);             \
     break;
   switch (dpl) {
     KVAD_TILED(1) KVAD_TILED(2) KVAD_TILED(3) KVAD_TILED(4) KVAD_TILED(5) KVAD_TILED(6) KVAD_TILED(7) KVAD_TILED(8)

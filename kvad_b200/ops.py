@@ -80,7 +80,7 @@ _SIGNATURES = {
         "kvad_attention_simt": [c_int, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_int,
                                 c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p],
         "kvad_attention_tiled": [c_int, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
-                                 c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p],
+                                 c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_void_p],
     },
     "attention_prefill": {
         "kvad_attention_prefill": [c_void_p, c_int64, c_int, c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_int,
@@ -142,7 +142,7 @@ _SIGNATURES = {
     "attention_scored_wide": {
         "kvad_attention_scored_wide": [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
                                        c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_float, c_int, c_int,
-                                       c_int, c_int, c_void_p],
+                                       c_int, c_int, c_int, c_void_p],
         "kvad_attention_scored_wide_takes": [c_int, c_int, c_int],
         "kvad_attention_scored_wide_status": [],
         "kvad_attention_scored_wide_test_hooks": [c_uint, c_int],
@@ -410,7 +410,7 @@ class Ops:
         the key under which a step's CUDA graph is kept."""
         return (_switch_epoch, self.tensor_core_linear, self.tensor_core_prefill, self.fast_decode,
                 self.rows_linear_max, self.qkv_sums, self.SUMS_MIN_K, self.tiled_prompt, self.split_linear, self.pieces_linear, self.scored_prompt, self.scored_wide, self.chunked_recurrences,
-                self.SPLIT_MIN_ROWS, self.PIECES_MIN_ROWS, self.PIECES_MIN_K, self.PIECES_ONE_TILE, self.PIECES_WORK_BYTES, self.SCORED_PROMPT_MIN_NEW, self.CHUNK_MIN_ROWS, self.CHUNK_SHORT_ROWS, self.CHUNK_WORK_BYTES,
+                self.SPLIT_MIN_ROWS, self.PIECES_MIN_ROWS, self.PIECES_MIN_K, self.PIECES_ONE_TILE, self.PIECES_WORK_BYTES, self.SCORED_PROMPT_MIN_NEW, self.SHORT_PROMPT_KEYS, self.SHORT_PROMPT_MAX, self.CHUNK_MIN_ROWS, self.CHUNK_SHORT_ROWS, self.CHUNK_WORK_BYTES,
                 self.ROWS_LINEAR_MAX_OUT, self.ROWS_BLOCKS_MAX, self.HEADS_LINEAR_MAX_ROWS)
 
     def begin_step(self) -> None:
@@ -683,15 +683,29 @@ class Ops:
         if q.dtype != self.dtype or out.dtype != self.dtype or k_pages.dtype != self.dtype:
             raise KernelError(f"attention_prompt: tensors must be {self.dtype}")
         if self.scored_wide and max_new >= self.SCORED_PROMPT_MIN_NEW and self._wide_takes(q, out, k_pages, v_pages, hd, hd, page, ld_q, ld_o, n_seqs, n_heads, max_new):
+            # more blocks than SMs of short prompts: sequences of a page at most stay on the CUDA cores
+            together = 1                # heads a block (as the kernel has it)
+            while together < 16 and (n_heads // n_kv) % (2 * together) == 0:
+                together *= 2
+            blocks = n_seqs * (n_heads // together) * -(-int(max_new) * together // 128)
+            short = self.SHORT_PROMPT_KEYS if blocks > sm_count() and max_new * hd <= self.SHORT_PROMPT_MAX and n_seqs <= 65535 and n_heads <= 65535 else 0
             h = lib("attention_scored_wide")
             _check(h.kvad_attention_scored_wide(_ptr(q), ld_q, _ptr(out), ld_o, None, 0, 0, None, _ptr(seq_starts), _ptr(kv_lens), _ptr(page_table),
                                                 page_table.shape[1], _ptr(k_pages), _ptr(v_pages), int(n_seqs), n_heads, n_kv, hd, hd, page, int(max_new),
-                                                float(scale), 0.0, 0.0, int(window or 0), 0, 0, 1, _stream()), h)
-            return
+                                                float(scale), 0.0, 0.0, int(window or 0), 0, 0, 1, short, _stream()), h)
+            if not short:
+                return
+        else:
+            short = 0
         h = lib("attention_simt")
         _check(h.kvad_attention_tiled(self.code, _ptr(q), ld_q, _ptr(out), ld_o, _ptr(seq_starts), _ptr(kv_lens), _ptr(page_table),
                                       page_table.shape[1], _ptr(k_pages), _ptr(v_pages), int(n_seqs), n_heads, n_kv, hd, page,
-                                      int(max_new), float(scale), int(window or 0), _stream()), h)
+                                      int(max_new), float(scale), int(window or 0), short, _stream()), h)
+
+    # 32-bit prompts of more blocks than SMs and so many (new rows a sequence x entries of a head) at most: sequences of up to SHORT_PROMPT_KEYS positions run on the CUDA
+    # cores, four blocks an SM, where the tensor-core kernel's one block an SM takes 9 us whatever it has to do; the launch for the longer ones passes them by.  (12 heads of 64, us so, by
+    # the tensor cores alone and by the CUDA cores alone: 16 sequences of 17: 19, 21, 15; 32 of 17: 22, 31, 17; 64 of 32: 41, 63, 32; 16 of 8 behind 200 positions: 36, 33, 44.)
+    SHORT_PROMPT_KEYS, SHORT_PROMPT_MAX = 64, 2048
 
     PREFILL_HEAD_SIZES = (16, 32, 48, 64, 80, 96, 112, 128)
 
@@ -1223,7 +1237,7 @@ class Ops:
             _check(h.kvad_attention_scored_wide(_ptr(q), ld_q, _ptr(out), ld_o, _ptr(gate), ld_g, int(gate_heads), _ptr(sinks), _ptr(seq_starts), _ptr(kv_lens),
                                                 _ptr(page_table), page_table.shape[1], _ptr(k_pages), _ptr(v_ptr), int(n_seqs), int(n_heads), n_kv, dk, dv,
                                                 page, int(max_new), float(scale), float(softcap or 0.0), float(slope_span or 0.0), int(window or 0),
-                                                int(keep_first or 0), int(chunk or 0), int(key_maps), _stream()), h)
+                                                int(keep_first or 0), int(chunk or 0), int(key_maps), 0, _stream()), h)
             return
         h = lib("attention_scored")
         _check(h.kvad_attention_scored(self.code, _ptr(q), ld_q, _ptr(out), ld_o, _ptr(gate), ld_g, _ptr(seq_starts), _ptr(kv_lens),

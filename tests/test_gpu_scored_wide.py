@@ -159,3 +159,22 @@ def test_numbers_of_one_sign(H, G, dk, dv, alias, scale):
         far, bias = zip(*[(float((x - want).norm() / want.norm()), float(((x - want) / want).mean())) for x in (c.run(ops), c.run(cores))])
         # 2^-23: exponentials good to 2 units in the last place; a page's sums truncate at their last four steps, 2^-25 of the sum each on the average
         assert far[0] < max(1.1 * far[1], 2.0 ** -23) and abs(bias[0]) < 2.0 ** -23, (far, bias)
+
+
+@pytest.mark.parametrize("H,d,window", [(12, 64, 0), (12, 64, 20), (25, 32, 0)])
+def test_short_prompts_beside_longer_ones(H, d, window):
+    """More blocks than SMs: sequences of a page at most go to the CUDA cores, the others to the tensor cores; no place is left out or written twice."""
+    ops, cores = Ops(torch.float32), Ops(torch.float32)
+    cores.scored_wide = False
+    c = Case([(0, 32), (60, 4), (61, 4), (0, 1), (33, 31), (33, 32), (200, 20)] * 4, H, H, d, d)      # (of 32 new rows at most)
+    outs = []
+    for o in (ops, cores):
+        out = torch.full((c.out[0], H * d), float("nan"), device="cuda")
+        o.attention_prompt(c.q, out, c.starts, c.lens, len(c.seqs), c.max_new, c.table, c.kp, c.vp, H, c.scale, window)
+        outs.append(out)
+    assert outs[0].isfinite().all() and float((outs[0] - outs[1]).abs().max()) < 1e-5
+    at = 0
+    for cached, new in c.seqs:                           # (the same kernel: the same bits; another: not)
+        same = torch.equal(outs[0][at:at + new], outs[1][at:at + new])
+        assert same == (cached + new <= 64) or new == 1
+        at += new
