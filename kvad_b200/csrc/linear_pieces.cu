@@ -153,11 +153,6 @@ __global__ void __launch_bounds__(THREADS, 1) linear_pieces_kernel(const uint8_t
   const int mine = (int)blockIdx.x < tiles ? (tiles - (int)blockIdx.x - 1) / (int)gridDim.x + 1 : 0, blocks = mine * num_kb;      // of this CTA
   pdl_wait();
 
-  auto wait = [&](uint64_t* bar, uint32_t parity) {
-    if (mbar_wait(bar, parity)) return true;
-    *failed = 1;
-    return false;
-  };
   if (warp < 4) {
     regs_fewer<32>();
     if (warp == 0 && lane == 0) {
@@ -167,7 +162,7 @@ __global__ void __launch_bounds__(THREADS, 1) linear_pieces_kernel(const uint8_t
       for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
         const uint8_t* w_at = w_pieces + (int64_t)(t % tiles_n) * num_kb * T::STAGE;
         for (int kb = 0; kb < num_kb; ++kb, ++j, w_at += T::STAGE) {
-          if (j >= RING && !wait(&done[s], turn ^ 1)) { ok = false; break; }
+          if (j >= RING && !mbar_wait(&done[s], turn ^ 1)) { ok = false; break; }
           if (!(p.skip_copy && j == 0)) {
             mbar_expect_tx(&ready[s], T::STAGE);
             bulk_load(smem + s * T::STAGE, w_at, T::STAGE, &ready[s]);
@@ -182,7 +177,7 @@ __global__ void __launch_bounds__(THREADS, 1) linear_pieces_kernel(const uint8_t
       int s = 0, acc = 0;
       uint32_t turn = 0;
       for (int j = 0; j < blocks; ++j) {
-        if (!wait(&ready[s], turn)) break;
+        if (!mbar_wait(&ready[s], turn)) break;
         tc_fence_after();
         const uint64_t w = w0 + (uint32_t)s * (T::STAGE >> 4);
         const uint32_t d = tmem_base + (uint32_t)(acc * BN), a = tmem_a + (uint32_t)(s * A_COLS);
@@ -224,7 +219,7 @@ __global__ void __launch_bounds__(THREADS, 1) linear_pieces_kernel(const uint8_t
     fetch();
     for (int j = group; j < blocks; j += 2) {
       const int ring = j % RING;
-      if (j >= RING && !wait(&done[ring], ((j / RING) & 1) ^ 1)) break;
+      if (j >= RING && !mbar_wait(&done[ring], ((j / RING) & 1) ^ 1)) break;
       tc_fence_after();
 #pragma unroll
       for (int pair = 0; pair < 2; ++pair) {    // 16 rows: i = 2 pair and 2 pair + 1
@@ -266,7 +261,7 @@ __global__ void __launch_bounds__(THREADS, 1) linear_pieces_kernel(const uint8_t
 #pragma unroll
       for (int i = 0; i < SHARE; ++i) sum[i] = 0.f;
       for (int kb = 0; kb < num_kb; ++kb, ++j) {
-        if (!wait(&done[j % RING], (j / RING) & 1)) { ok = false; break; }
+        if (!mbar_wait(&done[j % RING], (j / RING) & 1)) { ok = false; break; }
         tc_fence_after();
         {
           uint32_t v[32];
@@ -316,6 +311,7 @@ __global__ void __launch_bounds__(THREADS, 1) linear_pieces_kernel(const uint8_t
         }
       }
     }
+    if (!ok) *failed = 1;                       // (whichever role gave up: then there are products that this one has waited for in vain)
   }
   tc_fence_before();
   __syncthreads();
