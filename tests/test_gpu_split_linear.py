@@ -20,11 +20,14 @@ def randn(g, *shape):
 # more tiles than SMs (a CTA goes round its slots over several tiles)
 @pytest.mark.parametrize("m,n,k", [(33, 64, 4), (64, 65, 32), (127, 128, 36), (128, 200, 128), (129, 63, 160), (300, 1031, 96), (1500, 2309, 200), (70, 5, 772)])
 @pytest.mark.parametrize("tile", [64, 128])
-def test_split_product_is_no_further_off_than_the_fmaf_chain(m, n, k, tile):
+@pytest.mark.parametrize("pieces", [False, True])
+def test_split_product_is_no_further_off_than_the_fmaf_chain(m, n, k, tile, pieces):
+    """Either road by itself: weights cut where they are used (linear_split), or by a pass before (linear_pieces)."""
     g = torch.Generator(device="cuda")
     g.manual_seed(m * n + k)
     ops, chain = Ops(torch.float32), Ops(torch.float32)
     chain.split_linear, chain.rows_linear_max, ops.SPLIT_MIN_ROWS = False, 0, 1
+    ops.pieces_linear, ops.PIECES_MIN_ROWS, ops.PIECES_MIN_K = pieces, 1, 1
     wide = randn(g, m, k + 8)
     a, w, b, old = wide[:, 4:4 + k], randn(g, n, k) * 0.3, randn(g, n), randn(g, m, n + 3)[:, :n]
     exact = a.double() @ w.double().t()
@@ -43,7 +46,7 @@ def test_split_product_is_no_further_off_than_the_fmaf_chain(m, n, k, tile):
             outs.append(rel(out[:, :n], want))
         # six products leave out less than 2^-23 of |a||w|; single roundings of the result are 2^-25 on average
         assert outs[0] < max(1.1 * outs[1], 1.5e-7), (epi, outs)
-    assert lib("linear_split").kvad_linear_split_status() == 0
+    assert lib("linear_split").kvad_linear_split_status() == 0 and lib("linear_pieces").kvad_linear_pieces_status() == 0
 
 
 def test_split_product_of_values_that_bfloat16_cannot_hold():

@@ -38,7 +38,11 @@ def test_a_constant_that_chooses_a_kernel_is_part_of_a_captured_step():
     import torch
     ops = Ops(torch.bfloat16)
     for name in ("SPLIT_MIN_ROWS", "SCORED_PROMPT_MIN_NEW", "CHUNK_MIN_ROWS", "CHUNK_SHORT_ROWS", "CHUNK_WORK_BYTES", "SUMS_MIN_K", "ROWS_LINEAR_MAX_OUT",
-                 "ROWS_BLOCKS_MAX", "HEADS_LINEAR_MAX_ROWS", "split_linear", "scored_prompt", "chunked_recurrences"):
+                 "ROWS_BLOCKS_MAX", "HEADS_LINEAR_MAX_ROWS", "split_linear", "scored_prompt", "chunked_recurrences", "pieces_linear", "scored_wide", "PIECES_MIN_ROWS", "PIECES_MIN_K",
+                 "PIECES_WORK_BYTES", "SHORT_PROMPT_KEYS", "SHORT_PROMPT_MAX"):
         before = ops.path_key()
         setattr(ops, name, getattr(ops, name) + 1)
         assert ops.path_key() != before, name
+    before = ops.path_key()
+    ops.PIECES_ONE_TILE = (256, *ops.PIECES_ONE_TILE[1:])
+    assert ops.path_key() != before
