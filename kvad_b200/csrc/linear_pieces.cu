@@ -156,6 +156,7 @@ __global__ void __launch_bounds__(THREADS, 1) linear_pieces_kernel(const uint8_t
   if (warp < 4) {
     regs_fewer<32>();
     if (warp == 0 && lane == 0) {
+      const int from = p.skip_copy ? 1 : 0;
       int s = 0, j = 0;
       uint32_t turn = 0;
       bool ok = true;
@@ -163,7 +164,7 @@ __global__ void __launch_bounds__(THREADS, 1) linear_pieces_kernel(const uint8_t
         const uint8_t* w_at = w_pieces + (int64_t)(t % tiles_n) * num_kb * T::STAGE;
         for (int kb = 0; kb < num_kb; ++kb, ++j, w_at += T::STAGE) {
           if (j >= RING && !mbar_wait(&done[s], turn ^ 1)) { ok = false; break; }
-          if (!(p.skip_copy && j == 0)) {
+          if (j >= from) {
             mbar_expect_tx(&ready[s], T::STAGE);
             bulk_load(smem + s * T::STAGE, w_at, T::STAGE, &ready[s]);
           }
