@@ -19,9 +19,9 @@
 // 128 x 128 x 16 (64), 2300 cycles, and runs in 2850.  Values of up to 64: the weights, ~1000 instructions a row and page, 1400 cycles a page; then the
 // start of a block (~5 us with the first page's chain), of which two go one after another where there are more than 148 tiles.
 // Graph-replayed launches, us: 2 x 1024 rows of 16 heads over a latent of 256: 1100 on the CUDA cores, 127 by mma.sync, 40 here; 16 heads of 64 on 4 key heads, capped,
-// window 512: 358, 55, 27; without cap and window 46, 23.  64 new rows of 4 sequences with 300 cached positions: latent 47.6, 17.7; 16 heads of 64: 15.4, 10.4; 2 new rows:
-// 38.4, 14.7; 12.3, 9.5.  The mma.sync kernel was ahead nowhere and is gone.  (On the way: products issued by a branch of one lane 64, by the
-// whole warp 50, S and P V by warps of their own with wide P V 40.)
+// window 512: 358, 55, 28 (42 where scores lie beyond 0.45 caps); without cap and window 46, 23.  64 new rows of 4 sequences with 300 cached positions: latent 47.6, 17.7; 16 heads of 64: 15.4, 10.4;
+// 2 new rows: 38.4, 14.0; 12.3, 9.1.  With a head a group many short sequences were faster by mma.sync, two blocks an SM: 32 of 2 rows 14, 26; of 32 rows 17, 26.  (On the way: products issued by a
+// branch of one lane 64, by the whole warp 50, S and P V by warps of their own with wide P V 40.)
 #include <algorithm>
 #include <type_traits>
 

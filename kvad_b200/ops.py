@@ -704,7 +704,7 @@ class Ops:
 
     # 32-bit prompts of more blocks than SMs and so many (new rows a sequence x entries of a head) at most: sequences of up to SHORT_PROMPT_KEYS positions run on the CUDA
     # cores, four blocks an SM, where the tensor-core kernel's one block an SM takes 9 us whatever it has to do; the launch for the longer ones passes them by.  (12 heads of 64, us so, by
-    # the tensor cores alone and by the CUDA cores alone: 16 sequences of 17: 19, 21, 15; 32 of 17: 22, 31, 17; 64 of 32: 41, 63, 32; 16 of 8 behind 200 positions: 36, 33, 44.)
+    # the tensor cores alone and by the CUDA cores alone: 16 sequences of 17: 18, 20, 15; 32 of 17: 23, 30, 17; 64 of 32: 42, 60, 32; 16 of 8 behind 200 positions: 36, 33, 44.)
     SHORT_PROMPT_KEYS, SHORT_PROMPT_MAX = 64, 2048
 
     PREFILL_HEAD_SIZES = (16, 32, 48, 64, 80, 96, 112, 128)
@@ -1171,9 +1171,10 @@ class Ops:
         if gate is not None:
             self.gate_mul(gate, out, out, "sigmoid")
 
-    # New rows a sequence from which bfloat16 goes to attention_scored_prompt.cu: all but single-token rows, whose keys may be split over blocks.  (16 heads on
-    # 4 key heads of 64, two new rows: 6.3 us against the CUDA cores' 15.9 without a cache, 15.2 against 89.8 behind 500 positions, 90 against 668 behind
-    # 4000; one head a group and heads of 128 and 256 likewise, 2 to 8 times.)
+    # New rows a sequence from which prompts go to attention_scored_prompt.cu (bfloat16) and attention_scored_wide.cu (32-bit): all but single-token rows, whose keys may be split over
+    # blocks.  (16 heads of 64 on 4 key heads, two new rows of four sequences, us here and on the CUDA cores: without a cache 7.0, 15, behind 500 positions 12, 87; 32 sequences 7.9, 30 and
+    # 13, 180; 32-bit 9.7, 15 and 25, 84; 11, 29 and 29, 172.  One block an SM: with a head a group many sequences take turns, 32 of two rows 26, 30, of 32 rows 26, 37, behind 500 positions 45, 180;
+    # 32-bit 37, 29; 40, 35; 118, 184.)
     SCORED_PROMPT_MIN_NEW = 2
 
     def attention_scored(self, q, out, seq_starts, kv_lens, n_seqs: int, max_new: int, page_table, k_pages, v_pages, n_heads: int,
